@@ -26,6 +26,8 @@
 // that build is for measurements only.
 #include "rowwise.cuh"
 
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 namespace b200 {
@@ -318,7 +320,7 @@ softmax_resident_kernel(const SoftmaxParams p) {
   softmax_finish<Tout, CH, V, G, FASTEXP, EXACT>(v, mx, mx_raw, y, nv, lane, gs, p.log_mode != 0, valid, red);
 }
 
-// Element-wise kernel for rows that do not fit in registers or break the vector-path alignment
+// Element-wise kernel for masked rows of more than 8192 elements that break the vector-path alignment
 // rules: one CTA per row and three sweeps (max, sum of exp, write). Only the first sweep of a
 // row comes from DRAM when the row fits in L2.
 template <typename Tin, bool PACKED>
@@ -334,6 +336,48 @@ __device__ __forceinline__ float softmax_logit(const SoftmaxParams& p, const Tin
     if (PACKED) t = round_through<Tin>(t);
   }
   return t;
+}
+
+// Rows with a mask (or short ones) that the vector path cannot take: a warp per row (n <= 512) or a
+// CTA per row, E elements per thread at a distance of the group, held in registers: one read of the
+// row and of its mask instead of the three sweeps below, every access of a warp one coalesced stretch
+// whatever the alignment. Bound by the number of 2-byte accesses and the exponentials. Measured: fp16
+// [49152, 333] with a key mask 404 us with the three sweeps, 59 us here; bf16 [24576, 1201] 795 -> 98 us.
+template <typename Tin, typename Tout, bool PACKED, int E, int G>
+__global__ void __launch_bounds__(G == 0 ? 1024 : 256) softmax_ragged_kernel(const SoftmaxParams p) {
+  __shared__ float red[32];
+  const int lane = glane<G>(), gs = gsize<G>();
+  long long row = grow<G>();
+  const bool valid = row < p.rows;  // warps of a partly filled last CTA compute on the last row
+  if (!valid) row = p.rows - 1;
+  const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
+  const Tin* m = p.mask ? reinterpret_cast<const Tin*>(p.mask) + row_offset(p.mmap, row) : nullptr;
+  Tout* y = reinterpret_cast<Tout*>(p.y) + row_offset(p.ymap, row);
+  float t[E];
+  float mx = -INFINITY;
+#pragma unroll
+  for (int e = 0; e < E; ++e) t[e] = e * gs + lane < p.n ? softmax_logit<Tin, PACKED>(p, x, m, e * gs + lane) : -INFINITY;
+#pragma unroll
+  for (int e = 0; e < E; ++e) mx = fmaxf(mx, t[e]);
+  mx = greduce<FastMax, G>(mx, red);
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    if (e * gs + lane < p.n) {
+      t[e] = t[e] - mx;  // log_softmax keeps the difference, softmax the exponential
+      const float v = expf(t[e]);
+      s += v;
+      if (!p.log_mode) t[e] = v;
+    }
+  }
+  s = greduce<SumOp, G>(s, red);
+  if (!valid) return;
+  const float ls = logf(s), inv = __frcp_rn(s);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = e * gs + lane;
+    if (i < p.n) y[i] = Elem<Tout>::from_f32(p.log_mode ? t[e] - ls : (sizeof(Tout) == 4 ? t[e] / s : t[e] * inv));
+  }
 }
 
 template <typename Tin, typename Tout, bool PACKED>
@@ -371,8 +415,339 @@ __global__ void __launch_bounds__(1024) softmax_streaming_kernel(const SoftmaxPa
 }
 
 // ----------------------------------------------------------------------------------------------
-// Long or ragged rows (rows that do not fit the register-resident kernel, or whose length is not a
-// whole number of 16-byte vectors): one CTA per row, two sweeps instead of three.
+// Rows that the register-resident kernel above does not take (longer than 4096 vectors, a length that
+// is no whole number of vectors, or a start off the 16-byte grid; no mask): the row is held in
+// registers as the raw 16-byte vectors that were loaded, so that it crosses HBM once whatever its
+// alignment.
+//   * A CTA of at most 512 threads holds up to CH = 8 vectors per thread (4096 vectors); longer rows,
+//     and rows of a tensor with few of them, are split over a thread-block cluster of S <= 8 CTAs
+//     that exchange one (maximum, sum) pair each through distributed shared memory.
+//   * The body of the row is loaded from the first 16-byte boundary on; the at most V - 1 elements in
+//     front of it and behind the last whole vector are held one per thread by the first CTA.
+//   * The output row has an alignment of its own (fp32 rows of 20 005 elements start on any multiple
+//     of four bytes). The outputs of a thread's vector are handed over by warp shuffles to where the
+//     next aligned chunk of the output starts, so stores are whole chunks; only a warp's first and
+//     last elements leave one by one.
+// Bound by HBM: the exponentials cost 18 us of the SFU pipe on the case below, the traffic 75 us.
+// Measured: bf16 [4096, 20005] (rows 20 008 apart) -> fp32 log_softmax 183.7 us with the two-sweep
+// kernel below, 103.3 us (4.76 TB/s) here; bf16 [2000, 32001] softmax 192.6 -> 57.6 us.
+// ----------------------------------------------------------------------------------------------
+// Stores a thread's V outputs, the first of which goes to `y`. `shift` (warp-uniform, below the chunk
+// length VO) counts the elements from y to the next chunk boundary of the output; the lane above
+// supplies what this lane's last chunk lacks, the lane below takes the first `shift` elements.
+// Every lane of the warp calls it. has_next: the lane above holds the vector that follows this one.
+template <typename Tout, int V>
+__device__ __forceinline__ void store_shifted(Tout* y, const f32x2 (&o)[V / 2], int shift, int lane, bool valid,
+                                              bool has_next) {
+  constexpr int VO = V * (int)sizeof(Tout) <= 16 ? V : 16 / (int)sizeof(Tout);  // elements of a chunk
+  if (shift == 0) {
+    if (valid) store_pairs<Tout, V>(y, o);
+    return;
+  }
+  if constexpr (sizeof(Tout) == 4) {
+    float e[V + 3];
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) unpack2(o[i], e[2 * i], e[2 * i + 1]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) e[V + i] = __shfl_down_sync(0xffffffffu, e[i], 1);
+    float* out = reinterpret_cast<float*>(y);
+    if (lane == 0 && valid) {
+      out[0] = e[0];
+      if (shift > 1) out[1] = e[1];
+      if (shift > 2) out[2] = e[2];
+    }
+    if (shift & 1) {
+#pragma unroll
+      for (int i = 0; i < V + 2; ++i) e[i] = e[i + 1];
+    }
+    if (shift & 2) {
+#pragma unroll
+      for (int i = 0; i < V + 1; ++i) e[i] = e[i + 2];
+    }
+    if (!valid) return;
+    out += shift;
+#pragma unroll
+    for (int k = 0; k < V / VO; ++k) {
+      if (k < V / VO - 1 || has_next) {
+        st_stream(out + k * VO, make_uint4(__float_as_uint(e[k * VO]), __float_as_uint(e[k * VO + 1]),
+                                           __float_as_uint(e[k * VO + 2]), __float_as_uint(e[k * VO + 3])));
+      } else {
+#pragma unroll
+        for (int i = 0; i < VO - 1; ++i)
+          if (i < VO - shift) out[k * VO + i] = e[k * VO + i];
+      }
+    }
+  } else {
+    constexpr int W = V / 2;  // 32-bit words of a thread's outputs
+    uint32_t w[2 * W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) w[i] = Pairs<Tout>::narrow(o[i]);
+#pragma unroll
+    for (int i = 0; i < W; ++i) w[W + i] = __shfl_down_sync(0xffffffffu, w[i], 1);
+    unsigned short* out = reinterpret_cast<unsigned short*>(y);
+    if (lane == 0 && valid) {
+#pragma unroll
+      for (int i = 0; i < V - 1; ++i)
+        if (i < shift) out[i] = (unsigned short)(w[i / 2] >> (16 * (i & 1)));
+    }
+    if (W == 4 && (shift & 4)) {
+#pragma unroll
+      for (int i = 0; i + 2 < 2 * W; ++i) w[i] = w[i + 2];
+    }
+    if (shift & 2) {
+#pragma unroll
+      for (int i = 0; i + 1 < 2 * W; ++i) w[i] = w[i + 1];
+    }
+    if (shift & 1) {
+#pragma unroll
+      for (int i = 0; i < W; ++i) w[i] = __byte_perm(w[i], w[i + 1], 0x5432);
+    }
+    if (!valid) return;
+    out += shift;
+    if (has_next) {
+      if constexpr (W == 4) st_stream(out, make_uint4(w[0], w[1], w[2], w[3]));
+      else asm volatile("st.global.cs.v2.u32 [%0], {%1,%2};" ::"l"(out), "r"(w[0]), "r"(w[1]) : "memory");
+    } else {
+#pragma unroll
+      for (int i = 0; i < V - 1; ++i)
+        if (i < V - shift) out[i] = (unsigned short)(w[i / 2] >> (16 * (i & 1)));
+    }
+  }
+}
+
+template <typename Tin, typename Tout, int CH, bool CLUSTER>
+__global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParams p, const int S) {
+  constexpr int V = Elem<Tin>::V;
+  constexpr int P = V / 2;
+  constexpr int VO = V * (int)sizeof(Tout) <= 16 ? V : 16 / (int)sizeof(Tout);
+  constexpr float kFloor = -1e30f;  // differences from the maximum are clamped here: the exponential needs finite ones
+  __shared__ float red[32];
+  __shared__ float pairs[2][8];  // cluster: (maximum, sum) of every CTA of the row
+  const int tid = threadIdx.x, lane = tid & 31, T_ = blockDim.x;
+  // a CTA's shared memory may be written from another one only once it runs: arrive here, wait before the write
+  if constexpr (CLUSTER) cooperative_groups::this_cluster().barrier_arrive();
+  const int rank = CLUSTER ? (int)(blockIdx.x % (unsigned)S) : 0;
+  const long long row = CLUSTER ? (long long)(blockIdx.x / (unsigned)S) : (long long)blockIdx.x;
+  const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
+  Tout* y = reinterpret_cast<Tout*>(p.y) + row_offset(p.ymap, row);
+
+  // body: whole vectors from the first 16-byte boundary on; edge: what is in front of it and behind it
+  int head = (int)(((16u - (unsigned)(reinterpret_cast<uintptr_t>(x) & 15u)) & 15u) / sizeof(Tin));
+  if (head > p.n) head = p.n;
+  const int nvec = (p.n - head) / V;
+  const int tail0 = head + nvec * V;
+  const int edges = head + (p.n - tail0);
+  const int per = CLUSTER ? (nvec + S - 1) / S : nvec;
+  const int v0 = CLUSTER ? rank * per : 0;
+  const int cnt = nvec - v0 < per ? nvec - v0 : per;  // vectors of this CTA (may be negative: none)
+  const Tin* xb = x + head + (long long)v0 * V;
+  Tout* yb = y + head + (long long)v0 * V;
+
+  uint4 raw[CH];
+#pragma unroll
+  for (int c = 0; c < CH; ++c)
+    if (c * T_ + tid < cnt) raw[c] = ld_stream(xb + (long long)(c * T_ + tid) * V);
+  const bool has_edge = rank == 0 && tid < edges;
+  const int edge_at = tid < head ? tid : tail0 + (tid - head);
+  const f32x2 scale2 = splat2(p.scale);
+  const bool scaled = p.has_scale != 0;
+  float edge = -INFINITY;
+  if (has_edge) {
+    edge = Elem<Tin>::to_f32(x[edge_at]);
+    if (scaled) edge = edge * p.scale;
+  }
+  auto logits = [&](int c, f32x2 (&t)[P]) {
+    Pairs<Tin>::unpack(raw[c], t);
+    if (scaled) {
+#pragma unroll
+      for (int i = 0; i < P; ++i) t[i] = mul2(t[i], scale2);
+    }
+  };
+
+  // ---- maximum (a NaN anywhere makes it NaN) ------------------------------------------------------
+  float m = edge;
+  bool in_fp32 = true;
+  if constexpr (sizeof(Tin) == 2) {
+    if (!scaled) {  // a maximum is exact in the input type: packed pairs, no conversion
+      using P2 = typename Pair<Tin>::type;
+      P2 m2 = Pair<Tin>::splat(-INFINITY);
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        if (c * T_ + tid < cnt) {
+          const uint32_t w[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) m2 = MaxOp::apply2(m2, *reinterpret_cast<const P2*>(&w[i]));
+        }
+      }
+      const float2 f = Pair<Tin>::widen(m2);
+      m = MaxOp::apply(m, MaxOp::apply(f.x, f.y));
+      in_fp32 = false;
+    }
+  }
+  if (in_fp32) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (c * T_ + tid < cnt) {
+        f32x2 t[P];
+        logits(c, t);
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          float a, b;
+          unpack2(t[i], a, b);
+          m = MaxOp::apply(m, MaxOp::apply(a, b));
+        }
+      }
+    }
+  }
+  float M = block_reduce<MaxOp>(m, red);
+
+  // ---- sum of the exponentials --------------------------------------------------------------------
+  // log_softmax takes the compensated exponential for fp32 outputs too: only the logarithm of the sum
+  // sees it, where its 3.5e-7 is below the rounding of (x - max) - log(sum).
+  const bool log_mode = p.log_mode != 0;
+  auto difference = [&](f32x2 t, f32x2 M2) {
+    float a, b;
+    unpack2(sub2(t, M2), a, b);
+    return pack2(fmaxf(a, kFloor), fmaxf(b, kFloor));  // a NaN is lost here: the maximum has caught it
+  };
+  auto exp_exact = [](f32x2 d) {
+    float a, b;
+    unpack2(d, a, b);
+    return pack2(expf(a), expf(b));
+  };
+  auto add_up = [&](auto exponential) {
+    const f32x2 M2 = splat2(M);
+    f32x2 sum = splat2(0.f);
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (c * T_ + tid < cnt) {
+        f32x2 t[P];
+        logits(c, t);
+        f32x2 part = exponential(difference(t[0], M2));
+#pragma unroll
+        for (int i = 1; i < P; ++i) part = add2(part, exponential(difference(t[i], M2)));
+        sum = add2(sum, part);
+      }
+    }
+    float s = hsum2(sum);
+    if (has_edge) s += expf(fmaxf(edge - M, kFloor));
+    return s;
+  };
+  float s;
+  if (sizeof(Tout) == 2 || log_mode) s = add_up([](f32x2 d) { return exp_pair_compensated(d); });
+  else s = add_up(exp_exact);
+  float sum = block_reduce<SumOp>(s, red);
+  if constexpr (CLUSTER) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_wait();
+    if (tid < S) {  // this CTA's pair into the table of CTA `tid`
+      float* far = cluster.map_shared_rank(&pairs[0][0], tid);
+      far[rank] = M;
+      far[8 + rank] = sum;
+    }
+    cluster.sync();  // all pairs are in place; no CTA touches another's memory after this
+    M = pairs[0][0];
+    for (int r = 1; r < S; ++r) M = MaxOp::apply(M, pairs[0][r]);
+    sum = 0.f;
+    for (int r = 0; r < S; ++r) {
+      // a CTA whose elements are all -inf (or that has none) adds nothing
+      if (pairs[0][r] > -INFINITY) sum += pairs[1][r] * expf(fmaxf(pairs[0][r] - M, kFloor));
+    }
+  }
+  // aten: x - max is NaN for a row of -inf and for +inf elements; a NaN logit poisons the row
+  if (!(fabsf(M) < INFINITY)) sum = NAN;
+
+  // ---- outputs ------------------------------------------------------------------------------------
+  const float log_sum = logf(sum), inv = __frcp_rn(sum);
+  const f32x2 M2 = splat2(M), log_sum2 = splat2(log_sum), inv2 = splat2(inv);
+  const int shift = (int)(((0u - (unsigned)reinterpret_cast<uintptr_t>(yb)) & (VO * (unsigned)sizeof(Tout) - 1u)) /
+                          sizeof(Tout));
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int j = c * T_ + tid;
+    if (j - lane >= cnt) break;  // warp-uniform: no lane of this warp has a vector here
+    f32x2 t[P], o[P];
+    const bool valid = j < cnt;
+    if (!valid) raw[c] = make_uint4(0u, 0u, 0u, 0u);
+    logits(c, t);
+    if (log_mode) {
+#pragma unroll
+      for (int i = 0; i < P; ++i) o[i] = sub2(sub2(t[i], M2), log_sum2);
+    } else if constexpr (sizeof(Tout) == 4) {
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        float a, b;
+        unpack2(exp_exact(difference(t[i], M2)), a, b);
+        o[i] = pack2(a / sum, b / sum);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < P; ++i) o[i] = mul2(exp_pair_compensated(difference(t[i], M2)), inv2);
+    }
+    store_shifted<Tout, V>(yb + (long long)j * V, o, shift, lane, valid, lane < 31 && j + 1 < cnt);
+  }
+  if (has_edge) {
+    float o;
+    if (log_mode) {
+      o = (edge - M) - log_sum;
+    } else {
+      const float e = expf(fmaxf(edge - M, kFloor));
+      o = sizeof(Tout) == 4 ? e / sum : e * inv;
+    }
+    y[edge_at] = Elem<Tout>::from_f32(o);
+  }
+}
+
+// Returns false when the row does not fit (more than 8 CTAs of 4096 vectors: 64 registers a thread
+// hold 8 vectors and what is computed from them, and a cluster has at most 8 CTAs everywhere).
+template <typename Tin, typename Tout>
+static bool try_launch_softmax_rows(const SoftmaxParams& p, cudaStream_t st, int* rc) {
+  constexpr int V = Elem<Tin>::V;
+  const long long nvec = p.n / V + 1;  // an upper bound whatever the alignment of a row
+  if (nvec > 8 * 4096) return false;
+  int S = 1;
+  while (nvec > 4096LL * S) S *= 2;
+  // few rows: as many CTAs per row as give every SM two, while each still has work for 128 threads
+  while (S < 8 && p.rows * S < 2LL * device_info().sm_count && nvec / (2 * S) >= 512) S *= 2;
+  if (p.rows * S > 0x7fffffffLL) return false;
+  const long long per = (nvec + S - 1) / S;
+  const int ch = per > 512 ? 8 : (per > 128 ? 4 : 2);
+  const int threads = (int)((per + ch - 1) / ch + 31) / 32 * 32;
+  if (S == 1) {
+    set_path_tag("two sweeps over a row in registers, any alignment");
+    const unsigned grid = (unsigned)p.rows;
+    if (ch == 8) softmax_rows_kernel<Tin, Tout, 8, false><<<grid, threads, 0, st>>>(p, 1);
+    else if (ch == 4) softmax_rows_kernel<Tin, Tout, 4, false><<<grid, threads, 0, st>>>(p, 1);
+    else softmax_rows_kernel<Tin, Tout, 2, false><<<grid, threads, 0, st>>>(p, 1);
+    *rc = launch_status("b200_softmax");
+    return true;
+  }
+  set_path_tag("two sweeps over a row in the registers of a cluster, any alignment");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.rows * S));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = ch == 8 ? cudaLaunchKernelEx(&cfg, softmax_rows_kernel<Tin, Tout, 8, true>, p, S)
+                                : cudaLaunchKernelEx(&cfg, softmax_rows_kernel<Tin, Tout, 4, true>, p, S);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *rc = fail((int)e, "b200_softmax: cluster launch failed: %s", cudaGetErrorString(e));
+    return true;
+  }
+  *rc = launch_status("b200_softmax");
+  return true;
+}
+
+// ----------------------------------------------------------------------------------------------
+// Rows beyond 32768 vectors (more than 262 144 16-bit columns): one CTA per row, two sweeps.
 //   sweep 1: every thread keeps a running maximum m and the sum of exp(t - m) of its elements,
 //            rescaling the sum when the maximum grows; the CTA then combines the (m, s) pairs:
 //            M = max m_i, S = sum s_i * exp(m_i - M)
@@ -602,14 +977,26 @@ static int launch_softmax(const SoftmaxParams& p, bool vector_ok, cudaStream_t s
 #undef B200_SM_LAUNCH
     }
   } else if (p.mask == nullptr && !PACKED && p.n >= 256) {
+    int rc = B200_OK;
+    if (try_launch_softmax_rows<Tin, Tout>(p, st, &rc)) return rc;
     int threads = (int)((p.n / V + 3) / 4);
     threads = (threads + 31) / 32 * 32;
     threads = threads < 128 ? 128 : (threads > 1024 ? 1024 : threads);
     set_path_tag("two sweeps, CTA per row");
     softmax_long_kernel<Tin, Tout><<<(unsigned)p.rows, threads, 0, st>>>(p);
+  } else if (p.n <= 8192) {
+    set_path_tag("elements in registers");
+    if (p.n <= 512) {
+      const unsigned grid = (unsigned)((p.rows + 7) / 8);
+      if (p.n <= 64) softmax_ragged_kernel<Tin, Tout, PACKED, 2, 32><<<grid, 256, 0, st>>>(p);
+      else if (p.n <= 256) softmax_ragged_kernel<Tin, Tout, PACKED, 8, 32><<<grid, 256, 0, st>>>(p);
+      else softmax_ragged_kernel<Tin, Tout, PACKED, 16, 32><<<grid, 256, 0, st>>>(p);
+    } else {
+      const int threads = ((p.n + 7) / 8 + 31) / 32 * 32;
+      softmax_ragged_kernel<Tin, Tout, PACKED, 8, 0><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    }
   } else {
-    int threads = 1024;
-    while (threads > 64 && threads / 2 >= p.n) threads /= 2;
+    const int threads = 1024;
     set_path_tag("element-wise, three passes");
     softmax_streaming_kernel<Tin, Tout, PACKED><<<(unsigned)p.rows, threads, 0, st>>>(p);
   }

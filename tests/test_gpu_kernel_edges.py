@@ -1,0 +1,59 @@
+"""GPU parity at the edges of the kernels' ranges: row lengths and starts off the vector grid, ends of
+tiles and groups, the smallest and largest sizes a variant takes.
+
+Tolerances: a 16-bit result may differ from the fp64 value by half a step of its type (2^-8 of the value
+for bf16, 2^-11 for fp16) plus what the fp32 arithmetic before it loses; fp32 results by a few fp32 ulps
+(2^-23) times the length of the summation tree, far below the bounds used here.
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+STEP = {torch.float32: 2.0 ** -21, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+def _kernels():
+    import better_benchmark_b200.kernels as k
+    return k
+
+
+def _randn(shape, dtype, seed, scale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(shape, generator=g) * scale).to(dtype).cuda()
+
+
+def _near(got, want64, what, floor=1e-6):
+    """|got - want| within half a step of got's type (a whole one for fp32 rounding before it) of the value."""
+    err = (got.double() - want64).abs()
+    bound = STEP[got.dtype] * want64.abs() + floor
+    worst = (err - bound).max().item()
+    assert worst <= 0, f"{what}: beyond the bound by {worst:.3e}"
+
+
+@pytest.mark.parametrize("log", [False, True])
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16),
+                                       (torch.float16, torch.float32), (torch.float32, torch.float32),
+                                       (torch.float32, torch.float16)])
+@pytest.mark.parametrize("rows,n,stride", [(3, 257, 257), (5, 1003, 1005), (2, 4097, 4099), (2, 32769, 32771),
+                                           (300, 8195, 8195), (1, 131075, 131075)])
+def test_softmax_rows_of_any_alignment(rows, n, stride, dtype, out, log):
+    """The row held in registers, one CTA or a cluster per row: consecutive rows start on every residue
+    of the 16-byte grid, and so do their outputs."""
+    base = _randn((rows, stride), dtype, n, 3.0)
+    x = base[:, stride - n:]
+    got = _kernels().softmax(x, log=log, out_dtype=out)
+    d = x.double()
+    want = torch.log_softmax(d, -1) if log else torch.softmax(d, -1)
+    _near(got, want, f"softmax {rows}x{n} {dtype}->{out} log={log}", floor=2e-6 if log else 1e-7)
+
+
+@pytest.mark.parametrize("scale", [None, 0.125])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("keys", [1, 31, 33, 65, 255, 257, 511, 513, 1201, 8191])
+def test_masked_softmax_of_ragged_rows(keys, dtype, scale):
+    x, keep = _randn((2, 3, 5, keys), dtype, keys, 2.0), torch.rand(2, 1, 1, keys, device="cuda") < 0.8
+    keep[..., 0] = True
+    mask = torch.where(keep, 0.0, -10000.0).to(dtype)
+    got = _kernels().softmax(x, mask=mask, scale=scale)
+    _near(got, torch.softmax(x.double() * (scale or 1.0) + mask.double(), -1), f"masked softmax {keys} {dtype}", floor=1e-7)
