@@ -13,6 +13,7 @@
 // Pointwise semantics follow aten: the value is converted to fp32, multiplied by the scale (when
 // given) and rounded once to the output dtype.
 #include "rowwise.cuh"
+#include "tile_stream.cuh"
 
 #include <type_traits>
 #include <cstdlib>
@@ -193,73 +194,227 @@ __global__ void __launch_bounds__(256) transpose16_tile_kernel(const TransposePa
   st_stream(reinterpret_cast<__half*>(o + p.P), hi);
 }
 
-// Batched transpose of SMALL matrices without conversion (a [P, C] matrix and its transpose fit in
-// shared memory; e.g. the [49, 128] and [196, 64] attention tiles of
-// repros/canonical/pointwise_021e90d9c17d/shapes.json, whose 49 rows fill a 64 x 64 tile only to
-// three quarters and whose output rows of 49 elements do not start on 16-byte boundaries). The
-// input matrix and the output matrix of one batch entry are each ONE contiguous block, so both are
-// moved with 16-byte accesses as flat arrays; the transposition is the shared-memory gather in
+// Transpose of 16-bit elements without conversion for every shape that is not made of whole 64 x 64
+// tiles: the tile is kept transposed in shared memory as words of two consecutive input rows, one
+// word row per input column, so that an output row is written as 4-byte words whatever its parity
+// (an output row of an odd length P starts on a 2-byte boundary: its first and last element then
+// leave alone). A thread turns the words of rows 2r and 2r + 1 into the words of columns 2c and 2c + 1
+// with two byte permutes; column c lives in row (c / 2) + 32 (c & 1), which keeps the writes of a warp
+// in 32 different banks.
+// pairs: rows start on 4-byte boundaries and C is even, so a warp reads a tile row as 32 words.
+// Bound by HBM (half of the lines are touched by two CTAs). Measured against 2-byte accesses through a
+// tile of floats: f16 [200, 501, 768] 173.6 -> 82.0 us, [300, 500, 333] 119.1 -> 56.3 us.
+__global__ void __launch_bounds__(256) transpose16_ragged_kernel(const TransposeParams p, const int pairs) {
+  __shared__ uint32_t tile[64 * 33];
+  const long long b = blockIdx.z;
+  const int p0 = (int)blockIdx.y * 64, c0 = (int)blockIdx.x * 64;
+  const int np = p.P - p0 < 64 ? (int)(p.P - p0) : 64, nc = p.C - c0 < 64 ? (int)(p.C - c0) : 64;
+  const unsigned short* src =
+      reinterpret_cast<const unsigned short*>(p.x) + b * p.in_batch_stride + (long long)p0 * p.in_row_stride + c0;
+  unsigned short* dst = reinterpret_cast<unsigned short*>(p.y) + b * p.P * p.C + (long long)c0 * p.P + p0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (pairs) {
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {  // rows 2 (4 warp + i / 2) + (i & 1)
+      const int r = warp * 8 + i;
+      w[i] = r < np && 2 * lane < nc
+                 ? __ldg(reinterpret_cast<const uint32_t*>(src + (long long)r * p.in_row_stride) + lane) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      tile[lane * 33 + warp * 4 + i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x5410);
+      tile[(lane + 32) * 33 + warp * 4 + i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x7632);
+    }
+  } else {
+    unsigned short e[2][8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = warp * 8 + i, c = lane + 32 * h;
+        e[h][i] = r < np && c < nc ? __ldg(src + (long long)r * p.in_row_stride + c) : (unsigned short)0;
+      }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = lane + 32 * h;
+        tile[((c >> 1) + 32 * (c & 1)) * 33 + warp * 4 + i] = (uint32_t)e[h][2 * i] | ((uint32_t)e[h][2 * i + 1] << 16);
+      }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = warp * 8 + i;
+    if (c >= nc) break;  // warp-uniform
+    unsigned short* out = dst + (long long)c * p.P;
+    const int odd = (int)((reinterpret_cast<uintptr_t>(out) >> 1) & 1u);
+    const uint32_t* row = tile + ((c >> 1) + 32 * (c & 1)) * 33;
+    uint32_t w = row[lane];
+    const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);
+    if (odd) {
+      if (lane == 0) out[0] = (unsigned short)w;
+      w = __byte_perm(w, next, 0x5432);  // elements 2 lane + 1 and 2 lane + 2; the second is missing in lane 31
+    }
+    const int at = 2 * lane + odd;
+    if (at + 1 < np) *reinterpret_cast<uint32_t*>(out + at) = w;
+    else if (at < np) out[at] = (unsigned short)w;
+  }
+}
+
+// Batched transpose of SMALL 16-bit matrices without conversion (e.g. the [49, 128] and [196, 64]
+// attention tiles of repros/canonical/pointwise_021e90d9c17d/shapes.json, whose 49 rows fill a 64 x 64
+// tile only to three quarters and whose output rows of 49 elements start on 2-byte boundaries). One
+// matrix, or a group of consecutive ones, is one contiguous block on both sides, so it crosses HBM as
+// flat 16-byte vectors: asynchronous copies into a ring of `stages` shared-memory blocks, the
+// transposition from shared memory to shared memory, one bulk store of the finished block.
+//
+// The transposition moves 4-byte words only. The output rows of columns 2c and 2c + 1 are 2 P
+// consecutive elements, P whole words whether P is even or odd:
+//   even P: word k of row 2c is (in[2k][2c], in[2k+1][2c]), the same for row 2c + 1
+//   odd P : row 2c ends in the middle of a word, which row 2c + 1 completes; the latter's words pair
+//           input rows (1, 2), (3, 4), ...
+// so a thread that walks the words (2c, 2c + 1) of the input rows writes both. Neighbouring lanes take
+// neighbouring column pairs: they read neighbouring words, and write words P apart - different banks
+// when P is odd; for even P each lane starts its walk one word later than its neighbour, which makes
+// the distance odd as well.
+// What bounds it: HBM, with the shared-memory passes (copy in, read, write, copy out: about 390 cycles
+// for a [49, 128] matrix, a third of the time its bytes take) behind it. Measured on bf16 [16384, 49, 128]:
+// 141.4 us with two-byte gathers (four-way bank conflicts), 74.1 us (5.55 TB/s) here.
+__device__ __forceinline__ void copy_async16(uint32_t smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+
+template <bool ODD>
+__global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposeParams p, const int group, const int stages,
+                                                              const int split, const FastDiv by_tasks,
+                                                              const FastDiv by_pairs) {
+  extern __shared__ __align__(128) unsigned char pairs_smem[];
+  const int P = (int)p.P, C = (int)p.C, CW = C / 2;
+  const int elems = P * C;
+  const int span = group * elems * 2;  // bytes of a whole group, a multiple of 16
+  const uint32_t ring = smem_u32(pairs_smem);
+  unsigned char* const done = pairs_smem + (size_t)stages * span;  // the transposed group
+  uint32_t* const out = reinterpret_cast<uint32_t*>(done);
+  const long long groups = (p.batch + group - 1) / group;
+  const int tid = threadIdx.x;
+  auto bytes_of = [&](long long g) {
+    const long long left = p.batch - g * group;
+    return (int)(left < group ? left : group) * elems * 2;
+  };
+  auto load = [&](long long g, int slot) {
+    if (g < groups) {
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(p.x) + g * group * p.in_batch_stride * 2;
+      const int whole = bytes_of(g) & ~15;
+      for (int at = tid * 16; at < whole; at += 256 * 16) copy_async16(ring + (uint32_t)(slot * span + at), src + at);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  long long g = blockIdx.x;
+  for (int s = 0; s < stages - 1; ++s) load(g + (long long)s * gridDim.x, s);
+  int slot = 0;
+  for (; g < groups; g += gridDim.x) {
+    const int ahead = slot == 0 ? stages - 1 : slot - 1;
+    load(g + (long long)(stages - 1) * gridDim.x, ahead);  // its last reader passed the barrier below
+    if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 1;" ::: "memory");
+    const int bytes = bytes_of(g), whole = bytes & ~15;
+    const unsigned char* block = pairs_smem + (size_t)slot * span;
+    if (tid * 2 < bytes - whole)  // the last group may end between two 16-byte boundaries
+      *reinterpret_cast<unsigned short*>(pairs_smem + (size_t)slot * span + whole + tid * 2) =
+          __ldg(reinterpret_cast<const unsigned short*>(reinterpret_cast<const unsigned char*>(p.x) +
+                                                        g * group * p.in_batch_stride * 2 + whole) + tid);
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the block before has left
+    __syncthreads();
+    const uint32_t* in = reinterpret_cast<const uint32_t*>(block);
+    const int here = bytes / (elems * 2);
+    const int tasks = group * CW, steps = P / 2;
+    for (int t = tid; t < tasks * split; t += 256) {
+      const int q = (int)fast_div((unsigned)t, by_tasks);
+      const int u = t - q * tasks;
+      const int m = (int)fast_div((unsigned)u, by_pairs);
+      if (m >= here) continue;
+      const int cp = u - m * CW;
+      const int j0 = steps * q / split, j1 = steps * (q + 1) / split;
+      const uint32_t* src = in + m * (elems / 2) + cp;
+      uint32_t* dst = out + m * (elems / 2) + cp * P;
+      if constexpr (ODD) {
+        uint32_t a = src[2 * j0 * CW];
+#pragma unroll 4
+        for (int j = j0; j < j1; ++j) {
+          const uint32_t b = src[(2 * j + 1) * CW], n = src[(2 * j + 2) * CW];
+          dst[j] = __byte_perm(a, b, 0x5410);
+          dst[(P + 1) / 2 + j] = __byte_perm(b, n, 0x7632);
+          a = n;
+        }
+        if (q == split - 1) dst[P / 2] = __byte_perm(src[(P - 1) * CW], src[0], 0x7610);
+      } else {
+        const int len = j1 - j0;
+        int r = len > 0 ? cp % len : 0;
+#pragma unroll 4
+        for (int j = 0; j < len; ++j) {
+          const int k = j0 + r;
+          const uint32_t a = src[2 * k * CW], b = src[(2 * k + 1) * CW];
+          dst[k] = __byte_perm(a, b, 0x5410);
+          dst[P / 2 + k] = __byte_perm(a, b, 0x7632);
+          if (++r == len) r = 0;
+        }
+      }
+    }
+    fence_proxy_async_smem();  // the bulk store reads what the threads wrote
+    __syncthreads();
+    unsigned char* y = reinterpret_cast<unsigned char*>(p.y) + g * span;
+    if (tid == 0 && whole > 0) {
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(y), "r"(smem_u32(done)), "r"(whole)
+                   : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    if (tid * 2 < bytes - whole)
+      reinterpret_cast<unsigned short*>(y + whole)[tid] = reinterpret_cast<const unsigned short*>(done + whole)[tid];
+    if (++slot == stages) slot = 0;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory outlives the store
+}
+
+// Batched transpose of small 32-bit matrices (a [P, C] matrix fits in shared memory): both sides are
+// moved with 16-byte accesses as flat arrays, the transposition is the shared-memory gather in
 // between: output element o = c * P + p comes from [p][c]. A CTA takes matrices b, b + grid, ...
-template <typename E>  // E: unsigned short (16-bit elements) or unsigned int (32-bit elements)
 __global__ void __launch_bounds__(256) transpose_small_kernel(const TransposeParams p, const int pitch) {
-  constexpr int VE = 16 / (int)sizeof(E);
   extern __shared__ __align__(16) unsigned char small_smem[];
-  E* tile = reinterpret_cast<E*>(small_smem);  // [P][pitch]
+  uint32_t* tile = reinterpret_cast<uint32_t*>(small_smem);  // [P][pitch]
   const int P = (int)p.P, C = (int)p.C;
-  const int nvec = P * C / VE;
+  const int nvec = P * C / 4;
   for (long long b = blockIdx.x; b < p.batch; b += gridDim.x) {
-    const E* src = reinterpret_cast<const E*>(p.x) + b * p.in_batch_stride;
-    E* dst = reinterpret_cast<E*>(p.y) + b * (long long)P * C;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(p.x) + b * p.in_batch_stride;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(p.y) + b * (long long)P * C;
     for (int j0 = threadIdx.x; j0 < nvec; j0 += 4 * 256) {  // four loads in flight per thread
       uint4 raws[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int j = j0 + u * 256;
-        if (j < nvec) raws[u] = ld_stream(reinterpret_cast<const float*>(src) + (size_t)j * 4);
+        if (j < nvec) raws[u] = ld_stream(src + (size_t)j * 4);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int j = j0 + u * 256;
         if (j >= nvec) continue;
-        const uint4 raw = raws[u];
-        const int e0 = j * VE;
-        const int r = e0 / C, c0 = e0 - r * C;  // C is a multiple of VE: the vector stays in one row
-        E* t = tile + r * pitch + c0;
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-        if constexpr (sizeof(E) == 2) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            t[2 * k] = (E)(w[k] & 0xffffu);
-            t[2 * k + 1] = (E)(w[k] >> 16);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) t[k] = (E)w[k];
-        }
+        const int r = j * 4 / C, c0 = j * 4 - r * C;  // C is a multiple of 4: the vector stays in one row
+        uint32_t* t = tile + r * pitch + c0;
+        t[0] = raws[u].x; t[1] = raws[u].y; t[2] = raws[u].z; t[3] = raws[u].w;
       }
     }
     __syncthreads();
     for (int j = threadIdx.x; j < nvec; j += 256) {
-      int o = j * VE;
-      int c = o / P, r = o - c * P;
+      int c = j * 4 / P, r = j * 4 - c * P;
       uint32_t w[4];
-      if constexpr (sizeof(E) == 2) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t lo = tile[r * pitch + c];
-          if (++r == P) { r = 0; ++c; }
-          const uint32_t hi = tile[r * pitch + c];
-          if (++r == P) { r = 0; ++c; }
-          w[k] = lo | (hi << 16);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          w[k] = tile[r * pitch + c];
-          if (++r == P) { r = 0; ++c; }
-        }
+      for (int k = 0; k < 4; ++k) {
+        w[k] = tile[r * pitch + c];
+        if (++r == P) { r = 0; ++c; }
       }
-      st_stream(reinterpret_cast<float*>(dst) + (size_t)j * 4, make_uint4(w[0], w[1], w[2], w[3]));
+      st_stream(dst + (size_t)j * 4, make_uint4(w[0], w[1], w[2], w[3]));
     }
     __syncthreads();  // the tile is overwritten by the next matrix
   }
@@ -355,35 +510,79 @@ static int launch_permute(const PermuteParams& p, bool vec, cudaStream_t st) {
   return launch_status("b200_permute_copy");
 }
 
+// Groups of small 16-bit matrices through transpose_pairs_kernel; false when the shape does not fit.
+static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st, int* rc) {
+  const long long elems = p.P * p.C;
+  if (p.C % 2 != 0 || p.P < 2 || elems * 2 > 32 * 1024 || p.in_row_stride != p.C || !aligned16(p.x) || !aligned16(p.y))
+    return false;
+  int group = 1;  // the smallest group that is a whole number of 16-byte vectors
+  while (group * elems % 8 != 0) group *= 2;
+  if (group * elems * 2 > 32 * 1024) return false;
+  if (p.in_batch_stride == elems || p.batch == 1) {
+    // small matrices: larger groups (up to 12 KB a block), but no fewer than four blocks per SM
+    while (2 * group * elems * 2 <= 12 * 1024 && p.batch / (2 * group) >= 4LL * device_info().sm_count) group *= 2;
+  } else if (group != 1 || p.in_batch_stride % 8 != 0) {
+    return false;
+  }
+  const int span = (int)(group * elems * 2);
+  const int stages = span <= 16 * 1024 ? 3 : 2;
+  const size_t smem = (size_t)(stages + 1) * span;
+  const int tasks = (int)(group * (p.C / 2));
+  int split = 256 / tasks;  // threads that share a pair of columns
+  if (split > p.P / 2) split = (int)(p.P / 2);
+  if (split < 1) split = 1;
+  auto kernel = p.P % 2 ? transpose_pairs_kernel<true> : transpose_pairs_kernel<false>;
+  const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  int per_sm = (int)((size_t)device_info().max_smem_optin / (smem + 1024));
+  if (per_sm > 8) per_sm = 8;
+  if (per_sm < 1) per_sm = 1;
+  long long grid = (p.batch + group - 1) / group;
+  if (grid > (long long)device_info().sm_count * per_sm) grid = (long long)device_info().sm_count * per_sm;
+  kernel<<<(unsigned)grid, 256, smem, st>>>(p, group, stages, split, make_fast_div(tasks), make_fast_div(p.C / 2));
+  *rc = launch_status("b200_transpose_copy [small matrices, word pairs]");
+  return true;
+}
+
 template <typename Tin, typename Tout>
 static int launch_transpose(const TransposeParams& p, cudaStream_t st) {
-  if constexpr (std::is_same<Tin, Tout>::value) {
-    // small matrices that are not made of whole 64 x 64 tiles: flat 16-byte copies around a
-    // shared-memory gather
-    constexpr int VE = 16 / (int)sizeof(Tin);
-    const long long elems = p.P * p.C;
-    const bool tiles64 = sizeof(Tin) == 2 && p.P % 64 == 0 && p.C % 64 == 0;
-    if (!p.has_scale && !tiles64 && elems * (long long)sizeof(Tin) <= 32 * 1024 && p.C % VE == 0 && elems % VE == 0 &&
-        p.in_row_stride == p.C && p.in_batch_stride % VE == 0 && aligned16(p.x) && aligned16(p.y) && p.batch >= 1) {
-      const int pitch = (int)p.C + 1;
-      const size_t smem = (size_t)p.P * pitch * sizeof(Tin);
-      if (smem <= 48 * 1024) {
-        long long grid = p.batch;
-        const long long cap = (long long)device_info().sm_count * 8;
-        if (grid > cap) grid = cap;
-        if constexpr (sizeof(Tin) == 2) transpose_small_kernel<unsigned short><<<(unsigned)grid, 256, smem, st>>>(p, pitch);
-        else transpose_small_kernel<unsigned int><<<(unsigned)grid, 256, smem, st>>>(p, pitch);
-        return launch_status("b200_transpose_copy [small matrices, flat 16-byte copies]");
+  dim3 grid((unsigned)((p.C + 63) / 64), (unsigned)((p.P + 63) / 64), (unsigned)p.batch);
+  if constexpr (std::is_same<Tin, Tout>::value && sizeof(Tin) == 2) {
+    if (!p.has_scale) {
+      const bool whole = p.P % 64 == 0 && p.C % 64 == 0 && p.in_row_stride % 8 == 0 && p.in_batch_stride % 8 == 0 &&
+                         aligned16(p.x) && aligned16(p.y);
+      if (whole) {
+        transpose16_tile_kernel<<<grid, 256, 0, st>>>(p);
+        return launch_status("b200_transpose_copy [16-byte tiles]");
+      }
+      int rc = B200_OK;
+      if (try_launch_transpose_pairs(p, st, &rc)) return rc;
+      const bool words = p.C % 2 == 0 && p.in_row_stride % 2 == 0 && p.in_batch_stride % 2 == 0 &&
+                         (reinterpret_cast<uintptr_t>(p.x) & 3u) == 0;
+      if (p.P <= 0x7fffffffLL && p.C <= 0x7fffffffLL) {
+        transpose16_ragged_kernel<<<grid, 256, 0, st>>>(p, words ? 1 : 0);
+        return launch_status("b200_transpose_copy [ragged 16-bit tiles]");
       }
     }
   }
-  dim3 grid((unsigned)((p.C + 63) / 64), (unsigned)((p.P + 63) / 64), (unsigned)p.batch);
-  if constexpr (std::is_same<Tin, Tout>::value && sizeof(Tin) == 2) {
-    const bool whole = p.P % 64 == 0 && p.C % 64 == 0 && !p.has_scale && p.in_row_stride % 8 == 0 &&
-                       p.in_batch_stride % 8 == 0 && aligned16(p.x) && aligned16(p.y);
-    if (whole) {
-      transpose16_tile_kernel<<<grid, 256, 0, st>>>(p);
-      return launch_status("b200_transpose_copy [16-byte tiles]");
+  if constexpr (std::is_same<Tin, Tout>::value && sizeof(Tin) == 4) {
+    // small matrices: flat 16-byte copies around a shared-memory gather
+    const long long elems = p.P * p.C;
+    if (!p.has_scale && elems * 4 <= 32 * 1024 && p.C % 4 == 0 && p.in_row_stride == p.C && p.in_batch_stride % 4 == 0 &&
+        aligned16(p.x) && aligned16(p.y) && p.batch >= 1) {
+      const int pitch = (int)p.C + 1;
+      const size_t smem = (size_t)p.P * pitch * sizeof(Tin);
+      if (smem <= 48 * 1024) {
+        long long ctas = p.batch;
+        const long long cap = (long long)device_info().sm_count * 8;
+        if (ctas > cap) ctas = cap;
+        transpose_small_kernel<<<(unsigned)ctas, 256, smem, st>>>(p, pitch);
+        return launch_status("b200_transpose_copy [small matrices, flat 16-byte copies]");
+      }
     }
   }
   transpose_tile_kernel<Tin, Tout><<<grid, 256, 0, st>>>(p);

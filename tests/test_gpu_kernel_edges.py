@@ -57,3 +57,17 @@ def test_masked_softmax_of_ragged_rows(keys, dtype, scale):
     mask = torch.where(keep, 0.0, -10000.0).to(dtype)
     got = _kernels().softmax(x, mask=mask, scale=scale)
     _near(got, torch.softmax(x.double() * (scale or 1.0) + mask.double(), -1), f"masked softmax {keys} {dtype}", floor=1e-7)
+
+
+@pytest.mark.parametrize("batch,rows,cols", [(1, 2, 2), (7, 49, 128), (5, 196, 64), (33, 3, 10), (2000, 5, 6), (9, 64, 66),
+                                             (3, 129, 126), (2, 16, 1024), (2, 63, 65), (3, 65, 63), (2, 500, 333),
+                                             (2, 501, 768), (1, 1, 300), (2, 300, 1), (1300, 33, 64)])
+def test_transpose_of_ragged_16_bit_matrices(batch, rows, cols):
+    """Groups of small matrices (a last group that ends between two 16-byte boundaries among them) and
+    64 x 64 tiles with ragged ends on either side; a view that starts off the 4-byte grid."""
+    k = _kernels()
+    x = _randn((batch, rows, cols), torch.float16, rows)
+    assert torch.equal(k.permute_copy(x, (0, 2, 1)), x.transpose(1, 2).contiguous())
+    flat = _randn((batch * rows * cols + 1,), torch.bfloat16, cols)
+    y = flat[1:].view(batch, rows, cols)
+    assert torch.equal(k.permute_copy(y, (0, 2, 1)), y.transpose(1, 2).contiguous())
