@@ -71,3 +71,15 @@ def test_transpose_of_ragged_16_bit_matrices(batch, rows, cols):
     flat = _randn((batch * rows * cols + 1,), torch.bfloat16, cols)
     y = flat[1:].view(batch, rows, cols)
     assert torch.equal(k.permute_copy(y, (0, 2, 1)), y.transpose(1, 2).contiguous())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_silu_over_the_whole_range(dtype):
+    """Every 16-bit pattern above -10000 against fp64 (below, the clamped exponential leaves x * 6e-39), +inf and NaN."""
+    x = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).cuda().view(dtype)
+    got = _kernels().cast_scale(x, dtype, activation="silu")
+    want = (x.double() * torch.sigmoid(x.double()))
+    finite = torch.isfinite(x) & (x > -1e4)
+    _near(got[finite], want[finite], f"silu {dtype}", floor=1.2e-7 if dtype == torch.float16 else 1e-34)
+    assert torch.isnan(got[torch.isnan(x)]).all()
+    assert torch.equal(got[x == float("inf")], x[x == float("inf")])
