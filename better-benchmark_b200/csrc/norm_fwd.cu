@@ -15,6 +15,7 @@
 #include "tile_stream.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace b200 {
 
@@ -596,6 +597,254 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
   return false;
 }
 
+// ----------------------------------------------------------------------------------------------
+// Residual add -> LayerNorm, rows of 65..128 vectors: a warp per row, every warp with its own ring of
+// copy stages (a row of x and a row of the residual, brought in by two bulk copies that lane 0 issues),
+// no CTA barrier in the row loop. The stage is refilled as soon as the sums are in registers, so two
+// stages keep a row in flight per warp. Weight and bias are converted to fp32 once per CTA, in a
+// [slot][pair][lane] layout that a warp reads without bank conflicts. BOTH (res_round == 2): the choice
+// between the two forms is made on the packed 16-bit results: round both, compare |full| > 3, select.
+// All forms take this kernel, so that an element of the both-forms result has the bits of the form it
+// was taken from.
+// What bounds it: HBM, with about 38 instructions per pair of elements (two complete normalisations and
+// the roundings between them, 57 % of the issue slots) behind it. The resident kernel converts weight
+// and bias in every row on top and overlaps its load and store phases less; it keeps the rows of up to
+// 64 vectors, of which it puts two into a warp. Measured on bf16 [65536, 768] with the sum kept: 82.5 ->
+// 76.8 us back to back (64 us, 6.25 TB/s, from a clean L2); f16 [46251, 448]: 34.9 us there, 36.9 us here.
+// ----------------------------------------------------------------------------------------------
+constexpr int kResWarps = 8;  // warps per CTA
+
+// |a| > 3 per 16-bit half: all ones or zeros (zeros for NaN)
+template <typename T>
+__device__ __forceinline__ uint32_t beyond_three(uint32_t a) {
+  if constexpr (std::is_same<T, __half>::value) {
+    return __hgt2_mask(__habs2(*reinterpret_cast<const __half2*>(&a)), __float2half2_rn(3.0f));
+  } else {
+    return __hgt2_mask(__habs2(*reinterpret_cast<const __nv_bfloat162*>(&a)), __float2bfloat162_rn(3.0f));
+  }
+}
+
+template <typename T, int CH, bool EXACT, bool BOTH>
+__global__ void __launch_bounds__(kResWarps * 32, 3)
+residual_norm_warp_kernel(const NormFwdParams p, const int stages) {
+  constexpr int V = Elem<T>::V;
+  constexpr int P = V / 2;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nv = p.n / V;
+  const uint32_t row_bytes = (uint32_t)nv * 16u, stage_bytes = 2u * row_bytes;
+  // layout: [kResWarps][stages][x row | residual row] | mbarriers [kResWarps][4] | weight, bias [CH][P][32] fp32 pairs
+  unsigned char* ring = smem + (size_t)warp * stages * stage_bytes;
+  unsigned char* behind = smem + (size_t)kResWarps * stages * stage_bytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(behind) + warp * 4;
+  f32x2* wsm = reinterpret_cast<f32x2*>(behind + kResWarps * 4 * sizeof(uint64_t));
+  f32x2* bsm = wsm + CH * P * 32;
+  const int rows = (int)p.rows;  // the launcher admits fewer than 2^31 rows
+  const int gwarp = (int)blockIdx.x * kResWarps + warp, gstep = (int)gridDim.x * kResWarps;
+  const int my_rows = rows > gwarp ? (rows - gwarp + gstep - 1) / gstep : 0;
+  const T* xg = reinterpret_cast<const T*>(p.x);
+  const T* rg = reinterpret_cast<const T*>(p.res);
+  auto issue = [&](int k, int slot) {  // lane 0 only
+    const long long off = ((long long)gwarp + (long long)k * gstep) * p.x_row_stride;
+    unsigned char* dst = ring + (size_t)slot * stage_bytes;
+    mbar_arrive_expect_tx(&full[slot], stage_bytes);
+    bulk_load(dst, xg + off, row_bytes, &full[slot]);
+    bulk_load(dst + row_bytes, rg + off, row_bytes, &full[slot]);
+  };
+  if (lane == 0) {  // the first rows are on their way before the weights are staged
+    for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
+    mbar_init_fence();
+    for (int k = 0; k < my_rows && k < stages; ++k) issue(k, k);
+  }
+  for (int q = threadIdx.x; q < CH * 32; q += blockDim.x) {  // q = slot * 32 + lane: vector q of the row
+    float wf[V], bf[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      wf[i] = 1.f;
+      bf[i] = 0.f;
+    }
+    if (q < nv && p.w) load_param<V>(p.w, p.w_dtype, (long long)q * V, wf);
+    if (q < nv && p.b) load_param<V>(p.b, p.w_dtype, (long long)q * V, bf);
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      wsm[((q >> 5) * P + i) * 32 + (q & 31)] = pack2(wf[2 * i], wf[2 * i + 1]);
+      bsm[((q >> 5) * P + i) * 32 + (q & 31)] = pack2(bf[2 * i], bf[2 * i + 1]);
+    }
+  }
+  __syncthreads();  // barriers initialised (seen by every lane), weights in place
+
+  const uint32_t ring_addr = smem_u32(ring) + (uint32_t)lane * 16u;
+  const f32x2* w_lane = wsm + lane;
+  const f32x2* b_lane = bsm + lane;
+  int slot = 0;
+  uint32_t phase = 0;
+  long long row = gwarp;
+  for (int k = 0; k < my_rows; ++k, row += gstep) {
+    const bool arrived = __all_sync(0xffffffffu, mbar_wait(&full[slot], phase));
+    if (!arrived) {  // stop; none of this warp's copies may be in flight at exit
+      if (lane == 0) {
+        note_wait_timeout();
+        int ds = slot;
+        uint32_t dp = phase;
+        for (int d = k; d < my_rows && d < k + stages; ++d) {
+          mbar_wait(&full[ds], dp);
+          if (++ds == stages) { ds = 0; dp ^= 1u; }
+        }
+      }
+      return;
+    }
+    const uint32_t sx = ring_addr + (uint32_t)slot * stage_bytes, sr = sx + row_bytes;
+    f32x2 v[CH][P];
+    uint4 pr[BOTH ? CH : 1];  // the rounded sums
+    f32x2 s2 = splat2(0.f), t2 = splat2(0.f);
+    T* so = p.sum_out ? reinterpret_cast<T*>(p.sum_out) + row * (long long)p.n + lane * V : nullptr;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (EXACT || c * 32 + lane < nv) {
+        f32x2 r[P];
+        Pairs<T>::unpack(lds128(sx + c * 512), v[c]);
+        Pairs<T>::unpack(lds128(sr + c * 512), r);
+#pragma unroll
+        for (int i = 0; i < P; ++i) v[c][i] = add2(v[c][i], r[i]);
+        const uint4 packed = Pairs<T>::pack(v[c]);
+        if (so) st_stream(so + c * 32 * V, packed);
+        if constexpr (BOTH) {
+          pr[c] = packed;
+          Pairs<T>::unpack(packed, r);
+#pragma unroll
+          for (int i = 0; i < P; ++i) t2 = add2(t2, r[i]);
+        } else if (p.res_round == 1) {
+          Pairs<T>::unpack(packed, v[c]);
+        }
+#pragma unroll
+        for (int i = 0; i < P; ++i) s2 = add2(s2, v[c][i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < P; ++i) v[c][i] = splat2(0.f);
+        if constexpr (BOTH) pr[c] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    __syncwarp();  // every lane has read the stage
+    if (lane == 0 && k + stages < my_rows) {
+      fence_proxy_async_smem();
+      issue(k + stages, slot);
+    }
+    if (++slot == stages) {
+      slot = 0;
+      phase ^= 1u;
+    }
+    float s = hsum2(s2), t = hsum2(t2);
+    greduce_sum2<32>(s, t, nullptr);
+    const float mean = s * p.inv_n, mean_r = t * p.inv_n;
+    const f32x2 mean2 = splat2(mean), mean_r2 = splat2(mean_r);
+    f32x2 q2 = splat2(0.f), u2 = splat2(0.f);
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (EXACT || c * 32 + lane < nv) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          v[c][i] = sub2(v[c][i], mean2);  // the centred value: the output needs it again
+          q2 = fma2(v[c][i], v[c][i], q2);
+        }
+        if constexpr (BOTH) {
+          f32x2 r[P];
+          Pairs<T>::unpack(pr[c], r);
+#pragma unroll
+          for (int i = 0; i < P; ++i) {
+            r[i] = sub2(r[i], mean_r2);
+            u2 = fma2(r[i], r[i], u2);
+          }
+        }
+      }
+    }
+    float q = hsum2(q2), u = hsum2(u2);
+    greduce_sum2<32>(q, u, nullptr);
+    const float var = q * p.inv_denom;
+    const float rstd = precise_rsqrt(var + p.eps), rstd_r = precise_rsqrt(u * p.inv_denom + p.eps);
+    if (lane == 0) {
+      if (p.mean_out) p.mean_out[row] = mean;
+      if (p.rstd_out) p.rstd_out[row] = rstd;
+      if (p.var_out) p.var_out[row] = var;
+    }
+    const f32x2 rstd2 = splat2(rstd), rstd_r2 = splat2(rstd_r);
+    T* y = reinterpret_cast<T*>(p.y) + row * p.y_row_stride + lane * V;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (EXACT || c * 32 + lane < nv) {
+        f32x2 o[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+          o[i] = add2(mul2(mul2(v[c][i], rstd2), w_lane[(c * P + i) * 32]), b_lane[(c * P + i) * 32]);
+        if constexpr (BOTH) {
+          f32x2 r[P];
+          uint32_t out[P];
+          Pairs<T>::unpack(pr[c], r);
+#pragma unroll
+          for (int i = 0; i < P; ++i) {
+            r[i] = add2(mul2(mul2(sub2(r[i], mean_r2), rstd_r2), w_lane[(c * P + i) * 32]), b_lane[(c * P + i) * 32]);
+            const uint32_t full16 = Pairs<T>::narrow(o[i]), round16 = Pairs<T>::narrow(r[i]);
+            const uint32_t pick = beyond_three<T>(full16);
+            out[i] = (full16 & pick) | (round16 & ~pick);
+          }
+          st_stream(y + c * 32 * V, make_uint4(out[0], out[1], out[2], out[3]));
+        } else {
+          st_stream(y + c * 32 * V, Pairs<T>::pack(o));
+        }
+      }
+    }
+  }
+}
+
+// Returns false when the shape does not fit (the caller takes the resident kernel).
+template <typename T>
+static bool try_launch_residual_norm_warp(const NormFwdParams& p, cudaStream_t st, int* rc) {
+  constexpr int V = Elem<T>::V;
+  const long long nv = p.n / V;
+  if (streaming_disabled() || p.rms || p.prologue || !p.y || nv <= 64 || nv > 128 ||
+      p.rows >= 0x7fffffffLL) return false;
+  const DeviceInfo& dev = device_info();
+  const int ch = (int)((nv + 31) / 32);
+  const size_t stage_bytes = 2 * (size_t)nv * 16;
+  const size_t fixed = kResWarps * 4 * sizeof(uint64_t) + 2 * (size_t)ch * (V / 2) * 32 * sizeof(f32x2);
+  const size_t per_cta = ((size_t)dev.max_smem_optin - 1024 * 3) / 3;
+  int stages = (int)((per_cta - fixed) / (kResWarps * stage_bytes));
+  if (stages > 4) stages = 4;
+  if (stages < 2) return false;
+  const size_t smem = kResWarps * stages * stage_bytes + fixed;
+  long long grid = 3LL * dev.sm_count;
+  const long long useful = (p.rows + kResWarps - 1) / kResWarps;
+  if (grid > useful) grid = useful;
+  const bool exact = nv == 32LL * ch;
+  auto launch = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      *rc = fail((int)e, "b200_norm_fwd: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+      return;
+    }
+    kernel<<<(unsigned)grid, kResWarps * 32, smem, st>>>(p, stages);
+    *rc = launch_status("b200_norm_fwd [residual add, warp per row, warp rings]");
+  };
+  auto pick = [&](auto both_tag) {
+    constexpr bool BOTH = decltype(both_tag)::value;
+    if (ch == 3) {
+      if (exact) launch(residual_norm_warp_kernel<T, 3, true, BOTH>);
+      else launch(residual_norm_warp_kernel<T, 3, false, BOTH>);
+    } else {
+      if (exact) launch(residual_norm_warp_kernel<T, 4, true, BOTH>);
+      else launch(residual_norm_warp_kernel<T, 4, false, BOTH>);
+    }
+  };
+  if constexpr (sizeof(T) == 2) {
+    if (p.res_round == 2) pick(std::true_type{});
+    else pick(std::false_type{});
+  } else {
+    pick(std::false_type{});
+  }
+  return true;
+}
+
 // Element-wise kernel for ragged, unaligned or very long rows: one CTA per row, sweeps over
 // global memory (the second and third sweep of a row that fits in L2 are served from there).
 template <typename Tin, typename Tout>
@@ -684,6 +933,10 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
   if (vector_ok && p.n % V == 0 && !p.res) {  // the ring kernel streams one tensor
     int rc = B200_OK;
     if (try_launch_norm_fwd_stream<Tin, Tout>(p, st, &rc)) return rc;
+  }
+  if constexpr (kResBuilt) {
+    int rc = B200_OK;
+    if (vector_ok && p.n % V == 0 && p.res && try_launch_residual_norm_warp<Tin>(p, st, &rc)) return rc;
   }
   if (vector_ok && p.n % V == 0 && pick_row_geometry(p.n / V, &g)) {
     set_path_tag(g.block ? (p.res ? "residual add, vector, row resident, CTA per row" : "vector, row resident, CTA per row")

@@ -59,6 +59,32 @@ def test_masked_softmax_of_ragged_rows(keys, dtype, scale):
     _near(got, torch.softmax(x.double() * (scale or 1.0) + mask.double(), -1), f"masked softmax {keys} {dtype}", floor=1e-7)
 
 
+def _layer_norm64(d, w, b, eps, rms):
+    c = d if rms else d - d.mean(-1, keepdim=True)
+    y = c * torch.rsqrt(c.square().mean(-1, keepdim=True) + eps) * w.double()
+    return y if b is None else y + b.double()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,n", [(1, 264), (9, 512), (1, 520), (13, 520), (4000, 768), (11, 776), (3, 1024), (5, 449), (3, 1023)])
+def test_residual_layer_norm_forms(rows, n, dtype):
+    """A warp per row with its own copy ring (65..128 vectors), and ragged rows: the element-wise choice
+    between the two forms is bit for bit a choice between the two single forms."""
+    k = _kernels()
+    x, r = _randn((rows, n), dtype, n, 2.0), _randn((rows, n), dtype, n + 1)
+    w, b = _randn((n,), dtype, n + 2, 2.0), _randn((n,), dtype, n + 3)
+    kw = dict(eps=1e-6, residual=r, want_sum=True, want_mean=True, want_rstd=True)
+    full, mean, rstd, _, total = k.norm_fwd(x, w, b, **kw)
+    rounded = k.norm_fwd(x, w, b, round_sum=True, **kw)[0]
+    both, mean2, rstd2, _, total2 = k.norm_fwd(x, w, b, round_sum="both", **kw)
+    s = x.float() + r.float()
+    assert torch.equal(total, s.to(dtype)) and torch.equal(total2, total)
+    assert torch.equal(mean, mean2) and torch.equal(rstd, rstd2)
+    assert torch.equal(both, torch.where(full.float().abs() > 3, full, rounded))
+    _near(full, _layer_norm64(x.double() + r.double(), w, b, 1e-6, False), f"fp32 form {rows}x{n} {dtype}", floor=4e-5)
+    _near(rounded, _layer_norm64(s.to(dtype).double(), w, b, 1e-6, False), f"rounded form {rows}x{n} {dtype}", floor=4e-5)
+
+
 @pytest.mark.parametrize("batch,rows,cols", [(1, 2, 2), (7, 49, 128), (5, 196, 64), (33, 3, 10), (2000, 5, 6), (9, 64, 66),
                                              (3, 129, 126), (2, 16, 1024), (2, 63, 65), (3, 65, 63), (2, 500, 333),
                                              (2, 501, 768), (1, 1, 300), (2, 300, 1), (1300, 33, 64)])
