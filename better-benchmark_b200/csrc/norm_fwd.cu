@@ -923,6 +923,106 @@ __global__ void __launch_bounds__(1024) norm_fwd_streaming_kernel(const NormFwdP
   }
 }
 
+// Ragged or unaligned rows that fit in registers: a warp per row (n <= 512) or a CTA per row, E
+// elements per thread at a distance of the group, so that every access of a warp is one coalesced
+// stretch of 2- or 4-byte elements whatever the row's alignment. The row is read once; the element-wise
+// sweeps below read it two to six times and are left with rows of more than 16 384 elements (16 a thread).
+// Bound by the number of those accesses: about 1.6 TB/s for 16-bit elements, 3.3 TB/s for fp32.
+// Measured against the sweeps: LayerNorm bf16 [20000, 769] 461.6 -> 73.8 us, RMSNorm f32 [20000, 1001]
+// 329.8 -> 49.2 us, residual LayerNorm f16 [46251, 449] 795.6 -> 106.9 us.
+// G: 32 = a warp per row, 0 = the CTA.
+template <typename Tin, typename Tout, int E, int G>
+__global__ void __launch_bounds__(G == 0 ? 1024 : 256) norm_fwd_ragged_kernel(const NormFwdParams p) {
+  __shared__ float red[64];
+  constexpr bool DUAL = std::is_same<Tin, Tout>::value && sizeof(Tin) == 2;
+  const int lane = glane<G>(), gs = gsize<G>();
+  long long row = grow<G>();
+  const bool valid = row < p.rows;  // warps of a partly filled last CTA recompute the last row
+  if (!valid) row = p.rows - 1;
+  const Tin* x = reinterpret_cast<const Tin*>(p.x) + row * p.x_row_stride;
+  const Tin* res = p.res ? reinterpret_cast<const Tin*>(p.res) + row * p.x_row_stride : nullptr;
+  const bool both = DUAL && res != nullptr && p.res_round == 2;
+  const int n = p.n;
+  float f[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) f[e] = e * gs + lane < n ? Elem<Tin>::to_f32(__ldg(x + e * gs + lane)) : 0.f;
+  if (res) {
+    float r[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) r[e] = e * gs + lane < n ? Elem<Tin>::to_f32(__ldg(res + e * gs + lane)) : 0.f;
+    Tin* so = p.sum_out && valid ? reinterpret_cast<Tin*>(p.sum_out) + row * (long long)n : nullptr;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      f[e] = f[e] + r[e];
+      if (so && e * gs + lane < n) so[e * gs + lane] = Elem<Tin>::from_f32(f[e]);
+      if (p.res_round == 1) f[e] = round_through<Tin>(f[e]);
+    }
+  }
+  if (p.prologue == 1) {  // gelu(0) = 0: the padding stays zero
+#pragma unroll
+    for (int e = 0; e < E; ++e) f[e] = gelu_erf_rounded<Tin>(f[e]);
+  }
+  float s = 0.f, t = 0.f;  // t: the sum over the rounded values (both forms)
+#pragma unroll
+  for (int e = 0; e < E; ++e) s += p.rms ? f[e] * f[e] : f[e];
+  if constexpr (DUAL) {
+    if (both) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) t += round_through<Tin>(f[e]);
+    }
+  }
+  greduce_sum2<G>(s, t, red);
+  float mean = 0.f, var = s * p.inv_n, rstd_r = 0.f;
+  const float mean_r = t * p.inv_n;
+  if (!p.rms) {
+    mean = s * p.inv_n;
+    float q = 0.f, u = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (e * gs + lane < n) {
+        const float d = f[e] - mean;
+        q += d * d;
+        if constexpr (DUAL) {
+          if (both) {
+            const float dr = round_through<Tin>(f[e]) - mean_r;
+            u += dr * dr;
+          }
+        }
+      }
+    }
+    greduce_sum2<G>(q, u, red);
+    var = q * p.inv_denom;
+    rstd_r = precise_rsqrt(u * p.inv_denom + p.eps);
+  }
+  const float rstd = precise_rsqrt(var + p.eps);
+  if (lane == 0 && valid) {
+    if (p.mean_out) p.mean_out[row] = mean;
+    if (p.rstd_out) p.rstd_out[row] = rstd;
+    if (p.var_out) p.var_out[row] = var;
+  }
+  if (p.y == nullptr || !valid) return;
+  Tout* y = reinterpret_cast<Tout*>(p.y) + row * p.y_row_stride;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = e * gs + lane;
+    if (i < n) {
+      const float w = p.w ? load_param1(p.w, p.w_dtype, i) : 1.f;
+      const float b = p.b ? load_param1(p.b, p.w_dtype, i) : 0.f;
+      float o = (f[e] - mean) * rstd;
+      if (p.w) o = o * w;
+      if (p.b) o = o + b;
+      if constexpr (DUAL) {
+        if (both && !(fabsf(round_through<Tout>(o)) > 3.0f)) {
+          o = (round_through<Tin>(f[e]) - mean_r) * rstd_r;
+          if (p.w) o = o * w;
+          if (p.b) o = o + b;
+        }
+      }
+      y[i] = Elem<Tout>::from_f32(o);
+    }
+  }
+}
+
 template <typename Tin, typename Tout>
 static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t st) {
   constexpr int V = Elem<Tin>::V;
@@ -974,11 +1074,24 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
       else B200_NF_LAUNCH(0, 8);
     }
 #undef B200_NF_LAUNCH
+  } else if (p.n <= 16384) {
+    set_path_tag(p.res ? "residual add, elements in registers" : "elements in registers");
+    if (p.n <= 512) {  // a warp per row
+      const unsigned grid = (unsigned)((p.rows + 7) / 8);
+      if (p.n <= 64) norm_fwd_ragged_kernel<Tin, Tout, 2, 32><<<grid, 256, 0, st>>>(p);
+      else if (p.n <= 128) norm_fwd_ragged_kernel<Tin, Tout, 4, 32><<<grid, 256, 0, st>>>(p);
+      else if (p.n <= 256) norm_fwd_ragged_kernel<Tin, Tout, 8, 32><<<grid, 256, 0, st>>>(p);
+      else norm_fwd_ragged_kernel<Tin, Tout, 16, 32><<<grid, 256, 0, st>>>(p);
+    } else if (p.n <= 8192) {
+      const int threads = ((p.n + 7) / 8 + 31) / 32 * 32;
+      norm_fwd_ragged_kernel<Tin, Tout, 8, 0><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    } else {
+      const int threads = ((p.n + 15) / 16 + 31) / 32 * 32;
+      norm_fwd_ragged_kernel<Tin, Tout, 16, 0><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    }
   } else {
-    int threads = 1024;
-    while (threads > 64 && threads / 2 >= p.n) threads /= 2;
     set_path_tag(p.res ? "residual add, element-wise, CTA per row" : "element-wise, CTA per row");
-    norm_fwd_streaming_kernel<Tin, Tout><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    norm_fwd_streaming_kernel<Tin, Tout><<<(unsigned)p.rows, 1024, 0, st>>>(p);
   }
   return launch_status("b200_norm_fwd");
 }

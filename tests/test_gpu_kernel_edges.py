@@ -65,6 +65,16 @@ def _layer_norm64(d, w, b, eps, rms):
     return y if b is None else y + b.double()
 
 
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,n", [(3, 2), (9, 33), (7, 65), (10, 129), (5, 257), (3, 511), (3, 513), (2, 8191),
+                                    (2, 8193), (2, 16383), (2, 16385)])
+def test_norm_fwd_of_ragged_rows(rows, n, dtype, rms):
+    x, w, b = _randn((rows, n), dtype, n), _randn((n,), dtype, n + 1), None if rms else _randn((n,), dtype, n + 2)
+    y = _kernels().norm_fwd(x, w, b, eps=1e-5, rms=rms)[0]
+    _near(y, _layer_norm64(x.double(), w, b, 1e-5, rms), f"norm {rows}x{n} {dtype} rms={rms}", floor=2e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows,n", [(1, 264), (9, 512), (1, 520), (13, 520), (4000, 768), (11, 776), (3, 1024), (5, 449), (3, 1023)])
 def test_residual_layer_norm_forms(rows, n, dtype):
