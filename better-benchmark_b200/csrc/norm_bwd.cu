@@ -199,10 +199,7 @@ norm_bwd_kernel(const NormBwdParams p) {
   }
   if (p.fused) {
     const bool ok = grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) {
-      if (p.dw) finalize_columns(p.partials, p.groups, p.n, p.dw, fin);
-      if (LN && p.db) finalize_columns(p.partials + (long long)p.groups * p.n, p.groups, p.n, p.db, fin);
-    }
+    if (ok) finalize_sectors(p, LN && p.db, fin);
     grid_barrier_depart(p.bar);
   }
 }
@@ -436,10 +433,7 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
   }
   if (p.fused) {
     const bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) {
-      if (p.dw) finalize_columns(p.partials, p.groups, p.n, p.dw, fin);
-      if (LN && p.db) finalize_columns(p.partials + (long long)p.groups * p.n, p.groups, p.n, p.db, fin);
-    }
+    if (ok) finalize_sectors(p, LN && p.db, fin);
     grid_barrier_depart(p.bar);
   }
 }
@@ -740,23 +734,8 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
     }
   }
   if (p.fused) {
-    bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
-    const int chunks = (p.n + 63) / 64;
-    const int slices = (int)gridDim.x / chunks;
-    if (ok && p.level2 != nullptr && slices >= 2) {
-      double* l2w = p.level2;
-      double* l2b = p.level2 + (long long)slices * p.n;
-      if (p.dw) finalize_level1(p.partials, p.groups, p.n, l2w, slices, fin);
-      if (LN && p.db) finalize_level1(p.partials + (long long)p.groups * p.n, p.groups, p.n, l2b, slices, fin);
-      ok = grid_barrier(p.bar, 2u, &bar_ok);
-      if (ok) {
-        if (p.dw) finalize_level2(l2w, slices, p.n, p.dw);
-        if (LN && p.db) finalize_level2(l2b, slices, p.n, p.db);
-      }
-    } else if (ok) {
-      if (p.dw) finalize_columns(p.partials, p.groups, p.n, p.dw, fin);
-      if (LN && p.db) finalize_columns(p.partials + (long long)p.groups * p.n, p.groups, p.n, p.db, fin);
-    }
+    const bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
+    if (ok) finalize_sectors(p, LN && p.db, fin);
     grid_barrier_depart(p.bar);
   }
 }
@@ -963,15 +942,6 @@ static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratc
   }
   p.groups = (int)grid;
   p.fused = cooperative ? 1 : 0;
-  p.level2 = nullptr;
-  if (cooperative && (p.dw || p.db)) {  // room for the second level of the finalize behind the partial planes?
-    const long long chunks = (p.n + 63) / 64;
-    const long long slices = grid / chunks;
-    const long long planes = 256 + 2LL * grid * p.n * (long long)sizeof(float);
-    const long long need = (planes + 7) / 8 * 8 + 2LL * slices * p.n * (long long)sizeof(double);
-    if (slices >= 2 && (long long)scratch_bytes >= need)
-      p.level2 = reinterpret_cast<double*>(reinterpret_cast<char*>(p.bar) + (planes + 7) / 8 * 8);
-  }
   int tg_arg = tg, groups_arg = groups_per_cta, wpg_inv_arg = (65536 + tg / 32 - 1) / (tg / 32);
   if (cooperative) {
     int stages_arg = stages;
@@ -1120,8 +1090,8 @@ extern "C" int64_t b200_norm_bwd_wait_timeouts(void) {
 }
 
 // Bytes of scratch that let every path run its largest grid for rows of n elements: the barrier
-// words, two planes (dweight, dbias) of one fp32 partial row per group, and the fp64 second level
-// of the fused finalize. A group is a CTA (at most eight resident per SM), except in the
+// words, two planes (dweight, dbias) of one fp32 partial row per group, and 64 fp64 values per
+// group that nothing uses any more (the size that callers have been told stays). A group is a CTA (at most eight resident per SM), except in the
 // warp-per-row register kernel that takes rows of up to 256 elements, where it is a warp (64 per
 // SM). The launchers shrink their grids to whatever scratch they are given, so a smaller buffer
 // costs speed, never correctness.
@@ -1167,7 +1137,7 @@ extern "C" int b200_norm_bwd(const void* x, const void* dy, const void* weight, 
   p.n_f = (float)n;
   p.bar = reinterpret_cast<unsigned int*>(scratch);
   p.partials = scratch ? reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + 256) : nullptr;
-  p.groups = 0; p.fused = 0; p.level2 = nullptr;
+  p.groups = 0; p.fused = 0;
   const bool cooperative = (flags & 1) == 0 && (dweight || dbias);
 
   const int eb = dtype_size(x_dtype), wb = dtype_size(w_dtype);

@@ -28,7 +28,6 @@ struct NormBwdParams {
   long long dx_batch_stride, dx_seq_stride, dx_head_stride;
   float n_f;
   float* partials;    // [groups][n] for dw, followed by [groups][n] for db
-  double* level2;     // [2][slices][n]: second level of the fused finalize (may be null)
   unsigned int* bar;  // grid barrier words (cooperative variant)
   int groups;
   int fused;  // 1: barrier + finalize inside this launch
@@ -80,66 +79,58 @@ __device__ __forceinline__ void finalize_columns(const float* partials, int grou
   }
 }
 
-// Two-level variant for grids much larger than the number of 64-column chunks (narrow rows): with
-// one chunk per CTA only n/64 CTAs would add up all the partial rows while the rest of the grid
-// idles. Level 1: CTA b sums chunk b % chunks over the partial rows slice, slice + slices, ...
-// (slice = b / chunks) and writes fp64 sums; a grid barrier; level 2: the first `chunks` CTAs add
-// the slices in order. `which` selects the dw (0) or db (1) plane of `level2`.
-__device__ __forceinline__ void finalize_level1(const float* partials, int groups, int n, double* level2, int slices,
-                                                double* smem /* [warps][64] */) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int chunks = (n + 63) / 64;
-  if ((int)blockIdx.x >= chunks * slices) return;
-  const int chunk = blockIdx.x % chunks, slice = blockIdx.x / chunks;
-  const int c0 = chunk * 64 + lane, c1 = c0 + 32;
-  double a0 = 0.0, a1 = 0.0;
-  for (int k0 = warp; slice + slices * k0 < groups; k0 += 4 * nwarps) {
-    float v0[4], v1[4];
+// The same inside a cooperative launch, after its grid barrier, for rows of n % 4 == 0 columns: the
+// columns of dw and db are dealt out in 32-byte sectors (eight columns), so that the whole grid takes
+// part (192 CTAs for 768 columns of both) and no second level, with a second grid barrier, is needed
+// (LayerNorm backward bf16 [32768, 768], together with the copies that start before the weights are
+// staged: 45.1 us with the two levels, 39.0 us so).
+// Two threads share a sector of a partial row; the CTA's threads split the partial rows. fp64, fixed
+// order.
+__device__ __forceinline__ void finalize_sectors(const NormBwdParams& p, bool with_db, double* smem /* [warps][8] */) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int n = p.n, groups = p.groups;
+  const int sectors = (n + 7) / 8, rows_at_once = blockDim.x >> 1;
+  const int total = sectors * ((p.dw ? 1 : 0) + (with_db ? 1 : 0));
+  for (int s = blockIdx.x; s < total; s += gridDim.x) {
+    const bool is_db = !p.dw || s >= sectors;
+    const int col = (p.dw && s >= sectors ? s - sectors : s) * 8;
+    const int c = col + 4 * (tid & 1);
+    const float* src = p.partials + (is_db ? (long long)groups * n : 0) + c;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (c < n) {
+      for (int g0 = tid >> 1; g0 < groups; g0 += 4 * rows_at_once) {
+        float4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int g = slice + slices * (k0 + u * nwarps);
-      const float* row = partials + (long long)g * n;
-      v0[u] = (g < groups && c0 < n) ? __ldcg(row + c0) : 0.f;
-      v1[u] = (g < groups && c1 < n) ? __ldcg(row + c1) : 0.f;
+        for (int u = 0; u < 4; ++u) {
+          const int g = g0 + u * rows_at_once;
+          v[u] = g < groups ? __ldcg(reinterpret_cast<const float4*>(src + (long long)g * n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          acc[0] += (double)v[u].x;
+          acc[1] += (double)v[u].y;
+          acc[2] += (double)v[u].z;
+          acc[3] += (double)v[u].w;
+        }
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      a0 += (double)v0[u];
-      a1 += (double)v1[u];
+    for (int o = 16; o >= 2; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+    if (lane < 2) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) smem[warp * 8 + lane * 4 + i] = acc[i];
     }
-  }
-  smem[warp * 64 + lane] = a0;
-  smem[warp * 64 + 32 + lane] = a1;
-  __syncthreads();
-  if (warp == 0) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int w = 0; w < nwarps; ++w) {
-      s0 += smem[w * 64 + lane];
-      s1 += smem[w * 64 + 32 + lane];
+    __syncthreads();
+    if (tid < 8 && col + tid < n) {
+      double t = 0.0;
+      for (int w = 0; w < nwarps; ++w) t += smem[w * 8 + tid];
+      (is_db ? p.db : p.dw)[col + tid] = (float)t;
     }
-    if (c0 < n) level2[(long long)slice * n + c0] = s0;
-    if (c1 < n) level2[(long long)slice * n + c1] = s1;
+    __syncthreads();
   }
-  __syncthreads();
 }
-
-__device__ __forceinline__ void finalize_level2(const double* level2, int slices, int n, float* out) {
-  const int chunks = (n + 63) / 64;
-  if ((int)blockIdx.x >= chunks || threadIdx.x >= 64) return;
-  const int c = blockIdx.x * 64 + threadIdx.x;
-  if (c >= n) return;
-  double s = 0.0;
-  for (int k0 = 0; k0 < slices; k0 += 8) {  // eight loads in flight, added in order
-    double v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      v[u] = k0 + u < slices ? __ldcg(level2 + (long long)(k0 + u) * n + c) : 0.0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) s += v[u];
-  }
-  out[c] = (float)s;
-}
-
 
 // Warp reduction of N (2, 4 or 8) values per lane at once: in every step a lane keeps one half of
 // its values and hands the other half to its partner, so N values need N - 1 + log2(32 / N)

@@ -19,9 +19,8 @@
 //   * Two sweeps over the stage: row sums first (one batched warp reduction), then dx and the
 //     gradient sums. The stage is refilled as soon as the second sweep has read it.
 //   * At the end the warps of a CTA fold their sums in a fixed order through shared memory into
-//     ONE fp32 partial row per CTA; after the grid barrier the partial rows are added in fp64
-//     (two-level when the grid is much larger than the number of 64-column chunks). No atomics:
-//     results are bit-reproducible.
+//     ONE fp32 partial row per CTA; after the grid barrier the partial rows are added in fp64 by
+//     the whole grid. No atomics: results are bit-reproducible.
 // Every wait is bounded; a wait that runs out makes the warp stop, wait (bounded) for its own
 // copies and raise the error word of the grid barrier, so that all CTAs leave.
 #include "norm_bwd.cuh"
@@ -59,8 +58,8 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   if (threadIdx.x == 0) cta_failed = 0;
   if (lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
+    mbar_init_fence();
   }
-  mbar_init_fence();
 
   const T* xg = reinterpret_cast<const T*>(p.x);
   const T* dyg = reinterpret_cast<const T*>(p.dy);
@@ -71,6 +70,13 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     bulk_load(dst, xg + row * p.x_row_stride, row_bytes, &full[slot]);
     if constexpr (!DYS) bulk_load(dst + row_bytes, dyg + row * p.dy_row_stride, row_bytes, &full[slot]);
   };
+  // a warp's first rows are on their way before the weights are staged; the other lanes first touch
+  // the barriers after the __syncthreads below
+  int issued = 0;
+  if (lane == 0) {
+    for (; issued < my_rows && issued < stages; ++issued) issue(issued, issued);
+  }
+  issued = __shfl_sync(0xffffffffu, issued, 0);
   const f32x2 dy_all = splat2(DYS ? Elem<T>::to_f32(__ldg(dyg)) : 0.f);
 
   // weight slice: registers (RMSNorm) or shared memory (LayerNorm, which already keeps two
@@ -116,7 +122,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
       for (int i = 0; i < P; ++i) wv[c][i] = pack2(wf[2 * i], wf[2 * i + 1]);
     }
   }
-  __syncthreads();  // barriers initialised, weight slice in place
+  __syncthreads();  // barriers initialised (seen by every lane), weight slice in place
 
   // LayerNorm with a scalar dy: g = dy * w is the same in every row, and so are sum(g) and the
   // term g * n - sum(g) of dx. They are computed once: sum(g) by every warp (same order, same
@@ -140,12 +146,6 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     }
     __syncthreads();
   }
-
-  int issued = 0;
-  if (lane == 0) {
-    for (; issued < my_rows && issued < stages; ++issued) issue(issued, issued);
-  }
-  issued = __shfl_sync(0xffffffffu, issued, 0);
 
   f32x2 acc_w[CH][P], acc_b[LN ? CH : 1][P];
   uint32_t dx_col[CH];
@@ -397,24 +397,9 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     __syncthreads();  // the fold area doubles as the fp64 area of the finalize
   }
   if (p.fused) {
-    double* fin = reinterpret_cast<double*>(smem);  // [warps][64] fp64, inside the ring
-    bool ok = !any_failed && grid_barrier(p.bar, 1u, &bar_ok);
-    const int chunks = (p.n + 63) / 64;
-    const int slices = (int)gridDim.x / chunks;
-    if (ok && p.level2 != nullptr && slices >= 2) {
-      double* l2w = p.level2;
-      double* l2b = p.level2 + (long long)slices * p.n;
-      if (p.dw) finalize_level1(p.partials, p.groups, p.n, l2w, slices, fin);
-      if (LN && p.db) finalize_level1(p.partials + (long long)p.groups * p.n, p.groups, p.n, l2b, slices, fin);
-      ok = grid_barrier(p.bar, 2u, &bar_ok);
-      if (ok) {
-        if (p.dw) finalize_level2(l2w, slices, p.n, p.dw);
-        if (LN && p.db) finalize_level2(l2b, slices, p.n, p.db);
-      }
-    } else if (ok) {
-      if (p.dw) finalize_columns(p.partials, p.groups, p.n, p.dw, fin);
-      if (LN && p.db) finalize_columns(p.partials + (long long)p.groups * p.n, p.groups, p.n, p.db, fin);
-    }
+    double* fin = reinterpret_cast<double*>(smem);  // [warps][8] fp64, inside the ring
+    const bool ok = !any_failed && grid_barrier(p.bar, 1u, &bar_ok);
+    if (ok) finalize_sectors(p, LN && p.db, fin);
     grid_barrier_depart(p.bar);
   }
 }
@@ -463,15 +448,6 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
   }
   p.groups = (int)grid;
   p.fused = 1;
-  p.level2 = nullptr;
-  if (p.dw || p.db) {  // room for the second level of the finalize behind the partial planes?
-    const long long chunks = (p.n + 63) / 64;
-    const long long slices = grid / chunks;
-    const long long planes = 256 + 2LL * grid * p.n * (long long)sizeof(float);
-    const long long need = (planes + 7) / 8 * 8 + 2LL * slices * p.n * (long long)sizeof(double);
-    if (slices >= 2 && (long long)scratch_bytes >= need)
-      p.level2 = reinterpret_cast<double*>(reinterpret_cast<char*>(p.bar) + (planes + 7) / 8 * 8);
-  }
   int stages_arg = stages, ring_arg = (int)ring_bytes;
   void* args[] = {&p, &stages_arg, &ring_arg};
   e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), dim3(kWarps * 32),

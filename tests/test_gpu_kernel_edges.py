@@ -95,6 +95,31 @@ def test_residual_layer_norm_forms(rows, n, dtype):
     _near(rounded, _layer_norm64(s.to(dtype).double(), w, b, 1e-6, False), f"rounded form {rows}x{n} {dtype}", floor=4e-5)
 
 
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,n", [(1, 3), (7, 129), (600, 257), (9, 511), (700, 513), (5, 4095),   # ragged rows
+                                    (600, 132), (40, 520), (5000, 264), (3, 4104)])                  # last sector half full
+def test_norm_bwd_edges(rows, n, dtype, rms):
+    x, dy, w = _randn((rows, n), dtype, n), _randn((rows, n), dtype, n + 1), _randn((n,), torch.float32, n + 2)
+    d, g = x.double(), dy.double() * w.double()
+    mean = None if rms else x.float().mean(-1)
+    c = d if rms else d - mean.double()[:, None]
+    rstd = torch.rsqrt(c.square().mean(-1) + 1e-5).float()
+    dx, dw, db = _kernels().norm_bwd(x, dy, w, rstd, mean=mean, rms=rms, want_dbias=not rms)
+    xhat = c * rstd.double()[:, None]
+    want = g - xhat * (g * xhat).mean(-1, keepdim=True)
+    if not rms:
+        want = want - g.mean(-1, keepdim=True)
+    want = want * rstd.double()[:, None]
+    scale = want.abs().max().item()
+    _near(dx, want, f"dx {rows}x{n} {dtype}", floor=4e-6 * max(scale, 1.0))
+    # fp32 chains per thread, fp64 above them: a few fp32 ulps of the largest partial sum
+    floor = 2.0 ** -21 * max(1.0, rows ** 0.5) * 8
+    _near(dw, (dy.double() * xhat).sum(0), f"dweight {rows}x{n}", floor=floor)
+    if not rms:
+        _near(db, dy.double().sum(0), f"dbias {rows}x{n}", floor=floor)
+
+
 @pytest.mark.parametrize("batch,rows,cols", [(1, 2, 2), (7, 49, 128), (5, 196, 64), (33, 3, 10), (2000, 5, 6), (9, 64, 66),
                                              (3, 129, 126), (2, 16, 1024), (2, 63, 65), (3, 65, 63), (2, 500, 333),
                                              (2, 501, 768), (1, 1, 300), (2, 300, 1), (1300, 33, 64)])
