@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256) transpose_small_kernel(const TransposePar
 // the activations' code (the erf and exp sequences cost registers and instruction-cache lines that a 5 us
 // parameter cast would pay for without using them).
 template <typename Tin, typename Tout, bool VEC, int ACT>
-__global__ void __launch_bounds__(256, ACT >= 4 ? 3 : 4) cast_scale_kernel(const void* x, void* y, long long n, float scale,
+__global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const void* x, void* y, long long n, float scale,
                                                                             int mode_word) {
   const int has_scale = mode_word & 1;
   constexpr int VIN = VEC ? Elem<Tin>::V : 1;
@@ -435,7 +435,9 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 3 : 4) cast_scale_kernel(const
   if constexpr (VEC) {
     // A CTA takes blocks of U * blockDim consecutive vectors (block b, b + grid, ...): its U loads
     // in flight per thread fall into one contiguous stretch of memory.
-    constexpr int U = 4;
+    // GELU and SiLU: two loads and five CTAs per SM (48 registers) instead of four and three - their
+    // arithmetic needs the warps more than the loads in flight (SiLU bf16 [32768, 1536] 47.1 -> 42.5 us).
+    constexpr int U = ACT >= 4 ? 2 : 4;
     const long long stride = blockDim.x;
     const long long block = (long long)U * blockDim.x;
     for (long long u0 = (long long)blockIdx.x * block + threadIdx.x; u0 < units; u0 += (long long)gridDim.x * block) {
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 3 : 4) cast_scale_kernel(const
             // and keeps its reciprocal a normal number up to exp(88). The argument is clamped to the range in
             // which the result does not depend on it any more (the exponential needs finite inputs).
             // The SFU pipe (two exponentials and two reciprocals a pair) is what bounds it. Measured on
-            // bf16 [32768, 1536]: 63.5 us with the correctly rounded software reciprocal, 47.1 us here.
+            // bf16 [32768, 1536]: 63.5 us with the correctly rounded software reciprocal, 47.1 us with this one.
 #pragma unroll
             for (int i = 0; i < VIN / 2; ++i) {
               const float a = f[2 * i], b = f[2 * i + 1];
