@@ -55,7 +55,10 @@ def _require_cuda(*tensors: torch.Tensor) -> torch.device:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of the current stream of the current device: what
+    # torch.cuda.current_stream().cuda_stream returns, without building a Stream object on every
+    # call (3.3 us against 0.2 us; a small kernel launch as a whole takes 4 us)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t):
@@ -206,6 +209,8 @@ def _rows_2d(t: torch.Tensor, what: str):
     n = t.shape[-1]
     if n > 1 and t.stride(-1) != 1:
         raise UnsupportedLayout(f"{what}: the last dimension must be contiguous")
+    if n > 0 and t.is_contiguous():  # the usual case, without the general collapse
+        return t.numel() // n, n, n
     oshape, ostr = _outer(t)
     dims, (s,) = collapse_outer(oshape, [ostr])
     if dims[1] != 1 or dims[2] != 1:
@@ -260,7 +265,7 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
     y = None
     y_stride = n
     if want_y:
-        y = torch.empty(x.shape, dtype=out_dtype, device=x.device)
+        y = torch.empty_like(x, dtype=out_dtype, memory_format=torch.contiguous_format)
     stat_shape = list(x.shape[:-1]) + ([1] if keepdim else [])
 
     def stat(flag):

@@ -151,6 +151,10 @@ def check(status: int, what: str) -> None:
     raise KernelLaunchError(f"{what}: CUDA error {status}: {text}")
 
 
+_I64_ARRAYS = {n: c_int64 * n for n in (3, 4)}   # building an array type costs more than filling it
+
+
 def i64_array(values) -> ctypes.Array:
     vals = [int(v) for v in values]
-    return (c_int64 * len(vals))(*vals)
+    kind = _I64_ARRAYS.get(len(vals)) or c_int64 * len(vals)
+    return kind(*vals)
