@@ -12,9 +12,9 @@
 //   c1 = sum_dy * (1/N);  c2 = (dot * (1/N)) * (invstd * invstd);  gs = invstd * w
 //   dx = cast(((float(dy') - (float(x) - mean) * c2) - c1) * gs)
 //
-// Three launches: sums (a thread's own short chain in fp32, everything above it in fp64; per-CTA
-// partials over a fixed split of the rows), finalize (fixed order, coefficient table), apply (each
-// CTA walks its part of the rows backwards, so that it starts in what the sums pass left in L2).
+// Three launches, chained by programmatic dependent launch: sums (a thread's own short chains in fp32,
+// everything above them in fp64; per-CTA partials), finalize (fixed order, coefficient table), apply
+// (from the end of the tensors to their front, so that it starts in what the sums pass left in L2).
 // No atomics: bit-reproducible.
 // Channels-last tensors whose channel count is a multiple of the 16-byte vector (at most 256
 // vectors per row) take the vector kernels; every other layout the strided element-wise ones.
@@ -23,6 +23,7 @@
 #include <cooperative_groups.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace b200 {
 
@@ -73,18 +74,24 @@ __device__ __forceinline__ void bn_bwd_prologue(f32x2 (&g)[Elem<T>::V / 2], cons
 // Channels-last sums: the tensors are flat [rows * C] arrays of 16-byte vectors, whatever C is. A
 // vector may straddle the end of a row; the pattern of channels under a vector repeats every
 // PV = C / gcd(C, V) vectors: vector i has phase i % PV and its element j belongs to channel
-// (phase * V + j) % C. blockDim.x and the CTA's range [b*per, (b+1)*per) are multiples of PV, so a
-// thread keeps its phase - its V channels - for the whole launch.
-template <typename T>
-__global__ void __launch_bounds__(256) bn_bwd_sums_cl_kernel(const BnBwdParams p, long long vecs_per_cta, int PV) {
+// (phase * V + j) % C. blockDim.x, and with it a chunk of kChunk * blockDim.x vectors, is a multiple
+// of PV, so a thread keeps its phase - its V channels - for the whole launch.
+// All CTAs of the grid are resident and take chunks b, b + grid, ...: the launch moves through the
+// tensors from front to back as a whole, so what it leaves in L2 is their last part, which is where
+// the apply kernel begins. What bounds it: 4.8 TB/s of reads, the loads of a round being waited for
+// before the next are issued (more, smaller CTAs per SM were slower: 4 of 64 registers 119 us, 3 of 80
+// registers 107 us for the whole call). Measured on bf16 [256, 64, 56, 56] (sums, finalize, apply):
+// 105.5 us with 8 CTAs per SM on contiguous ranges, 102.5 us so; bf16 [64, 256, 14, 14] with the
+// activation 31.9 -> 27.4 us; f32 [121, 485, 16, 16], element-wise before, 345 -> 64 us.
+constexpr int kChunk = 4;  // vectors of each tensor in flight per thread
+
+// MAXT: 256 threads, or 512 for patterns of more than 256 vectors (one CTA per SM of as many threads).
+template <typename T, bool ACT, int MAXT>
+__global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_sums_cl_kernel(const BnBwdParams p, long long total, int PV) {
   constexpr int V = Elem<T>::V;
-  __shared__ float red[2 * 256 * 8 / 8 * 8];  // [2][threads][V] fp32, V <= 8
+  __shared__ float red[2 * MAXT * V];  // [2][threads][V]
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
   const int ph = tid % PV;
-  const long long total = p.rows * C / V;
-  const long long v0 = (long long)blockIdx.x * vecs_per_cta;
-  long long v1 = v0 + vecs_per_cta;
-  if (v1 > total) v1 = total;
   const uint4* dy = reinterpret_cast<const uint4*>(p.dy);
   const uint4* x = reinterpret_cast<const uint4*>(p.x);
   const uint4* act = reinterpret_cast<const uint4*>(p.act);
@@ -94,36 +101,46 @@ __global__ void __launch_bounds__(256) bn_bwd_sums_cl_kernel(const BnBwdParams p
     mean2[i] = pack2(__ldg(p.mean + (ph * V + 2 * i) % C), __ldg(p.mean + (ph * V + 2 * i + 1) % C));
     s1[i] = s2[i] = splat2(0.f);
   }
-  constexpr int U = 4;  // vectors of each tensor in flight per thread
-  for (long long v = v0 + tid; v < v1; v += (long long)U * T_) {
-    uint4 rg[U], rx[U], ra[U];
+  const long long step = (long long)gridDim.x * kChunk * T_;
+  for (long long v = (long long)blockIdx.x * kChunk * T_ + tid; v < total; v += step) {
+    uint4 rg[kChunk], rx[kChunk], ra[ACT ? kChunk : 1];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < kChunk; ++u) {
       const long long i = v + (long long)u * T_;
-      if (i < v1) {
+      if (i < total) {
         rg[u] = ld_stream(reinterpret_cast<const T*>(dy + i));
         rx[u] = ld_stream(reinterpret_cast<const T*>(x + i));
-        if (act) ra[u] = ld_stream(reinterpret_cast<const T*>(act + i));
+        if constexpr (ACT) ra[u] = ld_stream(reinterpret_cast<const T*>(act + i));
       }
     }
+    // the chunk's own short sums first: the chain over the chunks is then kChunk times shorter
+    f32x2 t1[V / 2], t2[V / 2];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (v + (long long)u * T_ < v1) {
+    for (int i = 0; i < V / 2; ++i) t1[i] = t2[i] = splat2(0.f);
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      if (v + (long long)u * T_ < total) {
         f32x2 g[V / 2], xv[V / 2];
         Pairs<T>::unpack(rg[u], g);
         Pairs<T>::unpack(rx[u], xv);
-        if (act) bn_bwd_prologue<T>(g, ra[u], p.slope);
+        if constexpr (ACT) bn_bwd_prologue<T>(g, ra[u], p.slope);
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) {
-          s1[i] = add2(s1[i], g[i]);
-          s2[i] = add2(s2[i], mul2(g[i], sub2(xv[i], mean2[i])));
+          t1[i] = add2(t1[i], g[i]);
+          t2[i] = add2(t2[i], mul2(g[i], sub2(xv[i], mean2[i])));
         }
       }
     }
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {
+      s1[i] = add2(s1[i], t1[i]);
+      s2[i] = add2(s2[i], t2[i]);
+    }
   }
-  // fold the threads of a column (tid, tid + vpr, ...) in a fixed order
+  let_next_kernel_start();
+  // fold the threads of a phase (tid, tid + PV, ...) in a fixed order
   float* r1 = red;
-  float* r2 = red + 256 * V;
+  float* r2 = red + MAXT * V;
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) {
     unpack2(s1[i], r1[tid * V + 2 * i], r1[tid * V + 2 * i + 1]);
@@ -159,14 +176,16 @@ __global__ void __launch_bounds__(256) bn_bwd_finalize_kernel(const BnBwdParams 
     mean = __ldg(p.mean + c);
     if (p.weight) w = load_param1(p.weight, p.w_dtype, c);
   }
+  wait_for_previous_kernel();
+  let_next_kernel_start();
   double s1 = 0.0, s2 = 0.0;
   for (int g0 = tid; g0 < p.splits; g0 += 256 * 4) {
     double a[4], b[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int g = g0 + u * 256;
-      a[u] = g < p.splits ? p.partials[((long long)g * 2) * p.channels + c] : 0.0;
-      b[u] = g < p.splits ? p.partials[((long long)g * 2 + 1) * p.channels + c] : 0.0;
+      a[u] = g < p.splits ? __ldcg(p.partials + ((long long)g * 2) * p.channels + c) : 0.0;
+      b[u] = g < p.splits ? __ldcg(p.partials + ((long long)g * 2 + 1) * p.channels + c) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -200,59 +219,63 @@ __global__ void __launch_bounds__(256) bn_bwd_finalize_kernel(const BnBwdParams 
   }
 }
 
-// Apply pass. CTA b takes the same vectors [b*per, (b+1)*per) as in the sums pass but walks them
-// from the end to the start: what the sums pass read last is what is still in L2, so the first
-// part of this pass is served from there instead of DRAM (the two inputs together are larger than
-// the L2, so walking forward again would find nothing). blockDim.x and `per` are multiples of vpr,
-// so a thread stays in one vector column here too.
-template <typename T>
-__global__ void __launch_bounds__(256) bn_bwd_apply_cl_kernel(const BnBwdParams p, long long vecs_per_cta, int PV) {
+// Apply pass: the chunks of the sums pass from the last to the first. The sums pass ended with the end
+// of the tensors, so the first part of this pass is served from L2 (what is left of the two inputs there);
+// dx is written with streaming stores that do not push it out. The first chunk is requested before
+// the coefficients are there.
+template <typename T, bool ACT, int MAXT>
+__global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_apply_cl_kernel(const BnBwdParams p, long long total, int PV) {
   constexpr int V = Elem<T>::V;
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
-  const int ph = PV - 1 - tid % PV;  // the range ends on a multiple of PV: its last vector has phase PV - 1
-  const long long total = p.rows * C / V;
-  const long long v0 = (long long)blockIdx.x * vecs_per_cta;
-  long long v1 = v0 + vecs_per_cta;
-  if (v1 > total) v1 = total;
+  const int ph = tid % PV;
   const uint4* dy = reinterpret_cast<const uint4*>(p.dy);
   const uint4* x = reinterpret_cast<const uint4*>(p.x);
   const uint4* act = reinterpret_cast<const uint4*>(p.act);
   uint4* dx = reinterpret_cast<uint4*>(p.dx);
+  const long long chunk = (long long)kChunk * T_, step = (long long)gridDim.x * chunk;
+  const long long last = (total - 1) / chunk * chunk;  // first vector of the last chunk
+  long long v = last - (long long)blockIdx.x * chunk + tid;
+  uint4 rg[kChunk], rx[kChunk], ra[ACT ? kChunk : 1];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      const long long i = v + (long long)u * T_;
+      if (i >= 0 && i < total) {
+        rg[u] = ld_stream(reinterpret_cast<const T*>(dy + i));
+        rx[u] = ld_stream(reinterpret_cast<const T*>(x + i));
+        if constexpr (ACT) ra[u] = ld_stream(reinterpret_cast<const T*>(act + i));
+      }
+    }
+  };
+  fetch();
+  wait_for_previous_kernel();
   f32x2 c1[V / 2], c2[V / 2], gs[V / 2], mean2[V / 2];
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) {
     const int c = (ph * V + 2 * i) % C, d = (ph * V + 2 * i + 1) % C;
-    c1[i] = pack2(p.coef[c], p.coef[d]);
-    c2[i] = pack2(p.coef[C + c], p.coef[C + d]);
-    gs[i] = pack2(p.coef[2 * C + c], p.coef[2 * C + d]);
-    mean2[i] = pack2(p.coef[3 * C + c], p.coef[3 * C + d]);
+    c1[i] = pack2(__ldcg(p.coef + c), __ldcg(p.coef + d));
+    c2[i] = pack2(__ldcg(p.coef + C + c), __ldcg(p.coef + C + d));
+    gs[i] = pack2(__ldcg(p.coef + 2 * C + c), __ldcg(p.coef + 2 * C + d));
+    mean2[i] = pack2(__ldcg(p.coef + 3 * C + c), __ldcg(p.coef + 3 * C + d));
   }
-  constexpr int U = 4;
-  for (long long v = v1 - 1 - tid; v >= v0; v -= (long long)U * T_) {
-    uint4 rg[U], rx[U], ra[U];
+  for (; v >= 0; v -= step) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long i = v - (long long)u * T_;
-      if (i >= v0) {
-        rg[u] = ld_stream(reinterpret_cast<const T*>(dy + i));
-        rx[u] = ld_stream(reinterpret_cast<const T*>(x + i));
-        if (act) ra[u] = ld_stream(reinterpret_cast<const T*>(act + i));
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long i = v - (long long)u * T_;
-      if (i >= v0) {
+    for (int u = 0; u < kChunk; ++u) {
+      const long long i = v + (long long)u * T_;
+      if (i < total) {
         f32x2 g[V / 2], xv[V / 2], o[V / 2];
         Pairs<T>::unpack(rg[u], g);
         Pairs<T>::unpack(rx[u], xv);
-        if (act) bn_bwd_prologue<T>(g, ra[u], p.slope);
+        if constexpr (ACT) bn_bwd_prologue<T>(g, ra[u], p.slope);
 #pragma unroll
         for (int k = 0; k < V / 2; ++k)
           o[k] = mul2(sub2(sub2(g[k], mul2(sub2(xv[k], mean2[k]), c2[k])), c1[k]), gs[k]);
         st_stream(reinterpret_cast<T*>(dx + i), Pairs<T>::pack(o));
       }
     }
+    v -= step;
+    fetch();
+    v += step;
   }
 }
 
@@ -716,29 +739,34 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
     long long g = p.channels, h = V;  // gcd(C, V)
     while (h) { const long long t = g % h; g = h; h = t; }
     const int vpr = (int)(p.channels / g);  // PV: vectors after which the channel pattern repeats
-    const int threads = 256 / vpr * vpr;  // a multiple of PV: a thread keeps its phase
+    const int threads = vpr <= 256 ? 256 / vpr * vpr : vpr;  // a multiple of PV: a thread keeps its phase
     const long long total = p.rows * p.channels / V;
-    long long splits = 8LL * dev.sm_count;  // eight CTAs per SM
+    long long splits = (threads <= 256 ? 2LL : 1LL) * dev.sm_count;  // all CTAs resident
     // at least two rounds of loads (8 vectors of each tensor) per thread: small tensors get few
     // partial rows and a short finalize
     if (splits * threads * 8 > total) splits = (total + threads * 8 - 1) / (threads * 8);
     if (splits < 1) splits = 1;
-    long long per = (total + splits - 1) / splits;
-    per = (per + vpr - 1) / vpr * vpr;  // whole rows per CTA: the column of a thread stays fixed
-    splits = (total + per - 1) / per;
     const long long need = splits * 2 * p.channels * (long long)sizeof(double) + coef_floats * (long long)sizeof(float);
     if ((long long)scratch_bytes < need)
       return fail(B200_ERR_WORKSPACE, "b200_batch_norm_bwd: scratch of %zu bytes, need %lld", scratch_bytes, need);
     p.splits = (int)splits;
     p.coef = reinterpret_cast<float*>(p.partials + splits * 2 * p.channels);
-    bn_bwd_sums_cl_kernel<T><<<(unsigned)splits, threads, 0, st>>>(p, per, vpr);
-    int rc = launch_status("b200_batch_norm_bwd sums");
-    if (rc != B200_OK) return rc;
-    bn_bwd_finalize_kernel<<<p.channels, 256, 0, st>>>(p);
-    rc = launch_status("b200_batch_norm_bwd finalize");
-    if (rc != B200_OK || !p.dx) return rc;
-    bn_bwd_apply_cl_kernel<T><<<(unsigned)splits, threads, 0, st>>>(p, per, vpr);
-    return launch_status("b200_batch_norm_bwd apply [channels-last, vector]");
+    auto run = [&](auto act_tag, auto maxt_tag) {
+      constexpr bool ACT = decltype(act_tag)::value;
+      constexpr int MAXT = decltype(maxt_tag)::value;
+      bn_bwd_sums_cl_kernel<T, ACT, MAXT><<<(unsigned)splits, threads, 0, st>>>(p, total, vpr);
+      int rc = launch_status("b200_batch_norm_bwd sums");
+      if (rc != B200_OK) return rc;
+      launch_dependent(bn_bwd_finalize_kernel, dim3((unsigned)p.channels), dim3(256), st, p);
+      rc = launch_status("b200_batch_norm_bwd finalize");
+      if (rc != B200_OK || !p.dx) return rc;
+      launch_dependent(bn_bwd_apply_cl_kernel<T, ACT, MAXT>, dim3((unsigned)splits), dim3((unsigned)threads), st, p, total, vpr);
+      return launch_status("b200_batch_norm_bwd apply [channels-last, vector]");
+    };
+    using Narrow = std::integral_constant<int, 256>;
+    using Wide = std::integral_constant<int, 512>;
+    if (p.act) return threads <= 256 ? run(std::true_type{}, Narrow{}) : run(std::true_type{}, Wide{});
+    return threads <= 256 ? run(std::false_type{}, Narrow{}) : run(std::false_type{}, Wide{});
   }
   {  // contiguous NCHW: one launch, a cluster of CTAs per channel
     int rc = B200_OK;
@@ -806,11 +834,11 @@ extern "C" int b200_batch_norm_bwd_ex(const void* dy, const void* x, const void*
   const int v = 16 / eb;
   const bool cl = stride_c == 1 && stride_s == channels && stride_n == spatial * channels;
   // vectors after which the pattern of channels under a vector repeats: C / gcd(C, v); the flat
-  // kernels need whole periods and at most 256 vectors in one
+  // kernels need whole periods and at most 512 vectors in one
   long long g = channels, h = v;
   while (h) { const long long t = g % h; g = h; h = t; }
   const long long pv = channels / g;
-  const bool fast = cl && pv >= 1 && pv <= 256 && (batch * spatial * channels) % (pv * v) == 0 && aligned16(dy) &&
+  const bool fast = cl && pv >= 1 && pv <= 512 && (batch * spatial * channels) % (pv * v) == 0 && aligned16(dy) &&
                     aligned16(x) && (!act || aligned16(act)) && (!dx || aligned16(dx));
   p.rows = fast ? batch * spatial : batch;
   switch (x_dtype) {

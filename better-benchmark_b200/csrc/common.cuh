@@ -355,6 +355,28 @@ __device__ __forceinline__ void grid_barrier_depart(unsigned int* bar) {
   }
 }
 
+// Programmatic dependent launch between the kernels of ONE call (statistics -> finalize -> apply): a
+// kernel launched by launch_dependent may start while the kernel before it drains. Whatever it does
+// before wait_for_previous_kernel must not depend on that kernel's results; after it, all of them are
+// visible. let_next_kernel_start lets the next launch_dependent kernel begin as soon as every CTA of
+// this one has called it or left (without it: when this kernel has ended).
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Formal, typename... Actual>
+inline cudaError_t launch_dependent(void (*kernel)(Formal...), dim3 grid, dim3 block, cudaStream_t st, Actual... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, Formal(args)...);
+}
+
 // The occupancy query is a host-side calculation; cached per (kernel, block size, smem).
 inline int cached_occupancy(const void* fn, int threads, size_t smem = 0) {
   struct Entry { const void* fn; int threads; size_t smem; int blocks; };
