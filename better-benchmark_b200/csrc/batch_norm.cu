@@ -924,11 +924,12 @@ __global__ void __launch_bounds__(256) batch_norm_apply_general_kernel(const Bat
 //   apply     the same ranges walked from the end (what the sums pass read last is what L2 still
 //             holds), y written with streaming stores
 // ----------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256, 3) batch_norm_sums_cl_flat_kernel(const BatchNormParams p, long long vecs_per_cta,
+// MAXT: 256 threads, or 512 for patterns of more than 256 vectors.
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1) batch_norm_sums_cl_flat_kernel(const BatchNormParams p, long long vecs_per_cta,
                                                                       int PV, int rows_shift) {
   constexpr int V = Elem<T>::V;
-  __shared__ float red[2 * 256 * V];  // [2][threads][V]
+  __shared__ float red[2 * MAXT * V];  // [2][threads][V]
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
   const int ph = tid % PV;
   const long long total = p.rows * C / V;
@@ -939,7 +940,7 @@ __global__ void __launch_bounds__(256, 3) batch_norm_sums_cl_flat_kernel(const B
   const uint4* x = reinterpret_cast<const uint4*>(p.x);
   // The shift of every channel (bn_shift_scalar: mean of its first sixteen rows, eight significant
   // bits; the finalize kernel forms the same value) is computed once per CTA into shared memory,
-  // at most 2 * 256 * V channels per round, and every thread picks up its V channels.
+  // at most 2 * MAXT * V channels per round, and every thread picks up its V channels.
   f32x2 shift[V / 2], s1[V / 2], s2[V / 2];
   f32x2 upper[V / 2];  // a thread's sum of squares moves here every 16 vectors: two short chains instead of one long one
 #pragma unroll
@@ -949,16 +950,16 @@ __global__ void __launch_bounds__(256, 3) batch_norm_sums_cl_flat_kernel(const B
     for (int i = 0; i < V / 2; ++i)
       shift[i] = pack2(Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i) % C)), Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i + 1) % C)));
   }
-  for (int c0 = 0; rows_shift && c0 < C; c0 += 2 * 256 * V) {
-    for (int c = c0 + tid; c < C && c < c0 + 2 * 256 * V; c += T_) red[c - c0] = bn_shift_scalar<T>(xe, c, C, p.rows);
+  for (int c0 = 0; rows_shift && c0 < C; c0 += 2 * MAXT * V) {
+    for (int c = c0 + tid; c < C && c < c0 + 2 * MAXT * V; c += T_) red[c - c0] = bn_shift_scalar<T>(xe, c, C, p.rows);
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < V / 2; ++i) {
       const int ca = (ph * V + 2 * i) % C, cb = (ph * V + 2 * i + 1) % C;
       float lo, hi;
       unpack2(shift[i], lo, hi);
-      if (ca >= c0 && ca < c0 + 2 * 256 * V) lo = red[ca - c0];
-      if (cb >= c0 && cb < c0 + 2 * 256 * V) hi = red[cb - c0];
+      if (ca >= c0 && ca < c0 + 2 * MAXT * V) lo = red[ca - c0];
+      if (cb >= c0 && cb < c0 + 2 * MAXT * V) hi = red[cb - c0];
       shift[i] = pack2(lo, hi);
     }
     __syncthreads();
@@ -994,7 +995,7 @@ __global__ void __launch_bounds__(256, 3) batch_norm_sums_cl_flat_kernel(const B
     }
   }
   float* r1 = red;
-  float* r2 = red + 256 * V;
+  float* r2 = red + MAXT * V;
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) {
     unpack2(s1[i], r1[tid * V + 2 * i], r1[tid * V + 2 * i + 1]);
@@ -1016,8 +1017,8 @@ __global__ void __launch_bounds__(256, 3) batch_norm_sums_cl_flat_kernel(const B
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256, 3) batch_norm_apply_cl_flat_kernel(const BatchNormParams p, long long vecs_per_cta,
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1) batch_norm_apply_cl_flat_kernel(const BatchNormParams p, long long vecs_per_cta,
                                                                        int PV) {
   constexpr int V = Elem<T>::V;
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
@@ -1077,9 +1078,9 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
   while (h) { const long long t = g % h; g = h; h = t; }
   const long long PV = C / g;
   const long long elems = p.rows * C;
-  if (PV > 256 || elems % (PV * V) != 0) return false;  // whole periods only: every range ends on a multiple of PV
+  if (PV > 512 || elems % (PV * V) != 0) return false;  // whole periods only: every range ends on a multiple of PV
   const long long total = elems / V;
-  const int threads = (int)(256 / PV * PV);
+  const int threads = (int)(PV <= 256 ? 256 / PV * PV : PV);
   const long long stats_floats = 2 * C;
   const long long room = ((long long)scratch_bytes - 256) / (long long)sizeof(float) - stats_floats;
   if (room < 2 * C) return false;
@@ -1094,13 +1095,15 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
   splits = (total + per - 1) / per;
   p.stats = p.partials + splits * 2 * C;
   const int rows_shift = per > 32LL * threads ? 1 : 0;  // more than 32 vectors per thread
-  batch_norm_sums_cl_flat_kernel<T><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV, rows_shift);
+  if (threads <= 256) batch_norm_sums_cl_flat_kernel<T, 256><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV, rows_shift);
+  else batch_norm_sums_cl_flat_kernel<T, 512><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV, rows_shift);
   *rc = launch_status("b200_batch_norm_fwd sums [channels-last, flat vectors]");
   if (*rc != B200_OK) return true;
   batch_norm_finalize_general_kernel<T><<<(p.channels + 7) / 8, 256, 0, st>>>(p, (int)splits, rows_shift);
   *rc = launch_status("b200_batch_norm_fwd finalize");
   if (*rc != B200_OK || !p.y) return true;
-  batch_norm_apply_cl_flat_kernel<T><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV);
+  if (threads <= 256) batch_norm_apply_cl_flat_kernel<T, 256><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV);
+  else batch_norm_apply_cl_flat_kernel<T, 512><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV);
   *rc = launch_status("b200_batch_norm_fwd apply [channels-last, flat vectors]");
   return true;
 }

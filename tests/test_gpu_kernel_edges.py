@@ -144,3 +144,32 @@ def test_silu_over_the_whole_range(dtype):
     _near(got[finite], want[finite], f"silu {dtype}", floor=1.2e-7 if dtype == torch.float16 else 1e-34)
     assert torch.isnan(got[torch.isnan(x)]).all()
     assert torch.equal(got[x == float("inf")], x[x == float("inf")])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,c,hw", [(8, 64, 49), (8, 257, 64), (16, 511, 16), (8, 1022, 16), (33, 24, 7), (64, 100, 196)])
+def test_batch_norm_channels_last_of_any_channel_count(n, c, hw, dtype):
+    """Channel patterns of up to 512 vectors, tensors of one chunk and of several per CTA, forward and
+    backward against fp64."""
+    k = _kernels()
+    x = _randn((n, c, hw, 1), dtype, c, 2.0).contiguous(memory_format=torch.channels_last)
+    dy = _randn((n, c, hw, 1), dtype, c + 1).contiguous(memory_format=torch.channels_last)
+    act = _randn((n, c, hw, 1), dtype, c + 2).contiguous(memory_format=torch.channels_last)
+    w, b = _randn((c,), torch.float32, c + 3), _randn((c,), torch.float32, c + 4)
+    col = lambda t: t.double().view(1, c, 1, 1)  # noqa: E731
+    d = x.double()
+    mean64, var64 = d.mean((0, 2, 3)), d.var((0, 2, 3), unbiased=False)
+    y, mean, invstd = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1, relu=True)
+    _near(mean, mean64, "mean", floor=2e-6)
+    _near(invstd, torch.rsqrt(var64 + 1e-5), "invstd", floor=2e-6)
+    _near(y, torch.relu((d - col(mean64)) * col(torch.rsqrt(var64 + 1e-5)) * col(w) + col(b)), f"y {n}x{c}x{hw}", floor=2e-5)
+    for a in (None, act):
+        dx, dw, db = k.batch_norm_bwd(dy, x, mean, invstd, w, act=a, slope=0.25)
+        g = dy.double() if a is None else torch.where(a > 0, dy, dy * 0.25).double()
+        xhat = (d - col(mean)) * col(invstd)
+        s1, s2 = g.sum((0, 2, 3)), (g * xhat).sum((0, 2, 3))
+        floor = 2.0 ** -21 * (n * hw) ** 0.5 * 8   # fp32 chains per thread, fp64 above them
+        _near(db, s1, "dbias", floor=floor)
+        _near(dw, s2, "dweight", floor=floor)
+        want = (g - col(s1) / (n * hw) - xhat * col(s2) / (n * hw)) * col(w) * col(invstd)
+        _near(dx, want, f"dx {n}x{c}x{hw}", floor=1e-5)
