@@ -58,16 +58,22 @@ struct NormFwdParams {
 // (repros/canonical/var_mean_af505388b035/repro.py:27-33): (x * 0.5) * (erf(x * 0.7071067811865476) + 1)
 // in fp32, in that order, then rounded to the tensor dtype - the graph materialises the
 // activation as a 16-bit tensor before the statistics are taken.
-template <typename Tin>
-__device__ __forceinline__ float gelu_erf_rounded(float x) {
-  const float g = (x * 0.5f) * (erff(x * 0.7071067811865476f) + 1.0f);
-  return round_through<Tin>(g);
-}
+// (16-bit tensors: gelu_pair, whose fp32 result is as close to the fp64 one as that expression's.)
 template <typename Tin>
 __device__ __forceinline__ f32x2 gelu_erf_rounded2(f32x2 v) {
+  if constexpr (sizeof(Tin) == 2) {
+    return Pairs<Tin>::word(Pairs<Tin>::narrow(gelu_pair(v)));
+  } else {
+    float a, b;
+    unpack2(v, a, b);
+    return pack2((a * 0.5f) * (erff(a * 0.7071067811865476f) + 1.0f), (b * 0.5f) * (erff(b * 0.7071067811865476f) + 1.0f));
+  }
+}
+template <typename Tin>
+__device__ __forceinline__ float gelu_erf_rounded(float x) {
   float a, b;
-  unpack2(v, a, b);
-  return pack2(gelu_erf_rounded<Tin>(a), gelu_erf_rounded<Tin>(b));
+  unpack2(gelu_erf_rounded2<Tin>(splat2(x)), a, b);
+  return a;
 }
 
 // rsqrtf is the 2-ulp hardware approximation aten's CUDA rsqrt uses as well.
@@ -960,7 +966,7 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256) norm_fwd_ragged_kernel(co
   }
   if (p.prologue == 1) {  // gelu(0) = 0: the padding stays zero
 #pragma unroll
-    for (int e = 0; e < E; ++e) f[e] = gelu_erf_rounded<Tin>(f[e]);
+    for (int e = 0; e < E; e += 2) unpack2(gelu_erf_rounded2<Tin>(pack2(f[e], f[e + 1])), f[e], f[e + 1]);
   }
   float s = 0.f, t = 0.f;  // t: the sum over the rounded values (both forms)
 #pragma unroll

@@ -479,6 +479,9 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const
               r = fma2(r, fma2(fma2(e, splat2(-0.25f), splat2(-0.25f)), r, splat2(1.0f)), r);
               unpack2(mul2(mul2(pack2(a, b), splat2(0.25f)), r), f[2 * i], f[2 * i + 1]);
             }
+          } else if constexpr (ACT == 4 && sizeof(Tout) == 2) {
+#pragma unroll
+            for (int i = 0; i < VIN / 2; ++i) unpack2(gelu_pair(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
           } else if constexpr (ACT != 0) {
 #pragma unroll
             for (int i = 0; i < VIN; ++i) f[i] = apply_activation<ACT>(f[i]);

@@ -219,6 +219,41 @@ __device__ __forceinline__ f32x2 exp_pair_fast(f32x2 x) {
   return r;
 }
 
+// Exact (erf-form) GELU of a pair, x * Phi(x), for results that are rounded to a 16-bit type afterwards.
+//
+// With a = |x| and Q(a) = erfc(a / sqrt 2) / 2 the normal distribution is Phi(x) = Q(a) for x < 0 and
+// 1 - Q(a) otherwise, and Q(a) = exp(-a^2 / 2) * P(t), t = 1 / (1 + 0.305 a), P a polynomial without a
+// constant term: the form of Hastings' approximations (Abramowitz & Stegun 26.2.17), here of degree
+// eight with coefficients fitted to erfcx by iteratively reweighted least squares (relative error of Q
+// below 9.5e-8 for 0 <= a <= 14). Over standard normal inputs the fp32 result is 3.9e-8 (2-norm) off
+// the fp64 one, the (x / 2) * (erff(x / sqrt 2) + 1) it replaces 3.7e-8; rounded to 16 bits both are
+// equally close, and for x < -3, where erff + 1 cancels, only this form keeps the value (within half a
+// 16-bit step over every bf16 and normal fp16 input). Fewer than half the instructions of erff. Measured:
+// GELU bf16 [32768, 1536] 69.6 -> 50.1 us, GELU -> LayerNorm bf16 [65536, 768] 81.2 -> 67.4 us.
+// a is clamped to 64 for the exponential, which needs finite arguments (Q(64) = 0); the product takes x
+// itself, so that inf, -inf (NaN, as -inf * 0) and NaN come out as the graph has them.
+__device__ __forceinline__ f32x2 gelu_pair(f32x2 x) {
+  float x0, x1, r0, r1, q0, q1, u0, u1;
+  unpack2(x, x0, x1);
+  const f32x2 a = pack2(fminf(fabsf(x0), 64.f), fminf(fabsf(x1), 64.f));
+  const f32x2 e = exp_pair_compensated(mul2(mul2(a, a), splat2(-0.5f)));
+  unpack2(fma2(a, splat2(0.305f), splat2(1.0f)), r0, r1);
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(r0));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(r1));
+  const f32x2 t = pack2(r0, r1);
+  f32x2 h = fma2(splat2(0.03669983148574829f), t, splat2(-0.1529906988143921f));
+  h = fma2(h, t, splat2(0.1857205182313919f));
+  h = fma2(h, t, splat2(-0.037979673594236374f));
+  h = fma2(h, t, splat2(0.12102290987968445f));
+  h = fma2(h, t, splat2(0.10342058539390564f));
+  h = fma2(h, t, splat2(0.12246684730052948f));
+  h = fma2(h, t, splat2(0.12163973599672318f));
+  const f32x2 q = mul2(e, mul2(h, t));
+  unpack2(q, q0, q1);
+  unpack2(sub2(splat2(1.0f), q), u0, u1);
+  return mul2(x, pack2(x0 < 0.f ? q0 : u0, x1 < 0.f ? q1 : u1));
+}
+
 template <bool BLOCK>
 __device__ __forceinline__ int group_lane() {
   return BLOCK ? (int)threadIdx.x : (int)(threadIdx.x & 31);

@@ -173,3 +173,17 @@ def test_batch_norm_channels_last_of_any_channel_count(n, c, hw, dtype):
         _near(dw, s2, "dweight", floor=floor)
         want = (g - col(s1) / (n * hw) - xhat * col(s2) / (n * hw)) * col(w) * col(invstd)
         _near(dx, want, f"dx {n}x{c}x{hw}", floor=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gelu_over_the_whole_range(dtype):
+    """Every 16-bit pattern against x * erfc(-x / sqrt 2) / 2 in fp64; -inf and NaN give NaN, as
+    (x / 2) * (erf(x / sqrt 2) + 1) does, +inf itself."""
+    x = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).cuda().view(dtype)
+    got = _kernels().cast_scale(x, dtype, activation="gelu_erf")
+    d = x.double()
+    want = 0.5 * d * torch.special.erfc(-d * 0.5 ** 0.5)
+    finite = torch.isfinite(x)
+    _near(got[finite], want[finite], f"gelu {dtype}", floor=6e-8 if dtype == torch.float16 else 1e-35)
+    assert torch.isnan(got[torch.isnan(x) | (x == float("-inf"))]).all()
+    assert torch.equal(got[x == float("inf")], x[x == float("inf")])
