@@ -746,8 +746,9 @@ __global__ void __launch_bounds__(512) norm_bwd_finalize_kernel(const NormBwdPar
   if (p.db) finalize_columns(p.partials + (long long)p.groups * p.n, p.groups, p.n, p.db, fin);
 }
 
-// Element-wise kernels for rows the vector path cannot take (ragged n, unaligned pointers, a head
-// size that is not a multiple of the vector length). Correct for every layout, not tuned.
+// Element-wise kernels for rows that neither the vector kernels nor the ragged one below can take (more
+// than 4096 elements, or a head size that is not a multiple of the vector length). Correct for every
+// layout, not tuned.
 template <typename T, bool LN>
 __global__ void __launch_bounds__(256) norm_bwd_rows_general_kernel(const NormBwdParams p) {
   __shared__ float red[32];
