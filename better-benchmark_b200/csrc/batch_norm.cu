@@ -33,6 +33,33 @@
 
 namespace b200 {
 
+// ReLU of a packed vector after the cast, as the graph has it; NaN stays NaN.
+template <typename T>
+__device__ __forceinline__ uint4 relu_packed(uint4 packed) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    const __nv_bfloat162 z = __float2bfloat162_rn(0.f);
+    uint32_t* w = reinterpret_cast<uint32_t*>(&packed);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      __nv_bfloat162 h = __hmax2_nan(*reinterpret_cast<__nv_bfloat162*>(&w[i]), z);
+      w[i] = *reinterpret_cast<uint32_t*>(&h);
+    }
+  } else if constexpr (std::is_same<T, __half>::value) {
+    const __half2 z = __float2half2_rn(0.f);
+    uint32_t* w = reinterpret_cast<uint32_t*>(&packed);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      __half2 h = __hmax2_nan(*reinterpret_cast<__half2*>(&w[i]), z);
+      w[i] = *reinterpret_cast<uint32_t*>(&h);
+    }
+  } else {
+    float* w = reinterpret_cast<float*>(&packed);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = w[i] < 0.f ? 0.f : w[i];  // NaN < 0 is false: NaN stays
+  }
+  return packed;
+}
+
 template <typename T, bool VECTOR>
 __device__ __forceinline__ void bn_finalize_channel(const BatchNormParams& p, int c, int num_partials,
                                                     float shift) {
@@ -748,29 +775,7 @@ batch_norm_cl_warp_kernel(const BatchNormParams p, const int stages, const int r
 #pragma unroll
       for (int i = 0; i < V / 2; ++i) o[i] = add2(mul2(mul2(sub2(f[i], mean2[i]), inv2[i]), w2[i]), b2[i]);
       uint4 packed = Pairs<T>::pack(o);
-      if (relu) {  // ReLU after the cast, as the graph has it; NaN stays NaN
-        if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-          const __nv_bfloat162 z = __float2bfloat162_rn(0.f);
-          uint32_t* w = reinterpret_cast<uint32_t*>(&packed);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            __nv_bfloat162 h = __hmax2_nan(*reinterpret_cast<__nv_bfloat162*>(&w[i]), z);
-            w[i] = *reinterpret_cast<uint32_t*>(&h);
-          }
-        } else if constexpr (std::is_same<T, __half>::value) {
-          const __half2 z = __float2half2_rn(0.f);
-          uint32_t* w = reinterpret_cast<uint32_t*>(&packed);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            __half2 h = __hmax2_nan(*reinterpret_cast<__half2*>(&w[i]), z);
-            w[i] = *reinterpret_cast<uint32_t*>(&h);
-          }
-        } else {
-          float* w = reinterpret_cast<float*>(&packed);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) w[i] = w[i] < 0.f ? 0.f : w[i];  // NaN < 0 is false: NaN stays
-        }
-      }
+      if (relu) packed = relu_packed<T>(packed);
       st_stream(reinterpret_cast<T*>(dst), packed);
     };
     const int resident_from = n_chunks - (n_chunks < stages ? n_chunks : stages);  // chunks >= this are in smem
@@ -1108,6 +1113,318 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
   return true;
 }
 
+// ----------------------------------------------------------------------------------------------
+// The same three steps for large tensors:
+//   sums      all CTAs are resident and take chunks b, b + grid, ...: the launch moves through the tensor
+//             from front to back as a whole, and what it leaves in L2 is the tensor's last part
+//   finalize  a CTA per channel
+//   apply     the chunks from the last to the first, so that it starts with what is in L2
+// Both passes bring x in through a ring of each thread's own in shared memory (asynchronous 16-byte
+// copies, read only by the thread that issued them: no barrier, no registers), which keeps about 160 KB
+// per SM on the way whatever the arithmetic does. The three kernels are chained by programmatic
+// dependent launch; apply fills its ring before the statistics are there.
+// Bound by HBM: bf16 [128, 96, 56, 56] takes 20 us for the sums (77 MB, next to the write-back of the
+// previous y), 4 for the finalize, 31 for the apply (writes settle near 3.4 TB/s in every kernel here).
+// Measured against the kernels above: that tensor 80.8 -> 53.5 us, [256, 92, 28, 28] (37 MB) 53.3 -> 42.7,
+// f32 [121, 485, 16, 16] (60 MB) 76 -> 37; bf16 [64, 120, 28, 28] (12 MB) 24.8 there, 31.8 here. Power-of-two
+// vector counts from 8 MB up stay with the cooperative kernel (bf16 [256, 64, 56, 56] 59.1 us, 61.3 here).
+// ----------------------------------------------------------------------------------------------
+constexpr long long kRingFromBytes = 32000000;  // between the two sides measured: 12 MB and 37 MB
+
+constexpr int kRingU = 4;  // vectors per thread in a stage
+constexpr int kRingS = 6;  // stages
+constexpr int kRingBytesPerThread = kRingS * kRingU * 16;  // 384
+
+// Brings vectors v, v + T_, ... that lie in [0, total) into stage s; always one group.
+__device__ __forceinline__ void bn_ring_issue(const uint4* x, uint32_t mine, int s, long long v, long long total, int T_) {
+  const uint32_t dst = mine + (uint32_t)(s * kRingU * T_) * 16u;
+#pragma unroll
+  for (int u = 0; u < kRingU; ++u) {
+    const long long i = v + (long long)u * T_;
+    if (i >= 0 && i < total) copy_async16(dst + (uint32_t)(u * T_) * 16u, x + i);
+  }
+  copy_async_commit();
+}
+
+// MAXT: 256 threads, or 512 for patterns of more than 256 vectors.
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total,
+                                                                                   int PV, int rows_shift) {
+  constexpr int V = Elem<T>::V;
+  extern __shared__ __align__(128) unsigned char smem[];
+  float* red = reinterpret_cast<float*>(smem + (size_t)kRingBytesPerThread * MAXT);  // [MAXT * V]: the shifts
+  const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
+  const int ph = tid % PV;
+  const T* xe = reinterpret_cast<const T*>(p.x);
+  const uint4* x = reinterpret_cast<const uint4*>(p.x);
+  const uint32_t mine = smem_u32(smem) + (uint32_t)tid * 16u;
+  const long long step = (long long)gridDim.x * kRingU * T_;
+  long long v = (long long)blockIdx.x * kRingU * T_ + tid;
+#pragma unroll
+  for (int s = 0; s < kRingS - 1; ++s) bn_ring_issue(x, mine, s, v + s * step, total, T_);
+  // The shift of every channel (bn_shift_scalar: mean of its first sixteen rows, eight significant
+  // bits; the finalize kernel forms the same value) is computed once per CTA into shared memory,
+  // at most MAXT * V channels per round, and every thread picks up its V channels.
+  f32x2 shift[V / 2], s1[V / 2], s2[V / 2], t1[V / 2], t2[V / 2];
+  f32x2 upper[V / 2];
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) shift[i] = s1[i] = s2[i] = t1[i] = t2[i] = upper[i] = splat2(0.f);
+  if (!rows_shift) {  // short chains (small tensors): the channel's element of row 0 will do
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i)
+      shift[i] = pack2(Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i) % C)), Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i + 1) % C)));
+  }
+  for (int c0 = 0; rows_shift && c0 < C; c0 += MAXT * V) {
+    for (int c = c0 + tid; c < C && c < c0 + MAXT * V; c += T_) red[c - c0] = bn_shift_scalar<T>(xe, c, C, p.rows);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {
+      const int ca = (ph * V + 2 * i) % C, cb = (ph * V + 2 * i + 1) % C;
+      float lo, hi;
+      unpack2(shift[i], lo, hi);
+      if (ca >= c0 && ca < c0 + MAXT * V) lo = red[ca - c0];
+      if (cb >= c0 && cb < c0 + MAXT * V) hi = red[cb - c0];
+      shift[i] = pack2(lo, hi);
+    }
+    __syncthreads();
+  }
+  // Additions of squares of 16-bit values are biased, in proportion to the length of the chain they
+  // join: two stages' squares are summed by themselves, sixteen of those join one chain, the chains a third.
+  int slot = 0, round = 0;
+  for (; v < total; v += step) {
+    bn_ring_issue(x, mine, slot == 0 ? kRingS - 1 : slot - 1, v + (kRingS - 1) * step, total, T_);
+    copy_async_wait<kRingS - 1>();
+    const uint32_t src = mine + (uint32_t)(slot * kRingU * T_) * 16u;
+#pragma unroll
+    for (int u = 0; u < kRingU; ++u) {
+      if (v + (long long)u * T_ < total) {
+        f32x2 f[V / 2];
+        Pairs<T>::unpack(lds128(src + (uint32_t)(u * T_) * 16u), f);
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i) {
+          const f32x2 d = sub2(f[i], shift[i]);
+          t1[i] = add2(t1[i], d);
+          t2[i] = fma2(d, d, t2[i]);
+        }
+      }
+    }
+    ++round;
+    if ((round & 1) == 0) {
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) {
+        s1[i] = add2(s1[i], t1[i]);
+        s2[i] = add2(s2[i], t2[i]);
+        t1[i] = t2[i] = splat2(0.f);
+      }
+    }
+    if ((round & 31) == 0) {
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) {
+        upper[i] = add2(upper[i], s2[i]);
+        s2[i] = splat2(0.f);
+      }
+    }
+    if (++slot == kRingS) slot = 0;
+  }
+  let_next_kernel_start();
+  __syncthreads();  // every thread has read its ring: the memory is reused
+  float* r1 = reinterpret_cast<float*>(smem);  // [2][MAXT][V]
+  float* r2 = r1 + MAXT * V;
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) {
+    unpack2(add2(s1[i], t1[i]), r1[tid * V + 2 * i], r1[tid * V + 2 * i + 1]);
+    unpack2(add2(upper[i], add2(s2[i], t2[i])), r2[tid * V + 2 * i], r2[tid * V + 2 * i + 1]);
+  }
+  __syncthreads();
+  const int period = PV * V;  // elements; a multiple of C
+  for (int c = tid; c < C; c += T_) {
+    double a = 0.0, b = 0.0;
+    for (int idx = c; idx < period; idx += C) {  // every (phase, element) that lands on channel c
+      const int col = idx / V, e = idx % V;
+      for (int t = col; t < T_; t += PV) {
+        a += (double)r1[t * V + e];
+        b += (double)r2[t * V + e];
+      }
+    }
+    p.partials[((long long)blockIdx.x * 2) * C + c] = (float)a;
+    p.partials[((long long)blockIdx.x * 2 + 1) * C + c] = (float)b;
+  }
+}
+
+// Finalize: a CTA per channel, all partial rows of it in flight at once, fp64 in a fixed
+// order. Everything but the partial rows (the shift) is requested before the sums are there. The sixteen
+// values of the shift are added in the order of bn_shift_scalar: the same bits.
+template <typename T>
+__global__ void __launch_bounds__(256) batch_norm_finalize_ring_kernel(const BatchNormParams p, int splits, int rows_shift) {
+  __shared__ double red[2][8];
+  __shared__ float first_rows[BN_SHIFT_ROWS];
+  const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const T* x = reinterpret_cast<const T*>(p.x);
+  if (tid < BN_SHIFT_ROWS) {
+    const long long r = rows_shift ? (tid < p.rows ? tid : p.rows - 1) : 0;
+    first_rows[tid] = Elem<T>::to_f32(__ldg(x + r * p.channels + c));
+  }
+  wait_for_previous_kernel();
+  let_next_kernel_start();
+  float old_mean = 0.f, old_var = 0.f;
+  if (tid == 0 && p.running_mean) {
+    old_mean = __ldcg(p.running_mean + c);
+    old_var = __ldcg(p.running_var + c);
+  }
+  double s1 = 0.0, s2 = 0.0;
+  for (int g0 = tid; g0 < splits; g0 += 4 * 256) {
+    float a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int g = g0 + u * 256;
+      a[u] = g < splits ? __ldcg(p.partials + ((long long)g * 2) * p.channels + c) : 0.f;
+      b[u] = g < splits ? __ldcg(p.partials + ((long long)g * 2 + 1) * p.channels + c) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s1 += (double)a[u];
+      s2 += (double)b[u];
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+  if (lane == 0) {
+    red[0][warp] = s1;
+    red[1][warp] = s2;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    s1 = s2 = 0.0;
+    for (int w = 0; w < 8; ++w) {
+      s1 += red[0][w];
+      s2 += red[1][w];
+    }
+    float shift = first_rows[0];
+    if (rows_shift) {
+      shift = 0.f;
+      for (int r = 0; r < BN_SHIFT_ROWS; ++r) shift = __fadd_rn(shift, first_rows[r]);
+      shift = bn_round_shift(__fmul_rn(shift, 1.0f / BN_SHIFT_ROWS));
+    }
+    float mean, invstd;
+    bn_channel_stats(p, c, s1, s2, shift, true, &mean, &invstd, true, old_mean, old_var);
+    p.stats[c] = mean;
+    p.stats[p.channels + c] = invstd;
+  }
+}
+
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_apply_cl_ring_kernel(const BatchNormParams p, long long total,
+                                                                                    int PV) {
+  constexpr int V = Elem<T>::V;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
+  const int ph = tid % PV;
+  const uint4* x = reinterpret_cast<const uint4*>(p.x);
+  uint4* y = reinterpret_cast<uint4*>(p.y);
+  const uint32_t mine = smem_u32(smem) + (uint32_t)tid * 16u;
+  const long long chunk = (long long)kRingU * T_, step = (long long)gridDim.x * chunk;
+  long long v = (total - 1) / chunk * chunk - (long long)blockIdx.x * chunk + tid;  // from the last chunk down
+#pragma unroll
+  for (int s = 0; s < kRingS - 1; ++s) bn_ring_issue(x, mine, s, v - s * step, total, T_);
+  f32x2 mean2[V / 2], inv2[V / 2], w2[V / 2], b2[V / 2];
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) {
+    const int c0 = (ph * V + 2 * i) % C, c1 = (ph * V + 2 * i + 1) % C;
+    w2[i] = p.weight ? pack2(load_param1(p.weight, p.w_dtype, c0), load_param1(p.weight, p.w_dtype, c1)) : splat2(1.f);
+    b2[i] = p.bias ? pack2(load_param1(p.bias, p.w_dtype, c0), load_param1(p.bias, p.w_dtype, c1)) : splat2(0.f);
+  }
+  wait_for_previous_kernel();
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) {
+    const int c0 = (ph * V + 2 * i) % C, c1 = (ph * V + 2 * i + 1) % C;
+    mean2[i] = pack2(__ldcg(p.stats + c0), __ldcg(p.stats + c1));
+    inv2[i] = pack2(__ldcg(p.stats + C + c0), __ldcg(p.stats + C + c1));
+  }
+  const bool relu = p.relu != 0;
+  int slot = 0;
+  for (; v >= 0; v -= step) {
+    bn_ring_issue(x, mine, slot == 0 ? kRingS - 1 : slot - 1, v - (kRingS - 1) * step, total, T_);
+    copy_async_wait<kRingS - 1>();
+    const uint32_t src = mine + (uint32_t)(slot * kRingU * T_) * 16u;
+#pragma unroll
+    for (int u = 0; u < kRingU; ++u) {
+      const long long i = v + (long long)u * T_;
+      if (i < total) {
+        f32x2 f[V / 2];
+        Pairs<T>::unpack(lds128(src + (uint32_t)(u * T_) * 16u), f);
+#pragma unroll
+        for (int k = 0; k < V / 2; ++k) f[k] = add2(mul2(mul2(sub2(f[k], mean2[k]), inv2[k]), w2[k]), b2[k]);
+        uint4 packed = Pairs<T>::pack(f);
+        if (relu) packed = relu_packed<T>(packed);
+        st_stream(reinterpret_cast<T*>(y + i), packed);
+      }
+    }
+    if (++slot == kRingS) slot = 0;
+  }
+  copy_async_wait<0>();
+}
+
+// Returns false when the shape does not fit, or is below kRingFromBytes (the caller takes the kernels above).
+template <typename T>
+static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_bytes, cudaStream_t st, int* rc) {
+  constexpr int V = Elem<T>::V;
+  const DeviceInfo& dev = device_info();
+  const long long C = p.channels;
+  long long g = C, h = V;  // gcd(C, V)
+  while (h) { const long long t = g % h; g = h; h = t; }
+  const long long PV = C / g;
+  const long long elems = p.rows * C;
+  if (PV > 512 || elems % (PV * V) != 0) return false;  // whole periods only
+  if (elems * (long long)sizeof(T) < kRingFromBytes) return false;
+  const long long total = elems / V;
+  const int threads = (int)(PV <= 256 ? 256 / PV * PV : PV);
+  const long long stats_floats = 2 * C;
+  const long long room = ((long long)scratch_bytes - 256) / (long long)sizeof(float) - stats_floats;
+  if (room < 2 * C) return false;
+  long long splits = (threads <= 256 ? 2LL : 1LL) * dev.sm_count;  // all CTAs resident
+  // at least 8 vectors per thread: small tensors get few partial rows and a short finalize
+  if (splits * threads * 8 > total) splits = (total + threads * 8 - 1) / (threads * 8);
+  if (splits > room / (2 * C)) return false;  // the kernels above make do with fewer partial rows
+  if (splits < 1) splits = 1;
+  p.stats = p.partials + splits * 2 * C;
+  const int rows_shift = total > 32LL * threads * splits ? 1 : 0;  // more than 32 vectors per thread
+  auto run = [&](auto maxt_tag) {
+    constexpr int MAXT = decltype(maxt_tag)::value;
+    auto sums = batch_norm_sums_cl_ring_kernel<T, MAXT>;
+    auto apply = batch_norm_apply_cl_ring_kernel<T, MAXT>;
+    const size_t ring = (size_t)kRingBytesPerThread * MAXT;  // 96 KB, or 192 KB: two CTAs, or one, per SM
+    const size_t with_shifts = ring + (size_t)MAXT * V * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(sums), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)with_shifts);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(reinterpret_cast<const void*>(apply), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+    // the finalize kernel uses next to no shared memory: asked to keep the split of its neighbours, it does
+    // not make every SM drain and re-partition twice a call
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(reinterpret_cast<const void*>(batch_norm_finalize_ring_kernel<T>),
+                               cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      *rc = fail((int)e, "b200_batch_norm_fwd: cannot reserve %zu bytes of shared memory: %s", with_shifts, cudaGetErrorString(e));
+      return;
+    }
+    sums<<<(unsigned)splits, threads, with_shifts, st>>>(p, total, (int)PV, rows_shift);
+    *rc = launch_status("b200_batch_norm_fwd sums [channels-last, flat vectors, copy rings]");
+    if (*rc != B200_OK) return;
+    launch_dependent(batch_norm_finalize_ring_kernel<T>, dim3((unsigned)p.channels), dim3(256), 0, st, p, (int)splits, rows_shift);
+    *rc = launch_status("b200_batch_norm_fwd finalize");
+    if (*rc != B200_OK || !p.y) return;
+    launch_dependent(apply, dim3((unsigned)splits), dim3((unsigned)threads), ring, st, p, total, (int)PV);
+    *rc = launch_status("b200_batch_norm_fwd apply [channels-last, flat vectors, copy rings]");
+  };
+  if (threads <= 256) run(std::integral_constant<int, 256>{});
+  else run(std::integral_constant<int, 512>{});
+  return true;
+}
+
 // Channels-last tensors smaller than this take the three flat launches: a cooperative launch with
 // its grid-wide barriers costs more than two extra plain launches until the tensor is tens of MB.
 constexpr long long kFlatBelowBytes = 8000000;  // measured: 3.2 MB 16.3 us flat / 21.3 us fused, 12.8 MB 27.5 / 24.1
@@ -1255,6 +1572,7 @@ static int launch_batch_norm(BatchNormParams p, bool channels_last_fast, bool ch
     BatchNormParams q = p;
     q.rows = p.rows * p.spatial;
     int rc = B200_OK;
+    if (try_launch_batch_norm_cl_ring<T>(q, scratch_bytes, st, &rc)) return rc;
     if (try_launch_batch_norm_cl_flat<T>(q, scratch_bytes, st, &rc)) return rc;
   }
   {  // contiguous NCHW: one launch, a cluster of CTAs per channel (batch_norm_nchw.cu)

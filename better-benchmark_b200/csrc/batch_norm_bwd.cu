@@ -757,10 +757,10 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
       bn_bwd_sums_cl_kernel<T, ACT, MAXT><<<(unsigned)splits, threads, 0, st>>>(p, total, vpr);
       int rc = launch_status("b200_batch_norm_bwd sums");
       if (rc != B200_OK) return rc;
-      launch_dependent(bn_bwd_finalize_kernel, dim3((unsigned)p.channels), dim3(256), st, p);
+      launch_dependent(bn_bwd_finalize_kernel, dim3((unsigned)p.channels), dim3(256), 0, st, p);
       rc = launch_status("b200_batch_norm_bwd finalize");
       if (rc != B200_OK || !p.dx) return rc;
-      launch_dependent(bn_bwd_apply_cl_kernel<T, ACT, MAXT>, dim3((unsigned)splits), dim3((unsigned)threads), st, p, total, vpr);
+      launch_dependent(bn_bwd_apply_cl_kernel<T, ACT, MAXT>, dim3((unsigned)splits), dim3((unsigned)threads), 0, st, p, total, vpr);
       return launch_status("b200_batch_norm_bwd apply [channels-last, vector]");
     };
     using Narrow = std::integral_constant<int, 256>;

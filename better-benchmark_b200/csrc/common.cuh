@@ -364,10 +364,12 @@ __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("gridd
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... Formal, typename... Actual>
-inline cudaError_t launch_dependent(void (*kernel)(Formal...), dim3 grid, dim3 block, cudaStream_t st, Actual... args) {
+inline cudaError_t launch_dependent(void (*kernel)(Formal...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                    Actual... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

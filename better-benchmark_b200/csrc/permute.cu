@@ -282,10 +282,6 @@ __global__ void __launch_bounds__(256) transpose16_ragged_kernel(const Transpose
 // What bounds it: HBM, with the shared-memory passes (copy in, read, write, copy out: about 390 cycles
 // for a [49, 128] matrix, a third of the time its bytes take) behind it. Measured on bf16 [16384, 49, 128]:
 // 141.4 us with two-byte gathers (four-way bank conflicts), 74.1 us (5.55 TB/s) here.
-__device__ __forceinline__ void copy_async16(uint32_t smem_dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
-}
-
 template <bool ODD>
 __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposeParams p, const int group, const int stages,
                                                               const int split, const FastDiv by_tasks,

@@ -74,6 +74,18 @@ __device__ __forceinline__ void bulk_load_hint(void* smem_dst, const void* gmem_
       : "memory");
 }
 
+// 16-byte asynchronous copies that a thread issues for itself. They complete in groups; a thread that
+// only ever reads its own slots needs no barrier after copy_async_wait (which leaves the N newest groups
+// in flight).
+__device__ __forceinline__ void copy_async16(uint32_t smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Bounded wait for the phase with the given parity. Returns false when the bound ran out.
 // ~2M polls with back-off: far beyond any legitimate copy latency, well under a second.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {

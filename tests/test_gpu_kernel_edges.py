@@ -147,7 +147,8 @@ def test_silu_over_the_whole_range(dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("n,c,hw", [(8, 64, 49), (8, 257, 64), (16, 511, 16), (8, 1022, 16), (33, 24, 7), (64, 100, 196)])
+@pytest.mark.parametrize("n,c,hw", [(8, 64, 49), (8, 257, 64), (16, 511, 16), (8, 1022, 16), (33, 24, 7), (64, 100, 196),
+                                    (1001, 92, 196), (64, 511, 512)])   # the last two: copy rings (32 MB and more)
 def test_batch_norm_channels_last_of_any_channel_count(n, c, hw, dtype):
     """Channel patterns of up to 512 vectors, tensors of one chunk and of several per CTA, forward and
     backward against fp64."""
