@@ -22,6 +22,7 @@
 //           the most recently read ones, which are the likeliest to still be in L2; y is written
 //           with streaming stores so that it does not push x out of L2.
 // DRAM traffic therefore approaches one read of x plus one write of y.
+// Channels-last tensors that this kernel does not take go through three launches over flat vectors.
 // Contiguous NCHW tensors take the single-launch cluster kernel of batch_norm_nchw.cu. Any other
 // layout takes the three-launch general path: strided statistics, finalize, strided normalise.
 #include "batch_norm.cuh"

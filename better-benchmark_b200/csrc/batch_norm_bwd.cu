@@ -16,8 +16,8 @@
 // everything above them in fp64; per-CTA partials), finalize (fixed order, coefficient table), apply
 // (from the end of the tensors to their front, so that it starts in what the sums pass left in L2).
 // No atomics: bit-reproducible.
-// Channels-last tensors whose channel count is a multiple of the 16-byte vector (at most 256
-// vectors per row) take the vector kernels; every other layout the strided element-wise ones.
+// Channels-last tensors whose channel pattern repeats within 512 vectors of 16 bytes take the vector
+// kernels, contiguous NCHW tensors the cluster kernel; every other layout the strided element-wise ones.
 #include "rowwise.cuh"
 
 #include <cooperative_groups.h>
