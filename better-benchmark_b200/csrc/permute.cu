@@ -454,27 +454,8 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const
             for (int i = 0; i < VIN; ++i) f[i] = f[i] * scale;
           }
           if constexpr (ACT == 8 && sizeof(Tout) == 2) {
-            // SiLU for a 16-bit result: x / (exp(-x) + 1) with the compensated pair exponential (the
-            // accuracy class of expf) and a hardware reciprocal refined by one Newton step (correctly
-            // rounded but for rare last-bit cases): 1.5 fp32 ulp, three orders of magnitude below half
-            // an ulp of the output. The denominator is formed as (e + 1) / 4, which rounds like e + 1
-            // and keeps its reciprocal a normal number up to exp(88). The argument is clamped to the range in
-            // which the result does not depend on it any more (the exponential needs finite inputs).
-            // The SFU pipe (two exponentials and two reciprocals a pair) is what bounds it. Measured on
-            // bf16 [32768, 1536]: 63.5 us with the correctly rounded software reciprocal, 47.1 us with this one.
 #pragma unroll
-            for (int i = 0; i < VIN / 2; ++i) {
-              const float a = f[2 * i], b = f[2 * i + 1];
-              const f32x2 e = exp_pair_compensated(pack2(fminf(fmaxf(-a, -87.f), 88.f), fminf(fmaxf(-b, -87.f), 88.f)));
-              const f32x2 d = fma2(e, splat2(0.25f), splat2(0.25f));
-              float da, db, ra, rb;
-              unpack2(d, da, db);
-              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ra) : "f"(da));
-              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rb) : "f"(db));
-              f32x2 r = pack2(ra, rb);
-              r = fma2(r, fma2(fma2(e, splat2(-0.25f), splat2(-0.25f)), r, splat2(1.0f)), r);
-              unpack2(mul2(mul2(pack2(a, b), splat2(0.25f)), r), f[2 * i], f[2 * i + 1]);
-            }
+            for (int i = 0; i < VIN / 2; ++i) unpack2(silu_pair(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
           } else if constexpr (ACT == 4 && sizeof(Tout) == 2) {
 #pragma unroll
             for (int i = 0; i < VIN / 2; ++i) unpack2(gelu_pair(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);

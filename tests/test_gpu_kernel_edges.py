@@ -136,14 +136,23 @@ def test_transpose_of_ragged_16_bit_matrices(batch, rows, cols):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_silu_over_the_whole_range(dtype):
-    """Every 16-bit pattern above -10000 against fp64 (below, the clamped exponential leaves x * 6e-39), +inf and NaN."""
+    """Every 16-bit pattern against fp64: finite values down to the type's lowest (where the result is -0), infinities and NaN."""
     x = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).cuda().view(dtype)
     got = _kernels().cast_scale(x, dtype, activation="silu")
     want = (x.double() * torch.sigmoid(x.double()))
-    finite = torch.isfinite(x) & (x > -1e4)
+    finite = torch.isfinite(x)
     _near(got[finite], want[finite], f"silu {dtype}", floor=1.2e-7 if dtype == torch.float16 else 1e-34)
-    assert torch.isnan(got[torch.isnan(x)]).all()
+    assert torch.isnan(got[torch.isnan(x) | (x == float("-inf"))]).all()
     assert torch.equal(got[x == float("inf")], x[x == float("inf")])
+
+
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float16])
+def test_silu_where_the_exponential_overflows(out):
+    """fp32 inputs around -88.72, where exp(-x) leaves fp32, and far below: -0 as x / inf gives it, never x times a residue."""
+    x = torch.cat([torch.linspace(-90.0, -87.0, 4096), -torch.logspace(2, 38, 4096)]).cuda()
+    got = _kernels().cast_scale(x, out, activation="silu")
+    _near(got, x.double() * torch.sigmoid(x.double()), f"silu f32 -> {out}", floor=6e-8 if out == torch.float16 else 3e-37)
+    assert (got[x < -89] == 0).all()
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
