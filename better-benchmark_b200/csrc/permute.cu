@@ -37,19 +37,28 @@ struct PermuteParams {
 // (repros/canonical/pointwise_795cdbe23b17/repro.py:26-29).
 // One activation per launch; ACT is its bit (0: none), so that each instantiation carries only the
 // code it uses.
-template <int ACT>
-__device__ __forceinline__ float apply_activation(float f) {
-  if constexpr (ACT == 2) f = f < 0.f ? 0.f : f;
-  if constexpr (ACT == 4) f = (f * 0.5f) * (erff(f * 0.7071067811865476f) + 1.0f);
-  if constexpr (ACT == 8) f = f / (expf(-f) + 1.0f);
-  return f;
+// For 16-bit results GELU and SiLU are evaluated by the pair forms of rowwise.cuh, in the vector loop and for
+// single elements alike: a result does not depend on an element's position or on the tensor's alignment.
+template <typename Tout, int ACT>
+__device__ __forceinline__ f32x2 apply_activation2(f32x2 v) {
+  if constexpr (ACT == 4 && sizeof(Tout) == 2) return gelu_pair(v);
+  if constexpr (ACT == 8 && sizeof(Tout) == 2) return silu_pair(v);
+  float a, b;
+  unpack2(v, a, b);
+  auto one = [](float f) {
+    if constexpr (ACT == 2) f = f < 0.f ? 0.f : f;
+    if constexpr (ACT == 4) f = (f * 0.5f) * (erff(f * 0.7071067811865476f) + 1.0f);
+    if constexpr (ACT == 8) f = f / (expf(-f) + 1.0f);
+    return f;
+  };
+  return pack2(one(a), one(b));
 }
 
 template <typename Tin, typename Tout, int ACT = 0>
 __device__ __forceinline__ Tout convert_scaled(Tin v, float scale, int has_scale) {
-  float f = Elem<Tin>::to_f32(v);
+  float f = Elem<Tin>::to_f32(v), unused;
   if (has_scale & 1) f = f * scale;
-  f = apply_activation<ACT>(f);
+  unpack2(apply_activation2<Tout, ACT>(splat2(f)), f, unused);
   return Elem<Tout>::from_f32(f);
 }
 
@@ -453,15 +462,10 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const
 #pragma unroll
             for (int i = 0; i < VIN; ++i) f[i] = f[i] * scale;
           }
-          if constexpr (ACT == 8 && sizeof(Tout) == 2) {
+          if constexpr (ACT != 0) {
 #pragma unroll
-            for (int i = 0; i < VIN / 2; ++i) unpack2(silu_pair(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
-          } else if constexpr (ACT == 4 && sizeof(Tout) == 2) {
-#pragma unroll
-            for (int i = 0; i < VIN / 2; ++i) unpack2(gelu_pair(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
-          } else if constexpr (ACT != 0) {
-#pragma unroll
-            for (int i = 0; i < VIN; ++i) f[i] = apply_activation<ACT>(f[i]);
+            for (int i = 0; i < VIN / 2; ++i)
+              unpack2(apply_activation2<Tout, ACT>(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
           }
           store_converted<Tout, VIN>(dst + u * VIN, f);
         }

@@ -197,3 +197,19 @@ def test_gelu_over_the_whole_range(dtype):
     _near(got[finite], want[finite], f"gelu {dtype}", floor=6e-8 if dtype == torch.float16 else 1e-35)
     assert torch.isnan(got[torch.isnan(x) | (x == float("-inf"))]).all()
     assert torch.equal(got[x == float("inf")], x[x == float("inf")])
+
+
+@pytest.mark.parametrize("activation", ["silu", "gelu_erf"])
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16),
+                                       (torch.float32, torch.bfloat16), (torch.float32, torch.float16)])
+def test_activations_do_not_depend_on_position_or_alignment(dtype, out, activation):
+    """Vectors, a tail behind the last whole vector, and a view off the 16-byte grid give the same bits."""
+    bits = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).cuda()
+    x = bits.view(dtype) if dtype != torch.float32 else bits.view(torch.bfloat16).float()
+    run = lambda t: _kernels().cast_scale(t, out, activation=activation).view(torch.int16)  # noqa: E731
+    want = run(x)
+    shifted = torch.cat([x[:1], x])[1:]
+    assert torch.equal(run(shifted), want)
+    for start in (0, 32768 - 11, 65536 - 1024):   # every length modulo a vector
+        for n in range(1, 20):
+            assert torch.equal(run(x[start:].clone()[:n]), want[start:start + n]), (start, n)
