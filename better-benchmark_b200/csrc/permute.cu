@@ -462,7 +462,21 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const
 #pragma unroll
             for (int i = 0; i < VIN; ++i) f[i] = f[i] * scale;
           }
-          if constexpr (ACT != 0) {
+          // SiLU: a vector without an element beyond 88 takes the form without clamps (bf16 [32768, 1536],
+          // graph replay: 42.8 us with the clamps on every element, 40.8 us so)
+          bool plain = false;
+          if constexpr (ACT == 8 && sizeof(Tout) == 2) {
+            float largest = fabsf(f[0]);
+#pragma unroll
+            for (int i = 1; i < VIN; ++i) largest = fmaxf(largest, fabsf(f[i]));
+            plain = largest <= 88.f;
+            if (plain) {
+#pragma unroll
+              for (int i = 0; i < VIN / 2; ++i)
+                unpack2(silu_pair<false>(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
+            }
+          }
+          if (ACT != 0 && !plain) {
 #pragma unroll
             for (int i = 0; i < VIN / 2; ++i)
               unpack2(apply_activation2<Tout, ACT>(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
