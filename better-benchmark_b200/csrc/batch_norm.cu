@@ -1610,9 +1610,23 @@ using namespace b200;
 // operation). Synchronises the device.
 extern "C" int64_t b200_batch_norm_wait_timeouts(void) { return (int64_t)read_wait_timeouts(); }
 
-extern "C" int64_t b200_batch_norm_scratch_bytes(int64_t channels) {
+static int64_t batch_norm_scratch_for(int64_t rows, int64_t channels) {  // so many partial rows, and the statistics
+  return 256 + (rows * 2 * channels + 2 * channels) * (int64_t)sizeof(float);
+}
+
+// What every path makes do with: a partial row per SM (or per split of the general path).
+static int64_t batch_norm_least_scratch_bytes(int64_t channels) {
   const int sms = device_info().sm_count;
-  return 256 + ((int64_t)(sms > 64 ? sms : 64) * 2 * channels + 2 * channels) * (int64_t)sizeof(float);
+  return batch_norm_scratch_for(sms > 64 ? sms : 64, channels);
+}
+
+// What lets every path run its largest grid: the flat channels-last kernels take eight partial rows per SM
+// (the copy rings two); their patterns of at most 512 vectors end at 4096 channels. With less scratch they
+// run on fewer CTAs, which changes the order of the sums.
+extern "C" int64_t b200_batch_norm_scratch_bytes(int64_t channels) {
+  const int64_t rows = channels <= 4096 ? 8LL * device_info().sm_count : 0, least = batch_norm_least_scratch_bytes(channels);
+  const int64_t largest = batch_norm_scratch_for(rows, channels);
+  return largest > least ? largest : least;
 }
 
 // b200_batch_norm_fwd with the factor that turns the biased batch variance into the value blended
@@ -1721,7 +1735,7 @@ extern "C" int b200_batch_norm_fwd(const void* x, void* y, const void* weight, c
 // callers must order them.
 // ----------------------------------------------------------------------------------------------
 #define B200_BN_STATIC_MAX_CHANNELS 1024
-#define B200_BN_STATIC_MAX_GROUPS 160  // partial rows: one per CTA (<= SM count) or per split (<= 64)
+#define B200_BN_STATIC_MAX_GROUPS 160  // partial rows at 1024 channels: one per CTA (<= SM count) or per split (<= 64)
 
 namespace b200 {
 
@@ -1767,11 +1781,11 @@ extern "C" int b200_batch_norm_fwd_static_scratch(const void* x, void* y, const 
                 "b200_batch_norm_fwd_static_scratch: %lld channels exceed the built-in scratch (max %d); "
                 "use b200_batch_norm_fwd with a caller-provided scratch buffer",
                 (long long)channels, B200_BN_STATIC_MAX_CHANNELS);
-  if (channels > 0 && b200_batch_norm_scratch_bytes(channels) > (int64_t)kBnStaticScratchBytes)
+  if (channels > 0 && batch_norm_least_scratch_bytes(channels) > (int64_t)kBnStaticScratchBytes)
     return fail(B200_ERR_UNSUPPORTED,
                 "b200_batch_norm_fwd_static_scratch: this device needs %lld scratch bytes for %lld channels, "
                 "the built-in array holds %zu",
-                (long long)b200_batch_norm_scratch_bytes(channels), (long long)channels, kBnStaticScratchBytes);
+                (long long)batch_norm_least_scratch_bytes(channels), (long long)channels, kBnStaticScratchBytes);
   void* scratch = nullptr;
   int rc = bn_static_scratch_address(&scratch);
   if (rc != B200_OK) return rc;

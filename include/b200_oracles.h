@@ -150,7 +150,8 @@ int32_t b200_norm_bwd(const void* x, const void* dy, const void* weight, const f
 /* Same counter for b200_batch_norm_fwd's fused kernel. */
 int64_t b200_batch_norm_wait_timeouts(void);
 
-/* Scratch bytes b200_batch_norm_fwd needs for `channels` channels. */
+/* Scratch bytes that let b200_batch_norm_fwd run its largest grid for `channels` channels. With less (down
+ * to a partial row per SM) channels-last tensors run on fewer CTAs, whose sums are added in another order. */
 int64_t b200_batch_norm_scratch_bytes(int64_t channels);
 
 /* BatchNorm2d training forward (+ ReLU when relu != 0): x and y are [batch, channels, spatial]
@@ -292,6 +293,7 @@ int32_t b200_batch_norm_bwd_ex(const void* dy, const void* x, const void* act, c
  * (about 1.3 MB) until the process exits. The first call on each device looks up the array's
  * device address and should be made before any stream capture. All calls on a device share the
  * array: calls that overlap on the GPU race and must be ordered by the caller. Allocates nothing.
+ * Above 512 channels the array is smaller than b200_batch_norm_scratch_bytes: see there.
  * The caller has no scratch pointer to hand to b200_check_status here (and the barrier words are
  * cleared at every call): a bounded device-side wait that ran out shows in
  * b200_batch_norm_wait_timeouts(), which stays at 0 in normal operation.

@@ -213,3 +213,20 @@ def test_activations_do_not_depend_on_position_or_alignment(dtype, out, activati
     for start in (0, 32768 - 11, 65536 - 1024):   # every length modulo a vector
         for n in range(1, 20):
             assert torch.equal(run(x[start:].clone()[:n]), want[start:start + n]), (start, n)
+
+
+@pytest.mark.parametrize("dtype,n,c,hw", [(torch.bfloat16, 1001, 92, 196), (torch.bfloat16, 336, 92, 196),
+                                          (torch.float32, 80, 485, 256), (torch.bfloat16, 64, 1022, 49)])
+def test_batch_norm_takes_the_same_path_with_the_advertised_scratch(dtype, n, c, hw):
+    """A scratch buffer of exactly the advertised size gives the bits that the larger default buffer gives."""
+    from better_benchmark_b200 import native
+    k = _kernels()
+    x = _randn((n, c, hw, 1), dtype, c).contiguous(memory_format=torch.channels_last)
+    w, b = _randn((c,), torch.float32, 1), _randn((c,), torch.float32, 2)
+    scratch = torch.zeros(int(native.load().b200_batch_norm_scratch_bytes(c)), dtype=torch.uint8, device="cuda")
+    want = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1)
+    path = native.load().b200_last_kernel()
+    got = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1, scratch=scratch)
+    assert native.load().b200_last_kernel() == path
+    for g, v in zip(got, want):
+        assert torch.equal(g, v)
