@@ -33,6 +33,45 @@ const DeviceInfo& device_info() {
   return info[dev];
 }
 
+cudaError_t set_function_attribute_once(const void* kernel, cudaFuncAttribute attr, int value) {
+  struct Entry { const void* kernel; int attr, device; };
+  static Entry done[512];
+  static int used = 0;
+  static std::mutex mu;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  for (int i = 0; i < used; ++i)
+    if (done[i].kernel == kernel && done[i].attr == (int)attr && done[i].device == dev) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, attr, value);
+  // a full table only means that the same value is set again
+  if (e == cudaSuccess && used < 512) done[used++] = Entry{kernel, (int)attr, dev};
+  return e;
+}
+
+cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes) {
+  struct Entry { const void* kernel; int device; size_t limit; };
+  static Entry done[256];
+  static int used = 0;
+  static std::mutex mu;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const size_t optin = (size_t)device_info().max_smem_optin;
+  std::lock_guard<std::mutex> lock(mu);
+  for (int i = 0; i < used; ++i)
+    if (done[i].kernel == kernel && done[i].device == dev) return bytes <= done[i].limit ? cudaSuccess : cudaErrorInvalidValue;
+  cudaFuncAttributes attr;
+  e = cudaFuncGetAttributes(&attr, kernel);
+  if (e != cudaSuccess) return e;
+  const size_t limit = optin > attr.sharedSizeBytes ? optin - attr.sharedSizeBytes : 0;
+  if (bytes > limit) return cudaErrorInvalidValue;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+  if (e == cudaSuccess && used < 256) done[used++] = Entry{kernel, dev, limit};
+  return e;
+}
+
 static std::atomic<long long> g_launches{0};
 static thread_local const char* t_path_tag = nullptr;
 static thread_local char t_last_kernel[160] = {0};

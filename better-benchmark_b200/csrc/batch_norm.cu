@@ -1398,15 +1398,14 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
     auto apply = batch_norm_apply_cl_ring_kernel<T, MAXT>;
     const size_t ring = (size_t)kRingBytesPerThread * MAXT;  // 96 KB, or 192 KB: two CTAs, or one, per SM
     const size_t with_shifts = ring + (size_t)MAXT * V * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(sums), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)with_shifts);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(sums), with_shifts);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(reinterpret_cast<const void*>(apply), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+      e = allow_dynamic_smem(reinterpret_cast<const void*>(apply), ring);
     // the finalize kernel uses next to no shared memory: asked to keep the split of its neighbours, it does
     // not make every SM drain and re-partition twice a call
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(reinterpret_cast<const void*>(batch_norm_finalize_ring_kernel<T>),
-                               cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      e = set_function_attribute_once(reinterpret_cast<const void*>(batch_norm_finalize_ring_kernel<T>),
+                                      cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) {
       cudaGetLastError();
       *rc = fail((int)e, "b200_batch_norm_fwd: cannot reserve %zu bytes of shared memory: %s", with_shifts, cudaGetErrorString(e));
@@ -1483,7 +1482,7 @@ static bool try_launch_batch_norm_warp(BatchNormParams p, size_t scratch_bytes, 
   }
   const void* kernel = big ? reinterpret_cast<const void*>(batch_norm_cl_warp_kernel<T, 4>)
                            : reinterpret_cast<const void*>(batch_norm_cl_warp_kernel<T, 2>);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(kernel, smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -1550,8 +1549,7 @@ static int launch_batch_norm(BatchNormParams p, bool channels_last_fast, bool ch
     if (stages > 8) stages = 8;
     const size_t smem = (size_t)stages * tile_bytes + red_bytes + 8 * sizeof(uint64_t);
     p.smem_tiles = stages;
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail((int)e, "b200_batch_norm_fwd: cannot reserve %zu bytes of shared memory: %s", smem,

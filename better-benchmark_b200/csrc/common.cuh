@@ -379,6 +379,15 @@ inline cudaError_t launch_dependent(void (*kernel)(Formal...), dim3 grid, dim3 b
   return cudaLaunchKernelEx(&cfg, kernel, Formal(args)...);
 }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory. The limit is an attribute of the function, not of
+// a launch: set to each launch's own size, one host thread would lower it between another's set and launch.
+// So it is set once per kernel and device, to all that the device leaves beside the kernel's static
+// shared memory. cudaErrorInvalidValue when `bytes` is more than that. Both in abi.cu.
+cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
+
+// Sets a function attribute that is the same for every launch, once per kernel and device.
+cudaError_t set_function_attribute_once(const void* kernel, cudaFuncAttribute attr, int value);
+
 // The occupancy query is a host-side calculation; cached per (kernel, block size, smem).
 inline int cached_occupancy(const void* fn, int threads, size_t smem = 0) {
   struct Entry { const void* fn; int threads; size_t smem; int blocks; };

@@ -962,8 +962,7 @@ static bool try_launch_norm_bwd_stream(NormBwdParams p, int threads, size_t scra
   if (stages > 8) stages = 8;
   const size_t smem = (size_t)stages * 2 * row_bytes + fixed;
   auto kernel = norm_bwd_stream_kernel<T, CH, LN>;
-  cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -1040,8 +1039,7 @@ static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratc
       (size_t)stages * stage_bytes < 2 * (size_t)groups_per_cta * p.n * sizeof(float)) return false;
   const size_t smem = (size_t)stages * stage_bytes + fixed;
   auto kernel = groups_per_cta > 1 ? norm_bwd_tile_kernel<T, R, LN, true> : norm_bwd_tile_kernel<T, R, LN, false>;
-  cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;

@@ -430,8 +430,7 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
   const size_t smem = ring_bytes + fixed;
   if (smem > (size_t)dev.max_smem_optin) return false;
   auto kernel = norm_bwd_warp_kernel<T, CH, LN, DYS>;
-  cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;

@@ -584,8 +584,7 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
   const bool exact = nv == (long long)g * ch;
 
   auto launch = [&](auto kernel) {
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) {
       cudaGetLastError();
       *rc = fail((int)e, "b200_norm_fwd: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
@@ -822,8 +821,7 @@ static bool try_launch_residual_norm_warp(const NormFwdParams& p, cudaStream_t s
   if (grid > useful) grid = useful;
   const bool exact = nv == 32LL * ch;
   auto launch = [&](auto kernel) {
-    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) {
       cudaGetLastError();
       *rc = fail((int)e, "b200_norm_fwd: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));

@@ -540,8 +540,7 @@ static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st
   if (split > p.P / 2) split = (int)(p.P / 2);
   if (split < 1) split = 1;
   auto kernel = p.P % 2 ? transpose_pairs_kernel<true> : transpose_pairs_kernel<false>;
-  const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;

@@ -230,3 +230,36 @@ def test_batch_norm_takes_the_same_path_with_the_advertised_scratch(dtype, n, c,
     assert native.load().b200_last_kernel() == path
     for g, v in zip(got, want):
         assert torch.equal(g, v)
+
+
+def test_threads_launch_one_kernel_with_different_shared_memory_sizes():
+    """Host threads, each on its own stream, call one instantiation with rings of different sizes through the C ABI:
+    a limit set for one launch must not reject another's."""
+    import threading
+    from better_benchmark_b200 import kernels, native
+    lib = native.load()
+    failures = []
+
+    def work(x):
+        y = torch.empty(x.shape[0], x.shape[2], x.shape[1], dtype=x.dtype, device="cuda")
+        b, r, c = x.shape
+        with torch.cuda.stream(torch.cuda.Stream()):
+            args = (x.data_ptr(), y.data_ptr(), b, r, c, r * c, c, kernels._code(x), kernels._code(x), 1.0, 0,
+                    torch.cuda.current_stream().cuda_stream)
+            for _ in range(20000):
+                if lib.b200_transpose_copy(*args) != 0:
+                    failures.append(native.last_error())
+                    return
+            torch.cuda.current_stream().synchronize()
+        if not torch.equal(y, x.transpose(1, 2)):
+            failures.append("wrong values")
+
+    # odd row counts: one instantiation, rings of 49 KB and 94 KB
+    inputs = [_randn(shape, torch.bfloat16, shape[1]) for shape in [(8, 49, 128), (4, 201, 80)] * 2]
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(x,)) for x in inputs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
