@@ -72,6 +72,27 @@ cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes) {
   return e;
 }
 
+int cached_occupancy(const void* fn, int threads, size_t smem) {
+  struct Entry { const void* fn; int threads, device; size_t smem; int blocks; };
+  static Entry cache[256];
+  static int used = 0;
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+  std::lock_guard<std::mutex> lock(mu);
+  for (int i = 0; i < used; ++i)
+    if (cache[i].fn == fn && cache[i].threads == threads && cache[i].smem == smem && cache[i].device == dev)
+      return cache[i].blocks;
+  int blocks = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, threads, smem) != cudaSuccess) {
+    cudaGetLastError();
+    blocks = 1;
+  }
+  if (blocks < 1) blocks = 1;
+  if (used < 256) cache[used++] = Entry{fn, threads, dev, smem, blocks};
+  return blocks;
+}
+
 static std::atomic<long long> g_launches{0};
 static thread_local const char* t_path_tag = nullptr;
 static thread_local char t_last_kernel[160] = {0};

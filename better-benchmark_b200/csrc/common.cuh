@@ -388,21 +388,7 @@ cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
 // Sets a function attribute that is the same for every launch, once per kernel and device.
 cudaError_t set_function_attribute_once(const void* kernel, cudaFuncAttribute attr, int value);
 
-// The occupancy query is a host-side calculation; cached per (kernel, block size, smem).
-inline int cached_occupancy(const void* fn, int threads, size_t smem = 0) {
-  struct Entry { const void* fn; int threads; size_t smem; int blocks; };
-  static Entry cache[256];
-  static int used = 0;
-  for (int i = 0; i < used; ++i)
-    if (cache[i].fn == fn && cache[i].threads == threads && cache[i].smem == smem) return cache[i].blocks;
-  int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, threads, smem) != cudaSuccess) {
-    cudaGetLastError();
-    blocks = 1;
-  }
-  if (blocks < 1) blocks = 1;
-  if (used < 256) cache[used++] = Entry{fn, threads, smem, blocks};
-  return blocks;
-}
+// Resident CTAs per SM (at least 1): a host-side calculation, cached per (kernel, block size, smem, device). In abi.cu.
+int cached_occupancy(const void* fn, int threads, size_t smem = 0);
 
 }  // namespace b200

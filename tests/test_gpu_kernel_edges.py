@@ -263,3 +263,34 @@ def test_threads_launch_one_kernel_with_different_shared_memory_sizes():
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+def test_threads_ask_for_occupancies_at_the_same_time():
+    """First calls of many kernel / block-size pairs from several host threads (each with its own stream and
+    scratch) give the bits that the same calls give afterwards, one by one."""
+    import threading
+    k = _kernels()
+    sizes = [list(range(600 + 40 * t, 3400, 173)) for t in range(4)]
+    data = {n: (_randn((7, n), torch.float16, n), _randn((7, n), torch.float16, n + 1), _randn((n,), torch.float32, n))
+            for group in sizes for n in group}
+    rstd = torch.ones(7, device="cuda")
+    torch.cuda.synchronize()
+    results, start = {}, threading.Barrier(len(sizes))
+
+    def work(group):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            scratch = torch.zeros(64 << 20, dtype=torch.uint8, device="cuda")
+            start.wait()
+            for n in group:
+                x, dy, w = data[n]
+                results[n] = k.norm_bwd(x, dy, w, rstd, rms=True, scratch=scratch)[:2]
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(group,)) for group in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for n, (x, dy, w) in data.items():
+        for got, want in zip(results[n], k.norm_bwd(x, dy, w, rstd, rms=True)[:2]):
+            assert torch.equal(got, want), n
