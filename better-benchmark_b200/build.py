@@ -53,10 +53,9 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
 
     def compile_one(job):
         src, obj = job
-        cmd = [nvcc, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
+        cmd = [nvcc, *NVCC_FLAGS, "-Xptxas=-v", "-c", str(src), "-o", str(obj)]
         res = subprocess.run(cmd, capture_output=True, text=True)
+        obj.with_suffix(".ptxas").write_text(res.stderr)   # registers and spills of every kernel
         return src, res
 
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as pool:

@@ -79,10 +79,14 @@ __device__ __forceinline__ float gelu_erf_rounded(float x) {
 // rsqrtf is the 2-ulp hardware approximation aten's CUDA rsqrt uses as well.
 __device__ __forceinline__ float precise_rsqrt(float v) { return rsqrtf(v); }
 
-template <typename Tin, typename Tout, int CH, int G, bool RES = false>
+template <typename Tin, typename Tout, int CH, int G, bool GELU, bool RES>
 // Residual instantiations with sub-warp rows: three CTAs of 256 threads per SM (80 registers, a few
 // spilled words) measured faster than two at 119 registers: 57.1 -> 45.8 us on [65536, 768] bf16
 // under the reference's cold-L2 protocol.
+// The GELU prologue is a template parameter: as a branch at run time its registers were the plain kernels'
+// too (bf16, CTA per row of up to 1024 vectors 120, now 64; sub-warp rows of up to 128 vectors 138, now 54).
+// RMSNorm bf16 [16384, 4096] 66.7 -> 44.2 us, [2048, 768] 5.0 -> 3.6; LayerNorm 83.5 -> 52.5 and 6.2 -> 4.5;
+// GELU -> LayerNorm 112.5 -> 96.8 and 7.6 -> 5.6.
 __global__ void __launch_bounds__(G == 0 ? 512 : 256, (RES && G != 0) ? 3 : 1)
 norm_fwd_resident_kernel(const NormFwdParams p) {
   constexpr int V = Elem<Tin>::V;
@@ -139,7 +143,7 @@ norm_fwd_resident_kernel(const NormFwdParams p) {
 #pragma unroll
     for (int i = 0; i < V / 2; ++i) v[c][i] = pack2(f[2 * i], f[2 * i + 1]);
   }
-  if (p.prologue == 1) {  // gelu(0) = 0: the padding slots stay zero
+  if constexpr (GELU) {  // gelu(0) = 0: the padding slots stay zero
 #pragma unroll
     for (int c = 0; c < CH; ++c)
 #pragma unroll
@@ -302,7 +306,7 @@ norm_fwd_resident_kernel(const NormFwdParams p) {
 // per tile: it makes the bounded-wait outcome CTA-uniform and, at the same time, proves that the
 // previous tile's stage is free to be refilled.
 // ----------------------------------------------------------------------------------------------
-template <typename Tin, typename Tout, int CH, int G, bool EXACT>
+template <typename Tin, typename Tout, int CH, int G, bool EXACT, bool GELU>
 __global__ void __launch_bounds__(256, 4)
 norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contiguous) {
   constexpr int V = Elem<Tin>::V;
@@ -425,7 +429,7 @@ norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contig
         for (int i = 0; i < V / 2; ++i) v[c][i] = splat2(0.f);
       }
     }
-    if (p.prologue == 1) {  // gelu(0) = 0: the padding slots stay zero
+    if constexpr (GELU) {  // gelu(0) = 0: the padding slots stay zero
 #pragma unroll
       for (int c = 0; c < CH; ++c)
 #pragma unroll
@@ -593,7 +597,17 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
     kernel<<<(unsigned)grid, threads, smem, st>>>(p, stages, contiguous);
     *rc = launch_status("b200_norm_fwd [streaming ring, sub-warp rows]");
   };
-#define B200_NFS(GG, CC)                                                            if (g == GG && ch == CC) {                                                          if (exact) launch(norm_fwd_stream_kernel<Tin, Tout, CC, GG, true>);               else launch(norm_fwd_stream_kernel<Tin, Tout, CC, GG, false>);                    return true;                                                                    }
+#define B200_NFS(GG, CC)                                                                  \
+  if (g == GG && ch == CC) {                                                              \
+    if (p.prologue) {                                                                     \
+      if (exact) launch(norm_fwd_stream_kernel<Tin, Tout, CC, GG, true, true>);           \
+      else launch(norm_fwd_stream_kernel<Tin, Tout, CC, GG, false, true>);                \
+    } else {                                                                              \
+      if (exact) launch(norm_fwd_stream_kernel<Tin, Tout, CC, GG, true, false>);          \
+      else launch(norm_fwd_stream_kernel<Tin, Tout, CC, GG, false, false>);               \
+    }                                                                                     \
+    return true;                                                                          \
+  }
   B200_NFS(8, 1) B200_NFS(8, 2) B200_NFS(8, 3) B200_NFS(8, 4) B200_NFS(16, 3) B200_NFS(16, 4) B200_NFS(32, 3) B200_NFS(32, 4)
   if constexpr (V == 4) {
     B200_NFS(32, 6) B200_NFS(32, 8)
@@ -1045,15 +1059,17 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
   if (vector_ok && p.n % V == 0 && pick_row_geometry(p.n / V, &g)) {
     set_path_tag(g.block ? (p.res ? "residual add, vector, row resident, CTA per row" : "vector, row resident, CTA per row")
                          : (p.res ? "residual add, vector, row resident, sub-warp rows" : "vector, row resident, sub-warp rows"));
-#define B200_NF_LAUNCH(GG, CC)                                                                       \
-  do {                                                                                               \
-    if constexpr (kResBuilt) {                                                                       \
-      if (p.res) {                                                                                   \
-        norm_fwd_resident_kernel<Tin, Tout, CC, GG, true><<<grid, g.threads, 0, st>>>(p);            \
-        break;                                                                                       \
-      }                                                                                              \
-    }                                                                                                \
-    norm_fwd_resident_kernel<Tin, Tout, CC, GG><<<grid, g.threads, 0, st>>>(p);                      \
+#define B200_NF_LAUNCH(GG, CC)                                                                              \
+  do {                                                                                                      \
+    if constexpr (kResBuilt) {                                                                              \
+      if (p.res) {                                                                                          \
+        if (p.prologue) norm_fwd_resident_kernel<Tin, Tout, CC, GG, true, true><<<grid, g.threads, 0, st>>>(p); \
+        else norm_fwd_resident_kernel<Tin, Tout, CC, GG, false, true><<<grid, g.threads, 0, st>>>(p);       \
+        break;                                                                                              \
+      }                                                                                                     \
+    }                                                                                                       \
+    if (p.prologue) norm_fwd_resident_kernel<Tin, Tout, CC, GG, true, false><<<grid, g.threads, 0, st>>>(p); \
+    else norm_fwd_resident_kernel<Tin, Tout, CC, GG, false, false><<<grid, g.threads, 0, st>>>(p);          \
   } while (0)
     if (!g.block) {
       if (p.res) {  // CTAs of 128 threads for the residual kernels (measured: 45.8 -> 44.3 us on the case above)
