@@ -78,11 +78,11 @@ __device__ __forceinline__ void bn_bwd_prologue(f32x2 (&g)[Elem<T>::V / 2], cons
 // of PV, so a thread keeps its phase - its V channels - for the whole launch.
 // All CTAs of the grid are resident and take chunks b, b + grid, ...: the launch moves through the
 // tensors from front to back as a whole, so what it leaves in L2 is their last part, which is where
-// the apply kernel begins. What bounds it: 4.8 TB/s of reads, the loads of a round being waited for
-// before the next are issued (more, smaller CTAs per SM were slower: 4 of 64 registers 119 us, 3 of 80
-// registers 107 us for the whole call). Measured on bf16 [256, 64, 56, 56] (sums, finalize, apply):
-// 105.5 us with 8 CTAs per SM on contiguous ranges, 102.5 us so; bf16 [64, 256, 14, 14] with the
-// activation 31.9 -> 27.4 us; f32 [121, 485, 16, 16], element-wise before, 345 -> 64 us.
+// the apply kernel begins. What bounds it: the reads, the loads of a round being waited for before the next
+// are issued. Measured (sums, finalize, apply) against 8 CTAs per SM on contiguous ranges: bf16
+// [256, 64, 56, 56] 106 -> 91 us, [328, 92, 14, 14] 21.5 -> 17.6, [992, 1024, 7, 7] 112 -> 90;
+// f32 [200, 485, 8, 8], element-wise before, 145 -> 28. The same kernels with 8 CTAs per SM in turn: 93.6 us
+// where these take 85.9 (bf16 [992, 64, 28, 28]).
 constexpr int kChunk = 4;  // vectors of each tensor in flight per thread
 
 // MAXT: 256 threads, or 512 for patterns of more than 256 vectors (one CTA per SM of as many threads).
@@ -249,14 +249,17 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_apply_cl_kernel(const
   };
   fetch();
   wait_for_previous_kernel();
+  // through L1: a thread reads 4 V values, and the 256 threads of a CTA read the same few lines (past L1
+  // this alone made the call on bf16 [328, 92, 14, 14] 40.5 us instead of 17.6). Nothing of the table can be in L1
+  // from before: the sums kernel started after it was last read, and the finalize kernel only writes it.
   f32x2 c1[V / 2], c2[V / 2], gs[V / 2], mean2[V / 2];
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) {
     const int c = (ph * V + 2 * i) % C, d = (ph * V + 2 * i + 1) % C;
-    c1[i] = pack2(__ldcg(p.coef + c), __ldcg(p.coef + d));
-    c2[i] = pack2(__ldcg(p.coef + C + c), __ldcg(p.coef + C + d));
-    gs[i] = pack2(__ldcg(p.coef + 2 * C + c), __ldcg(p.coef + 2 * C + d));
-    mean2[i] = pack2(__ldcg(p.coef + 3 * C + c), __ldcg(p.coef + 3 * C + d));
+    c1[i] = pack2(p.coef[c], p.coef[d]);
+    c2[i] = pack2(p.coef[C + c], p.coef[C + d]);
+    gs[i] = pack2(p.coef[2 * C + c], p.coef[2 * C + d]);
+    mean2[i] = pack2(p.coef[3 * C + c], p.coef[3 * C + d]);
   }
   for (; v >= 0; v -= step) {
 #pragma unroll
@@ -742,9 +745,11 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
     const int threads = vpr <= 256 ? 256 / vpr * vpr : vpr;  // a multiple of PV: a thread keeps its phase
     const long long total = p.rows * p.channels / V;
     long long splits = (threads <= 256 ? 2LL : 1LL) * dev.sm_count;  // all CTAs resident
-    // at least two rounds of loads (8 vectors of each tensor) per thread: small tensors get few
-    // partial rows and a short finalize
-    if (splits * threads * 8 > total) splits = (total + threads * 8 - 1) / (threads * 8);
+    // Small tensors: a chunk per CTA while that makes fewer (with two: bf16 [16, 256, 14, 14] 12.1 us, f32
+    // [24, 64, 28, 28] 11.4; so 8.5 and 9.5), and two for each where two are needed (343 chunks on 296 CTAs:
+    // bf16 [56, 256, 14, 14] 15.1 us, on 172: 14.2). From there on every resident CTA is wanted.
+    const long long chunks = (total + threads * kChunk - 1) / (threads * kChunk);
+    if (chunks <= 2 * splits) splits = chunks <= splits ? chunks : (chunks + 1) / 2;
     if (splits < 1) splits = 1;
     const long long need = splits * 2 * p.channels * (long long)sizeof(double) + coef_floats * (long long)sizeof(float);
     if ((long long)scratch_bytes < need)
