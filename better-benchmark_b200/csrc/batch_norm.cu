@@ -1115,7 +1115,7 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
 }
 
 // ----------------------------------------------------------------------------------------------
-// The same three steps for large tensors:
+// The same three steps as they are taken for most tensors:
 //   sums      all CTAs are resident and take chunks b, b + grid, ...: the launch moves through the tensor
 //             from front to back as a whole, and what it leaves in L2 is the tensor's last part
 //   finalize  a CTA per channel
@@ -1124,13 +1124,16 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
 // copies, read only by the thread that issued them: no barrier, no registers), which keeps about 160 KB
 // per SM on the way whatever the arithmetic does. The three kernels are chained by programmatic
 // dependent launch; apply fills its ring before the statistics are there.
-// Bound by HBM: bf16 [128, 96, 56, 56] takes 20 us for the sums (77 MB, next to the write-back of the
-// previous y), 4 for the finalize, 31 for the apply (writes settle near 3.4 TB/s in every kernel here).
-// Measured against the kernels above: that tensor 80.8 -> 53.5 us, [256, 92, 28, 28] (37 MB) 53.3 -> 42.7,
-// f32 [121, 485, 16, 16] (60 MB) 76 -> 37; bf16 [64, 120, 28, 28] (12 MB) 24.8 there, 31.8 here. Power-of-two
-// vector counts from 8 MB up stay with the cooperative kernel (bf16 [256, 64, 56, 56] 59.1 us, 61.3 here).
+// Measured against the kernels above: bf16 [672, 96, 28, 28] (101 MB) 87.7 -> 51.5 us, [1010, 92, 14, 14] (36 MB)
+// 48.1 -> 24.5, [161, 96, 28, 28] (24 MB) 34.6 -> 19.5, [64, 120, 28, 28] (12 MB) 20.4 -> 14.5, [40, 480, 7, 7]
+// (2 MB) 12.7 -> 8.6, [8, 24, 7, 7] (20 KB) 11.5 -> 9.3; f32 [1402, 92, 14, 14] (101 MB) 74.8 -> 51.3,
+// [168, 92, 14, 14] (12 MB) 18.3 -> 12.5.
+// With more than 1024 channels and less than 12 MB the CTAs of the finalize are the larger part of it, and the
+// kernels above stay (bf16 [40, 2040, 7, 7] 19.9 us there, 22.0 here; 16 MB: 33.7 and 27.6; 1020 channels, 8 MB:
+// 18.8 and 17.9; f32 1000 channels, 8 MB: 15.5 and 15.8). Power-of-two vector counts from 8 MB up stay with the
+// cooperative kernel.
 // ----------------------------------------------------------------------------------------------
-constexpr long long kRingFromBytes = 32000000;  // between the two sides measured: 12 MB and 37 MB
+static bool ring_is_slower(long long channels, long long bytes) { return channels > 1024 && bytes < 12000000; }
 
 constexpr int kRingU = 4;  // vectors per thread in a stage
 constexpr int kRingS = 6;  // stages
@@ -1371,7 +1374,7 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_apply_cl_ring_ker
   copy_async_wait<0>();
 }
 
-// Returns false when the shape does not fit, or is below kRingFromBytes (the caller takes the kernels above).
+// Returns false when the shape or the scratch does not fit, or the kernels above are faster (the caller takes them).
 template <typename T>
 static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_bytes, cudaStream_t st, int* rc) {
   constexpr int V = Elem<T>::V;
@@ -1382,7 +1385,7 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   const long long PV = C / g;
   const long long elems = p.rows * C;
   if (PV > 512 || elems % (PV * V) != 0) return false;  // whole periods only
-  if (elems * (long long)sizeof(T) < kRingFromBytes) return false;
+  if (ring_is_slower(C, elems * (long long)sizeof(T))) return false;
   const long long total = elems / V;
   const int threads = (int)(PV <= 256 ? 256 / PV * PV : PV);
   const long long stats_floats = 2 * C;
@@ -1392,7 +1395,6 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   // at least 8 vectors per thread: small tensors get few partial rows and a short finalize
   if (splits * threads * 8 > total) splits = (total + threads * 8 - 1) / (threads * 8);
   if (splits > room / (2 * C)) return false;  // the kernels above make do with fewer partial rows
-  if (splits < 1) splits = 1;
   p.stats = p.partials + splits * 2 * C;
   const int rows_shift = total > 32LL * threads * splits ? 1 : 0;  // more than 32 vectors per thread
   auto run = [&](auto maxt_tag) {

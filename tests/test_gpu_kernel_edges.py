@@ -157,7 +157,8 @@ def test_silu_where_the_exponential_overflows(out):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,c,hw", [(8, 64, 49), (8, 257, 64), (16, 511, 16), (8, 1022, 16), (33, 24, 7), (64, 100, 196),
-                                    (1001, 92, 196), (64, 511, 512)])   # the last two: copy rings (32 MB and more)
+                                    (1001, 92, 196), (64, 511, 512), (1, 24, 2),   # copy rings from one chunk to many
+                                     (16, 2040, 49), (8, 2044, 49)])   # many channels in a small tensor: the flat kernels
 def test_batch_norm_channels_last_of_any_channel_count(n, c, hw, dtype):
     """Channel patterns of up to 512 vectors, tensors of one chunk and of several per CTA, forward and
     backward against fp64."""
@@ -327,3 +328,13 @@ def test_batch_norm_bwd_costs_the_same_for_an_odd_channel_count():
     coefficients have to come from L1; fetched past it they cost 40.5 and 27.4 us."""
     odd, even = _bn_bwd_us(328, 92, 196), _bn_bwd_us(118, 64, 784)
     assert odd < 1.25 * even, (odd, even)
+
+
+@pytest.mark.parametrize("n,c,hw,rings", [(1, 24, 2, True), (64, 120, 784, True), (8, 1024, 49, True), (8, 2040, 49, False),
+                                          (80, 2040, 49, True)])
+def test_batch_norm_channels_last_takes_the_faster_kernels(n, c, hw, rings):
+    """Copy rings for every size, except for more than 1024 channels in less than 12 MB."""
+    k = _kernels()
+    x = _randn((n, c, hw, 1), torch.bfloat16, c).contiguous(memory_format=torch.channels_last)
+    k.batch_norm_fwd(x, None, None, None, None, eps=1e-5, momentum=0.1)
+    assert (b"copy rings" in k.load().b200_last_kernel()) == rings, k.load().b200_last_kernel()
