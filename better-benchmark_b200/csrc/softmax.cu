@@ -699,20 +699,39 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   }
 }
 
-// Returns false when the row does not fit (more than 8 CTAs of 4096 vectors: 64 registers a thread
-// hold 8 vectors and what is computed from them, and a cluster has at most 8 CTAs everywhere).
+// How many CTAs share a row of nvec whole vectors; 0: the two-sweep kernel below takes it. `aligned`: every row
+// starts and ends on the 16-byte grid, on both sides.
+//   * As few as hold the row: 64 registers a thread keep 8 vectors and what is computed from them, 512 threads 4096
+//     vectors, and a cluster has at most 8 CTAs everywhere. From 8192 vectors on all 8, whose 256 threads fit an
+//     SM four times (bf16 [1024, 131075]: 4 CTAs 193 us, 8 CTAs 182, two sweeps 317).
+//   * No more than half as many rows as SMs: 8 CTAs once a row has 1024 vectors (bf16 [8, 131072] 7.4 us, two
+//     sweeps 17.6; [64, 65536] 9.4 and 12.3; [16, 20005] 4.8, one CTA 5.7; f32 [16, 4099] 4.4 and 5.6).
+//   * Otherwise aligned rows of more than 8192 vectors are read twice: the second sweep finds the row in L2, and a
+//     CTA per row loads and stores at its own pace where a cluster waits for its slowest CTA twice a row
+//     (bf16 [1024, 131072]: two sweeps 134 us, clusters 144; [682, 196608] 132 and 188; [512, 262136] 143 and
+//     168; f32 [1024, 65536] 148 and 161). fp32 log-probabilities of 16-bit rows are the exception, their
+//     sweeps being bound by expf (bf16 -> f32 log [1024, 131072]: 246 and 180 us).
+//   * fp32 rows of more than 16 384 vectors are read twice on any alignment (f32 [682, 98307] 208 us, 231 as clusters).
 template <typename Tin, typename Tout>
-static bool try_launch_softmax_rows(const SoftmaxParams& p, cudaStream_t st, int* rc) {
-  constexpr int V = Elem<Tin>::V;
-  const long long nvec = p.n / V + 1;  // an upper bound whatever the alignment of a row
-  if (nvec > 8 * 4096) return false;
-  int S = 1;
-  while (nvec > 4096LL * S) S *= 2;
-  // few rows: as many CTAs per row as give every SM two, while each still has work for 128 threads
-  while (S < 8 && p.rows * S < 2LL * device_info().sm_count && nvec / (2 * S) >= 512) S *= 2;
-  if (p.rows * S > 0x7fffffffLL) return false;
+static int softmax_ctas_per_row(long long nvec, long long rows, bool aligned, bool log_mode) {
+  if (nvec > 8 * 4096) return 0;
+  if (2 * rows <= device_info().sm_count && nvec >= 1024) return 8;
+  if (nvec > 8192) {
+    if (aligned && !(log_mode && sizeof(Tin) == 2 && sizeof(Tout) == 4)) return 0;
+    if (sizeof(Tin) == 4 && nvec > 16384) return 0;
+    return 8;
+  }
+  return nvec > 4096 ? 2 : 1;
+}
+
+// Returns false when the two-sweep kernel is to take the rows.
+template <typename Tin, typename Tout>
+static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaStream_t st, int* rc) {
+  const long long nvec = p.n / Elem<Tin>::V;  // no row has more whole vectors, whatever its alignment
+  const int S = softmax_ctas_per_row<Tin, Tout>(nvec, p.rows, aligned, p.log_mode != 0);
+  if (S == 0 || p.rows * S > 0x7fffffffLL) return false;
   const long long per = (nvec + S - 1) / S;
-  const int ch = per > 512 ? 8 : (per > 128 ? 4 : 2);
+  const int ch = per > 512 ? 8 : (per > 128 || S > 1 ? 4 : 2);
   const int threads = (int)((per + ch - 1) / ch + 31) / 32 * 32;
   if (S == 1) {
     set_path_tag("two sweeps over a row in registers, any alignment");
@@ -978,7 +997,7 @@ static int launch_softmax(const SoftmaxParams& p, bool vector_ok, cudaStream_t s
     }
   } else if (p.mask == nullptr && !PACKED && p.n >= 256) {
     int rc = B200_OK;
-    if (try_launch_softmax_rows<Tin, Tout>(p, st, &rc)) return rc;
+    if (try_launch_softmax_rows<Tin, Tout>(p, vector_ok && p.n % V == 0, st, &rc)) return rc;
     int threads = (int)((p.n / V + 3) / 4);
     threads = (threads + 31) / 32 * 32;
     threads = threads < 128 ? 128 : (threads > 1024 ? 1024 : threads);
