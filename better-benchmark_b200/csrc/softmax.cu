@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(1024) softmax_streaming_kernel(const SoftmaxPa
 //     last elements leave one by one.
 // Bound by HBM: the exponentials cost 18 us of the SFU pipe on the case below, the traffic 75 us.
 // Measured: bf16 [4096, 20005] (rows 20 008 apart) -> fp32 log_softmax 183.7 us with the two-sweep
-// kernel below, 103.3 us (4.76 TB/s) here; bf16 [2000, 32001] softmax 192.6 -> 57.6 us.
+// kernel below, 109 us (4.5 TB/s) here; bf16 [2000, 32001] softmax 192.6 -> 57.6 us.
 // ----------------------------------------------------------------------------------------------
 // Stores a thread's V outputs, the first of which goes to `y`. `shift` (warp-uniform, below the chunk
 // length VO) counts the elements from y to the next chunk boundary of the output; the lane above
@@ -602,8 +602,9 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   float M = block_reduce<MaxOp>(m, red);
 
   // ---- sum of the exponentials --------------------------------------------------------------------
-  // log_softmax takes the compensated exponential for fp32 outputs too: only the logarithm of the sum
-  // sees it, where its 3.5e-7 is below the rounding of (x - max) - log(sum).
+  // fp32 results sum expf, log_softmax too: the compensated exponential would take 102 us instead of 109 on bf16
+  // [4096, 20005] -> fp32, but its errors have a mean of -4e-8, which the sum keeps (mean error of the
+  // log-probabilities of 1003 standard normals times two +2.7e-8, against -1.3e-8).
   const bool log_mode = p.log_mode != 0;
   auto difference = [&](f32x2 t, f32x2 M2) {
     float a, b;
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
     return s;
   };
   float s;
-  if (sizeof(Tout) == 2 || log_mode) s = add_up([](f32x2 d) { return exp_pair_compensated(d); });
+  if (sizeof(Tout) == 2) s = add_up([](f32x2 d) { return exp_pair_compensated(d); });
   else s = add_up(exp_exact);
   float sum = block_reduce<SumOp>(s, red);
   if constexpr (CLUSTER) {
@@ -710,7 +711,7 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
 //     CTA per row loads and stores at its own pace where a cluster waits for its slowest CTA twice a row
 //     (bf16 [1024, 131072]: two sweeps 134 us, clusters 144; [682, 196608] 132 and 188; [512, 262136] 143 and
 //     168; f32 [1024, 65536] 148 and 161). fp32 log-probabilities of 16-bit rows are the exception, their
-//     sweeps being bound by expf (bf16 -> f32 log [1024, 131072]: 246 and 180 us).
+//     sweeps being bound by expf (bf16 -> f32 log [1024, 131072]: 250 and 187 us, [682, 196608]: 246 and 241).
 //   * fp32 rows of more than 16 384 vectors are read twice on any alignment (f32 [682, 98307] 208 us, 231 as clusters).
 template <typename Tin, typename Tout>
 static int softmax_ctas_per_row(long long nvec, long long rows, bool aligned, bool log_mode) {

@@ -338,3 +338,17 @@ def test_batch_norm_channels_last_takes_the_faster_kernels(n, c, hw, rings):
     x = _randn((n, c, hw, 1), torch.bfloat16, c).contiguous(memory_format=torch.channels_last)
     k.batch_norm_fwd(x, None, None, None, None, eps=1e-5, momentum=0.1)
     assert (b"copy rings" in k.load().b200_last_kernel()) == rings, k.load().b200_last_kernel()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_log_softmax_in_fp32_has_no_biased_sum(dtype):
+    """Mean error of fp32 log-probabilities over 100 000 rows of 1003. An exponential whose errors have a mean shifts
+    every row alike: 2.7e-8 with the pair exponential of 16-bit results, 1.3e-8 with expf (rounding of the logits'
+    difference and of the logarithm alone). Rows scatter by 2.4e-7, their mean by 0.8e-9."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    total = 0.0
+    for _ in range(10):
+        x = (torch.randn((10000, 1003), generator=g, device="cuda") * 2).to(dtype)
+        got = _kernels().softmax(x, log=True, out_dtype=torch.float32)
+        total += (got.double() - torch.log_softmax(x.double(), -1)).mean().item() / 10
+    assert abs(total) < 2.1e-8, total
