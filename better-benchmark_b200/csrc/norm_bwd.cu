@@ -199,7 +199,7 @@ norm_bwd_kernel(const NormBwdParams p) {
   }
   if (p.fused) {
     const bool ok = grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_sectors(p, LN && p.db, fin);
+    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
     grid_barrier_depart(p.bar);
   }
 }
@@ -433,7 +433,7 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
   }
   if (p.fused) {
     const bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_sectors(p, LN && p.db, fin);
+    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
     grid_barrier_depart(p.bar);
   }
 }
@@ -735,7 +735,7 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
   }
   if (p.fused) {
     const bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_sectors(p, LN && p.db, fin);
+    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
     grid_barrier_depart(p.bar);
   }
 }

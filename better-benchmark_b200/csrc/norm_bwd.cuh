@@ -80,25 +80,31 @@ __device__ __forceinline__ void finalize_columns(const float* partials, int grou
 }
 
 // The same inside a cooperative launch, after its grid barrier, for rows of n % 4 == 0 columns: the
-// columns of dw and db are dealt out in 32-byte sectors (eight columns), so that the whole grid takes
+// columns of dw and db are dealt out in units of 8 (a 32-byte sector of a partial row), so that the whole grid takes
 // part (192 CTAs for 768 columns of both) and no second level, with a second grid barrier, is needed
 // (LayerNorm backward bf16 [32768, 768], together with the copies that start before the weights are
-// staged: 45.1 us with the two levels, 39.0 us so).
-// Two threads share a sector of a partial row; the CTA's threads split the partial rows. fp64, fixed
-// order.
-__device__ __forceinline__ void finalize_sectors(const NormBwdParams& p, bool with_db, double* smem /* [warps][8] */) {
+// staged: 45.1 us with the two levels, 39.0 us so). Where that makes more units than CTAs, units of 16, 32 or 64
+// columns: a unit is two barriers and a load latency, whatever its width (LayerNorm f32 [256, 8192]: 27.9 us with
+// 2048 units of 8, 17.2 us with two times 128 of 64).
+// width / 4 threads share a partial row's unit, the CTA's threads split the partial rows. fp64, fixed order.
+// Four loads in flight per thread and no more: with the loop over the partial rows unrolled, this needed more
+// registers than the kernels around it (the streaming kernel of fp32 RMSNorm 82 -> 120, so that one CTA of 288 threads
+// fitted an SM instead of two: f32 [16352, 2052] 86 -> 112 us).
+__device__ __forceinline__ void finalize_units(const float* partials, int groups, int n, float* dw, float* db,
+                                               const int width, double* smem /* [warps][width] */) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const int n = p.n, groups = p.groups;
-  const int sectors = (n + 7) / 8, rows_at_once = blockDim.x >> 1;
-  const int total = sectors * ((p.dw ? 1 : 0) + (with_db ? 1 : 0));
+  const int share = width / 4, units = (n + width - 1) / width, rows_at_once = blockDim.x / share;
+  const int sub = tid & (share - 1);
+  const int total = units * ((dw ? 1 : 0) + (db ? 1 : 0));
   for (int s = blockIdx.x; s < total; s += gridDim.x) {
-    const bool is_db = !p.dw || s >= sectors;
-    const int col = (p.dw && s >= sectors ? s - sectors : s) * 8;
-    const int c = col + 4 * (tid & 1);
-    const float* src = p.partials + (is_db ? (long long)groups * n : 0) + c;
+    const bool is_db = !dw || s >= units;
+    const int col = (dw && s >= units ? s - units : s) * width;
+    const int c = col + 4 * sub;
+    const float* src = partials + (is_db ? (long long)groups * n : 0) + c;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < n) {
-      for (int g0 = tid >> 1; g0 < groups; g0 += 4 * rows_at_once) {
+#pragma unroll 1
+      for (int g0 = tid / share; g0 < groups; g0 += 4 * rows_at_once) {
         float4 v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -115,21 +121,39 @@ __device__ __forceinline__ void finalize_sectors(const NormBwdParams& p, bool wi
       }
     }
 #pragma unroll
-    for (int o = 16; o >= 2; o >>= 1)
+    for (int o = 16; o >= 2; o >>= 1) {
+      if (o < share) break;
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-    if (lane < 2) {
+    }
+    if (lane < share) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) smem[warp * 8 + lane * 4 + i] = acc[i];
+      for (int i = 0; i < 4; ++i) smem[warp * width + lane * 4 + i] = acc[i];
     }
     __syncthreads();
-    if (tid < 8 && col + tid < n) {
+    for (int k = tid; k < width && col + k < n; k += blockDim.x) {
       double t = 0.0;
-      for (int w = 0; w < nwarps; ++w) t += smem[w * 8 + tid];
-      (is_db ? p.db : p.dw)[col + tid] = (float)t;
+      for (int w = 0; w < nwarps; ++w) t += smem[w * width + k];
+      (is_db ? db : dw)[col + k] = (float)t;
     }
     __syncthreads();
   }
+}
+
+// A call, so that the width that a few calls need stays out of the registers and the code of the kernels.
+static __device__ __noinline__ void finalize_wide_units(const float* partials, int groups, int n, float* dw, float* db,
+                                                        double* smem) {
+  const int planes = (dw ? 1 : 0) + (db ? 1 : 0);
+  int width = 16;
+  while (width < 64 && (n + width - 1) / width * planes > (int)gridDim.x) width *= 2;
+  finalize_units(partials, groups, n, dw, db, width, smem);
+}
+
+__device__ __forceinline__ void finalize_grid(const NormBwdParams& p, float* db, double* smem /* [warps][64] */) {
+  if ((p.n + 7) / 8 * ((p.dw ? 1 : 0) + (db ? 1 : 0)) <= (int)gridDim.x)
+    finalize_units(p.partials, p.groups, p.n, p.dw, db, 8, smem);
+  else
+    finalize_wide_units(p.partials, p.groups, p.n, p.dw, db, smem);
 }
 
 // Warp reduction of N (2, 4 or 8) values per lane at once: in every step a lane keeps one half of

@@ -397,9 +397,9 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     __syncthreads();  // the fold area doubles as the fp64 area of the finalize
   }
   if (p.fused) {
-    double* fin = reinterpret_cast<double*>(smem);  // [warps][8] fp64, inside the ring
+    double* fin = reinterpret_cast<double*>(smem);  // [warps][64] fp64, inside the ring
     const bool ok = !any_failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_sectors(p, LN && p.db, fin);
+    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
     grid_barrier_depart(p.bar);
   }
 }

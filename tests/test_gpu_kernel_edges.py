@@ -98,7 +98,8 @@ def test_residual_layer_norm_forms(rows, n, dtype):
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,n", [(1, 3), (7, 129), (600, 257), (9, 511), (700, 513), (5, 4095),   # ragged rows
-                                    (600, 132), (40, 520), (5000, 264), (3, 4104)])                  # last sector half full
+                                    (600, 132), (40, 520), (5000, 264), (3, 4104),                   # last unit of columns half full
+                                    (7, 4104), (150, 8196), (3, 8200), (2, 12040)])                  # units of 16 to 64 columns
 def test_norm_bwd_edges(rows, n, dtype, rms):
     x, dy, w = _randn((rows, n), dtype, n), _randn((rows, n), dtype, n + 1), _randn((n,), torch.float32, n + 2)
     d, g = x.double(), dy.double() * w.double()
@@ -118,6 +119,8 @@ def test_norm_bwd_edges(rows, n, dtype, rms):
     _near(dw, (dy.double() * xhat).sum(0), f"dweight {rows}x{n}", floor=floor)
     if not rms:
         _near(db, dy.double().sum(0), f"dbias {rows}x{n}", floor=floor)
+        alone = _kernels().norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dweight=False, want_dbias=True)
+        assert alone[1] is None and torch.equal(alone[2], db) and torch.equal(alone[0], dx)
 
 
 @pytest.mark.parametrize("batch,rows,cols", [(1, 2, 2), (7, 49, 128), (5, 196, 64), (33, 3, 10), (2000, 5, 6), (9, 64, 66),

@@ -27,6 +27,8 @@ def _resources(stem):
 LIMITS = [
     ("norm_fwd", r"norm_fwd_resident_kernel.*Li4ELi0ELb0ELb0E", 102, "CTA per row of 128 threads: five per SM"),
     ("norm_fwd", r"norm_fwd_resident_kernel.*Li4ELi(8|16|32)ELb0ELb0E", 85, "sub-warp rows, 256 threads: three CTAs per SM"),
+    ("norm_bwd", r"norm_bwd_stream_kernelIfLi2ELb0E", 93, "fp32 RMSNorm, streaming, up to 352 threads: two CTAs per SM"),
+    ("norm_bwd", r"norm_bwd_stream_kernelIfLi2ELb1E", 100, "fp32 LayerNorm, streaming, up to 320 threads: two CTAs per SM"),
 ]
 
 
