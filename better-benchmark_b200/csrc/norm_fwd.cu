@@ -948,9 +948,16 @@ __global__ void __launch_bounds__(1024) norm_fwd_streaming_kernel(const NormFwdP
 // Bound by the number of those accesses: about 1.6 TB/s for 16-bit elements, 3.3 TB/s for fp32.
 // Measured against the sweeps: LayerNorm bf16 [20000, 769] 461.6 -> 73.8 us, RMSNorm f32 [20000, 1001]
 // 329.8 -> 49.2 us, residual LayerNorm f16 [46251, 449] 795.6 -> 106.9 us.
+// Few rows (up to eight per SM of 129..512 elements, two per SM of up to 2048) take a CTA per row with two elements a
+// thread, as the longer chains of a thread are not hidden then: LayerNorm bf16 [148, 449] by warps 4.8 us, so 3.0;
+// [600, 257] 4.4 and 3.1 ([2400, 257] 4.8 by warps); [148, 769] with eight a thread 4.9, so 3.3.
+// Weight and bias are asked for in groups before the stores: one by one they cost [148, 449] 9.9 us.
 // G: 32 = a warp per row, 0 = the CTA.
 template <typename Tin, typename Tout, int E, int G>
-__global__ void __launch_bounds__(G == 0 ? 1024 : 256) norm_fwd_ragged_kernel(const NormFwdParams p) {
+// (Two CTAs of 1024 threads per SM for 16-bit rows, 32 registers; otherwise no minimum, which is not the same as 1:
+// that allows 64 registers, and fp32 rows of 5001 run one CTA per SM instead of two, [4800, 5001] 64.6 -> 101 us.)
+__global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 && sizeof(Tin) == 2 ? 2 : 0)
+norm_fwd_ragged_kernel(const NormFwdParams p) {
   __shared__ float red[64];
   constexpr bool DUAL = std::is_same<Tin, Tout>::value && sizeof(Tin) == 2;
   const int lane = glane<G>(), gs = gsize<G>();
@@ -1020,23 +1027,29 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256) norm_fwd_ragged_kernel(co
   }
   if (p.y == nullptr || !valid) return;
   Tout* y = reinterpret_cast<Tout*>(p.y) + row * p.y_row_stride;
+  // parameters in flight per thread: a CTA per row has other warps to hide them behind, and registers to save
+  constexpr int AT_ONCE = E < 8 ? E : (G != 0 ? 8 : (E == 8 && sizeof(Tin) == 4 ? 4 : 2));
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = e * gs + lane;
-    if (i < n) {
-      const float w = p.w ? load_param1(p.w, p.w_dtype, i) : 1.f;
-      const float b = p.b ? load_param1(p.b, p.w_dtype, i) : 0.f;
-      float o = (f[e] - mean) * rstd;
-      if (p.w) o = o * w;
-      if (p.b) o = o + b;
-      if constexpr (DUAL) {
-        if (both && !(fabsf(round_through<Tout>(o)) > 3.0f)) {
-          o = (round_through<Tin>(f[e]) - mean_r) * rstd_r;
-          if (p.w) o = o * w;
-          if (p.b) o = o + b;
+  for (int e0 = 0; e0 < E; e0 += AT_ONCE) {
+    float w[AT_ONCE], b[AT_ONCE];
+    if (p.w) load_params_strided(p.w, p.w_dtype, e0 * gs + lane, gs, n, w);
+    if (p.b) load_params_strided(p.b, p.w_dtype, e0 * gs + lane, gs, n, b);
+#pragma unroll
+    for (int k = 0; k < AT_ONCE; ++k) {
+      const int e = e0 + k, i = e * gs + lane;
+      if (i < n) {
+        float o = (f[e] - mean) * rstd;
+        if (p.w) o = o * w[k];
+        if (p.b) o = o + b[k];
+        if constexpr (DUAL) {
+          if (both && !(fabsf(round_through<Tout>(o)) > 3.0f)) {
+            o = (round_through<Tin>(f[e]) - mean_r) * rstd_r;
+            if (p.w) o = o * w[k];
+            if (p.b) o = o + b[k];
+          }
         }
+        y[i] = Elem<Tout>::from_f32(o);
       }
-      y[i] = Elem<Tout>::from_f32(o);
     }
   }
 }
@@ -1096,7 +1109,9 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
 #undef B200_NF_LAUNCH
   } else if (p.n <= 16384) {
     set_path_tag(p.res ? "residual add, elements in registers" : "elements in registers");
-    if (p.n <= 512) {  // a warp per row
+    if (p.n > 128 && p.n <= 2048 && p.rows <= (p.n <= 512 ? 8LL : 2LL) * device_info().sm_count) {
+      norm_fwd_ragged_kernel<Tin, Tout, 2, 0><<<(unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st>>>(p);
+    } else if (p.n <= 512) {  // a warp per row
       const unsigned grid = (unsigned)((p.rows + 7) / 8);
       if (p.n <= 64) norm_fwd_ragged_kernel<Tin, Tout, 2, 32><<<grid, 256, 0, st>>>(p);
       else if (p.n <= 128) norm_fwd_ragged_kernel<Tin, Tout, 4, 32><<<grid, 256, 0, st>>>(p);

@@ -394,6 +394,24 @@ __device__ __forceinline__ float load_param1(const void* base, int dtype, long l
   return __half2float(__ldg(reinterpret_cast<const __half*>(base) + idx));
 }
 
+// N parameters at a distance of `step`, those at n and beyond as 0: the type is asked for once, so that all loads are
+// on their way together (with load_param1 in a loop each waits for the one before it).
+template <int N>
+__device__ __forceinline__ void load_params_strided(const void* base, int dtype, int first, int step, int n, float (&out)[N]) {
+  auto load = [&](auto tag) {
+    using P = decltype(tag);
+    const P* p = reinterpret_cast<const P*>(base);
+    P raw[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) raw[e] = first + e * step < n ? __ldg(p + first + e * step) : Elem<P>::from_f32(0.f);
+#pragma unroll
+    for (int e = 0; e < N; ++e) out[e] = Elem<P>::to_f32(raw[e]);
+  };
+  if (dtype == B200_F32) load(float{});
+  else if (dtype == B200_BF16) load(__nv_bfloat16{});
+  else load(__half{});
+}
+
 // Round an fp32 value to T and back: the rounding boundary a 16-bit intermediate tensor imposes.
 template <typename T>
 __device__ __forceinline__ float round_through(float v) {

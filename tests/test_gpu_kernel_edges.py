@@ -68,7 +68,7 @@ def _layer_norm64(d, w, b, eps, rms):
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,n", [(3, 2), (9, 33), (7, 65), (10, 129), (5, 257), (3, 511), (3, 513), (2, 8191),
-                                    (2, 8193), (2, 16383), (2, 16385)])
+                                    (2, 8193), (2, 16383), (2, 16385), (1300, 257), (1185, 511), (400, 513), (297, 2047), (3, 2049)])
 def test_norm_fwd_of_ragged_rows(rows, n, dtype, rms):
     x, w, b = _randn((rows, n), dtype, n), _randn((n,), dtype, n + 1), None if rms else _randn((n,), dtype, n + 2)
     y = _kernels().norm_fwd(x, w, b, eps=1e-5, rms=rms)[0]
@@ -355,3 +355,16 @@ def test_log_softmax_in_fp32_has_no_biased_sum(dtype):
         got = _kernels().softmax(x, log=True, out_dtype=torch.float32)
         total += (got.double() - torch.log_softmax(x.double(), -1)).mean().item() / 10
     assert abs(total) < 2.1e-8, total
+
+
+def test_a_few_ragged_rows_cost_what_aligned_ones_do():
+    """LayerNorm forward of 148 rows: 449 columns (elements) against 448 (vectors), 3.0 and 4.0 us. One warp per row whose
+    16 weights and biases are fetched one after the other took 9.9."""
+    k = _kernels()
+
+    def us(n):
+        x, w, b = _randn((148, n), torch.bfloat16, 1), _randn((n,), torch.bfloat16, 2), _randn((n,), torch.bfloat16, 3)
+        return _graph_us(lambda: k.norm_fwd(x, w, b, eps=1e-5, want_rstd=True))
+
+    ragged, aligned = us(449), us(448)
+    assert ragged < 1.5 * aligned, (ragged, aligned)
