@@ -819,8 +819,8 @@ __global__ void __launch_bounds__(128) norm_bwd_cols_general_kernel(const NormBw
 // stretch whatever the alignment, a thread's columns are the same in every row, so its weights and its
 // sums of dweight / dbias stay in registers. One partial row per CTA, added up by the finalize launch.
 // Bound by the number of 2- and 4-byte accesses, about half of HBM speed. Measured against the three
-// passes: LayerNorm bf16 [20000, 449] 125.2 -> 47.0 us, RMSNorm f32 [10000, 1001] 112.8 -> 45.1 us, LayerNorm f16
-// [3000, 3001] 67.6 -> 53.2 us (71.7 us without the row ahead).
+// passes (with the finalize below): LayerNorm bf16 [20000, 449] 121 -> 34.4 us, [300, 513] 9.8 -> 6.8, [1397, 3001] 40.5 ->
+// 24.9, RMSNorm f32 [20000, 769] 191 -> 55 us.
 template <typename T, bool LN, int E, int G>
 __global__ void __launch_bounds__(G == 0 ? 512 : 256, G == 0 ? 1 : 2) norm_bwd_ragged_kernel(const NormBwdParams p) {
   extern __shared__ float fold[];  // warp per row: [warps][n] for dw, [warps][n] for db
@@ -830,9 +830,10 @@ __global__ void __launch_bounds__(G == 0 ? 512 : 256, G == 0 ? 1 : 2) norm_bwd_r
   const long long first = G == 0 ? (long long)blockIdx.x : (long long)blockIdx.x * nwarps + warp;
   const long long stride = G == 0 ? (long long)gridDim.x : (long long)gridDim.x * nwarps;
   float w[E], acc_w[E], acc_b[LN ? E : 1];
+  if (p.w) load_params_strided(p.w, p.w_dtype, lane, gs, n, w);
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    w[e] = p.w && e * gs + lane < n ? load_param1(p.w, p.w_dtype, e * gs + lane) : 1.f;
+    if (!p.w) w[e] = 1.f;
     acc_w[e] = 0.f;
     if constexpr (LN) acc_b[e] = 0.f;
   }
@@ -1123,6 +1124,35 @@ static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_byt
   return rc;
 }
 
+// The finalize of the ragged kernel: 16 columns of dw or db per CTA, so that short rows (n / 64 CTAs above) and
+// the many partial rows of a CTA per row do not meet in a handful of CTAs (LayerNorm bf16 [1200, 513] 31.9 us with the
+// kernel above, 10.5 so; [9341, 449] 29.9 and 19.5; fewer partial rows, that is fewer CTAs, gained nothing). fp64, fixed order.
+__global__ void __launch_bounds__(512) norm_bwd_finalize_ragged_kernel(const NormBwdParams p) {
+  __shared__ double part[16][16];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c = blockIdx.x * 16 + (tid & 15);
+  const bool is_db = !p.dw || blockIdx.y == 1;
+  const float* src = p.partials + (is_db ? (long long)p.groups * p.n : 0) + c;
+  double acc = 0.0;
+  if (c < p.n) {
+    for (int g0 = tid >> 4; g0 < p.groups; g0 += 8 * 32) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = g0 + u * 32 < p.groups ? __ldcg(src + (long long)(g0 + u * 32) * p.n) : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += (double)v[u];
+    }
+  }
+  acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+  if (lane < 16) part[warp][lane] = acc;
+  __syncthreads();
+  if (tid < 16 && c < p.n) {
+    double t = 0.0;
+    for (int w = 0; w < 16; ++w) t += part[w][tid];
+    (is_db ? p.db : p.dw)[c] = (float)t;
+  }
+}
+
 // Returns false when the shape does not fit (the caller takes the element-wise kernels).
 template <typename T, bool LN>
 static bool try_launch_norm_bwd_ragged(NormBwdParams p, size_t scratch_bytes, cudaStream_t st, int* rc) {
@@ -1144,7 +1174,7 @@ static bool try_launch_norm_bwd_ragged(NormBwdParams p, size_t scratch_bytes, cu
     kernel<<<(unsigned)grid, threads, smem, st>>>(p);
     *rc = launch_status("b200_norm_bwd [ragged rows, elements in registers]");
     if (*rc == B200_OK && sums) {
-      norm_bwd_finalize_kernel<<<(p.n + 63) / 64, 512, 0, st>>>(p);
+      norm_bwd_finalize_ragged_kernel<<<dim3((p.n + 15) / 16, (p.dw ? 1 : 0) + (p.db ? 1 : 0)), 512, 0, st>>>(p);
       *rc = launch_status("b200_norm_bwd finalize");
     }
     return true;

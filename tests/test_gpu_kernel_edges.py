@@ -368,3 +368,17 @@ def test_a_few_ragged_rows_cost_what_aligned_ones_do():
 
     ragged, aligned = us(449), us(448)
     assert ragged < 1.5 * aligned, (ragged, aligned)
+
+
+def test_ragged_norm_bwd_costs_what_aligned_rows_do():
+    """LayerNorm backward of 1200 rows: 513 columns (a CTA per row, 1200 partial rows) against 512, 10 us each.
+    With the partial rows added up by 9 CTAs it took 32."""
+    k = _kernels()
+
+    def us(n):
+        x, dy, w = _randn((1200, n), torch.bfloat16, 1), _randn((1200, n), torch.bfloat16, 2), torch.ones(n, device="cuda")
+        mean, rstd = torch.zeros(1200, device="cuda"), torch.ones(1200, device="cuda")
+        return _graph_us(lambda: k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True))
+
+    ragged, aligned = us(513), us(512)
+    assert ragged < 1.5 * aligned, (ragged, aligned)
