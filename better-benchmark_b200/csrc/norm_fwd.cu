@@ -623,8 +623,8 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
 // stages keep a row in flight per warp. Weight and bias are converted to fp32 once per CTA, in a
 // [slot][pair][lane] layout that a warp reads without bank conflicts. BOTH (res_round == 2): the choice
 // between the two forms is made on the packed 16-bit results: round both, compare |full| > 3, select.
-// All forms take this kernel, so that an element of the both-forms result has the bits of the form it
-// was taken from.
+// Which rows take it does not depend on the form, so that an element of the both-forms result has the bits of the
+// form it was taken from (residual_warp_rows below).
 // What bounds it: HBM, with about 38 instructions per pair of elements (two complete normalisations and
 // the roundings between them, 57 % of the issue slots) behind it. The resident kernel converts weight
 // and bias in every row on top and overlaps its load and store phases less; it keeps the rows of up to
@@ -814,13 +814,25 @@ residual_norm_warp_kernel(const NormFwdParams p, const int stages) {
   }
 }
 
+// Measured against the resident kernel (sum kept; fp32-sum form / both forms). 16-bit rows of up to 112 vectors: ahead
+// ([40000, 768] 44.7 / 51.6 -> 44.5 / 45.6 us, [2000, 520] 5.3 / 5.8 -> 5.1 / 5.7, [16000, 864] 23.8 / 27.1 -> 21.1 /
+// 24.2), but for one form of the widest large ones ([40000, 896] 51.0 / 59.5 -> 53.0 / 52.5). 113..128 vectors: ahead up
+// to 32 MB of x ([16000, 1024] 24.9 / 27.9 -> 24.4 / 25.9), behind from there ([40000, 1024] 53.5 / 60.8 -> 59.3 / 62.7).
+// fp32 rows: ahead with no more than a row per warp of one CTA per SM ([1000, 512] 4.9 -> 4.4, [1500, 512] 5.3 -> 5.5,
+// [40000, 512] 52.3 -> 58.1).
+template <typename T>
+static bool residual_warp_rows(long long rows, long long nv) {
+  if (sizeof(T) == 4) return rows <= 8LL * device_info().sm_count;
+  return nv <= 112 || rows * nv * 16 <= (32 << 20);
+}
+
 // Returns false when the shape does not fit (the caller takes the resident kernel).
 template <typename T>
 static bool try_launch_residual_norm_warp(const NormFwdParams& p, cudaStream_t st, int* rc) {
   constexpr int V = Elem<T>::V;
   const long long nv = p.n / V;
-  if (streaming_disabled() || p.rms || p.prologue || !p.y || nv <= 64 || nv > 128 ||
-      p.rows >= 0x7fffffffLL) return false;
+  if (streaming_disabled() || p.rms || p.prologue || !p.y || nv <= 64 || nv > 128 || p.rows >= 0x7fffffffLL ||
+      !residual_warp_rows<T>(p.rows, nv)) return false;
   const DeviceInfo& dev = device_info();
   const int ch = (int)((nv + 31) / 32);
   const size_t stage_bytes = 2 * (size_t)nv * 16;

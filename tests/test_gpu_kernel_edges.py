@@ -76,7 +76,8 @@ def test_norm_fwd_of_ragged_rows(rows, n, dtype, rms):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("rows,n", [(1, 264), (9, 512), (1, 520), (13, 520), (4000, 768), (11, 776), (3, 1024), (5, 449), (3, 1023)])
+@pytest.mark.parametrize("rows,n", [(1, 264), (9, 512), (1, 520), (13, 520), (4000, 768), (11, 776), (3, 1024), (5, 449), (3, 1023),
+                                    (1184, 512), (1185, 512), (16384, 1024), (16385, 1024)])  # the last of one kernel, the first of the other
 def test_residual_layer_norm_forms(rows, n, dtype):
     """A warp per row with its own copy ring (65..128 vectors), and ragged rows: the element-wise choice
     between the two forms is bit for bit a choice between the two single forms."""
@@ -382,3 +383,13 @@ def test_ragged_norm_bwd_costs_what_aligned_rows_do():
 
     ragged, aligned = us(513), us(512)
     assert ragged < 1.5 * aligned, (ragged, aligned)
+
+
+@pytest.mark.parametrize("rows,n,dtype,warp", [(16384, 1024, torch.bfloat16, True), (16385, 1024, torch.bfloat16, False),
+                                               (40000, 896, torch.float16, True), (1184, 512, torch.float32, True),
+                                               (1185, 512, torch.float32, False)])
+def test_residual_layer_norm_takes_the_faster_kernel(rows, n, dtype, warp):
+    k = _kernels()
+    x, w = torch.zeros((rows, n), dtype=dtype, device="cuda"), torch.ones(n, dtype=dtype, device="cuda")
+    k.norm_fwd(x, w, w, eps=1e-5, residual=x)
+    assert (b"warp rings" in k.load().b200_last_kernel()) == warp, k.load().b200_last_kernel()
