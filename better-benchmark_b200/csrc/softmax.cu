@@ -341,10 +341,13 @@ __device__ __forceinline__ float softmax_logit(const SoftmaxParams& p, const Tin
 // Rows with a mask (or short ones) that the vector path cannot take: a warp per row (n <= 512) or a
 // CTA per row, E elements per thread at a distance of the group, held in registers: one read of the
 // row and of its mask instead of the three sweeps below, every access of a warp one coalesced stretch
-// whatever the alignment. Bound by the number of 2-byte accesses and the exponentials. Measured: fp16
-// [49152, 333] with a key mask 404 us with the three sweeps, 59 us here; bf16 [24576, 1201] 795 -> 98 us.
+// whatever the alignment. Bound by the number of 2-byte accesses and the exponentials. Measured with a key mask: fp16
+// [24576, 333] 203 us with the three sweeps, 25.4 us here; fp32 [24576, 5001] 915 -> 496 us.
+// Few rows (up to four per SM of 65..512 elements, two per SM of up to 2048) take a CTA per row with two elements a
+// thread: fp16 [384, 333] by warps 3.7 us, so 3.2; [8, 511] 3.8 and 2.5. fp32 rows of eight elements a thread keep to 32
+// registers, two CTAs of 1024 threads per SM (50 registers: [24576, 5001] 1009 us).
 template <typename Tin, typename Tout, bool PACKED, int E, int G>
-__global__ void __launch_bounds__(G == 0 ? 1024 : 256) softmax_ragged_kernel(const SoftmaxParams p) {
+__global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 ? 2 : 0) softmax_ragged_kernel(const SoftmaxParams p) {
   __shared__ float red[32];
   const int lane = glane<G>(), gs = gsize<G>();
   long long row = grow<G>();
@@ -355,8 +358,26 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256) softmax_ragged_kernel(con
   Tout* y = reinterpret_cast<Tout*>(p.y) + row_offset(p.ymap, row);
   float t[E];
   float mx = -INFINITY;
+  {  // every load is on its way before the first value is looked at
+    Tin xv[E], mv[E];
 #pragma unroll
-  for (int e = 0; e < E; ++e) t[e] = e * gs + lane < p.n ? softmax_logit<Tin, PACKED>(p, x, m, e * gs + lane) : -INFINITY;
+    for (int e = 0; e < E; ++e)
+      if (e * gs + lane < p.n) xv[e] = __ldg(x + e * gs + lane);
+    if (m) {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (e * gs + lane < p.n) mv[e] = __ldg(m + e * gs + lane);
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      t[e] = -INFINITY;
+      if (e * gs + lane < p.n) {
+        t[e] = Elem<Tin>::to_f32(xv[e]);
+        if (p.has_scale) t[e] = PACKED ? round_through<Tin>(t[e] * p.scale) : t[e] * p.scale;
+        if (m) t[e] = PACKED ? round_through<Tin>(t[e] + Elem<Tin>::to_f32(mv[e])) : t[e] + Elem<Tin>::to_f32(mv[e]);
+      }
+    }
+  }
 #pragma unroll
   for (int e = 0; e < E; ++e) mx = fmaxf(mx, t[e]);
   mx = greduce<FastMax, G>(mx, red);
@@ -1006,9 +1027,12 @@ static int launch_softmax(const SoftmaxParams& p, bool vector_ok, cudaStream_t s
     softmax_long_kernel<Tin, Tout><<<(unsigned)p.rows, threads, 0, st>>>(p);
   } else if (p.n <= 8192) {
     set_path_tag("elements in registers");
-    if (p.n <= 512) {
+    if (p.n > 64 && p.n <= 2048 && p.rows <= (p.n <= 512 ? 4LL : 2LL) * device_info().sm_count) {
+      softmax_ragged_kernel<Tin, Tout, PACKED, 2, 0><<<(unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st>>>(p);
+    } else if (p.n <= 512) {
       const unsigned grid = (unsigned)((p.rows + 7) / 8);
       if (p.n <= 64) softmax_ragged_kernel<Tin, Tout, PACKED, 2, 32><<<grid, 256, 0, st>>>(p);
+      else if (p.n <= 128) softmax_ragged_kernel<Tin, Tout, PACKED, 4, 32><<<grid, 256, 0, st>>>(p);
       else if (p.n <= 256) softmax_ragged_kernel<Tin, Tout, PACKED, 8, 32><<<grid, 256, 0, st>>>(p);
       else softmax_ragged_kernel<Tin, Tout, PACKED, 16, 32><<<grid, 256, 0, st>>>(p);
     } else {
