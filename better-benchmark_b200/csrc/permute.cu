@@ -287,14 +287,18 @@ __global__ void __launch_bounds__(256) transpose16_ragged_kernel(const Transpose
 // so a thread that walks the words (2c, 2c + 1) of the input rows writes both. Neighbouring lanes take
 // neighbouring column pairs: they read neighbouring words, and write words P apart - different banks
 // when P is odd; for even P each lane starts its walk one word later than its neighbour, which makes
-// the distance odd as well.
+// the distance odd as well. Where P is a multiple of 8 that is not enough: 32 / gcd(P, 32) neighbours already
+// meet every bank there is, so only the next such run of lanes starts a word later (bf16 [7324, 8, 512] 30.5 -> 28.2 us,
+// [60000, 16, 32] 31.9 -> 29.4). P = 2 writes both words of a pair of columns at once ([14648, 2, 1024] 48.4 -> 25.0 us).
 // What bounds it: HBM, with the shared-memory passes (copy in, read, write, copy out: about 390 cycles
 // for a [49, 128] matrix, a third of the time its bytes take) behind it. Measured on bf16 [16384, 49, 128]:
-// 141.4 us with two-byte gathers (four-way bank conflicts), 74.1 us (5.55 TB/s) here.
-template <bool ODD>
-__global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposeParams p, const int group, const int stages,
-                                                              const int split, const FastDiv by_tasks,
-                                                              const FastDiv by_pairs) {
+// 139.5 us with two-byte gathers (four-way bank conflicts), 67.9 us (6.05 TB/s) here. The kernel divides by nothing but
+// precomputed reciprocals: the divisions of its first form cost a tenth of that, and a fifth of a 2 us call.
+template <int KIND>  // 0: P even, 1: P odd, 2: P = 2
+__global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposeParams p, const int group, const long long groups,
+                                                              const int stages, const int split, const FastDiv by_tasks,
+                                                              const FastDiv by_pairs, const FastDiv by_split,
+                                                              const FastDiv by_walk) {
   extern __shared__ __align__(128) unsigned char pairs_smem[];
   const int P = (int)p.P, C = (int)p.C, CW = C / 2;
   const int elems = P * C;
@@ -302,16 +306,17 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
   const uint32_t ring = smem_u32(pairs_smem);
   unsigned char* const done = pairs_smem + (size_t)stages * span;  // the transposed group
   uint32_t* const out = reinterpret_cast<uint32_t*>(done);
-  const long long groups = (p.batch + group - 1) / group;
   const int tid = threadIdx.x;
-  auto bytes_of = [&](long long g) {
+  // P a multiple of 8: rows of lanes whose words fall into the same banks start one word later than the row before
+  const int stagger = P % 8 == 0 ? 5 - min(__ffs(P) - 1, 5) : 0;
+  auto matrices_of = [&](long long g) {
     const long long left = p.batch - g * group;
-    return (int)(left < group ? left : group) * elems * 2;
+    return (int)(left < group ? left : group);
   };
   auto load = [&](long long g, int slot) {
     if (g < groups) {
       const unsigned char* src = reinterpret_cast<const unsigned char*>(p.x) + g * group * p.in_batch_stride * 2;
-      const int whole = bytes_of(g) & ~15;
+      const int whole = matrices_of(g) * elems * 2 & ~15;
       for (int at = tid * 16; at < whole; at += 256 * 16) copy_async16(ring + (uint32_t)(slot * span + at), src + at);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
     load(g + (long long)(stages - 1) * gridDim.x, ahead);  // its last reader passed the barrier below
     if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
     else asm volatile("cp.async.wait_group 1;" ::: "memory");
-    const int bytes = bytes_of(g), whole = bytes & ~15;
+    const int here = matrices_of(g), bytes = here * elems * 2, whole = bytes & ~15;
     const unsigned char* block = pairs_smem + (size_t)slot * span;
     if (tid * 2 < bytes - whole)  // the last group may end between two 16-byte boundaries
       *reinterpret_cast<unsigned short*>(pairs_smem + (size_t)slot * span + whole + tid * 2) =
@@ -333,7 +338,6 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
     if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the block before has left
     __syncthreads();
     const uint32_t* in = reinterpret_cast<const uint32_t*>(block);
-    const int here = bytes / (elems * 2);
     const int tasks = group * CW, steps = P / 2;
     for (int t = tid; t < tasks * split; t += 256) {
       const int q = (int)fast_div((unsigned)t, by_tasks);
@@ -341,10 +345,10 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
       const int m = (int)fast_div((unsigned)u, by_pairs);
       if (m >= here) continue;
       const int cp = u - m * CW;
-      const int j0 = steps * q / split, j1 = steps * (q + 1) / split;
+      const int j0 = (int)fast_div((unsigned)(steps * q), by_split), j1 = (int)fast_div((unsigned)(steps * (q + 1)), by_split);
       const uint32_t* src = in + m * (elems / 2) + cp;
       uint32_t* dst = out + m * (elems / 2) + cp * P;
-      if constexpr (ODD) {
+      if constexpr (KIND == 1) {
         uint32_t a = src[2 * j0 * CW];
 #pragma unroll 4
         for (int j = j0; j < j1; ++j) {
@@ -354,9 +358,12 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
           a = n;
         }
         if (q == split - 1) dst[P / 2] = __byte_perm(src[(P - 1) * CW], src[0], 0x7610);
+      } else if constexpr (KIND == 2) {  // P = 2: both words at once
+        const uint32_t a = src[0], b = src[CW];
+        *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
       } else {
-        const int len = j1 - j0;
-        int r = len > 0 ? cp % len : 0;
+        const int len = j1 - j0, x = cp >> stagger;
+        int r = x - (int)fast_div((unsigned)x, by_walk) * (int)by_walk.d;  // below the shortest walk
 #pragma unroll 4
         for (int j = 0; j < len; ++j) {
           const int k = j0 + r;
@@ -533,13 +540,15 @@ static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st
     return false;
   }
   const int span = (int)(group * elems * 2);
-  const int stages = span <= 16 * 1024 ? 3 : 2;
+  // three stages while four CTAs fit an SM with them (bf16 [16384, 49, 128]: 67.9 us, 72.8 with two), two from there on
+  // ([4185, 7, 1024] 21.1 us, 26.0 with three; [2441, 1024, 8] 20.8 and 23.4)
+  const int stages = 4 * ((size_t)4 * span + 1024) <= (size_t)device_info().max_smem_optin ? 3 : 2;
   const size_t smem = (size_t)(stages + 1) * span;
   const int tasks = (int)(group * (p.C / 2));
   int split = 256 / tasks;  // threads that share a pair of columns
   if (split > p.P / 2) split = (int)(p.P / 2);
   if (split < 1) split = 1;
-  auto kernel = p.P % 2 ? transpose_pairs_kernel<true> : transpose_pairs_kernel<false>;
+  auto kernel = p.P % 2 ? transpose_pairs_kernel<1> : (p.P == 2 ? transpose_pairs_kernel<2> : transpose_pairs_kernel<0>);
   const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -548,9 +557,11 @@ static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st
   int per_sm = (int)((size_t)device_info().max_smem_optin / (smem + 1024));
   if (per_sm > 8) per_sm = 8;
   if (per_sm < 1) per_sm = 1;
-  long long grid = (p.batch + group - 1) / group;
+  const long long groups = (p.batch + group - 1) / group;
+  long long grid = groups;
   if (grid > (long long)device_info().sm_count * per_sm) grid = (long long)device_info().sm_count * per_sm;
-  kernel<<<(unsigned)grid, 256, smem, st>>>(p, group, stages, split, make_fast_div(tasks), make_fast_div(p.C / 2));
+  kernel<<<(unsigned)grid, 256, smem, st>>>(p, group, groups, stages, split, make_fast_div(tasks), make_fast_div(p.C / 2),
+                                            make_fast_div(split), make_fast_div(p.P / 2 / split));
   *rc = launch_status("b200_transpose_copy [small matrices, word pairs]");
   return true;
 }

@@ -126,7 +126,9 @@ def test_norm_bwd_edges(rows, n, dtype, rms):
 
 @pytest.mark.parametrize("batch,rows,cols", [(1, 2, 2), (7, 49, 128), (5, 196, 64), (33, 3, 10), (2000, 5, 6), (9, 64, 66),
                                              (3, 129, 126), (2, 16, 1024), (2, 63, 65), (3, 65, 63), (2, 500, 333),
-                                             (2, 501, 768), (1, 1, 300), (2, 300, 1), (1300, 33, 64)])
+                                             (2, 501, 768), (1, 1, 300), (2, 300, 1), (1300, 33, 64),
+                                             (3, 2, 1024), (4001, 2, 6), (700, 4, 64), (9, 8, 1000), (50, 16, 130), (5000, 6, 34),
+                                             (2500, 12, 100), (4, 1024, 8), (1200, 32, 48)])   # even row counts: walks that start apart
 def test_transpose_of_ragged_16_bit_matrices(batch, rows, cols):
     """Groups of small matrices (a last group that ends between two 16-byte boundaries among them) and
     64 x 64 tiles with ragged ends on either side; a view that starts off the 4-byte grid."""
@@ -418,3 +420,12 @@ def test_a_few_ragged_softmax_rows_cost_what_aligned_ones_do():
 
     ragged, aligned = us(511), us(512)
     assert ragged < 1.25 * aligned, (ragged, aligned)
+
+
+def test_transposes_of_two_rows_cost_what_the_bytes_cost():
+    """The same 30 MB as [14648, 2, 1024] and [7324, 4, 1024] in 16 bits: 25 and 28 us. Two rows took 48 with a walk of
+    one step and its index arithmetic per column pair."""
+    k = _kernels()
+    two, four = (_graph_us(lambda x=_randn(shape, torch.bfloat16, 1): k.permute_copy(x, (0, 2, 1)))
+                 for shape in [(14648, 2, 1024), (7324, 4, 1024)])
+    assert two < 1.2 * four, (two, four)
