@@ -1270,17 +1270,13 @@ extern "C" int64_t b200_norm_bwd_wait_timeouts(void) {
 }
 
 // Bytes of scratch that let every path run its largest grid for rows of n elements: the barrier
-// words, two planes (dweight, dbias) of one fp32 partial row per group, and 64 fp64 values per
-// group that nothing uses any more (the size that callers have been told stays). A group is a CTA (at most eight resident per SM), except in the
-// warp-per-row register kernel that takes rows of up to 256 elements, where it is a warp (64 per
+// words and two planes (dweight, dbias) of one fp32 partial row per group. A group is a CTA (at most eight resident
+// per SM), except in the warp-per-row register kernel that takes rows of up to 256 elements, where it is a warp (64 per
 // SM). The launchers shrink their grids to whatever scratch they are given, so a smaller buffer
 // costs speed, never correctness.
 extern "C" int64_t b200_norm_bwd_scratch_bytes(int64_t n) {
-  const int64_t sms = device_info().sm_count;
-  const int64_t groups = (n <= 256 ? 64 : 8) * sms;
-  const int64_t planes = 2 * groups * n * (int64_t)sizeof(float);
-  const int64_t level2 = 2 * groups * 64 * (int64_t)sizeof(double);
-  return 256 + planes + 64 + level2;
+  const int64_t groups = (n <= 256 ? 64 : 8) * (int64_t)device_info().sm_count;
+  return 256 + 2 * groups * n * (int64_t)sizeof(float);
 }
 
 extern "C" int b200_norm_bwd(const void* x, const void* dy, const void* weight, const float* mean,

@@ -429,3 +429,19 @@ def test_transposes_of_two_rows_cost_what_the_bytes_cost():
     two, four = (_graph_us(lambda x=_randn(shape, torch.bfloat16, 1): k.permute_copy(x, (0, 2, 1)))
                  for shape in [(14648, 2, 1024), (7324, 4, 1024)])
     assert two < 1.2 * four, (two, four)
+
+
+@pytest.mark.parametrize("rows,n", [(20000, 64), (9000, 256), (20000, 129), (9000, 513), (9000, 768), (4000, 2052), (2000, 4096)])
+def test_norm_bwd_takes_its_largest_grid_with_the_advertised_scratch(rows, n):
+    """Exactly the advertised bytes give the bits that the larger default buffer gives, and they are what two planes of
+    partial rows take."""
+    from better_benchmark_b200 import native
+    lib = native.load()
+    x, dy, w = _randn((rows, n), torch.float32, n), _randn((rows, n), torch.float32, n + 1), torch.ones(n, device="cuda")
+    mean, rstd = torch.zeros(rows, device="cuda"), torch.ones(rows, device="cuda")
+    size = int(lib.b200_norm_bwd_scratch_bytes(n))
+    assert size <= 256 + 2 * (64 if n <= 256 else 8) * lib.b200_sm_count() * n * 4
+    kw = dict(mean=mean, rms=False, want_dbias=True)
+    want = _kernels().norm_bwd(x, dy, w, rstd, **kw)
+    got = _kernels().norm_bwd(x, dy, w, rstd, scratch=torch.zeros(size, dtype=torch.uint8, device="cuda"), **kw)
+    assert all(torch.equal(g, v) for g, v in zip(got, want))
