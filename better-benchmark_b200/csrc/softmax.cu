@@ -756,7 +756,7 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
   const int ch = per > 512 ? 8 : (per > 128 || S > 1 ? 4 : 2);
   const int threads = (int)((per + ch - 1) / ch + 31) / 32 * 32;
   if (S == 1) {
-    set_path_tag("two sweeps over a row in registers, any alignment");
+    set_path_tag("row in the registers of a CTA, any alignment");
     const unsigned grid = (unsigned)p.rows;
     if (ch == 8) softmax_rows_kernel<Tin, Tout, 8, false><<<grid, threads, 0, st>>>(p, 1);
     else if (ch == 4) softmax_rows_kernel<Tin, Tout, 4, false><<<grid, threads, 0, st>>>(p, 1);
@@ -764,7 +764,7 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
     *rc = launch_status("b200_softmax");
     return true;
   }
-  set_path_tag("two sweeps over a row in the registers of a cluster, any alignment");
+  set_path_tag("row in the registers of a cluster, any alignment");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.rows * S));
   cfg.blockDim = dim3((unsigned)threads);

@@ -445,3 +445,52 @@ def test_norm_bwd_takes_its_largest_grid_with_the_advertised_scratch(rows, n):
     want = _kernels().norm_bwd(x, dy, w, rstd, **kw)
     got = _kernels().norm_bwd(x, dy, w, rstd, scratch=torch.zeros(size, dtype=torch.uint8, device="cuda"), **kw)
     assert all(torch.equal(g, v) for g, v in zip(got, want))
+
+
+@pytest.mark.parametrize("log", [False, True])
+def test_masked_softmax_beyond_the_registers(log):
+    """More than 8192 keys off the vector grid: the three sweeps."""
+    k = _kernels()
+    x, keep = _randn((2, 1, 3, 9001), torch.float16, 3, 2.0), torch.rand(2, 1, 1, 9001, device="cuda") < 0.8
+    keep[..., 0] = True
+    mask = torch.where(keep, 0.0, -10000.0).to(torch.float16)
+    got = k.softmax(x, mask=mask, scale=0.5, log=log)
+    assert b"three passes" in k.load().b200_last_kernel()
+    t = x.double() * 0.5 + mask.double()
+    _near(got, torch.log_softmax(t, -1) if log else torch.softmax(t, -1), "9001 keys", floor=2e-6 if log else 1e-7)
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 40003), (torch.float32, 5001)])
+def test_softmax_rows_over_strided_outer_dimensions(dtype, n):
+    """Three outer dimensions that do not collapse, rows on every alignment: a CTA and a cluster per row."""
+    base = _randn((2, 3, 5, 4, n + 1), dtype, 5, 2.0)
+    for x in (base[:, ::2, 1:4, :, :n], base[:, :, ::2, 1:3, 1:]):
+        for rows in (x, x[:, :, :, :, :3001]):
+            got = _kernels().softmax(rows)
+            _near(got, torch.softmax(rows.double(), -1), f"strided softmax {tuple(rows.shape)}", floor=1e-7)
+
+
+def test_transpose_of_small_matrices_with_gaps_between_them():
+    """The batch stride is not rows * columns: one matrix per block."""
+    k = _kernels()
+    for dtype, rows, take, cols in ((torch.bfloat16, 60, 49, 128), (torch.float16, 10, 4, 96), (torch.bfloat16, 8, 2, 48)):
+        x = _randn((37, rows, cols), dtype, rows)[:, :take]
+        assert torch.equal(k.permute_copy(x, (0, 2, 1)), x.transpose(1, 2).contiguous())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_residual_layer_norm_of_strided_and_of_special_rows(dtype):
+    """Padded rows through the warp kernel's copies; NaN and infinities stay in their rows."""
+    k = _kernels()
+    n = 768 if dtype == torch.bfloat16 else 384
+    base, other = _randn((50, n + 32), dtype, 1, 2.0), _randn((50, n + 32), dtype, 2)
+    base[7, 3], base[8, n - 1], other[9, 0] = float("nan"), float("inf"), float("-inf")
+    x, r, w, b = base[:, :n], other[:, :n], _randn((n,), dtype, 3), _randn((n,), dtype, 4)
+    for form in (False, True, "both"):
+        y, total = [k.norm_fwd(x, w, b, eps=1e-6, residual=r, want_sum=True, round_sum=form)[i] for i in (0, 4)]
+        assert b"warp rings" in k.load().b200_last_kernel()
+        assert torch.equal(total.view(50, n)[:7], (x.float() + r.float()).to(dtype)[:7])
+        assert torch.isnan(y[7:10]).all() and torch.isfinite(y[:7]).all() and torch.isfinite(y[10:]).all()
+        if form is False:
+            rest = torch.cat([torch.arange(7), torch.arange(10, 50)]).cuda()
+            _near(y[rest], _layer_norm64((x.double() + r.double())[rest], w, b, 1e-6, False), "strided residual", floor=4e-5)

@@ -131,22 +131,27 @@ def test_softmax_output_dtype_and_strided_rows():
 
 
 @pytest.mark.parametrize("log", [False, True])
-@pytest.mark.parametrize("rows,n,stride,offset,dtype,out_dtype", [
-    (64, 20005, 20008, 0, torch.bfloat16, torch.float32),   # ragged length, aligned padded rows
-    (12, 262144, 262144, 0, torch.bfloat16, torch.bfloat16),  # rows far beyond the register-resident kernel
-    (33, 5001, 5004, 0, torch.float32, torch.float32),
-    (20, 4001, 4100, 3, torch.float16, torch.float16),     # unaligned row starts: element-wise sweeps
-    (7, 70000, 70000, 0, torch.float32, torch.bfloat16),
+@pytest.mark.parametrize("rows,n,stride,offset,dtype,out_dtype,path", [
+    (64, 20005, 20008, 0, torch.bfloat16, torch.float32, "registers of a cluster"),   # ragged length, aligned padded rows
+    (12, 262144, 262144, 0, torch.bfloat16, torch.bfloat16, "registers of a cluster"),  # the longest rows eight CTAs hold
+    (33, 5001, 5004, 0, torch.float32, torch.float32, "registers of a cluster"),
+    (20, 4001, 4100, 3, torch.float16, torch.float16, "registers of a CTA"),     # unaligned row starts
+    (7, 70000, 70000, 0, torch.float32, torch.bfloat16, "registers of a cluster"),
+    (90, 9001, 9001, 0, torch.bfloat16, torch.float32, "registers of a CTA"),    # more rows: as few CTAs as hold the row
+    (90, 40000, 40000, 0, torch.bfloat16, torch.bfloat16, "registers of a cluster"),
+    (80, 80000, 80000, 0, torch.bfloat16, torch.bfloat16, "two sweeps"),         # aligned and long
+    (80, 66000, 66001, 1, torch.float32, torch.float32, "two sweeps"),           # fp32 and long, unaligned
+    (4, 300001, 300004, 1, torch.bfloat16, torch.bfloat16, "two sweeps"),         # longer than eight CTAs hold
 ])
-def test_softmax_long_and_ragged_rows(rows, n, stride, offset, dtype, out_dtype, log):
-    """Rows the register-resident kernel cannot take go through the two-sweep kernel (running maximum
-    and rescaled sum, then a second read of the row)."""
+def test_softmax_long_and_ragged_rows(rows, n, stride, offset, dtype, out_dtype, path, log):
+    """Rows the register-resident kernel cannot take are held in registers by a CTA or by a cluster of them, or go through
+    the two-sweep kernel (running maximum and rescaled sum, then a second read of the row)."""
     from oracle.eager import MaskedScaledSoftmax
     k = _kernels()
     base = _randn((rows, stride + offset), dtype, n % 97, scale=3.0)
     view = base[:, offset:offset + n]
     got = k.softmax(base.cuda()[:, offset:offset + n], log=log, out_dtype=out_dtype)
-    assert b"two sweeps" in k.load().b200_last_kernel(), k.load().b200_last_kernel()
+    assert path.encode() in k.load().b200_last_kernel(), k.load().b200_last_kernel()
     want = MaskedScaledSoftmax(log=log, out_dtype=out_dtype)(view)
     assert_close(got, want, f"long softmax log={log} {dtype}->{out_dtype} {rows}x{n}")
     special = view.clone().float()
