@@ -58,13 +58,13 @@ cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const size_t optin = (size_t)device_info().max_smem_optin;
   std::lock_guard<std::mutex> lock(mu);
   for (int i = 0; i < used; ++i)
     if (done[i].kernel == kernel && done[i].device == dev) return bytes <= done[i].limit ? cudaSuccess : cudaErrorInvalidValue;
   cudaFuncAttributes attr;
   e = cudaFuncGetAttributes(&attr, kernel);
   if (e != cudaSuccess) return e;
+  const size_t optin = (size_t)device_info().max_smem_optin;
   const size_t limit = optin > attr.sharedSizeBytes ? optin - attr.sharedSizeBytes : 0;
   if (bytes > limit) return cudaErrorInvalidValue;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);

@@ -530,19 +530,20 @@ static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st
   const long long elems = p.P * p.C;
   if (p.C % 2 != 0 || p.P < 2 || elems * 2 > 32 * 1024 || p.in_row_stride != p.C || !aligned16(p.x) || !aligned16(p.y))
     return false;
+  const DeviceInfo& dev = device_info();
   int group = 1;  // the smallest group that is a whole number of 16-byte vectors
   while (group * elems % 8 != 0) group *= 2;
   if (group * elems * 2 > 32 * 1024) return false;
   if (p.in_batch_stride == elems || p.batch == 1) {
     // small matrices: larger groups (up to 12 KB a block), but no fewer than four blocks per SM
-    while (2 * group * elems * 2 <= 12 * 1024 && p.batch / (2 * group) >= 4LL * device_info().sm_count) group *= 2;
+    while (2 * group * elems * 2 <= 12 * 1024 && p.batch / (2 * group) >= 4LL * dev.sm_count) group *= 2;
   } else if (group != 1 || p.in_batch_stride % 8 != 0) {
     return false;
   }
   const int span = (int)(group * elems * 2);
   // three stages while four CTAs fit an SM with them (bf16 [16384, 49, 128]: 67.9 us, 72.8 with two), two from there on
   // ([4185, 7, 1024] 21.1 us, 26.0 with three; [2441, 1024, 8] 20.8 and 23.4)
-  const int stages = 4 * ((size_t)4 * span + 1024) <= (size_t)device_info().max_smem_optin ? 3 : 2;
+  const int stages = 4 * ((size_t)4 * span + 1024) <= (size_t)dev.max_smem_optin ? 3 : 2;
   const size_t smem = (size_t)(stages + 1) * span;
   const int tasks = (int)(group * (p.C / 2));
   int split = 256 / tasks;  // threads that share a pair of columns
@@ -554,12 +555,12 @@ static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st
     cudaGetLastError();
     return false;
   }
-  int per_sm = (int)((size_t)device_info().max_smem_optin / (smem + 1024));
+  int per_sm = (int)((size_t)dev.max_smem_optin / (smem + 1024));
   if (per_sm > 8) per_sm = 8;
   if (per_sm < 1) per_sm = 1;
   const long long groups = (p.batch + group - 1) / group;
   long long grid = groups;
-  if (grid > (long long)device_info().sm_count * per_sm) grid = (long long)device_info().sm_count * per_sm;
+  if (grid > (long long)dev.sm_count * per_sm) grid = (long long)dev.sm_count * per_sm;
   kernel<<<(unsigned)grid, 256, smem, st>>>(p, group, groups, stages, split, make_fast_div(tasks), make_fast_div(p.C / 2),
                                             make_fast_div(split), make_fast_div(p.P / 2 / split));
   *rc = launch_status("b200_transpose_copy [small matrices, word pairs]");
