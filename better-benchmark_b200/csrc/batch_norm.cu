@@ -914,8 +914,8 @@ __global__ void __launch_bounds__(256) batch_norm_apply_general_kernel(const Bat
 }
 
 // ----------------------------------------------------------------------------------------------
-// Channels-last tensors with ANY channel count: three launches over the tensor as a flat array of
-// 16-byte vectors (the corpus of the reference has channels-last BatchNorm points with 24, 36, 60,
+// Channels-last tensors whose channel pattern repeats within 512 vectors: three launches over the tensor as a flat
+// array of 16-byte vectors (the corpus of the reference has channels-last BatchNorm points with 24, 36, 60,
 // 92, 100, 480 ... channels; repros/canonical/var_mean_42fad1ece813/shapes.json).
 //
 // A vector holds V consecutive elements of the flat [rows * C] array, so it may straddle the end
@@ -1572,7 +1572,7 @@ static int launch_batch_norm(BatchNormParams p, bool channels_last_fast, bool ch
     note_launch("b200_batch_norm_fwd [fused, channels-last, CTA ring]");
     return B200_OK;
   }
-  if (channels_last) {  // any channel count: the tensor as a flat array of vectors, three launches
+  if (channels_last) {  // channel patterns of up to 512 vectors: the tensor as a flat array, three launches
     BatchNormParams q = p;
     q.rows = p.rows * p.spatial;
     int rc = B200_OK;

@@ -628,8 +628,8 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
 // What bounds it: HBM, with about 38 instructions per pair of elements (two complete normalisations and
 // the roundings between them, 57 % of the issue slots) behind it. The resident kernel converts weight
 // and bias in every row on top and overlaps its load and store phases less; it keeps the rows of up to
-// 64 vectors, of which it puts two into a warp. Measured on bf16 [65536, 768] with the sum kept: 82.5 ->
-// 76.8 us back to back (64 us, 6.25 TB/s, from a clean L2); f16 [46251, 448]: 34.9 us there, 36.9 us here.
+// 64 vectors, of which it puts two into a warp (f16 [46251, 448]: 34.9 us there, 36.9 us here). Measured on bf16
+// [65536, 768] with the sum kept: 82.5 -> 76.8 us back to back (64 us, 6.25 TB/s, from a clean L2).
 // ----------------------------------------------------------------------------------------------
 constexpr int kResWarps = 8;  // warps per CTA
 
@@ -958,8 +958,8 @@ __global__ void __launch_bounds__(1024) norm_fwd_streaming_kernel(const NormFwdP
 // stretch of 2- or 4-byte elements whatever the row's alignment. The row is read once; the element-wise
 // sweeps below read it two to six times and are left with rows of more than 16 384 elements (16 a thread).
 // Bound by the number of those accesses: about 1.6 TB/s for 16-bit elements, 3.3 TB/s for fp32.
-// Measured against the sweeps: LayerNorm bf16 [20000, 769] 461.6 -> 73.8 us, RMSNorm f32 [20000, 1001]
-// 329.8 -> 49.2 us, residual LayerNorm f16 [46251, 449] 795.6 -> 106.9 us.
+// Measured against the sweeps: LayerNorm bf16 [4800, 769] 114 -> 17.5 us, [4800, 8191] 246 -> 158, RMSNorm f32 [4800, 1001]
+// 82 -> 14.6 us, residual LayerNorm (both forms) bf16 [18682, 449] 322 -> 52 us.
 // Few rows (up to eight per SM of 129..512 elements, two per SM of up to 2048) take a CTA per row with two elements a
 // thread, as the longer chains of a thread are not hidden then: LayerNorm bf16 [148, 449] by warps 4.8 us, so 3.0;
 // [600, 257] 4.4 and 3.1 ([2400, 257] 4.8 by warps); [148, 769] with eight a thread 4.9, so 3.3.

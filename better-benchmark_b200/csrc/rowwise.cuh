@@ -225,9 +225,10 @@ __device__ __forceinline__ f32x2 exp_pair_fast(f32x2 x) {
 // 1 - Q(a) otherwise, and Q(a) = exp(-a^2 / 2) * P(t), t = 1 / (1 + 0.305 a), P a polynomial without a
 // constant term: the form of Hastings' approximations (Abramowitz & Stegun 26.2.17), here of degree
 // eight with coefficients fitted to erfcx by iteratively reweighted least squares (relative error of Q
-// below 9.5e-8 for 0 <= a <= 14). Over standard normal inputs the fp32 result is 3.9e-8 (2-norm) off
-// the fp64 one, the (x / 2) * (erff(x / sqrt 2) + 1) it replaces 3.7e-8; rounded to 16 bits both are
-// equally close, and for x < -3, where erff + 1 cancels, only this form keeps the value (within half a
+// below 9.5e-8 for 0 <= a <= 14). Over 2^24 standard normal inputs the 2-norm of the error of the 16-bit results agrees
+// in six digits with that of the (x / 2) * (erff(x / sqrt 2) + 1) it replaces, and fewer of them are not the nearest value
+// (bf16 5.5e-5 -> 0, fp16 2.7e-4 -> 6.1e-5; of fp16 inputs around 0.1, none -> 4.0e-4, by a
+// thousandth of half a step). For x < -3, where erff + 1 cancels, only this form keeps the value (within half a
 // 16-bit step over every bf16 and normal fp16 input). Fewer than half the instructions of erff. Measured:
 // GELU bf16 [32768, 1536] 69.6 -> 50.1 us, GELU -> LayerNorm bf16 [65536, 768] 81.2 -> 67.4 us.
 // a is clamped to 64 for the exponential, which needs finite arguments (Q(64) = 0); the product takes x

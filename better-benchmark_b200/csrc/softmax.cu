@@ -788,7 +788,8 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
 }
 
 // ----------------------------------------------------------------------------------------------
-// Rows beyond 32768 vectors (more than 262 144 16-bit columns): one CTA per row, two sweeps.
+// Rows that softmax_ctas_per_row leaves (beyond 32768 vectors, that is 262 144 16-bit columns; long aligned ones and long
+// fp32 ones when there are many): one CTA per row, two sweeps.
 //   sweep 1: every thread keeps a running maximum m and the sum of exp(t - m) of its elements,
 //            rescaling the sum when the maximum grows; the CTA then combines the (m, s) pairs:
 //            M = max m_i, S = sum s_i * exp(m_i - M)

@@ -253,8 +253,8 @@ int32_t b200_cast_scale(const void* x, void* y, int64_t n, int32_t in_dtype, int
  * sums only), dweight = sum(dy * (x - mean)) * invstd and dbias = sum(dy), fp32 [C] (each may be
  * NULL). `act` (may be NULL) enables the activation-backward prologue dy' = act > 0 ? dy : dy * slope
  * (slope 0: ReLU), rounded to the tensor dtype. One launch for contiguous NCHW tensors; three
- * launches (sums, fp64 finalize, apply) for channels-last tensors (flat 16-byte vectors, any channel
- * count) and for other strides (element-wise). No atomics. Scratch: b200_batch_norm_bwd_scratch_bytes(channels), 16-byte aligned, no initial state.
+ * launches (sums, fp64 finalize, apply) for channels-last tensors (flat 16-byte vectors where the channel
+ * pattern repeats within 512 of them) and for other strides (element-wise). No atomics. Scratch: b200_batch_norm_bwd_scratch_bytes(channels), 16-byte aligned, no initial state.
  * Replaces sum_sum_183b124c731f/oracle.py (partial sums, finalize, apply) and, with the prologue,
  * sum_sum_12fc8ebf8180/oracle.py. */
 int64_t b200_batch_norm_bwd_scratch_bytes(int64_t channels);
