@@ -26,11 +26,6 @@ struct BatchNormParams {
   int relu;
   float* partials;  // [P][2][C]
   float* stats;     // [2][C] mean, invstd (scratch copy every CTA reads)
-  unsigned int* bar;
-  long long rows_per_cta;  // contiguous row range of each CTA
-  int smem_tiles;          // stages of the shared-memory ring
-  int local_stats;         // 1: every CTA combines all partials itself (one grid barrier instead of two)
-  int deep;                // 1: a thread's chain of squares is long; it is carried in fp64 every 16 vectors
 };
 
 // The value every sum of a channel is shifted by. Any value works as long as all threads of all
@@ -38,8 +33,7 @@ struct BatchNormParams {
 // (s2 - s1 * s1 / n) / n cancels, and the cancellation multiplies the rounding error of s2 by
 // 1 + (shift - mean)^2 / var. The first element of the channel can sit three standard deviations
 // away (a factor of ten); the mean of the channel's first sixteen rows (rows beyond the last one
-// repeat it) rarely sits more than one. Both forms below add the same sixteen values in the same
-// order with the same roundings, so they agree to the bit.
+// repeat it) rarely sits more than one.
 constexpr int BN_SHIFT_ROWS = 16;
 
 // The shift is cut to eight significant bits (a bf16 value). With 16-bit inputs x - shift then
@@ -62,34 +56,6 @@ __device__ __forceinline__ float bn_shift_scalar(const T* x, int c, int channels
 #pragma unroll
   for (int r = 0; r < BN_SHIFT_ROWS; ++r) s = __fadd_rn(s, v[r]);
   return bn_round_shift(__fmul_rn(s, 1.0f / BN_SHIFT_ROWS));
-}
-
-// The same for the Elem<T>::V channels of vector column vc, as fp32 pairs.
-template <typename T>
-__device__ __forceinline__ void bn_shift_pairs(const T* x, int vc, int channels, long long rows,
-                                               f32x2 (&shift)[Elem<T>::V / 2]) {
-  constexpr int V = Elem<T>::V;
-  uint4 raw[BN_SHIFT_ROWS];
-#pragma unroll
-  for (int r = 0; r < BN_SHIFT_ROWS; ++r) {
-    const long long rr = r < rows ? r : rows - 1;
-    raw[r] = ld_keep(x + rr * channels + (long long)vc * V);
-  }
-#pragma unroll
-  for (int i = 0; i < V / 2; ++i) shift[i] = splat2(0.f);
-#pragma unroll
-  for (int r = 0; r < BN_SHIFT_ROWS; ++r) {
-    f32x2 f[V / 2];
-    Pairs<T>::unpack(raw[r], f);
-#pragma unroll
-    for (int i = 0; i < V / 2; ++i) shift[i] = add2(shift[i], f[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < V / 2; ++i) {
-    float lo, hi;
-    unpack2(mul2(shift[i], splat2(1.0f / BN_SHIFT_ROWS)), lo, hi);
-    shift[i] = pack2(bn_round_shift(lo), bn_round_shift(hi));
-  }
 }
 
 // Turns the fp64 totals of the shifted sums of one channel into mean / invstd and, for the one
@@ -125,42 +91,45 @@ __device__ __forceinline__ void bn_channel_stats(const BatchNormParams& p, int c
   }
 }
 
-// Many channels: the channels are dealt out to the WARPS of the grid (channel c to warp c / P of
-// CTA c % P, P = CTAs = partial rows), so that all of them are combined at the same time and no
-// CTA barrier is involved. The lanes split the partial rows, eight loads in flight each, fp64,
-// fixed order; lane 0 derives the statistics and publishes them in p.stats for the second grid barrier.
-template <typename T>
-__device__ __forceinline__ void bn_stats_by_warps(const BatchNormParams& p, const T* x, int P) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  // a trailing partial warp (block sizes that are no multiple of 32) takes no channel
-  for (int c = (int)blockIdx.x + warp * P; c < p.channels && warp < nwarps; c += P * nwarps) {
-    const float shift = lane == 0 ? bn_shift_scalar<T>(x, c, p.channels, p.rows) : 0.f;
-    double d1 = 0.0, d2 = 0.0;
-    for (int g0 = lane; g0 < P; g0 += 8 * 32) {
-      float a[8], b[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int g = g0 + u * 32;
-        a[u] = g < P ? __ldcg(p.partials + ((long long)g * 2) * p.channels + c) : 0.f;
-        b[u] = g < P ? __ldcg(p.partials + ((long long)g * 2 + 1) * p.channels + c) : 0.f;
+// Adds up what the threads of a CTA hold: `one` and `two` are flat arrays of blockDim.x * V values each, of
+// which value f belongs to channel f % channels (blockDim.x * V is a multiple of the channel count). As many
+// threads share a channel as there are; fp64, fixed order. `part`: 2 * blockDim.x doubles. One thread per channel
+// made this a chain of blockDim.x * V / channels additions: bf16 channels-last [N, 16, 7, 7] of 1 MB forward
+// 11.8 us, so 8.0 us.
+template <typename Out, int V>
+__device__ __forceinline__ void bn_fold_channels(const float* one, const float* two, double* part, int channels,
+                                                 Out* row_one, Out* row_two) {
+  const int tid = threadIdx.x, threads = blockDim.x, values = threads * V;
+  const int share = channels <= threads ? threads / channels : 1;  // threads per channel
+  if (share == 1) {
+    for (int c = tid; c < channels; c += threads) {
+      double a = 0.0, b = 0.0;
+      for (int f = c; f < values; f += channels) {
+        a += (double)one[f];
+        b += (double)two[f];
       }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        d1 += (double)a[u];
-        d2 += (double)b[u];
-      }
+      row_one[c] = (Out)a;
+      row_two[c] = (Out)b;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-      d2 += __shfl_xor_sync(0xffffffffu, d2, o);
+    return;
+  }
+  if (tid < share * channels) {
+    double a = 0.0, b = 0.0;
+    for (int f = tid; f < values; f += share * channels) {
+      a += (double)one[f];
+      b += (double)two[f];
     }
-    if (lane == 0) {
-      float mean, invstd;
-      bn_channel_stats(p, c, d1, d2, shift, true, &mean, &invstd);
-      p.stats[c] = mean;
-      p.stats[p.channels + c] = invstd;
-    }
+    part[tid] = a;
+    part[threads + tid] = b;
+  }
+  __syncthreads();
+  for (int i = tid; i < 2 * channels; i += threads) {  // both sums of a channel at the same time
+    const int c = i < channels ? i : i - channels;
+    const double* p = part + (i < channels ? 0 : threads) + c;
+    double a = 0.0;
+    for (int r = 0; r < share; ++r) a += p[r * channels];
+    if (i < channels) row_one[c] = (Out)a;
+    else row_two[c] = (Out)a;
   }
 }
 

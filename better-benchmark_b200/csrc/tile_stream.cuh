@@ -80,6 +80,10 @@ __device__ __forceinline__ void bulk_load_hint(void* smem_dst, const void* gmem_
 __device__ __forceinline__ void copy_async16(uint32_t smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
 }
+// The same with an L2 eviction-priority policy.
+__device__ __forceinline__ void copy_async16_hint(uint32_t smem_dst, const void* src, uint64_t policy) {
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(src), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void copy_async_wait() {

@@ -346,6 +346,31 @@ def test_batch_norm_channels_last_takes_the_faster_kernels(n, c, hw, rings):
     assert (b"copy rings" in k.load().b200_last_kernel()) == rings, k.load().b200_last_kernel()
 
 
+@pytest.mark.parametrize("n,c,hw,dtype", [(2, 1, 2056, torch.float16), (3, 4, 1022, torch.float32), (9, 8, 57345, torch.bfloat16),
+                                          (61, 16, 4099, torch.bfloat16), (41, 256, 441, torch.float32),
+                                          (340, 64, 196, torch.float16)])
+def test_batch_norm_channels_last_of_few_channels_and_power_of_two_counts(n, c, hw, dtype):
+    """Many threads share a channel in the fold of the partial sums; power-of-two counts on both sides of 8 MB."""
+    k = _kernels()
+    x = _randn((n, c, hw, 1), dtype, c, 2.0).contiguous(memory_format=torch.channels_last)
+    dy = _randn((n, c, hw, 1), dtype, c + 1).contiguous(memory_format=torch.channels_last)
+    w, b = _randn((c,), torch.float32, c + 3), _randn((c,), torch.float32, c + 4)
+    col = lambda t: t.double().view(1, c, 1, 1)  # noqa: E731
+    d = x.double()
+    mean64, var64 = d.mean((0, 2, 3)), d.var((0, 2, 3), unbiased=False)
+    y, mean, invstd = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1)
+    assert c < 4 or b"copy rings" in k.load().b200_last_kernel(), k.load().b200_last_kernel()
+    _near(mean, mean64, "mean", floor=2e-6)
+    _near(invstd, torch.rsqrt(var64 + 1e-5), "invstd", floor=2e-6)
+    _near(y, (d - col(mean64)) * col(torch.rsqrt(var64 + 1e-5)) * col(w) + col(b), f"y {n}x{c}x{hw}", floor=2e-5)
+    dx, dw, db = k.batch_norm_bwd(dy, x, mean, invstd, w)
+    xhat, floor = (d - col(mean)) * col(invstd), 2.0 ** -21 * (n * hw) ** 0.5 * 8   # as in the test above
+    s1, s2 = dy.double().sum((0, 2, 3)), (dy.double() * xhat).sum((0, 2, 3))
+    _near(db, s1, "dbias", floor=floor)
+    _near(dw, s2, "dweight", floor=floor)
+    _near(dx, (dy.double() - col(s1) / (n * hw) - xhat * col(s2) / (n * hw)) * col(w) * col(invstd), f"dx {n}x{c}x{hw}", floor=1e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_log_softmax_in_fp32_has_no_biased_sum(dtype):
     """Mean error of fp32 log-probabilities over 100 000 rows of 1003. An exponential whose errors have a mean shifts
