@@ -18,7 +18,7 @@
 // No atomics: bit-reproducible.
 // Channels-last tensors whose channel pattern repeats within 512 vectors of 16 bytes take the vector
 // kernels, contiguous NCHW tensors the cluster kernel; every other layout the strided element-wise ones.
-#include "rowwise.cuh"
+#include "batch_norm.cuh"
 
 #include <cooperative_groups.h>
 
@@ -84,12 +84,17 @@ __device__ __forceinline__ void bn_bwd_prologue(f32x2 (&g)[Elem<T>::V / 2], cons
 // f32 [200, 485, 8, 8], element-wise before, 145 -> 28. The same kernels with 8 CTAs per SM in turn: 93.6 us
 // where these take 85.9 (bf16 [992, 64, 28, 28]).
 constexpr int kChunk = 4;  // vectors of each tensor in flight per thread
+// What the apply kernel finds in L2: the tensors' last 80 MB, provided that nothing pushes them out. The rest is
+// loaded evict-first, and so is everything in the apply kernel without act: bf16
+// [256, 64, 56, 56] 90.4 -> 82.6 us, half of that size 53.3 -> 46.6 (60 MB a tensor).
+constexpr long long kStaysBytes = 80000000;
 
 // MAXT: 256 threads, or 512 for patterns of more than 256 vectors (one CTA per SM of as many threads).
 template <typename T, bool ACT, int MAXT>
 __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_sums_cl_kernel(const BnBwdParams p, long long total, int PV) {
   constexpr int V = Elem<T>::V;
-  __shared__ float red[2 * MAXT * V];  // [2][threads][V]
+  __shared__ __align__(16) float red[2 * MAXT * V];  // [2][threads][V]
+  __shared__ double part[2 * MAXT];
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
   const int ph = tid % PV;
   const uint4* dy = reinterpret_cast<const uint4*>(p.dy);
@@ -102,15 +107,18 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_sums_cl_kernel(const 
     s1[i] = s2[i] = splat2(0.f);
   }
   const long long step = (long long)gridDim.x * kChunk * T_;
+  const long long stays = total - kStaysBytes / 16 / (ACT ? 3 : 2);  // from here on L2 is to keep the vectors
+  const uint64_t keep = l2_policy_evict_normal(), drop = l2_policy_evict_first();
   for (long long v = (long long)blockIdx.x * kChunk * T_ + tid; v < total; v += step) {
     uint4 rg[kChunk], rx[kChunk], ra[ACT ? kChunk : 1];
+    const uint64_t policy = v >= stays ? keep : drop;
 #pragma unroll
     for (int u = 0; u < kChunk; ++u) {
       const long long i = v + (long long)u * T_;
       if (i < total) {
-        rg[u] = ld_stream(reinterpret_cast<const T*>(dy + i));
-        rx[u] = ld_stream(reinterpret_cast<const T*>(x + i));
-        if constexpr (ACT) ra[u] = ld_stream(reinterpret_cast<const T*>(act + i));
+        rg[u] = ld_policy(dy + i, policy);
+        rx[u] = ld_policy(x + i, policy);
+        if constexpr (ACT) ra[u] = ld_policy(act + i, policy);
       }
     }
     // the chunk's own short sums first: the chain over the chunks is then kChunk times shorter
@@ -147,19 +155,8 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_sums_cl_kernel(const 
     unpack2(s2[i], r2[tid * V + 2 * i], r2[tid * V + 2 * i + 1]);
   }
   __syncthreads();
-  const int period = PV * V;  // elements; a multiple of C
-  for (int c = tid; c < p.channels; c += T_) {
-    double a = 0.0, b = 0.0;
-    for (int idx = c; idx < period; idx += C) {  // every (phase, element) that lands on channel c
-      const int col = idx / V, e = idx % V;
-      for (int t = col; t < T_; t += PV) {
-        a += (double)r1[t * V + e];
-        b += (double)r2[t * V + e];
-      }
-    }
-    p.partials[((long long)blockIdx.x * 2) * p.channels + c] = a;
-    p.partials[((long long)blockIdx.x * 2 + 1) * p.channels + c] = b;
-  }
+  double* row = p.partials + ((long long)blockIdx.x * 2) * C;
+  bn_fold_channels<double, V>(r1, r2, part, C, row, row + C);
 }
 
 // One CTA per channel: the partials are read with every thread (all loads of a thread are in
@@ -236,14 +233,20 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_apply_cl_kernel(const
   const long long last = (total - 1) / chunk * chunk;  // first vector of the last chunk
   long long v = last - (long long)blockIdx.x * chunk + tid;
   uint4 rg[kChunk], rx[kChunk], ra[ACT ? kChunk : 1];
+  // nothing is read again (with act there are no registers left for the policy)
+  const uint64_t drop = ACT ? 0 : l2_policy_evict_first();
+  auto load = [&](const uint4* q) {
+    if constexpr (ACT) return ld_stream(q);
+    else return ld_policy(q, drop);
+  };
   auto fetch = [&]() {
 #pragma unroll
     for (int u = 0; u < kChunk; ++u) {
       const long long i = v + (long long)u * T_;
       if (i >= 0 && i < total) {
-        rg[u] = ld_stream(reinterpret_cast<const T*>(dy + i));
-        rx[u] = ld_stream(reinterpret_cast<const T*>(x + i));
-        if constexpr (ACT) ra[u] = ld_stream(reinterpret_cast<const T*>(act + i));
+        rg[u] = load(dy + i);
+        rx[u] = load(x + i);
+        if constexpr (ACT) ra[u] = load(act + i);
       }
     }
   };
