@@ -95,6 +95,7 @@ __device__ __forceinline__ void bn_finalize_channel(const BatchNormParams& p, in
 // ----------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) batch_norm_stats_general_kernel(const BatchNormParams p) {
+  wait_for_previous_kernel();
   __shared__ float red[32];
   const int c = blockIdx.x;
   const int split = blockIdx.y, splits = gridDim.y;
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(256) batch_norm_stats_general_kernel(const Bat
 template <typename T>
 __global__ void __launch_bounds__(256) batch_norm_finalize_general_kernel(const BatchNormParams p,
                                                                           int num_partials, int rows_shift) {
+  wait_for_previous_kernel();
   const int warps = blockDim.x >> 5;
   const int c = blockIdx.x * warps + (threadIdx.x >> 5);
   if (c >= p.channels) return;
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_general_kernel(const 
 
 template <typename T>
 __global__ void __launch_bounds__(256) batch_norm_apply_general_kernel(const BatchNormParams p) {
+  wait_for_previous_kernel();
   const int c = blockIdx.x;
   const T* x = reinterpret_cast<const T*>(p.x);
   T* y = reinterpret_cast<T*>(p.y);
@@ -174,6 +177,7 @@ __global__ void __launch_bounds__(256) batch_norm_apply_general_kernel(const Bat
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1) batch_norm_sums_cl_flat_kernel(const BatchNormParams p, long long vecs_per_cta,
                                                                       int PV, int rows_shift) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   __shared__ float red[2 * MAXT * V];  // [2][threads][V]
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
@@ -266,6 +270,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1) batch_norm_sums_cl_
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1) batch_norm_apply_cl_flat_kernel(const BatchNormParams p, long long vecs_per_cta,
                                                                        int PV) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
   const int ph = PV - 1 - tid % PV;  // the range ends on a multiple of PV: its last vector has phase PV - 1
@@ -341,15 +346,15 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
   splits = (total + per - 1) / per;
   p.stats = p.partials + splits * 2 * C;
   const int rows_shift = per > 32LL * threads ? 1 : 0;  // more than 32 vectors per thread
-  if (threads <= 256) batch_norm_sums_cl_flat_kernel<T, 256><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV, rows_shift);
-  else batch_norm_sums_cl_flat_kernel<T, 512><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV, rows_shift);
+  if (threads <= 256) launch_dependent(batch_norm_sums_cl_flat_kernel<T, 256>, (unsigned)splits, threads, 0, st, p, per, (int)PV, rows_shift);
+  else launch_dependent(batch_norm_sums_cl_flat_kernel<T, 512>, (unsigned)splits, threads, 0, st, p, per, (int)PV, rows_shift);
   *rc = launch_status("b200_batch_norm_fwd sums [channels-last, flat vectors]");
   if (*rc != B200_OK) return true;
-  batch_norm_finalize_general_kernel<T><<<(p.channels + 7) / 8, 256, 0, st>>>(p, (int)splits, rows_shift);
+  launch_dependent(batch_norm_finalize_general_kernel<T>, (p.channels + 7) / 8, 256, 0, st, p, (int)splits, rows_shift);
   *rc = launch_status("b200_batch_norm_fwd finalize");
   if (*rc != B200_OK || !p.y) return true;
-  if (threads <= 256) batch_norm_apply_cl_flat_kernel<T, 256><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV);
-  else batch_norm_apply_cl_flat_kernel<T, 512><<<(unsigned)splits, threads, 0, st>>>(p, per, (int)PV);
+  if (threads <= 256) launch_dependent(batch_norm_apply_cl_flat_kernel<T, 256>, (unsigned)splits, threads, 0, st, p, per, (int)PV);
+  else launch_dependent(batch_norm_apply_cl_flat_kernel<T, 512>, (unsigned)splits, threads, 0, st, p, per, (int)PV);
   *rc = launch_status("b200_batch_norm_fwd apply [channels-last, flat vectors]");
   return true;
 }
@@ -403,6 +408,7 @@ __device__ __forceinline__ void bn_ring_issue(const uint4* x, uint32_t mine, int
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total,
                                                                                    int PV, int rows_shift) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   extern __shared__ __align__(128) unsigned char smem[];
   float* red = reinterpret_cast<float*>(smem + (size_t)kRingBytesPerThread * MAXT);  // [MAXT * V]: the shifts
@@ -654,7 +660,7 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
       *rc = fail((int)e, "b200_batch_norm_fwd: cannot reserve %zu bytes of shared memory: %s", with_shifts, cudaGetErrorString(e));
       return;
     }
-    sums<<<(unsigned)splits, threads, with_shifts, st>>>(p, total, (int)PV, rows_shift);
+    launch_dependent(sums, (unsigned)splits, threads, with_shifts, st, p, total, (int)PV, rows_shift);
     *rc = launch_status("b200_batch_norm_fwd sums [channels-last, flat vectors, copy rings]");
     if (*rc != B200_OK) return;
     launch_dependent(batch_norm_finalize_ring_kernel<T>, dim3((unsigned)p.channels), dim3(256), 0, st, p, (int)splits, rows_shift);
@@ -691,14 +697,14 @@ static int launch_batch_norm(BatchNormParams p, bool channels_last, size_t scrat
   if ((long long)scratch_bytes < need)
     return fail(B200_ERR_WORKSPACE, "b200_batch_norm_fwd: scratch of %zu bytes, need %lld", scratch_bytes, need);
   p.stats = p.partials + splits * 2 * p.channels;
-  batch_norm_stats_general_kernel<T><<<dim3(p.channels, (unsigned)splits), 256, 0, st>>>(p);
+  launch_dependent(batch_norm_stats_general_kernel<T>, dim3(p.channels, (unsigned)splits), 256, 0, st, p);
   int rc = launch_status("b200_batch_norm_fwd stats [strided, element-wise]");
   if (rc != B200_OK) return rc;
-  batch_norm_finalize_general_kernel<T><<<(p.channels + 7) / 8, 256, 0, st>>>(p, (int)splits, 0);
+  launch_dependent(batch_norm_finalize_general_kernel<T>, (p.channels + 7) / 8, 256, 0, st, p, (int)splits, 0);
   rc = launch_status("b200_batch_norm_fwd finalize");
   if (rc != B200_OK) return rc;
   if (p.y) {
-    batch_norm_apply_general_kernel<T><<<dim3(p.channels, (unsigned)splits), 256, 0, st>>>(p);
+    launch_dependent(batch_norm_apply_general_kernel<T>, dim3(p.channels, (unsigned)splits), 256, 0, st, p);
     rc = launch_status("b200_batch_norm_fwd apply [strided, element-wise]");
   }
   return rc;

@@ -92,6 +92,7 @@ constexpr long long kStaysBytes = 80000000;
 // MAXT: 256 threads, or 512 for patterns of more than 256 vectors (one CTA per SM of as many threads).
 template <typename T, bool ACT, int MAXT>
 __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_sums_cl_kernel(const BnBwdParams p, long long total, int PV) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   __shared__ __align__(16) float red[2 * MAXT * V];  // [2][threads][V]
   __shared__ double part[2 * MAXT];
@@ -299,6 +300,7 @@ __device__ __forceinline__ float bn_bwd_dy_general(const BnBwdParams& p, long lo
 
 template <typename T>
 __global__ void __launch_bounds__(256) bn_bwd_sums_general_kernel(const BnBwdParams p) {
+  wait_for_previous_kernel();
   __shared__ double red[2][8];
   const int c = blockIdx.x;
   const long long total = p.rows * p.spatial;
@@ -338,6 +340,7 @@ __global__ void __launch_bounds__(256) bn_bwd_sums_general_kernel(const BnBwdPar
 
 template <typename T>
 __global__ void __launch_bounds__(256) bn_bwd_apply_general_kernel(const BnBwdParams p) {
+  wait_for_previous_kernel();
   const int c = blockIdx.x;
   const long long total = p.rows * p.spatial;
   const long long per = (total + gridDim.y - 1) / gridDim.y;
@@ -435,6 +438,7 @@ __device__ __forceinline__ void bn_bwd_visit_plane(const T* dyp, const T* xp, co
 template <typename T, bool HAS_ACT, bool CLUSTER>
 __global__ void __launch_bounds__(256)
 bn_bwd_nchw_cluster_kernel(const BnBwdParams p, const int imgs_per_cta, const int G) {
+  wait_for_previous_kernel();
   namespace cg = cooperative_groups;
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;
@@ -565,6 +569,7 @@ struct alignas(W * sizeof(T)) BwdPlaneVec {
 
 template <typename T, int K, int W, bool HAS_ACT>
 __global__ void __launch_bounds__(1024) bn_bwd_nchw_small_kernel(const BnBwdParams p, const FastDiv vpp_div) {
+  wait_for_previous_kernel();
   __shared__ float part[2][32];
   using Vec = BwdPlaneVec<T, W>;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
@@ -645,8 +650,8 @@ __global__ void __launch_bounds__(1024) bn_bwd_nchw_small_kernel(const BnBwdPara
 
 template <typename T, int K, int W>
 static void launch_bn_bwd_small_k(const BnBwdParams& p, int threads, const FastDiv& d, cudaStream_t st) {
-  if (p.act) bn_bwd_nchw_small_kernel<T, K, W, true><<<(unsigned)p.channels, threads, 0, st>>>(p, d);
-  else bn_bwd_nchw_small_kernel<T, K, W, false><<<(unsigned)p.channels, threads, 0, st>>>(p, d);
+  if (p.act) launch_dependent(bn_bwd_nchw_small_kernel<T, K, W, true>, (unsigned)p.channels, threads, 0, st, p, d);
+  else launch_dependent(bn_bwd_nchw_small_kernel<T, K, W, false>, (unsigned)p.channels, threads, 0, st, p, d);
 }
 
 // At most 8 elements of each tensor per thread; as few vectors per thread as 512 threads allow.
@@ -709,25 +714,14 @@ static bool try_launch_bn_bwd_nchw(const BnBwdParams& p, cudaStream_t st, int* r
   while (G > 2 && 256 / (G / 2) <= 2 * ipc && plane_vecs <= 4LL * (G / 2)) G /= 2;
   if (S == 1) {
     const dim3 grid(1, (unsigned)p.channels, 1);
-    if (p.act) bn_bwd_nchw_cluster_kernel<T, true, false><<<grid, 256, 0, st>>>(p, ipc, G);
-    else bn_bwd_nchw_cluster_kernel<T, false, false><<<grid, 256, 0, st>>>(p, ipc, G);
+    if (p.act) launch_dependent(bn_bwd_nchw_cluster_kernel<T, true, false>, grid, 256, 0, st, p, ipc, G);
+    else launch_dependent(bn_bwd_nchw_cluster_kernel<T, false, false>, grid, 256, 0, st, p, ipc, G);
     *rc = launch_status("b200_batch_norm_bwd [NCHW, one launch, CTA per channel]");
     return true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)S, (unsigned)p.channels, 1);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = p.act ? cudaLaunchKernelEx(&cfg, bn_bwd_nchw_cluster_kernel<T, true, true>, p, ipc, G)
-                        : cudaLaunchKernelEx(&cfg, bn_bwd_nchw_cluster_kernel<T, false, true>, p, ipc, G);
+  const dim3 grid = dim3((unsigned)S, (unsigned)p.channels, 1), block = dim3(256), cluster((unsigned)S, 1, 1);
+  cudaError_t e = p.act ? launch_clusters(cluster, bn_bwd_nchw_cluster_kernel<T, true, true>, grid, block, 0, st, p, ipc, G)
+                        : launch_clusters(cluster, bn_bwd_nchw_cluster_kernel<T, false, true>, grid, block, 0, st, p, ipc, G);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -762,7 +756,7 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
     auto run = [&](auto act_tag, auto maxt_tag) {
       constexpr bool ACT = decltype(act_tag)::value;
       constexpr int MAXT = decltype(maxt_tag)::value;
-      bn_bwd_sums_cl_kernel<T, ACT, MAXT><<<(unsigned)splits, threads, 0, st>>>(p, total, vpr);
+      launch_dependent(bn_bwd_sums_cl_kernel<T, ACT, MAXT>, (unsigned)splits, threads, 0, st, p, total, vpr);
       int rc = launch_status("b200_batch_norm_bwd sums");
       if (rc != B200_OK) return rc;
       launch_dependent(bn_bwd_finalize_kernel, dim3((unsigned)p.channels), dim3(256), 0, st, p);
@@ -789,13 +783,13 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
     return fail(B200_ERR_WORKSPACE, "b200_batch_norm_bwd: scratch of %zu bytes, need %lld", scratch_bytes, need);
   p.splits = (int)splits;
   p.coef = reinterpret_cast<float*>(p.partials + splits * 2 * p.channels);
-  bn_bwd_sums_general_kernel<T><<<dim3(p.channels, (unsigned)splits), 256, 0, st>>>(p);
+  launch_dependent(bn_bwd_sums_general_kernel<T>, dim3(p.channels, (unsigned)splits), 256, 0, st, p);
   int rc = launch_status("b200_batch_norm_bwd sums");
   if (rc != B200_OK) return rc;
-  bn_bwd_finalize_kernel<<<p.channels, 256, 0, st>>>(p);
+  launch_dependent(bn_bwd_finalize_kernel, p.channels, 256, 0, st, p);
   rc = launch_status("b200_batch_norm_bwd finalize");
   if (rc != B200_OK || !p.dx) return rc;
-  bn_bwd_apply_general_kernel<T><<<dim3(p.channels, (unsigned)splits), 256, 0, st>>>(p);
+  launch_dependent(bn_bwd_apply_general_kernel<T>, dim3(p.channels, (unsigned)splits), 256, 0, st, p);
   return launch_status("b200_batch_norm_bwd apply [strided, element-wise]");
 }
 

@@ -93,6 +93,7 @@ __device__ __forceinline__ void visit_plane(const T* plane, int hw, int lane, in
 template <typename T, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads)
 batch_norm_nchw_cluster_kernel(const BatchNormParams p, const int imgs_per_cta, const int G) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;
   __shared__ double warp_tot[kThreads / 32][2];
@@ -275,6 +276,7 @@ struct alignas(W * sizeof(T)) PlaneVec {
 template <typename T, int K, int W>
 __global__ void __launch_bounds__(1024)
 batch_norm_nchw_small_kernel(const BatchNormParams p, const FastDiv vpp_div) {
+  wait_for_previous_kernel();
   __shared__ float part[2][32];
   using Vec = PlaneVec<T, W>;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
@@ -363,11 +365,11 @@ static void launch_small(const BatchNormParams& p, cudaStream_t st) {
   threads = (threads + 31) / 32 * 32;
   const FastDiv d = make_fast_div(p.spatial / W);
   const unsigned grid = (unsigned)p.channels;
-  if (K == 1) batch_norm_nchw_small_kernel<T, 1, W><<<grid, threads, 0, st>>>(p, d);
-  if constexpr (KMAX >= 2) if (K == 2) batch_norm_nchw_small_kernel<T, 2, W><<<grid, threads, 0, st>>>(p, d);
-  if constexpr (KMAX >= 4) if (K == 4) batch_norm_nchw_small_kernel<T, 4, W><<<grid, threads, 0, st>>>(p, d);
-  if constexpr (KMAX >= 8) if (K == 8) batch_norm_nchw_small_kernel<T, 8, W><<<grid, threads, 0, st>>>(p, d);
-  if constexpr (KMAX >= 16) if (K == 16) batch_norm_nchw_small_kernel<T, 16, W><<<grid, threads, 0, st>>>(p, d);
+  if (K == 1) launch_dependent(batch_norm_nchw_small_kernel<T, 1, W>, grid, threads, 0, st, p, d);
+  if constexpr (KMAX >= 2) if (K == 2) launch_dependent(batch_norm_nchw_small_kernel<T, 2, W>, grid, threads, 0, st, p, d);
+  if constexpr (KMAX >= 4) if (K == 4) launch_dependent(batch_norm_nchw_small_kernel<T, 4, W>, grid, threads, 0, st, p, d);
+  if constexpr (KMAX >= 8) if (K == 8) launch_dependent(batch_norm_nchw_small_kernel<T, 8, W>, grid, threads, 0, st, p, d);
+  if constexpr (KMAX >= 16) if (K == 16) launch_dependent(batch_norm_nchw_small_kernel<T, 16, W>, grid, threads, 0, st, p, d);
 }
 
 }  // namespace
@@ -426,23 +428,12 @@ bool try_launch_batch_norm_nchw(const BatchNormParams& p, cudaStream_t st, int* 
   int G = 32;
   while (G > 2 && kThreads / (G / 2) <= 2 * ipc && plane_vecs <= 8LL * (G / 2)) G /= 2;
   if (S == 1) {
-    batch_norm_nchw_cluster_kernel<T, false><<<dim3(1, (unsigned)p.channels, 1), kThreads, 0, st>>>(p, ipc, G);
+    launch_dependent(batch_norm_nchw_cluster_kernel<T, false>, dim3(1, (unsigned)p.channels, 1), kThreads, 0, st, p, ipc, G);
     *rc = launch_status("b200_batch_norm_fwd [NCHW, one launch, CTA per channel]");
     return true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)S, (unsigned)p.channels, 1);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, batch_norm_nchw_cluster_kernel<T, true>, p, ipc, G);
+  const dim3 grid = dim3((unsigned)S, (unsigned)p.channels, 1), block = dim3(kThreads), cluster((unsigned)S, 1, 1);
+  cudaError_t e = launch_clusters(cluster, batch_norm_nchw_cluster_kernel<T, true>, grid, block, 0, st, p, ipc, G);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;  // the cluster launch was refused: the caller takes the three-launch path

@@ -52,6 +52,7 @@ __device__ __forceinline__ void store_out(void* out, int dtype, long long idx, f
 // CLUSTER: the gridDim.y CTAs that split one reduction are one cluster (cluster dims (1, splits, 1)).
 template <typename T, bool IS_MAX, bool VEC, bool CLUSTER>
 __global__ void __launch_bounds__(512) col_reduce_kernel(const ColReduceParams p) {
+  wait_for_previous_kernel();
   constexpr int V = VEC ? Elem<T>::V : 1;
   constexpr int U = 8;
   __shared__ float red[512 * V + 512];  // [TY][TX * V + 1]
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(512) col_reduce_kernel(const ColReduceParams p
 // with all their loads in flight together, and warp 0 adds the eight partial sums in order (fp64).
 template <bool IS_MAX>
 __global__ void __launch_bounds__(256) col_reduce_finalize_kernel(const ColReduceParams p) {
+  wait_for_previous_kernel();
   __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long total = p.batch * p.cols;
@@ -238,20 +240,9 @@ static int launch_col_reduce(ColReduceParams p, bool vec, size_t scratch_bytes, 
       ColReduceParams q = p;
       q.splits = (int)cs;
       q.rows_per_split = (p.rows + cs - 1) / cs;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)chunks, (unsigned)cs, (unsigned)p.batch);
-      cfg.blockDim = dim3(threads);
-      cfg.dynamicSmemBytes = 0;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1;
-      attr[0].val.clusterDim.y = (unsigned)cs;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      cudaError_t e = is_max ? cudaLaunchKernelEx(&cfg, col_reduce_kernel<T, true, true, true>, q)
-                             : cudaLaunchKernelEx(&cfg, col_reduce_kernel<T, false, true, true>, q);
+      const dim3 grid = dim3((unsigned)chunks, (unsigned)cs, (unsigned)p.batch), block = dim3(threads), cluster(1, (unsigned)cs, 1);
+      cudaError_t e = is_max ? launch_clusters(cluster, col_reduce_kernel<T, true, true, true>, grid, block, 0, st, q)
+                             : launch_clusters(cluster, col_reduce_kernel<T, false, true, true>, grid, block, 0, st, q);
       if (e == cudaSuccess) return launch_status("b200_col_reduce [vector, cluster of splits, DSMEM combine]");
       cudaGetLastError();  // the cluster launch was refused: take the two-launch path
     }
@@ -271,20 +262,9 @@ static int launch_col_reduce(ColReduceParams p, bool vec, size_t scratch_bytes, 
       q.tx_log2 = 3;
       q.splits = (int)cs;
       q.rows_per_split = (p.rows + cs - 1) / cs;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)chunks2, (unsigned)cs, (unsigned)p.batch);
-      cfg.blockDim = dim3(threads);
-      cfg.dynamicSmemBytes = 0;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1;
-      attr[0].val.clusterDim.y = (unsigned)cs;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      cudaError_t e = is_max ? cudaLaunchKernelEx(&cfg, col_reduce_kernel<T, true, true, true>, q)
-                             : cudaLaunchKernelEx(&cfg, col_reduce_kernel<T, false, true, true>, q);
+      const dim3 grid = dim3((unsigned)chunks2, (unsigned)cs, (unsigned)p.batch), block = dim3(threads), cluster(1, (unsigned)cs, 1);
+      cudaError_t e = is_max ? launch_clusters(cluster, col_reduce_kernel<T, true, true, true>, grid, block, 0, st, q)
+                             : launch_clusters(cluster, col_reduce_kernel<T, false, true, true>, grid, block, 0, st, q);
       if (e == cudaSuccess) return launch_status("b200_col_reduce [vector, narrow chunks, cluster of splits, DSMEM combine]");
       cudaGetLastError();
     }
@@ -292,17 +272,17 @@ static int launch_col_reduce(ColReduceParams p, bool vec, size_t scratch_bytes, 
   dim3 grid((unsigned)chunks, (unsigned)splits, (unsigned)p.batch);
   set_path_tag(vec ? "vector" : "element-wise");
   if (is_max) {
-    if (vec) col_reduce_kernel<T, true, true, false><<<grid, threads, 0, st>>>(p);
-    else col_reduce_kernel<T, true, false, false><<<grid, threads, 0, st>>>(p);
+    if (vec) launch_dependent(col_reduce_kernel<T, true, true, false>, grid, threads, 0, st, p);
+    else launch_dependent(col_reduce_kernel<T, true, false, false>, grid, threads, 0, st, p);
   } else {
-    if (vec) col_reduce_kernel<T, false, true, false><<<grid, threads, 0, st>>>(p);
-    else col_reduce_kernel<T, false, false, false><<<grid, threads, 0, st>>>(p);
+    if (vec) launch_dependent(col_reduce_kernel<T, false, true, false>, grid, threads, 0, st, p);
+    else launch_dependent(col_reduce_kernel<T, false, false, false>, grid, threads, 0, st, p);
   }
   int rc = launch_status("b200_col_reduce");
   if (rc != B200_OK || splits == 1) return rc;
   const long long total = p.batch * p.cols;
-  if (is_max) col_reduce_finalize_kernel<true><<<(unsigned)((total + 31) / 32), 256, 0, st>>>(p);
-  else col_reduce_finalize_kernel<false><<<(unsigned)((total + 31) / 32), 256, 0, st>>>(p);
+  if (is_max) launch_dependent(col_reduce_finalize_kernel<true>, (unsigned)((total + 31) / 32), 256, 0, st, p);
+  else launch_dependent(col_reduce_finalize_kernel<false>, (unsigned)((total + 31) / 32), 256, 0, st, p);
   return launch_status("b200_col_reduce finalize");
 }
 

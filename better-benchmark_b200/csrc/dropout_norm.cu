@@ -98,6 +98,7 @@ __device__ __forceinline__ void masks8(const uint32_t (&w)[8], uint32_t keep_fro
 
 template <typename T, int CH>
 __global__ void __launch_bounds__(128) dropout_rms_norm_kernel(DropoutNormParams p) {
+  wait_for_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int nv = p.cols >> 3;  // vectors of 8 elements per row
@@ -219,6 +220,7 @@ struct DropoutLayerNormParams {
 // Same row ownership as above; the variance is the centred sum of squares of the row in registers.
 template <typename T, int CH>
 __global__ void __launch_bounds__(128, min_ctas(CH)) dropout_layer_norm_kernel(DropoutLayerNormParams p) {
+  wait_for_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int nv = p.cols >> 3;
@@ -340,6 +342,7 @@ struct DropoutAddParams {
 // Flat over the elements, two vectors of 8 in flight per thread.
 template <typename T>
 __global__ void __launch_bounds__(256) dropout_add_kernel(DropoutAddParams p) {
+  wait_for_previous_kernel();
   const PhiloxKeys keys = philox_keys((unsigned long long)p.seeds[p.seed_index]);
   const f32x2 scale2 = splat2(p.scale);
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -402,12 +405,12 @@ int launch_dropout_rms_norm(const DropoutNormParams& p, cudaStream_t st) {
   const long long want = (p.rows + warps - 1) / warps;
   const long long cap = (long long)device_info().sm_count * 32;
   const int grid = (int)(want < cap ? want : cap);
-  if (nv <= 32) dropout_rms_norm_kernel<T, 1><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 64) dropout_rms_norm_kernel<T, 2><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 96) dropout_rms_norm_kernel<T, 3><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 128) dropout_rms_norm_kernel<T, 4><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 192) dropout_rms_norm_kernel<T, 6><<<grid, 32 * warps, 0, st>>>(p);
-  else dropout_rms_norm_kernel<T, 8><<<grid, 32 * warps, 0, st>>>(p);
+  if (nv <= 32) launch_dependent(dropout_rms_norm_kernel<T, 1>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 64) launch_dependent(dropout_rms_norm_kernel<T, 2>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 96) launch_dependent(dropout_rms_norm_kernel<T, 3>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 128) launch_dependent(dropout_rms_norm_kernel<T, 4>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 192) launch_dependent(dropout_rms_norm_kernel<T, 6>, grid, 32 * warps, 0, st, p);
+  else launch_dependent(dropout_rms_norm_kernel<T, 8>, grid, 32 * warps, 0, st, p);
   return launch_status("b200_dropout_rms_norm");
 }
 
@@ -418,12 +421,12 @@ int launch_dropout_layer_norm(const DropoutLayerNormParams& p, cudaStream_t st) 
   const long long want = (p.rows + warps - 1) / warps;
   const long long cap = (long long)device_info().sm_count * 32;
   const int grid = (int)(want < cap ? want : cap);
-  if (nv <= 32) dropout_layer_norm_kernel<T, 1><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 64) dropout_layer_norm_kernel<T, 2><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 96) dropout_layer_norm_kernel<T, 3><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 128) dropout_layer_norm_kernel<T, 4><<<grid, 32 * warps, 0, st>>>(p);
-  else if (nv <= 192) dropout_layer_norm_kernel<T, 6><<<grid, 32 * warps, 0, st>>>(p);
-  else dropout_layer_norm_kernel<T, 8><<<grid, 32 * warps, 0, st>>>(p);
+  if (nv <= 32) launch_dependent(dropout_layer_norm_kernel<T, 1>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 64) launch_dependent(dropout_layer_norm_kernel<T, 2>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 96) launch_dependent(dropout_layer_norm_kernel<T, 3>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 128) launch_dependent(dropout_layer_norm_kernel<T, 4>, grid, 32 * warps, 0, st, p);
+  else if (nv <= 192) launch_dependent(dropout_layer_norm_kernel<T, 6>, grid, 32 * warps, 0, st, p);
+  else launch_dependent(dropout_layer_norm_kernel<T, 8>, grid, 32 * warps, 0, st, p);
   return launch_status("b200_dropout_layer_norm");
 }
 
@@ -458,6 +461,7 @@ struct SoftmaxDropoutParams {
 
 template <typename T, int CH>
 __global__ void __launch_bounds__(128) softmax_dropout_kernel(SoftmaxDropoutParams p) {
+  wait_for_previous_kernel();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const PhiloxKeys keys = philox_keys((unsigned long long)p.seeds[p.seed_index]);
   const int nv = p.cols >> 3;
@@ -539,9 +543,9 @@ int launch_softmax_dropout(const SoftmaxDropoutParams& p, cudaStream_t st) {
   const long long want = (p.rows + 3) / 4;
   const long long cap = (long long)device_info().sm_count * 32;
   const int grid = (int)(want < cap ? want : cap);
-  if (nv <= 32) softmax_dropout_kernel<T, 1><<<grid, 128, 0, st>>>(p);
-  else if (nv <= 64) softmax_dropout_kernel<T, 2><<<grid, 128, 0, st>>>(p);
-  else softmax_dropout_kernel<T, 4><<<grid, 128, 0, st>>>(p);
+  if (nv <= 32) launch_dependent(softmax_dropout_kernel<T, 1>, grid, 128, 0, st, p);
+  else if (nv <= 64) launch_dependent(softmax_dropout_kernel<T, 2>, grid, 128, 0, st, p);
+  else launch_dependent(softmax_dropout_kernel<T, 4>, grid, 128, 0, st, p);
   return launch_status("b200_softmax_dropout");
 }
 
@@ -674,8 +678,8 @@ extern "C" int b200_dropout_add(const void* x, const void* residual, const int64
   const long long cap = (long long)device_info().sm_count * 32;
   const int grid = (int)(want < cap ? want : cap);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (x_dtype == B200_BF16) dropout_add_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(q);
-  else dropout_add_kernel<__half><<<grid, 256, 0, st>>>(q);
+  if (x_dtype == B200_BF16) launch_dependent(dropout_add_kernel<__nv_bfloat16>, grid, 256, 0, st, q);
+  else launch_dependent(dropout_add_kernel<__half>, grid, 256, 0, st, q);
   return launch_status("b200_dropout_add");
 }
 

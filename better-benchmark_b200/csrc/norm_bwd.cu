@@ -29,6 +29,7 @@ namespace b200 {
 template <typename T, int CH, bool BLOCK, bool LN>
 __global__ void __launch_bounds__(BLOCK ? 512 : 256)
 norm_bwd_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   __shared__ float2 red[2][16];
   __shared__ double fin[16 * 64];
@@ -215,6 +216,7 @@ norm_bwd_kernel(const NormBwdParams p) {
 template <typename T, int CH, bool LN>
 __global__ void __launch_bounds__(512, CH == 1 ? 2 : 1)
 norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(16) float2 red[2][16];
@@ -454,6 +456,7 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
 template <typename T, int R, bool LN, bool GROUPED>
 __global__ void __launch_bounds__(512, 2)
 norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, const int groups_arg, const int wpg_inv) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   constexpr int NVAL = R * (LN ? 2 : 1);  // row sums per tile: 2, 4 or 8
   constexpr int LPV = 32 / NVAL;          // lanes that share one value after the warp reduction
@@ -741,6 +744,7 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
 }
 
 __global__ void __launch_bounds__(512) norm_bwd_finalize_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
   __shared__ double fin[16 * 64];
   if (p.dw) finalize_columns(p.partials, p.groups, p.n, p.dw, fin);
   if (p.db) finalize_columns(p.partials + (long long)p.groups * p.n, p.groups, p.n, p.db, fin);
@@ -751,6 +755,7 @@ __global__ void __launch_bounds__(512) norm_bwd_finalize_kernel(const NormBwdPar
 // layout, not tuned.
 template <typename T, bool LN>
 __global__ void __launch_bounds__(256) norm_bwd_rows_general_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* x = reinterpret_cast<const T*>(p.x) + row * p.x_row_stride;
@@ -792,6 +797,7 @@ __global__ void __launch_bounds__(256) norm_bwd_rows_general_kernel(const NormBw
 // One thread per column, rows split over blockIdx.y; partial rows go to scratch like the fast path.
 template <typename T, bool LN>
 __global__ void __launch_bounds__(128) norm_bwd_cols_general_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= p.n) return;
   const long long per = (p.rows + gridDim.y - 1) / gridDim.y;
@@ -823,6 +829,7 @@ __global__ void __launch_bounds__(128) norm_bwd_cols_general_kernel(const NormBw
 // 24.9, RMSNorm f32 [20000, 769] 191 -> 55 us.
 template <typename T, bool LN, int E, int G>
 __global__ void __launch_bounds__(G == 0 ? 512 : 256, G == 0 ? 1 : 2) norm_bwd_ragged_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
   extern __shared__ float fold[];  // warp per row: [warps][n] for dw, [warps][n] for db
   __shared__ float red[64];
   const int lane = glane<G>(), gs = gsize<G>(), n = p.n;
@@ -980,10 +987,7 @@ static bool try_launch_norm_bwd_stream(NormBwdParams p, int threads, size_t scra
   p.groups = (int)grid;
   p.fused = cooperative ? 1 : 0;
   if (cooperative) {
-    int stages_arg = stages;
-    void* args[] = {&p, &stages_arg};
-    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), dim3(threads),
-                                    args, smem, st);
+    e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(threads), smem, st, p, stages);
     if (e != cudaSuccess) {
       cudaGetLastError();
       *rc = fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
@@ -993,10 +997,10 @@ static bool try_launch_norm_bwd_stream(NormBwdParams p, int threads, size_t scra
     *rc = B200_OK;
     return true;
   }
-  kernel<<<(unsigned)grid, threads, smem, st>>>(p, stages);
+  launch_dependent(kernel, (unsigned)grid, threads, smem, st, p, stages);
   *rc = launch_status("b200_norm_bwd (streaming)");
   if (*rc == B200_OK && (p.dw || p.db)) {
-    norm_bwd_finalize_kernel<<<(p.n + 63) / 64, 512, 0, st>>>(p);
+    launch_dependent(norm_bwd_finalize_kernel, (p.n + 63) / 64, 512, 0, st, p);
     *rc = launch_status("b200_norm_bwd finalize");
   }
   return true;
@@ -1059,10 +1063,7 @@ static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratc
   p.fused = cooperative ? 1 : 0;
   int tg_arg = tg, groups_arg = groups_per_cta, wpg_inv_arg = (65536 + tg / 32 - 1) / (tg / 32);
   if (cooperative) {
-    int stages_arg = stages;
-    void* args[] = {&p, &stages_arg, &tg_arg, &groups_arg, &wpg_inv_arg};
-    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), dim3(threads),
-                                    args, smem, st);
+    e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(threads), smem, st, p, stages, tg_arg, groups_arg, wpg_inv_arg);
     if (e != cudaSuccess) {
       cudaGetLastError();
       *rc = fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
@@ -1072,10 +1073,10 @@ static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratc
     *rc = B200_OK;
     return true;
   }
-  kernel<<<(unsigned)grid, threads, smem, st>>>(p, stages, tg_arg, groups_arg, wpg_inv_arg);
+  launch_dependent(kernel, (unsigned)grid, threads, smem, st, p, stages, tg_arg, groups_arg, wpg_inv_arg);
   *rc = launch_status("b200_norm_bwd (row tiles)");
   if (*rc == B200_OK && (p.dw || p.db)) {
-    norm_bwd_finalize_kernel<<<(p.n + 63) / 64, 512, 0, st>>>(p);
+    launch_dependent(norm_bwd_finalize_kernel, (p.n + 63) / 64, 512, 0, st, p);
     *rc = launch_status("b200_norm_bwd finalize");
   }
   return true;
@@ -1103,9 +1104,7 @@ static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_byt
   p.groups = (int)(grid * groups_per_cta);
   p.fused = cooperative ? 1 : 0;
   if (cooperative) {
-    void* args[] = {&p};
-    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid),
-                                                dim3(threads), args, 0, st);
+    const cudaError_t e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(threads), 0, st, p);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
@@ -1113,12 +1112,12 @@ static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_byt
     note_launch(BLOCK ? "b200_norm_bwd [registers, CTA per row, fused finalize]" : "b200_norm_bwd [registers, warp per row, fused finalize]");
     return B200_OK;
   }
-  kernel<<<(unsigned)grid, threads, 0, st>>>(p);
+  launch_dependent(kernel, (unsigned)grid, threads, 0, st, p);
   int rc = launch_status("b200_norm_bwd");
   if (rc != B200_OK) return rc;
   if (p.dw || p.db) {
     const int chunks = (p.n + 63) / 64;
-    norm_bwd_finalize_kernel<<<chunks, 512, 0, st>>>(p);
+    launch_dependent(norm_bwd_finalize_kernel, chunks, 512, 0, st, p);
     rc = launch_status("b200_norm_bwd finalize");
   }
   return rc;
@@ -1128,6 +1127,7 @@ static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_byt
 // the many partial rows of a CTA per row do not meet in a handful of CTAs (LayerNorm bf16 [1200, 513] 31.9 us with the
 // kernel above, 10.5 so; [9341, 449] 29.9 and 19.5; fewer partial rows, that is fewer CTAs, gained nothing). fp64, fixed order.
 __global__ void __launch_bounds__(512) norm_bwd_finalize_ragged_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
   __shared__ double part[16][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c = blockIdx.x * 16 + (tid & 15);
@@ -1171,10 +1171,10 @@ static bool try_launch_norm_bwd_ragged(NormBwdParams p, size_t scratch_bytes, cu
       if (grid > max_groups) grid = max_groups;
     }
     p.groups = (int)grid;
-    kernel<<<(unsigned)grid, threads, smem, st>>>(p);
+    launch_dependent(kernel, (unsigned)grid, threads, smem, st, p);
     *rc = launch_status("b200_norm_bwd [ragged rows, elements in registers]");
     if (*rc == B200_OK && sums) {
-      norm_bwd_finalize_ragged_kernel<<<dim3((p.n + 15) / 16, (p.dw ? 1 : 0) + (p.db ? 1 : 0)), 512, 0, st>>>(p);
+      launch_dependent(norm_bwd_finalize_ragged_kernel, dim3((p.n + 15) / 16, (p.dw ? 1 : 0) + (p.db ? 1 : 0)), 512, 0, st, p);
       *rc = launch_status("b200_norm_bwd finalize");
     }
     return true;
@@ -1243,7 +1243,7 @@ static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes
     if (try_launch_norm_bwd_ragged<T, LN>(p, scratch_bytes, st, &rc)) return rc;
   }
   // general path: rows kernel + column kernel + finalize
-  norm_bwd_rows_general_kernel<T, LN><<<(unsigned)p.rows, 256, 0, st>>>(p);
+  launch_dependent(norm_bwd_rows_general_kernel<T, LN>, (unsigned)p.rows, 256, 0, st, p);
   int rc = launch_status("b200_norm_bwd rows [element-wise]");
   if (rc != B200_OK || !(p.dw || p.db)) return rc;
   const long long plane = (long long)p.n * sizeof(float);
@@ -1252,10 +1252,10 @@ static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes
   if (splits > 64) splits = 64;
   if (splits > p.rows) splits = p.rows;
   p.groups = (int)splits;
-  norm_bwd_cols_general_kernel<T, LN><<<dim3((p.n + 127) / 128, (unsigned)splits), 128, 0, st>>>(p);
+  launch_dependent(norm_bwd_cols_general_kernel<T, LN>, dim3((p.n + 127) / 128, (unsigned)splits), 128, 0, st, p);
   rc = launch_status("b200_norm_bwd cols");
   if (rc != B200_OK) return rc;
-  norm_bwd_finalize_kernel<<<(p.n + 63) / 64, 512, 0, st>>>(p);
+  launch_dependent(norm_bwd_finalize_kernel, (p.n + 63) / 64, 512, 0, st, p);
   return launch_status("b200_norm_bwd finalize");
 }
 

@@ -37,6 +37,7 @@ constexpr int kWarps = 8;  // warps per CTA
 template <typename T, int CH, bool LN, bool DYS>
 __global__ void __launch_bounds__(kWarps * 32, (LN && DYS) ? 3 : 2)
 norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_bytes) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;  // fp32 pairs per vector
   extern __shared__ __align__(128) unsigned char smem[];
@@ -447,10 +448,7 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
   }
   p.groups = (int)grid;
   p.fused = 1;
-  int stages_arg = stages, ring_arg = (int)ring_bytes;
-  void* args[] = {&p, &stages_arg, &ring_arg};
-  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), dim3(kWarps * 32),
-                                  args, smem, st);
+  e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(kWarps * 32), smem, st, p, stages, (int)ring_bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *rc = fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));

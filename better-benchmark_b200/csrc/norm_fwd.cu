@@ -89,6 +89,7 @@ template <typename Tin, typename Tout, int CH, int G, bool GELU, bool RES>
 // GELU -> LayerNorm 112.5 -> 96.8 and 7.6 -> 5.6.
 __global__ void __launch_bounds__(G == 0 ? 512 : 256, (RES && G != 0) ? 3 : 1)
 norm_fwd_resident_kernel(const NormFwdParams p) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   __shared__ float red[64];
   const int lane = glane<G>();
@@ -309,6 +310,7 @@ norm_fwd_resident_kernel(const NormFwdParams p) {
 template <typename Tin, typename Tout, int CH, int G, bool EXACT, bool GELU>
 __global__ void __launch_bounds__(256, 4)
 norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contiguous) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   constexpr int PLANES = V / 4;  // fp32 copies of weight/bias are stored as planes of float4
   extern __shared__ __align__(128) unsigned char smem[];
@@ -594,7 +596,7 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
       *rc = fail((int)e, "b200_norm_fwd: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
       return;
     }
-    kernel<<<(unsigned)grid, threads, smem, st>>>(p, stages, contiguous);
+    launch_dependent(kernel, (unsigned)grid, threads, smem, st, p, stages, contiguous);
     *rc = launch_status("b200_norm_fwd [streaming ring, sub-warp rows]");
   };
 #define B200_NFS(GG, CC)                                                                  \
@@ -646,6 +648,7 @@ __device__ __forceinline__ uint32_t beyond_three(uint32_t a) {
 template <typename T, int CH, bool EXACT, bool BOTH>
 __global__ void __launch_bounds__(kResWarps * 32, 3)
 residual_norm_warp_kernel(const NormFwdParams p, const int stages) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -853,7 +856,7 @@ static bool try_launch_residual_norm_warp(const NormFwdParams& p, cudaStream_t s
       *rc = fail((int)e, "b200_norm_fwd: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
       return;
     }
-    kernel<<<(unsigned)grid, kResWarps * 32, smem, st>>>(p, stages);
+    launch_dependent(kernel, (unsigned)grid, kResWarps * 32, smem, st, p, stages);
     *rc = launch_status("b200_norm_fwd [residual add, warp per row, warp rings]");
   };
   auto pick = [&](auto both_tag) {
@@ -879,6 +882,7 @@ static bool try_launch_residual_norm_warp(const NormFwdParams& p, cudaStream_t s
 // global memory (the second and third sweep of a row that fits in L2 are served from there).
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(1024) norm_fwd_streaming_kernel(const NormFwdParams p) {
+  wait_for_previous_kernel();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const Tin* x = reinterpret_cast<const Tin*>(p.x) + row * p.x_row_stride;
@@ -970,6 +974,7 @@ template <typename Tin, typename Tout, int E, int G>
 // that allows 64 registers, and fp32 rows of 5001 run one CTA per SM instead of two, [4800, 5001] 64.6 -> 101 us.)
 __global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 && sizeof(Tin) == 2 ? 2 : 0)
 norm_fwd_ragged_kernel(const NormFwdParams p) {
+  wait_for_previous_kernel();
   __shared__ float red[64];
   constexpr bool DUAL = std::is_same<Tin, Tout>::value && sizeof(Tin) == 2;
   const int lane = glane<G>(), gs = gsize<G>();
@@ -1088,13 +1093,13 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
   do {                                                                                                      \
     if constexpr (kResBuilt) {                                                                              \
       if (p.res) {                                                                                          \
-        if (p.prologue) norm_fwd_resident_kernel<Tin, Tout, CC, GG, true, true><<<grid, g.threads, 0, st>>>(p); \
-        else norm_fwd_resident_kernel<Tin, Tout, CC, GG, false, true><<<grid, g.threads, 0, st>>>(p);       \
+        if (p.prologue) launch_dependent(norm_fwd_resident_kernel<Tin, Tout, CC, GG, true, true>, grid, g.threads, 0, st, p); \
+        else launch_dependent(norm_fwd_resident_kernel<Tin, Tout, CC, GG, false, true>, grid, g.threads, 0, st, p);       \
         break;                                                                                              \
       }                                                                                                     \
     }                                                                                                       \
-    if (p.prologue) norm_fwd_resident_kernel<Tin, Tout, CC, GG, true, false><<<grid, g.threads, 0, st>>>(p); \
-    else norm_fwd_resident_kernel<Tin, Tout, CC, GG, false, false><<<grid, g.threads, 0, st>>>(p);          \
+    if (p.prologue) launch_dependent(norm_fwd_resident_kernel<Tin, Tout, CC, GG, true, false>, grid, g.threads, 0, st, p); \
+    else launch_dependent(norm_fwd_resident_kernel<Tin, Tout, CC, GG, false, false>, grid, g.threads, 0, st, p);          \
   } while (0)
     if (!g.block) {
       if (p.res) {  // CTAs of 128 threads for the residual kernels (measured: 45.8 -> 44.3 us on the case above)
@@ -1122,23 +1127,23 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
   } else if (p.n <= 16384) {
     set_path_tag(p.res ? "residual add, elements in registers" : "elements in registers");
     if (p.n > 128 && p.n <= 2048 && p.rows <= (p.n <= 512 ? 8LL : 2LL) * device_info().sm_count) {
-      norm_fwd_ragged_kernel<Tin, Tout, 2, 0><<<(unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st>>>(p);
+      launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 2, 0>, (unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st, p);
     } else if (p.n <= 512) {  // a warp per row
       const unsigned grid = (unsigned)((p.rows + 7) / 8);
-      if (p.n <= 64) norm_fwd_ragged_kernel<Tin, Tout, 2, 32><<<grid, 256, 0, st>>>(p);
-      else if (p.n <= 128) norm_fwd_ragged_kernel<Tin, Tout, 4, 32><<<grid, 256, 0, st>>>(p);
-      else if (p.n <= 256) norm_fwd_ragged_kernel<Tin, Tout, 8, 32><<<grid, 256, 0, st>>>(p);
-      else norm_fwd_ragged_kernel<Tin, Tout, 16, 32><<<grid, 256, 0, st>>>(p);
+      if (p.n <= 64) launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 2, 32>, grid, 256, 0, st, p);
+      else if (p.n <= 128) launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 4, 32>, grid, 256, 0, st, p);
+      else if (p.n <= 256) launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 8, 32>, grid, 256, 0, st, p);
+      else launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 16, 32>, grid, 256, 0, st, p);
     } else if (p.n <= 8192) {
       const int threads = ((p.n + 7) / 8 + 31) / 32 * 32;
-      norm_fwd_ragged_kernel<Tin, Tout, 8, 0><<<(unsigned)p.rows, threads, 0, st>>>(p);
+      launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 8, 0>, (unsigned)p.rows, threads, 0, st, p);
     } else {
       const int threads = ((p.n + 15) / 16 + 31) / 32 * 32;
-      norm_fwd_ragged_kernel<Tin, Tout, 16, 0><<<(unsigned)p.rows, threads, 0, st>>>(p);
+      launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 16, 0>, (unsigned)p.rows, threads, 0, st, p);
     }
   } else {
     set_path_tag(p.res ? "residual add, element-wise, CTA per row" : "element-wise, CTA per row");
-    norm_fwd_streaming_kernel<Tin, Tout><<<(unsigned)p.rows, 1024, 0, st>>>(p);
+    launch_dependent(norm_fwd_streaming_kernel<Tin, Tout>, (unsigned)p.rows, 1024, 0, st, p);
   }
   return launch_status("b200_norm_fwd");
 }

@@ -66,6 +66,7 @@ __device__ __forceinline__ Tout convert_scaled(Tin v, float scale, int has_scale
 // sides are 16-byte friendly, so a thread moves VIN = 16 / sizeof(Tin) elements at once.
 template <typename Tin, typename Tout, bool VEC>
 __global__ void __launch_bounds__(256) permute_general_kernel(const PermuteParams p) {
+  wait_for_previous_kernel();
   constexpr int VIN = VEC ? Elem<Tin>::V : 1;
   constexpr int U = VEC ? 4 : 1;  // independent 16-byte loads in flight per thread
   const long long units = p.total / VIN;
@@ -143,6 +144,7 @@ struct TransposeParams {
 
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(256) transpose_tile_kernel(const TransposeParams p) {
+  wait_for_previous_kernel();
   constexpr int TILE = 64;
   __shared__ float tile[TILE][TILE + 1];
   const long long b = blockIdx.z;
@@ -175,6 +177,7 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const TransposePara
 // consecutive input rows, eight words that fall into eight different banks, and splits them into two
 // output vectors with byte permutes: eight consecutive elements of output row 2c and of row 2c + 1.
 __global__ void __launch_bounds__(256) transpose16_tile_kernel(const TransposeParams p) {
+  wait_for_previous_kernel();
   __shared__ __align__(16) uint32_t tile[64][32];
   const long long b = blockIdx.z;
   const long long p0 = (long long)blockIdx.y * 64, c0 = (long long)blockIdx.x * 64;
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(256) transpose16_tile_kernel(const TransposePa
 // Bound by HBM (half of the lines are touched by two CTAs). Measured against 2-byte accesses through a
 // tile of floats: f16 [200, 501, 768] 173.6 -> 82.0 us, [300, 500, 333] 119.1 -> 56.3 us.
 __global__ void __launch_bounds__(256) transpose16_ragged_kernel(const TransposeParams p, const int pairs) {
+  wait_for_previous_kernel();
   __shared__ uint32_t tile[64 * 33];
   const long long b = blockIdx.z;
   const int p0 = (int)blockIdx.y * 64, c0 = (int)blockIdx.x * 64;
@@ -299,6 +303,7 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
                                                               const int stages, const int split, const FastDiv by_tasks,
                                                               const FastDiv by_pairs, const FastDiv by_split,
                                                               const FastDiv by_walk) {
+  wait_for_previous_kernel();
   extern __shared__ __align__(128) unsigned char pairs_smem[];
   const int P = (int)p.P, C = (int)p.C, CW = C / 2;
   const int elems = P * C;
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
 // moved with 16-byte accesses as flat arrays, the transposition is the shared-memory gather in
 // between: output element o = c * P + p comes from [p][c]. A CTA takes matrices b, b + grid, ...
 __global__ void __launch_bounds__(256) transpose_small_kernel(const TransposeParams p, const int pitch) {
+  wait_for_previous_kernel();
   extern __shared__ __align__(16) unsigned char small_smem[];
   uint32_t* tile = reinterpret_cast<uint32_t*>(small_smem);  // [P][pitch]
   const int P = (int)p.P, C = (int)p.C;
@@ -439,6 +445,7 @@ __global__ void __launch_bounds__(256) transpose_small_kernel(const TransposePar
 template <typename Tin, typename Tout, bool VEC, int ACT>
 __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const void* x, void* y, long long n, float scale,
                                                                             int mode_word) {
+  wait_for_previous_kernel();
   const int has_scale = mode_word & 1;
   constexpr int VIN = VEC ? Elem<Tin>::V : 1;
   const long long units = n / VIN;
@@ -520,8 +527,8 @@ template <typename Tin, typename Tout>
 static int launch_permute(const PermuteParams& p, bool vec, cudaStream_t st) {
   const long long units = vec ? p.total / Elem<Tin>::V : p.total;
   set_path_tag(vec ? "vector gather" : "element-wise gather");
-  if (vec) permute_general_kernel<Tin, Tout, true><<<streaming_grid(units), 256, 0, st>>>(p);
-  else permute_general_kernel<Tin, Tout, false><<<streaming_grid(units), 256, 0, st>>>(p);
+  if (vec) launch_dependent(permute_general_kernel<Tin, Tout, true>, streaming_grid(units), 256, 0, st, p);
+  else launch_dependent(permute_general_kernel<Tin, Tout, false>, streaming_grid(units), 256, 0, st, p);
   return launch_status("b200_permute_copy");
 }
 
@@ -561,7 +568,7 @@ static bool try_launch_transpose_pairs(const TransposeParams& p, cudaStream_t st
   const long long groups = (p.batch + group - 1) / group;
   long long grid = groups;
   if (grid > (long long)dev.sm_count * per_sm) grid = (long long)dev.sm_count * per_sm;
-  kernel<<<(unsigned)grid, 256, smem, st>>>(p, group, groups, stages, split, make_fast_div(tasks), make_fast_div(p.C / 2),
+  launch_dependent(kernel, (unsigned)grid, 256, smem, st, p, group, groups, stages, split, make_fast_div(tasks), make_fast_div(p.C / 2),
                                             make_fast_div(split), make_fast_div(p.P / 2 / split));
   *rc = launch_status("b200_transpose_copy [small matrices, word pairs]");
   return true;
@@ -575,7 +582,7 @@ static int launch_transpose(const TransposeParams& p, cudaStream_t st) {
       const bool whole = p.P % 64 == 0 && p.C % 64 == 0 && p.in_row_stride % 8 == 0 && p.in_batch_stride % 8 == 0 &&
                          aligned16(p.x) && aligned16(p.y);
       if (whole) {
-        transpose16_tile_kernel<<<grid, 256, 0, st>>>(p);
+        launch_dependent(transpose16_tile_kernel, grid, 256, 0, st, p);
         return launch_status("b200_transpose_copy [16-byte tiles]");
       }
       int rc = B200_OK;
@@ -583,7 +590,7 @@ static int launch_transpose(const TransposeParams& p, cudaStream_t st) {
       const bool words = p.C % 2 == 0 && p.in_row_stride % 2 == 0 && p.in_batch_stride % 2 == 0 &&
                          (reinterpret_cast<uintptr_t>(p.x) & 3u) == 0;
       if (p.P <= 0x7fffffffLL && p.C <= 0x7fffffffLL) {
-        transpose16_ragged_kernel<<<grid, 256, 0, st>>>(p, words ? 1 : 0);
+        launch_dependent(transpose16_ragged_kernel, grid, 256, 0, st, p, words ? 1 : 0);
         return launch_status("b200_transpose_copy [ragged 16-bit tiles]");
       }
     }
@@ -599,12 +606,12 @@ static int launch_transpose(const TransposeParams& p, cudaStream_t st) {
         long long ctas = p.batch;
         const long long cap = (long long)device_info().sm_count * 8;
         if (ctas > cap) ctas = cap;
-        transpose_small_kernel<<<(unsigned)ctas, 256, smem, st>>>(p, pitch);
+        launch_dependent(transpose_small_kernel, (unsigned)ctas, 256, smem, st, p, pitch);
         return launch_status("b200_transpose_copy [small matrices, flat 16-byte copies]");
       }
     }
   }
-  transpose_tile_kernel<Tin, Tout><<<grid, 256, 0, st>>>(p);
+  launch_dependent(transpose_tile_kernel<Tin, Tout>, grid, 256, 0, st, p);
   return launch_status("b200_transpose_copy [element tiles]");
 }
 
@@ -615,8 +622,8 @@ static int launch_cast(const void* x, void* y, long long n, float scale, int has
   const unsigned grid = streaming_grid(units > 0 ? units : 1, 128);
   auto go = [&](auto act_tag) {
     constexpr int ACT = decltype(act_tag)::value;
-    if (vec) cast_scale_kernel<Tin, Tout, true, ACT><<<grid, 256, 0, st>>>(x, y, n, scale, has_scale);
-    else cast_scale_kernel<Tin, Tout, false, ACT><<<grid, 256, 0, st>>>(x, y, n, scale, has_scale);
+    if (vec) launch_dependent(cast_scale_kernel<Tin, Tout, true, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
+    else launch_dependent(cast_scale_kernel<Tin, Tout, false, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
   };
   switch (has_scale & 14) {
     case 0: go(std::integral_constant<int, 0>{}); break;

@@ -44,6 +44,7 @@ __device__ __forceinline__ void store_scalar(void* out, int dtype, long long idx
 template <typename Tin, typename Op, bool BLOCK, bool VEC>
 __global__ void __launch_bounds__(BLOCK ? 1024 : 256, BLOCK ? 1 : 8)
 row_reduce_kernel(const RowReduceParams p) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   constexpr int U = BLOCK ? 8 : 4;
   __shared__ __align__(8) float red[64];
@@ -170,12 +171,12 @@ static int launch_row_reduce(const RowReduceParams& p, bool vec, cudaStream_t st
   if (warp_mode) {
     const long long grid = (p.rows + 7) / 8;
     if (grid > 0x7fffffffLL) return fail(B200_ERR_UNSUPPORTED, "row_reduce: too many rows");
-    if (vec) row_reduce_kernel<Tin, Op, false, true><<<(unsigned)grid, 256, 0, st>>>(p);
-    else row_reduce_kernel<Tin, Op, false, false><<<(unsigned)grid, 256, 0, st>>>(p);
+    if (vec) launch_dependent(row_reduce_kernel<Tin, Op, false, true>, (unsigned)grid, 256, 0, st, p);
+    else launch_dependent(row_reduce_kernel<Tin, Op, false, false>, (unsigned)grid, 256, 0, st, p);
   } else {
     if (p.rows > 0x7fffffffLL) return fail(B200_ERR_UNSUPPORTED, "row_reduce: too many rows");
-    if (vec) row_reduce_kernel<Tin, Op, true, true><<<(unsigned)p.rows, threads, 0, st>>>(p);
-    else row_reduce_kernel<Tin, Op, true, false><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    if (vec) launch_dependent(row_reduce_kernel<Tin, Op, true, true>, (unsigned)p.rows, threads, 0, st, p);
+    else launch_dependent(row_reduce_kernel<Tin, Op, true, false>, (unsigned)p.rows, threads, 0, st, p);
   }
   return launch_status("b200_row_reduce");
 }

@@ -176,6 +176,7 @@ __device__ __forceinline__ void softmax_finish(f32x2 (&v)[CH][V / 2], float mx, 
 template <typename Tin, typename Tout, int CH, int G, bool PACKED, bool EXACT = false>
 __global__ void __launch_bounds__(G == 0 ? 512 : 256)
 softmax_resident_kernel(const SoftmaxParams p) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   constexpr bool FASTEXP = sizeof(Tout) == 2;
   __shared__ float red[32];
@@ -348,6 +349,7 @@ __device__ __forceinline__ float softmax_logit(const SoftmaxParams& p, const Tin
 // registers, two CTAs of 1024 threads per SM (50 registers: [24576, 5001] 1009 us).
 template <typename Tin, typename Tout, bool PACKED, int E, int G>
 __global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 ? 2 : 0) softmax_ragged_kernel(const SoftmaxParams p) {
+  wait_for_previous_kernel();
   __shared__ float red[32];
   const int lane = glane<G>(), gs = gsize<G>();
   long long row = grow<G>();
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 ? 2 : 0)
 
 template <typename Tin, typename Tout, bool PACKED>
 __global__ void __launch_bounds__(1024) softmax_streaming_kernel(const SoftmaxParams p) {
+  wait_for_previous_kernel();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
@@ -538,6 +541,7 @@ __device__ __forceinline__ void store_shifted(Tout* y, const f32x2 (&o)[V / 2], 
 
 template <typename Tin, typename Tout, int CH, bool CLUSTER>
 __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParams p, const int S) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   constexpr int P = V / 2;
   constexpr int VO = V * (int)sizeof(Tout) <= 16 ? V : 16 / (int)sizeof(Tout);
@@ -758,26 +762,16 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
   if (S == 1) {
     set_path_tag("row in the registers of a CTA, any alignment");
     const unsigned grid = (unsigned)p.rows;
-    if (ch == 8) softmax_rows_kernel<Tin, Tout, 8, false><<<grid, threads, 0, st>>>(p, 1);
-    else if (ch == 4) softmax_rows_kernel<Tin, Tout, 4, false><<<grid, threads, 0, st>>>(p, 1);
-    else softmax_rows_kernel<Tin, Tout, 2, false><<<grid, threads, 0, st>>>(p, 1);
+    if (ch == 8) launch_dependent(softmax_rows_kernel<Tin, Tout, 8, false>, grid, threads, 0, st, p, 1);
+    else if (ch == 4) launch_dependent(softmax_rows_kernel<Tin, Tout, 4, false>, grid, threads, 0, st, p, 1);
+    else launch_dependent(softmax_rows_kernel<Tin, Tout, 2, false>, grid, threads, 0, st, p, 1);
     *rc = launch_status("b200_softmax");
     return true;
   }
   set_path_tag("row in the registers of a cluster, any alignment");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.rows * S));
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)S;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = ch == 8 ? cudaLaunchKernelEx(&cfg, softmax_rows_kernel<Tin, Tout, 8, true>, p, S)
-                                : cudaLaunchKernelEx(&cfg, softmax_rows_kernel<Tin, Tout, 4, true>, p, S);
+  const dim3 grid = dim3((unsigned)(p.rows * S)), block = dim3((unsigned)threads), cluster((unsigned)S, 1, 1);
+  const cudaError_t e = ch == 8 ? launch_clusters(cluster, softmax_rows_kernel<Tin, Tout, 8, true>, grid, block, 0, st, p, S)
+                                : launch_clusters(cluster, softmax_rows_kernel<Tin, Tout, 4, true>, grid, block, 0, st, p, S);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *rc = fail((int)e, "b200_softmax: cluster launch failed: %s", cudaGetErrorString(e));
@@ -812,6 +806,7 @@ __device__ __forceinline__ f32x2 long_row_exp(f32x2 d) {
 
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(1024) softmax_long_kernel(const SoftmaxParams p) {
+  wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   constexpr int P = V / 2;
   constexpr int U = 4;  // vectors in flight per thread
@@ -998,9 +993,9 @@ static int launch_softmax(const SoftmaxParams& p, bool vector_ok, cudaStream_t s
 #define B200_SM_LAUNCH(GG, CC)                                                                   \
   do {                                                                                          \
     if (GG > 0 && p.n / V == (long long)GG * CC)                                                \
-      softmax_resident_kernel<Tin, Tout, CC, GG, PACKED, (GG > 0)><<<grid, g.threads, 0, st>>>(p); \
+      launch_dependent(softmax_resident_kernel<Tin, Tout, CC, GG, PACKED, (GG > 0)>, grid, g.threads, 0, st, p); \
     else                                                                                        \
-      softmax_resident_kernel<Tin, Tout, CC, GG, PACKED, false><<<grid, g.threads, 0, st>>>(p);   \
+      launch_dependent(softmax_resident_kernel<Tin, Tout, CC, GG, PACKED, false>, grid, g.threads, 0, st, p);   \
   } while (0)
       if (g.g == 8) {
         if (g.ch == 1) B200_SM_LAUNCH(8, 1);
@@ -1025,25 +1020,25 @@ static int launch_softmax(const SoftmaxParams& p, bool vector_ok, cudaStream_t s
     threads = (threads + 31) / 32 * 32;
     threads = threads < 128 ? 128 : (threads > 1024 ? 1024 : threads);
     set_path_tag("two sweeps, CTA per row");
-    softmax_long_kernel<Tin, Tout><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    launch_dependent(softmax_long_kernel<Tin, Tout>, (unsigned)p.rows, threads, 0, st, p);
   } else if (p.n <= 8192) {
     set_path_tag("elements in registers");
     if (p.n > 64 && p.n <= 2048 && p.rows <= (p.n <= 512 ? 4LL : 2LL) * device_info().sm_count) {
-      softmax_ragged_kernel<Tin, Tout, PACKED, 2, 0><<<(unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st>>>(p);
+      launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 2, 0>, (unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st, p);
     } else if (p.n <= 512) {
       const unsigned grid = (unsigned)((p.rows + 7) / 8);
-      if (p.n <= 64) softmax_ragged_kernel<Tin, Tout, PACKED, 2, 32><<<grid, 256, 0, st>>>(p);
-      else if (p.n <= 128) softmax_ragged_kernel<Tin, Tout, PACKED, 4, 32><<<grid, 256, 0, st>>>(p);
-      else if (p.n <= 256) softmax_ragged_kernel<Tin, Tout, PACKED, 8, 32><<<grid, 256, 0, st>>>(p);
-      else softmax_ragged_kernel<Tin, Tout, PACKED, 16, 32><<<grid, 256, 0, st>>>(p);
+      if (p.n <= 64) launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 2, 32>, grid, 256, 0, st, p);
+      else if (p.n <= 128) launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 4, 32>, grid, 256, 0, st, p);
+      else if (p.n <= 256) launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 8, 32>, grid, 256, 0, st, p);
+      else launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 16, 32>, grid, 256, 0, st, p);
     } else {
       const int threads = ((p.n + 7) / 8 + 31) / 32 * 32;
-      softmax_ragged_kernel<Tin, Tout, PACKED, 8, 0><<<(unsigned)p.rows, threads, 0, st>>>(p);
+      launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 8, 0>, (unsigned)p.rows, threads, 0, st, p);
     }
   } else {
     const int threads = 1024;
     set_path_tag("element-wise, three passes");
-    softmax_streaming_kernel<Tin, Tout, PACKED><<<(unsigned)p.rows, threads, 0, st>>>(p);
+    launch_dependent(softmax_streaming_kernel<Tin, Tout, PACKED>, (unsigned)p.rows, threads, 0, st, p);
   }
   return launch_status("b200_softmax");
 }
