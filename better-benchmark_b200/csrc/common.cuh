@@ -66,6 +66,7 @@ inline int launch_status(const char* what) {
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
 
 inline int dtype_size(int dt) { return dt == B200_F32 ? 4 : 2; }
 
@@ -197,6 +198,18 @@ __device__ __forceinline__ void st_stream(void* p, const uint4& v) {
                "r"(v.w)
                : "memory");
 #endif
+}
+
+// The same for 32 bytes at a 32-byte boundary: one instruction, and a warp's access is 1 KB of consecutive memory.
+__device__ __forceinline__ void ld_stream32(const void* p, uint4& a, uint4& b) {
+  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+               : "l"(p));
+}
+__device__ __forceinline__ void st_stream32(void* p, const uint4& a, const uint4& b) {
+  asm volatile("st.global.cs.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
 }
 
 __device__ __forceinline__ void st_default(void* p, const uint4& v) {

@@ -438,64 +438,116 @@ __global__ void __launch_bounds__(256) transpose_small_kernel(const TransposePar
   }
 }
 
+// Stores N values as Tout with the widest stores that their alignment (that of N * sizeof(Tout), at most 32 bytes) allows.
+template <typename Tout, int N>
+__device__ __forceinline__ void store_unit(Tout* p, const f32x2 (&o)[N / 2]) {
+  constexpr int BYTES = N * (int)sizeof(Tout);
+  if constexpr (BYTES <= 16) {
+    store_pairs<Tout, N>(p, o);
+  } else {
+    uint32_t w[BYTES / 4];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if constexpr (sizeof(Tout) == 2) {
+        w[i] = Pairs<Tout>::narrow(o[i]);
+      } else {
+        float a, b;
+        unpack2(o[i], a, b);
+        w[2 * i] = __float_as_uint(a);
+        w[2 * i + 1] = __float_as_uint(b);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < BYTES / 32; ++i)
+      st_stream32(reinterpret_cast<char*>(p) + 32 * i, make_uint4(w[8 * i], w[8 * i + 1], w[8 * i + 2], w[8 * i + 3]),
+                  make_uint4(w[8 * i + 4], w[8 * i + 5], w[8 * i + 6], w[8 * i + 7]));
+  }
+}
+
 // Contiguous cast / scale / activation (has_scale: bit 0 multiply by scale; bits 1..3 ReLU, exact GELU, SiLU after it).
 // ACT: the activation bit of the mode word (0: none); the plain cast / scale instantiation carries none of
 // the activations' code (the erf and exp sequences cost registers and instruction-cache lines that a 5 us
 // parameter cast would pay for without using them).
-template <typename Tin, typename Tout, bool VEC, int ACT>
+// BYTES: what a thread loads at once (0: one element). Bound by HBM; SiLU by the SFU pipe (22 us of 35) next to it. Measured,
+// 16 -> 32 bytes: SiLU bf16 [32768, 1536] 37.6 -> 35.0 us (5.75 TB/s), ReLU bf16 of 8 M elements 6.7 -> 6.4, f32 -> bf16 9.2 -> 8.6.
+template <typename Tin, typename Tout, int BYTES, int ACT>
 __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const void* x, void* y, long long n, float scale,
                                                                             int mode_word) {
   wait_for_previous_kernel();
   const int has_scale = mode_word & 1;
-  constexpr int VIN = VEC ? Elem<Tin>::V : 1;
-  const long long units = n / VIN;
+  constexpr int NV = BYTES == 0 ? 1 : BYTES / 16;                // vectors of a unit
+  constexpr int VIN = BYTES == 0 ? 1 : Elem<Tin>::V;             // elements of a vector
+  const long long units = n / (NV * VIN);
   const Tin* src = reinterpret_cast<const Tin*>(x);
   Tout* dst = reinterpret_cast<Tout*>(y);
-  if constexpr (VEC) {
-    // A CTA takes blocks of U * blockDim consecutive vectors (block b, b + grid, ...): its U loads
-    // in flight per thread fall into one contiguous stretch of memory.
-    // GELU and SiLU: two loads and five CTAs per SM (48 registers) instead of four and three - their
+  if constexpr (BYTES != 0) {
+    // A CTA takes blocks of U * blockDim consecutive units (block b, b + grid, ...): what its threads
+    // have in flight falls into one contiguous stretch of memory.
+    // GELU and SiLU: 32 bytes in flight and five CTAs per SM (48 registers) instead of 64 and three - their
     // arithmetic needs the warps more than the loads in flight (SiLU bf16 [32768, 1536] 47.1 -> 42.5 us).
-    constexpr int U = ACT >= 4 ? 2 : 4;
+    // They ask for their next block before they work on the one at hand (40.6 -> 37.6 us).
+    constexpr int U = (ACT >= 4 ? 2 : 4) / NV;
+    constexpr bool AHEAD = ACT >= 4;
     const long long stride = blockDim.x;
-    const long long block = (long long)U * blockDim.x;
-    for (long long u0 = (long long)blockIdx.x * block + threadIdx.x; u0 < units; u0 += (long long)gridDim.x * block) {
-      uint4 raw[U];
+    const long long block = (long long)U * blockDim.x, step = (long long)gridDim.x * block;
+    uint4 next[AHEAD ? U : 1][NV];
+    auto fetch = [&](long long u0, auto& raw) {
 #pragma unroll
       for (int k = 0; k < U; ++k) {
-        const long long u = u0 + k * stride;
-        if (u < units) raw[k] = ld_stream(src + u * VIN);
+        const Tin* p = src + (u0 + k * stride) * (NV * VIN);
+        if (u0 + k * stride < units) {
+          if constexpr (NV == 2) ld_stream32(p, raw[k][0], raw[k][1]);
+          else raw[k][0] = ld_stream(p);
+        }
+      }
+    };
+    const long long first = (long long)blockIdx.x * block + threadIdx.x;
+    if constexpr (AHEAD) fetch(first, next);
+    for (long long u0 = first; u0 < units; u0 += step) {
+      uint4 raw[U][NV];
+      if constexpr (AHEAD) {
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+#pragma unroll
+          for (int v = 0; v < NV; ++v) raw[k][v] = next[k][v];
+        fetch(u0 + step, next);
+      } else {
+        fetch(u0, raw);
       }
 #pragma unroll
       for (int k = 0; k < U; ++k) {
         const long long u = u0 + k * stride;
         if (u < units) {
-          float f[VIN];
-          Elem<Tin>::unpack(raw[k], f);
-          if (has_scale & 1) {
+          f32x2 o[NV * VIN / 2];
 #pragma unroll
-            for (int i = 0; i < VIN; ++i) f[i] = f[i] * scale;
-          }
-          // SiLU: a vector without an element beyond 88 takes the form without clamps (bf16 [32768, 1536],
-          // graph replay: 42.8 us with the clamps on every element, 40.8 us so)
-          bool plain = false;
-          if constexpr (ACT == 8 && sizeof(Tout) == 2) {
-            float largest = fabsf(f[0]);
+          for (int v = 0; v < NV; ++v) {
+            float f[VIN];
+            Elem<Tin>::unpack(raw[k][v], f);
+            if (has_scale & 1) {
 #pragma unroll
-            for (int i = 1; i < VIN; ++i) largest = fmaxf(largest, fabsf(f[i]));
-            plain = largest <= 88.f;
-            if (plain) {
+              for (int i = 0; i < VIN; ++i) f[i] = f[i] * scale;
+            }
+            // SiLU: a vector without an element beyond 88 takes the form without clamps (bf16 [32768, 1536],
+            // graph replay: 42.8 us with the clamps on every element, 40.8 us so)
+            bool plain = false;
+            if constexpr (ACT == 8 && sizeof(Tout) == 2) {
+              float largest = fabsf(f[0]);
+#pragma unroll
+              for (int i = 1; i < VIN; ++i) largest = fmaxf(largest, fabsf(f[i]));
+              plain = largest <= 88.f;
+              if (plain) {
+#pragma unroll
+                for (int i = 0; i < VIN / 2; ++i)
+                  o[v * (VIN / 2) + i] = silu_pair<false>(pack2(f[2 * i], f[2 * i + 1]));
+              }
+            }
+            if (!plain) {
 #pragma unroll
               for (int i = 0; i < VIN / 2; ++i)
-                unpack2(silu_pair<false>(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
+                o[v * (VIN / 2) + i] = apply_activation2<Tout, ACT>(pack2(f[2 * i], f[2 * i + 1]));
             }
           }
-          if (ACT != 0 && !plain) {
-#pragma unroll
-            for (int i = 0; i < VIN / 2; ++i)
-              unpack2(apply_activation2<Tout, ACT>(pack2(f[2 * i], f[2 * i + 1])), f[2 * i], f[2 * i + 1]);
-          }
-          store_converted<Tout, VIN>(dst + u * VIN, f);
+          store_unit<Tout, NV * VIN>(dst + u * (NV * VIN), o);
         }
       }
     }
@@ -504,14 +556,14 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const
          u += (long long)gridDim.x * blockDim.x)
       dst[u] = convert_scaled<Tin, Tout, ACT>(src[u], scale, has_scale);
   }
-  if constexpr (VEC) {  // ragged tail
-    const long long done = units * VIN;
+  if constexpr (BYTES != 0) {  // ragged tail
+    const long long done = units * (NV * VIN);
     const long long t = done + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) dst[t] = convert_scaled<Tin, Tout, ACT>(src[t], scale, has_scale);
   }
 }
 
-// Grid of the flat streaming kernels: one CTA per 256 units up to `per_sm` CTAs per SM, which then
+// Grid of the flat streaming kernels: one CTA per 256 units (the caller counts a block of several per thread as 256) up to `per_sm` CTAs per SM, which then
 // loop. Many small CTAs keep the window of addresses that are in flight at any moment narrow; for
 // the cast kernel 128 per SM measured best on a 262 M-element bf16 -> f32 cast (8: 331 us, 16: 299,
 // 32: 279, 64: 268, 128: 263, 256: 285, one CTA per block: 331). B200_STREAM_CTAS_PER_SM overrides both.
@@ -617,13 +669,21 @@ static int launch_transpose(const TransposeParams& p, cudaStream_t st) {
 
 template <typename Tin, typename Tout>
 static int launch_cast(const void* x, void* y, long long n, float scale, int has_scale, bool vec, cudaStream_t st) {
-  const long long units = vec ? n / Elem<Tin>::V : n;
-  set_path_tag(vec ? "vector" : "element-wise");
-  const unsigned grid = streaming_grid(units > 0 ? units : 1, 128);
+  constexpr int V = Elem<Tin>::V;
+  // 32 bytes a thread from 4096 units on, where that still makes 16 CTAs (SiLU bf16 of 1000 elements: 1.43 us, with
+  // 32 bytes 1.84; of 65 536: 1.97 and 1.90)
+  const bool wide = vec && aligned32(x) && aligned32(y) && n >= 4096 * 2 * V;
+  const long long units = wide ? n / (2 * V) : (vec ? n / V : n);
+  set_path_tag(wide ? "vector, 32 bytes" : (vec ? "vector" : "element-wise"));
   auto go = [&](auto act_tag) {
     constexpr int ACT = decltype(act_tag)::value;
-    if (vec) launch_dependent(cast_scale_kernel<Tin, Tout, true, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
-    else launch_dependent(cast_scale_kernel<Tin, Tout, false, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
+    // GELU and SiLU: 20 CTAs per SM, four times what is resident (SiLU bf16 [32768, 1536]: 5 per SM 36.3 us, 10 35.6, 20 35.0)
+    const long long per_cta = 256LL * (ACT >= 4 ? 2 : 4) / (wide ? 2 : 1);
+    const long long blocks = vec ? (units + per_cta - 1) / per_cta : (units + 255) / 256;
+    const unsigned grid = streaming_grid(256 * (blocks > 0 ? blocks : 1), ACT >= 4 && vec ? 20 : 128);
+    if (wide) launch_dependent(cast_scale_kernel<Tin, Tout, 32, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
+    else if (vec) launch_dependent(cast_scale_kernel<Tin, Tout, 16, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
+    else launch_dependent(cast_scale_kernel<Tin, Tout, 0, ACT>, grid, 256, 0, st, x, y, n, scale, has_scale);
   };
   switch (has_scale & 14) {
     case 0: go(std::integral_constant<int, 0>{}); break;

@@ -222,6 +222,24 @@ def test_activations_do_not_depend_on_position_or_alignment(dtype, out, activati
             assert torch.equal(run(x[start:].clone()[:n]), want[start:start + n]), (start, n)
 
 
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.float32), (torch.float32, torch.float16), (torch.float16, torch.float16),
+                                       (torch.float32, torch.float32)])
+@pytest.mark.parametrize("activation", [None, "relu", "silu"])
+def test_casts_on_both_sides_of_the_32_byte_path(dtype, out, activation):
+    """Lengths around its smallest size (4096 units) with every kind of rest, starts on 32-, 16- and 2- or 4-byte boundaries."""
+    unit = 32 // dtype.itemsize
+    x = _randn((400000,), dtype, 3, 2.0)
+    for n in (4096 * unit - 1, 4096 * unit, 4096 * unit + 1, 4099 * unit - 1, 399000):
+        for start in (0, unit // 2, 1):
+            t = x[start:start + n]
+            got = _kernels().cast_scale(t, out, activation=activation)
+            if activation == "silu":
+                d = t.double()
+                _near(got, d * torch.sigmoid(d), f"silu {n} {start}", floor=1.2e-7)
+            else:
+                assert torch.equal(got, (torch.relu(t) if activation else t).to(out)), (n, start)
+
+
 @pytest.mark.parametrize("dtype,n,c,hw", [(torch.bfloat16, 1001, 92, 196), (torch.bfloat16, 336, 92, 196),
                                           (torch.float32, 80, 485, 256), (torch.bfloat16, 64, 1022, 49)])
 def test_batch_norm_takes_the_same_path_with_the_advertised_scratch(dtype, n, c, hw):
