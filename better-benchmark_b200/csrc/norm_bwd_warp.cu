@@ -71,44 +71,19 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     bulk_load(dst, xg + row * p.x_row_stride, row_bytes, &full[slot]);
     if constexpr (!DYS) bulk_load(dst + row_bytes, dyg + row * p.dy_row_stride, row_bytes, &full[slot]);
   };
-  // a warp's first rows are on their way before the weights are staged; the other lanes first touch
-  // the barriers after the __syncthreads below
-  int issued = 0;
-  if (lane == 0) {
-    for (; issued < my_rows && issued < stages; ++issued) issue(issued, issued);
-  }
-  issued = __shfl_sync(0xffffffffu, issued, 0);
-  const f32x2 dy_all = splat2(DYS ? Elem<T>::to_f32(__ldg(dyg)) : 0.f);
-
-  // weight slice: registers (RMSNorm) or shared memory (LayerNorm, which already keeps two
-  // gradient sums per column in registers)
-  f32x2 wv[LN ? 1 : CH][P];
+  // The weights are asked for before the first rows (behind the copies of all CTAs, 60 MB, they took 4.7 us to arrive, and
+  // no row is worked on without them), and staged after the rows have been asked for.
+  static_assert(CH * 32 <= kWarps * 32, "a thread stages one vector of the row");
+  float wf_first[LN ? V : 1];
+  f32x2 wv[LN ? 1 : CH][P];  // RMSNorm: the lane's slice of the weight
   if constexpr (LN) {
-    // layout [vector slot c][pair i][lane] of fp32 pairs: the 32 lanes of a warp read 32 consecutive
-    // 8-byte words, one shared-memory wavefront without bank conflicts
-    for (int q = threadIdx.x; q < CH * 32; q += blockDim.x) {  // q = c * 32 + lane: vector q of the row
-      float wf[V];
-      if (p.w && q < nv) {
-        load_param<V>(p.w, p.w_dtype, (long long)q * V, wf);
-      } else {
 #pragma unroll
-        for (int i = 0; i < V; ++i) wf[i] = 1.f;
-      }
-      if constexpr (DYS) {  // one dy for the whole tensor: g = dy * w does not depend on the row
-        const float dyf = Elem<T>::to_f32(__ldg(dyg));
-#pragma unroll
-        for (int i = 0; i < V; ++i) wf[i] = __fmul_rn(dyf, wf[i]);
-      }
-      const int c = q >> 5, l = q & 31;
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        wsm[((c * P + i) * 32 + l) * 2] = wf[2 * i];
-        wsm[((c * P + i) * 32 + l) * 2 + 1] = wf[2 * i + 1];
-      }
-    }
+    for (int i = 0; i < V; ++i) wf_first[i] = 1.f;
+    if (p.w && (int)threadIdx.x < nv) load_param<V>(p.w, p.w_dtype, (long long)threadIdx.x * V, wf_first);
 #pragma unroll
     for (int i = 0; i < P; ++i) wv[0][i] = splat2(0.f);
   } else {
+    wf_first[0] = 0.f;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       const int j = c * 32 + lane;
@@ -121,6 +96,31 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
       }
 #pragma unroll
       for (int i = 0; i < P; ++i) wv[c][i] = pack2(wf[2 * i], wf[2 * i + 1]);
+    }
+  }
+  const float dyf = DYS ? Elem<T>::to_f32(__ldg(dyg)) : 0.f;
+  // the other lanes first touch the barriers after the __syncthreads below
+  int issued = 0;
+  if (lane == 0) {
+    for (; issued < my_rows && issued < stages; ++issued) issue(issued, issued);
+  }
+  issued = __shfl_sync(0xffffffffu, issued, 0);
+  const f32x2 dy_all = splat2(dyf);
+
+  // LayerNorm keeps its weight slice in shared memory (it already keeps two gradient sums per column in
+  // registers), in a layout [vector slot c][pair i][lane] of fp32 pairs: the 32 lanes of a warp read 32 consecutive
+  // 8-byte words, one shared-memory wavefront without bank conflicts
+  if constexpr (LN) {
+    if (threadIdx.x < CH * 32) {  // slot `warp`, lane `lane`
+      if constexpr (DYS) {  // one dy for the whole tensor: g = dy * w does not depend on the row
+#pragma unroll
+        for (int i = 0; i < V; ++i) wf_first[i] = __fmul_rn(dyf, wf_first[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        wsm[((warp * P + i) * 32 + lane) * 2] = wf_first[2 * i];
+        wsm[((warp * P + i) * 32 + lane) * 2 + 1] = wf_first[2 * i + 1];
+      }
     }
   }
   __syncthreads();  // barriers initialised (seen by every lane), weight slice in place
@@ -352,8 +352,9 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   __syncthreads();  // every warp is done with its rows (or gave up, with no copy in flight)
   const bool any_failed = cta_failed != 0;
   if (!any_failed && (p.dw || p.db)) {
-    float* fold_w = reinterpret_cast<float*>(smem);   // [kWarps][n]
-    float* fold_b = fold_w + (size_t)kWarps * p.n;    // [kWarps][n]
+    // [kWarps][CH][P][32] fp32 pairs for dw, then the same for db: a lane's pair at the lane's place, no bank conflicts
+    constexpr int kPlane = CH * P * 32;
+    f32x2* fold = reinterpret_cast<f32x2*>(smem);
     if constexpr (LN && DYS) {
 #pragma unroll
       for (int c = 0; c < CH; ++c) {
@@ -366,33 +367,30 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     }
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      const int j = c * 32 + lane;
-      if (j < nv) {
-        float* dw = fold_w + (size_t)warp * p.n + (size_t)j * V;
 #pragma unroll
-        for (int i = 0; i < P; ++i) unpack2(acc_w[c][i], dw[2 * i], dw[2 * i + 1]);
-        if constexpr (LN) {
-          float* db = fold_b + (size_t)warp * p.n + (size_t)j * V;
-#pragma unroll
-          for (int i = 0; i < P; ++i) unpack2(acc_b[c][i], db[2 * i], db[2 * i + 1]);
-        }
+      for (int i = 0; i < P; ++i) {
+        fold[warp * kPlane + (c * P + i) * 32 + lane] = acc_w[c][i];
+        if constexpr (LN) fold[(kWarps + warp) * kPlane + (c * P + i) * 32 + lane] = acc_b[c][i];
       }
     }
     __syncthreads();
-    float* pw = p.partials + (long long)blockIdx.x * p.n;
-    float* pb = p.partials + ((long long)p.groups + blockIdx.x) * p.n;
-    for (int c = threadIdx.x; c < p.n; c += blockDim.x) {
-      float a = fold_w[c];
+    // four columns a thread at a time
+    for (int q = threadIdx.x; q < (LN ? 2 : 1) * kPlane / 2; q += blockDim.x) {
+      const int l = q & 31, unit = q >> 5;  // unit = (plane * CH + c) * (P / 2) + h
+      const int h = unit % (P / 2), pc = unit / (P / 2), plane = pc / CH, c = pc - plane * CH;
+      const int col = (c * 32 + l) * V + 4 * h;
+      if (col < p.n && (plane == 0 || p.db)) {
+        const f32x2* src = fold + plane * kWarps * kPlane + (c * P + 2 * h) * 32 + l;
+        f32x2 lo = src[0], hi = src[32];
 #pragma unroll
-      for (int g = 1; g < kWarps; ++g) a += fold_w[(size_t)g * p.n + c];
-      pw[c] = a;
-      if constexpr (LN) {
-        if (p.db) {
-          float b = fold_b[c];
-#pragma unroll
-          for (int g = 1; g < kWarps; ++g) b += fold_b[(size_t)g * p.n + c];
-          pb[c] = b;
+        for (int g = 1; g < kWarps; ++g) {
+          lo = add2(lo, src[g * kPlane]);
+          hi = add2(hi, src[g * kPlane + 32]);
         }
+        float4 out;
+        unpack2(lo, out.x, out.y);
+        unpack2(hi, out.z, out.w);
+        *reinterpret_cast<float4*>(p.partials + ((long long)plane * p.groups + blockIdx.x) * p.n + col) = out;
       }
     }
     __syncthreads();  // the fold area doubles as the fp64 area of the finalize
@@ -413,8 +411,8 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
   const size_t stage_bytes = (DYS ? 1 : 2) * (size_t)nv * 16;
   // barriers (+ fp32 weight slots; a second table of the same size for LayerNorm with a scalar dy)
   const size_t fixed = kWarps * 8 * sizeof(uint64_t) + (LN ? (size_t)(DYS ? 2 : 1) * CH * 32 * V * sizeof(float) : 0);
-  // the ring doubles as the fold area [2][kWarps][n] fp32 and as the fp64 area of the finalize
-  size_t floor_bytes = 2 * (size_t)kWarps * p.n * sizeof(float);
+  // the ring doubles as the fold area [2][kWarps][CH * 32 * V] fp32 and as the fp64 area of the finalize
+  size_t floor_bytes = 2 * (size_t)kWarps * CH * 32 * V * sizeof(float);
   if (floor_bytes < 16 * 64 * sizeof(double)) floor_bytes = 16 * 64 * sizeof(double);
   int stages = 0, ctas_per_sm = (LN && DYS) ? 3 : 2;  // the scalar-dy LayerNorm form needs fewer registers
   for (; ctas_per_sm >= 1; --ctas_per_sm) {

@@ -351,6 +351,14 @@ norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contig
   // Thread 0 sets up the stage barriers and starts the first copies at once, before the CTA
   // converts weight and bias: HBM traffic begins with the CTA instead of after its prologue. (The
   // other threads first touch a barrier after the __syncthreads below.)
+  float wf[V], bf[V];
+  auto fetch_params = [&](int j) {
+    if (p.w && j < nv) load_param<V>(p.w, p.w_dtype, (long long)j * V, wf);
+    if (p.b && j < nv) load_param<V>(p.b, p.w_dtype, (long long)j * V, bf);
+  };
+  // Weight and bias are asked for first: behind the first copies of all CTAs (30 MB) they took 4 us to arrive, and no
+  // row is worked on before they are there.
+  fetch_params(threadIdx.x);
   int issued = 0;
   int issue_slot = 0;  // stage the next copy goes to
   if (threadIdx.x == 0) {
@@ -361,18 +369,12 @@ norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contig
   }
 
   for (int j = threadIdx.x; j < nv; j += blockDim.x) {
-    float f[V];
-    if (p.w) {
-      load_param<V>(p.w, p.w_dtype, (long long)j * V, f);
+    if (j != threadIdx.x) fetch_params(j);
 #pragma unroll
-      for (int q = 0; q < PLANES; ++q)
-        *reinterpret_cast<float4*>(wsm + ((size_t)q * nv + j) * 4) = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
-    }
-    if (p.b) {
-      load_param<V>(p.b, p.w_dtype, (long long)j * V, f);
-#pragma unroll
-      for (int q = 0; q < PLANES; ++q)
-        *reinterpret_cast<float4*>(bsm + ((size_t)q * nv + j) * 4) = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+    for (int q = 0; q < PLANES; ++q) {
+      const size_t at = ((size_t)q * nv + j) * 4;
+      if (p.w) *reinterpret_cast<float4*>(wsm + at) = make_float4(wf[4 * q], wf[4 * q + 1], wf[4 * q + 2], wf[4 * q + 3]);
+      if (p.b) *reinterpret_cast<float4*>(bsm + at) = make_float4(bf[4 * q], bf[4 * q + 1], bf[4 * q + 2], bf[4 * q + 3]);
     }
   }
   __syncthreads();
