@@ -47,22 +47,28 @@ struct RowMap {
   FastDiv d1, d2;
 };
 
-inline RowMap make_row_map(const int64_t* strides, long long d1, long long d2) {
-  RowMap m;
-  m.s0 = strides[0];
-  m.s1 = strides[1];
-  m.s2 = strides[2];
-  m.d1 = make_fast_div(d1);
-  m.d2 = make_fast_div(d2);
-  return m;
-}
-
 inline RowMap make_row_map_flat(long long row_stride) {
   RowMap m;
   m.s0 = row_stride;
   m.s1 = m.s2 = 0;
   m.d1 = make_fast_div(1);
   m.d2 = make_fast_div(1);
+  return m;
+}
+
+// A tensor whose rows lie at one distance gets the flat map although the call has several outer dimensions (another
+// operand, a broadcast mask, needs them): its loads then start without the divisions (softmax_resident_kernel).
+inline RowMap make_row_map(const int64_t* strides, long long d1, long long d2) {
+  if (d1 == 1 && d2 == 1) return make_row_map_flat(strides[0]);
+  if (d2 == 1 && strides[0] == strides[1] * d1) return make_row_map_flat(strides[1]);
+  if (d1 == 1 && strides[0] == strides[2] * d2) return make_row_map_flat(strides[2]);
+  if (strides[1] == strides[2] * d2 && strides[0] == strides[1] * d1) return make_row_map_flat(strides[2]);
+  RowMap m;
+  m.s0 = strides[0];
+  m.s1 = strides[1];
+  m.s2 = strides[2];
+  m.d1 = make_fast_div(d1);
+  m.d2 = make_fast_div(d2);
   return m;
 }
 

@@ -513,6 +513,22 @@ def test_softmax_rows_over_strided_outer_dimensions(dtype, n):
             _near(got, torch.softmax(rows.double(), -1), f"strided softmax {tuple(rows.shape)}", floor=1e-7)
 
 
+@pytest.mark.parametrize("mask_shape", [(1, 1, 1), (4, 1, 1), (1, 3, 1), (1, 1, 5), (4, 1, 5), (4, 3, 1), (1, 3, 5), (4, 3, 5)])
+@pytest.mark.parametrize("n", [64, 100, 1000])
+def test_softmax_of_every_broadcast_mask_and_outer_order(n, mask_shape):
+    """Rows at one distance take a flat map beside operands that need several dimensions: x contiguous, with gaps in each
+    outer dimension, and with its outer dimensions in another order; every row has the bits of the expanded call."""
+    k = _kernels()
+    m = _randn((*mask_shape, n), torch.float16, n)
+    big = _randn((8, 6, 10, n), torch.float16, n + 1, 2.0)
+    forms = (big[:4, :3, :5].contiguous(), big[::2, :3, :5], big[:4, ::2, :5], big[:4, :3, ::2],
+             big[:5, :3, :4].permute(2, 1, 0, 3), big[:3, :4, :5].permute(1, 0, 2, 3))
+    for x in forms:
+        want = k.softmax(x.contiguous().view(60, n), mask=m.expand(4, 3, 5, n).contiguous().view(60, n), scale=0.5)
+        assert torch.equal(k.softmax(x, mask=m, scale=0.5).reshape(60, n), want), (mask_shape, x.stride())
+        assert torch.equal(k.row_reduce(x, "sum").reshape(60), k.row_reduce(x.contiguous().view(60, n), "sum"))
+
+
 def test_transpose_of_small_matrices_with_gaps_between_them():
     """The batch stride is not rows * columns: one matrix per block."""
     k = _kernels()
