@@ -455,9 +455,12 @@ __global__ void __launch_bounds__(1024) softmax_streaming_kernel(const SoftmaxPa
 //     of four bytes). The outputs of a thread's vector are handed over by warp shuffles to where the
 //     next aligned chunk of the output starts, so stores are whole chunks; only a warp's first and
 //     last elements leave one by one.
-// Bound by HBM: the exponentials cost 18 us of the SFU pipe on the case below, the traffic 75 us.
-// Measured: bf16 [4096, 20005] (rows 20 008 apart) -> fp32 log_softmax 183.7 us with the two-sweep
-// kernel below, 109 us (4.5 TB/s) here; bf16 [2000, 32001] softmax 192.6 -> 57.6 us.
+// What bounds it: issue slots next to HBM (on the case below the traffic takes 75 us and the instructions about as long), with
+// three CTAs per SM that load, reduce twice and store; scale and log are template parameters, and nothing is clamped
+// unless a difference is infinite. Measured: bf16 [4096, 20005] (rows 20 008 apart) -> fp32 log_softmax 183.7 us with the
+// two-sweep kernel below, 109 us with run-time switches and clamps, 103 here; bf16 [2000, 32001] softmax 192.6 -> 54.6 us.
+// Not taken: the next row brought in by a bulk copy meanwhile (121 us: the loads are not what it waits for), stores
+// whose shift is known at compile time (98.6 us where these take 95.8, rows 20 005 apart).
 // ----------------------------------------------------------------------------------------------
 // Stores a thread's V outputs, the first of which goes to `y`. `shift` (warp-uniform, below the chunk
 // length VO) counts the elements from y to the next chunk boundary of the output; the lane above
@@ -542,7 +545,7 @@ __device__ __forceinline__ void store_shifted(Tout* y, const f32x2 (&o)[V / 2], 
   }
 }
 
-template <typename Tin, typename Tout, int CH, bool CLUSTER>
+template <typename Tin, typename Tout, int CH, bool CLUSTER, bool SCALED, bool LOG>
 __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParams p, const int S) {
   wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
@@ -557,7 +560,6 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   const int rank = CLUSTER ? (int)(blockIdx.x % (unsigned)S) : 0;
   const long long row = CLUSTER ? (long long)(blockIdx.x / (unsigned)S) : (long long)blockIdx.x;
   const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
-  Tout* y = reinterpret_cast<Tout*>(p.y) + row_offset(p.ymap, row);
 
   // body: whole vectors from the first 16-byte boundary on; edge: what is in front of it and behind it
   int head = (int)(((16u - (unsigned)(reinterpret_cast<uintptr_t>(x) & 15u)) & 15u) / sizeof(Tin));
@@ -569,24 +571,24 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   const int v0 = CLUSTER ? rank * per : 0;
   const int cnt = nvec - v0 < per ? nvec - v0 : per;  // vectors of this CTA (may be negative: none)
   const Tin* xb = x + head + (long long)v0 * V;
-  Tout* yb = y + head + (long long)v0 * V;
 
   uint4 raw[CH];
 #pragma unroll
   for (int c = 0; c < CH; ++c)
     if (c * T_ + tid < cnt) raw[c] = ld_stream(xb + (long long)(c * T_ + tid) * V);
+  Tout* y = reinterpret_cast<Tout*>(p.y) + row_offset(p.ymap, row);
+  Tout* yb = y + head + (long long)v0 * V;
   const bool has_edge = rank == 0 && tid < edges;
   const int edge_at = tid < head ? tid : tail0 + (tid - head);
   const f32x2 scale2 = splat2(p.scale);
-  const bool scaled = p.has_scale != 0;
   float edge = -INFINITY;
   if (has_edge) {
     edge = Elem<Tin>::to_f32(x[edge_at]);
-    if (scaled) edge = edge * p.scale;
+    if constexpr (SCALED) edge = edge * p.scale;
   }
   auto logits = [&](int c, f32x2 (&t)[P]) {
     Pairs<Tin>::unpack(raw[c], t);
-    if (scaled) {
+    if constexpr (SCALED) {
 #pragma unroll
       for (int i = 0; i < P; ++i) t[i] = mul2(t[i], scale2);
     }
@@ -594,25 +596,20 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
 
   // ---- maximum (a NaN anywhere makes it NaN) ------------------------------------------------------
   float m = edge;
-  bool in_fp32 = true;
-  if constexpr (sizeof(Tin) == 2) {
-    if (!scaled) {  // a maximum is exact in the input type: packed pairs, no conversion
-      using P2 = typename Pair<Tin>::type;
-      P2 m2 = Pair<Tin>::splat(-INFINITY);
+  if constexpr (sizeof(Tin) == 2 && !SCALED) {  // a maximum is exact in the input type: packed pairs, no conversion
+    using P2 = typename Pair<Tin>::type;
+    P2 m2 = Pair<Tin>::splat(-INFINITY);
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        if (c * T_ + tid < cnt) {
-          const uint32_t w[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+    for (int c = 0; c < CH; ++c) {
+      if (c * T_ + tid < cnt) {
+        const uint32_t w[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
 #pragma unroll
-          for (int i = 0; i < 4; ++i) m2 = MaxOp::apply2(m2, *reinterpret_cast<const P2*>(&w[i]));
-        }
+        for (int i = 0; i < 4; ++i) m2 = MaxOp::apply2(m2, *reinterpret_cast<const P2*>(&w[i]));
       }
-      const float2 f = Pair<Tin>::widen(m2);
-      m = MaxOp::apply(m, MaxOp::apply(f.x, f.y));
-      in_fp32 = false;
     }
-  }
-  if (in_fp32) {
+    const float2 f = Pair<Tin>::widen(m2);
+    m = MaxOp::apply(m, MaxOp::apply(f.x, f.y));
+  } else {
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (c * T_ + tid < cnt) {
@@ -630,14 +627,10 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   float M = block_reduce<MaxOp>(m, red);
 
   // ---- sum of the exponentials --------------------------------------------------------------------
-  // fp32 results sum expf, log_softmax too: the compensated exponential would take 102 us instead of 109 on bf16
-  // [4096, 20005] -> fp32, but its errors have a mean of -4e-8, which the sum keeps (mean error of the
-  // log-probabilities of 1003 standard normals times two +2.7e-8, against -1.3e-8).
-  const bool log_mode = p.log_mode != 0;
-  auto difference = [&](f32x2 t, f32x2 M2) {
+  auto clamped = [&](f32x2 d) {  // a NaN is lost here: the maximum has caught it
     float a, b;
-    unpack2(sub2(t, M2), a, b);
-    return pack2(fmaxf(a, kFloor), fmaxf(b, kFloor));  // a NaN is lost here: the maximum has caught it
+    unpack2(d, a, b);
+    return pack2(fmaxf(a, kFloor), fmaxf(b, kFloor));
   };
   auto exp_exact = [](f32x2 d) {
     float a, b;
@@ -645,26 +638,36 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
     return pack2(expf(a), expf(b));
   };
   auto add_up = [&](auto exponential) {
-    const f32x2 M2 = splat2(M);
+    const f32x2 own = splat2(M);
     f32x2 sum = splat2(0.f);
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (c * T_ + tid < cnt) {
         f32x2 t[P];
         logits(c, t);
-        f32x2 part = exponential(difference(t[0], M2));
+        f32x2 part = exponential(sub2(t[0], own));
 #pragma unroll
-        for (int i = 1; i < P; ++i) part = add2(part, exponential(difference(t[i], M2)));
+        for (int i = 1; i < P; ++i) part = add2(part, exponential(sub2(t[i], own)));
         sum = add2(sum, part);
       }
     }
-    float s = hsum2(sum);
-    if (has_edge) s += expf(fmaxf(edge - M, kFloor));
-    return s;
+    return hsum2(sum);
   };
+  // fp32 results sum expf, log_softmax too: the errors of the pair exponential have a mean of -4e-8, which the sum
+  // keeps (mean error of the log-probabilities of 1003 standard normals times two +2.7e-8, against -1.3e-8; without that
+  // mean it would take 4 % less, with errors up to 2 % larger in some cases and smaller in others). expf takes infinite
+  // differences as they are; the pair exponential does not: a thread whose sum is not a number takes its elements
+  // again with a floor under them.
   float s;
-  if (sizeof(Tout) == 2) s = add_up([](f32x2 d) { return exp_pair_compensated(d); });
-  else s = add_up(exp_exact);
+  bool finite = true;
+  if constexpr (sizeof(Tout) == 4) {
+    s = add_up(exp_exact);
+  } else {
+    s = add_up([](f32x2 d) { return exp_pair_compensated(d); });
+    finite = s == s;
+    if (!finite) s = add_up([&](f32x2 d) { return exp_pair_compensated(clamped(d)); });
+  }
+  if (has_edge) s += expf(fmaxf(edge - M, kFloor));
   float sum = block_reduce<SumOp>(s, red);
   if constexpr (CLUSTER) {
     namespace cg = cooperative_groups;
@@ -692,33 +695,45 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   const f32x2 M2 = splat2(M), log_sum2 = splat2(log_sum), inv2 = splat2(inv);
   const int shift = (int)(((0u - (unsigned)reinterpret_cast<uintptr_t>(yb)) & (VO * (unsigned)sizeof(Tout) - 1u)) /
                           sizeof(Tout));
+  auto store_all = [&](auto plain_tag) {
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int j = c * T_ + tid;
-    if (j - lane >= cnt) break;  // warp-uniform: no lane of this warp has a vector here
-    f32x2 t[P], o[P];
-    const bool valid = j < cnt;
-    if (!valid) raw[c] = make_uint4(0u, 0u, 0u, 0u);
-    logits(c, t);
-    if (log_mode) {
+    for (int c = 0; c < CH; ++c) {
+      const int j = c * T_ + tid;
+      if (j - lane >= cnt) break;  // warp-uniform: no lane of this warp has a vector here
+      f32x2 t[P], o[P];
+      const bool valid = j < cnt;
+      if (!valid) raw[c] = make_uint4(0u, 0u, 0u, 0u);
+      logits(c, t);
+      if constexpr (LOG) {
 #pragma unroll
-      for (int i = 0; i < P; ++i) o[i] = sub2(sub2(t[i], M2), log_sum2);
-    } else if constexpr (sizeof(Tout) == 4) {
+        for (int i = 0; i < P; ++i) o[i] = sub2(sub2(t[i], M2), log_sum2);
+      } else if constexpr (sizeof(Tout) == 4) {
 #pragma unroll
-      for (int i = 0; i < P; ++i) {
-        float a, b;
-        unpack2(exp_exact(difference(t[i], M2)), a, b);
-        o[i] = pack2(a / sum, b / sum);
+        for (int i = 0; i < P; ++i) {
+          float a, b;
+          unpack2(exp_exact(sub2(t[i], M2)), a, b);
+          o[i] = pack2(a / sum, b / sum);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          const f32x2 d = sub2(t[i], M2);
+          o[i] = mul2(exp_pair_compensated(decltype(plain_tag)::value ? d : clamped(d)), inv2);
+        }
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < P; ++i) o[i] = mul2(exp_pair_compensated(difference(t[i], M2)), inv2);
+      store_shifted<Tout, V>(yb + (long long)j * V, o, shift, lane, valid, lane < 31 && j + 1 < cnt);
     }
-    store_shifted<Tout, V>(yb + (long long)j * V, o, shift, lane, valid, lane < 31 && j + 1 < cnt);
+  };
+  if constexpr (sizeof(Tout) == 2 && !LOG) {
+    // the differences of the sum were finite; in a cluster they were taken from another maximum
+    if (!CLUSTER && __all_sync(0xffffffffu, finite)) store_all(std::true_type{});
+    else store_all(std::false_type{});
+  } else {
+    store_all(std::true_type{});
   }
   if (has_edge) {
     float o;
-    if (log_mode) {
+    if constexpr (LOG) {
       o = (edge - M) - log_sum;
     } else {
       const float e = expf(fmaxf(edge - M, kFloor));
@@ -731,7 +746,9 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
 // How many CTAs share a row of nvec whole vectors; 0: the two-sweep kernel below takes it. `aligned`: every row
 // starts and ends on the 16-byte grid, on both sides.
 //   * As few as hold the row: 64 registers a thread keep 8 vectors and what is computed from them, 512 threads 4096
-//     vectors, and a cluster has at most 8 CTAs everywhere. From 8192 vectors on all 8, whose 256 threads fit an
+//     vectors, and a cluster has at most 8 CTAs everywhere. fp32 log-probabilities of 16-bit rows go to two CTAs from 2560
+//     vectors on, where only two CTAs fit an SM (bf16 [2000, 30001] 89.1 -> 79.6 us, [2000, 21001] 62.1 -> 59.1; probabilities
+//     of the same rows 92.5 -> 98.5, 16-bit results 52.0 -> 59.0). From 8192 vectors on all 8, whose 256 threads fit an
 //     SM four times (bf16 [1024, 131075]: 4 CTAs 193 us, 8 CTAs 182, two sweeps 317).
 //   * No more than half as many rows as SMs: 8 CTAs once a row has 1024 vectors (bf16 [8, 131072] 7.4 us, two
 //     sweeps 17.6; [64, 65536] 9.4 and 12.3; [16, 20005] 4.8, one CTA 5.7; f32 [16, 4099] 4.4 and 5.6).
@@ -750,7 +767,7 @@ static int softmax_ctas_per_row(long long nvec, long long rows, bool aligned, bo
     if (sizeof(Tin) == 4 && nvec > 16384) return 0;
     return 8;
   }
-  return nvec > 4096 ? 2 : 1;
+  return nvec > (log_mode && sizeof(Tin) == 2 && sizeof(Tout) == 4 ? 2560 : 4096) ? 2 : 1;
 }
 
 // Returns false when the two-sweep kernel is to take the rows.
@@ -762,22 +779,23 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
   const long long per = (nvec + S - 1) / S;
   const int ch = per > 512 ? 8 : (per > 128 || S > 1 ? 4 : 2);
   const int threads = (int)((per + ch - 1) / ch + 31) / 32 * 32;
-  if (S == 1) {
-    set_path_tag("row in the registers of a CTA, any alignment");
-    const unsigned grid = (unsigned)p.rows;
-    if (ch == 8) launch_dependent(softmax_rows_kernel<Tin, Tout, 8, false>, grid, threads, 0, st, p, 1);
-    else if (ch == 4) launch_dependent(softmax_rows_kernel<Tin, Tout, 4, false>, grid, threads, 0, st, p, 1);
-    else launch_dependent(softmax_rows_kernel<Tin, Tout, 2, false>, grid, threads, 0, st, p, 1);
-    *rc = launch_status("b200_softmax");
-    return true;
-  }
-  set_path_tag("row in the registers of a cluster, any alignment");
-  const dim3 grid = dim3((unsigned)(p.rows * S)), block = dim3((unsigned)threads), cluster((unsigned)S, 1, 1);
-  const cudaError_t e = ch == 8 ? launch_clusters(cluster, softmax_rows_kernel<Tin, Tout, 8, true>, grid, block, 0, st, p, S)
-                                : launch_clusters(cluster, softmax_rows_kernel<Tin, Tout, 4, true>, grid, block, 0, st, p, S);
+  set_path_tag(S > 1 ? "row in the registers of a cluster, any alignment" : "row in the registers of a CTA, any alignment");
+  const dim3 grid((unsigned)(p.rows * S)), block((unsigned)threads), cluster((unsigned)S);
+  auto launch = [&](auto scaled_tag, auto log_tag) {
+    constexpr bool SCALED = decltype(scaled_tag)::value, LOG = decltype(log_tag)::value;
+    if (S > 1)
+      return ch == 8 ? launch_clusters(cluster, softmax_rows_kernel<Tin, Tout, 8, true, SCALED, LOG>, grid, block, 0, st, p, S)
+                     : launch_clusters(cluster, softmax_rows_kernel<Tin, Tout, 4, true, SCALED, LOG>, grid, block, 0, st, p, S);
+    if (ch == 8) return launch_dependent(softmax_rows_kernel<Tin, Tout, 8, false, SCALED, LOG>, grid, block, 0, st, p, S);
+    return ch == 4 ? launch_dependent(softmax_rows_kernel<Tin, Tout, 4, false, SCALED, LOG>, grid, block, 0, st, p, S)
+                   : launch_dependent(softmax_rows_kernel<Tin, Tout, 2, false, SCALED, LOG>, grid, block, 0, st, p, S);
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  const cudaError_t e = p.has_scale ? (p.log_mode ? launch(yes, yes) : launch(yes, no)) : (p.log_mode ? launch(no, yes) : launch(no, no));
   if (e != cudaSuccess) {
     cudaGetLastError();
-    *rc = fail((int)e, "b200_softmax: cluster launch failed: %s", cudaGetErrorString(e));
+    *rc = fail((int)e, "b200_softmax: launch failed: %s", cudaGetErrorString(e));
     return true;
   }
   *rc = launch_status("b200_softmax");

@@ -513,6 +513,29 @@ def test_softmax_rows_over_strided_outer_dimensions(dtype, n):
             _near(got, torch.softmax(rows.double(), -1), f"strided softmax {tuple(rows.shape)}", floor=1e-7)
 
 
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.float32), (torch.float16, torch.float16), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("n", [1003, 20483, 30001])   # one CTA a row, and on both sides of two (16-bit rows to fp32 logs)
+def test_softmax_rows_with_infinite_logits(n, dtype, out):
+    """-inf among finite logits has probability 0 and log-probability -inf; the other elements are as if it were not there."""
+    x = _randn((6, n), dtype, n, 2.0)
+    x[1, 3:200] = float("-inf")
+    x[2, 1:] = float("-inf")
+    x[3, :n // 2] = float("-inf")
+    x[4, n - 1] = float("nan")
+    x[5] = float("-inf")
+    d = x.double()
+    for scale in (None, 0.5):
+        for log in (False, True):
+            got = _kernels().softmax(x, log=log, out_dtype=out, scale=scale)
+            t = d if scale is None else d * scale
+            want = torch.log_softmax(t, -1) if log else torch.softmax(t, -1)
+            assert torch.isnan(got[4:]).all()
+            g, w = got[:4], want[:4]
+            assert torch.equal(torch.isinf(g), torch.isinf(w)) and not torch.isnan(g).any()
+            finite = torch.isfinite(w)
+            _near(g[finite], w[finite], f"softmax with -inf, {n} log={log} scale={scale}", floor=2e-6 if log else 1.2e-7)
+
+
 @pytest.mark.parametrize("mask_shape", [(1, 1, 1), (4, 1, 1), (1, 3, 1), (1, 1, 5), (4, 1, 5), (4, 3, 1), (1, 3, 5), (4, 3, 5)])
 @pytest.mark.parametrize("n", [64, 100, 1000])
 def test_softmax_of_every_broadcast_mask_and_outer_order(n, mask_shape):
