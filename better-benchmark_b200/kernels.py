@@ -7,6 +7,8 @@ nothing is ever copied, made contiguous or computed by torch behind the caller's
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import native
@@ -45,7 +47,8 @@ def _require_cuda(*tensors: torch.Tensor) -> torch.device:
             dev = t.device
         elif t.device != dev:
             raise native.KernelArgumentError("all tensors must be on one device")
-    if dev is not None and dev.index is not None and dev.index != torch.cuda.current_device():
+    # (torch._C._cuda_getDevice is what torch.cuda.current_device returns once CUDA is initialised, as it is for a CUDA tensor)
+    if dev is not None and dev.index is not None and dev.index != torch._C._cuda_getDevice():
         # the library launches on the current device's current stream and reads that device's
         # properties: pointers of another GPU would fault there, or silently cross NVLink
         raise native.KernelArgumentError(
@@ -99,7 +102,7 @@ def collapse_outer(shape, strides_list):
 def _is_dense(t: torch.Tensor) -> bool:
     """True when the tensor covers its storage range exactly once (some permutation of a
     contiguous layout), so an output may reuse its strides."""
-    if t.is_contiguous():
+    if t.is_contiguous() or (t.dim() == 4 and t.is_contiguous(memory_format=torch.channels_last)):
         return True
     expected = 1
     for size, stride in sorted(((sz, st) for sz, st in zip(t.shape, t.stride()) if sz != 1),
@@ -108,6 +111,16 @@ def _is_dense(t: torch.Tensor) -> bool:
             return False
         expected *= size
     return True
+
+
+@functools.lru_cache(maxsize=1024)
+def _scratch_bytes_on(device: int, entry: str, key: int) -> int:
+    return int(getattr(load(), entry)(key))
+
+
+def _scratch_bytes(entry: str, key: int) -> int:
+    """What the library asks for on the current device: one number per entry point, device and row or channel count."""
+    return _scratch_bytes_on(torch._C._cuda_getDevice(), entry, key)
 
 
 def _outer(t: torch.Tensor):
@@ -134,7 +147,7 @@ def row_reduce(x: torch.Tensor, op: str, *, keepdim: bool = False,
     oshape, ostrides = _outer(x)
     rows = _numel(oshape)
     out_shape = list(oshape) + ([1] if keepdim else [])
-    out = torch.empty(out_shape, dtype=out_dtype, device=x.device)
+    out = x.new_empty(out_shape, dtype=out_dtype)
     if rows == 0:
         return out
     if n == 0:
@@ -172,7 +185,7 @@ def softmax(x: torch.Tensor, *, mask: torch.Tensor | None = None, scale: float |
         if _is_dense(x):
             out = torch.empty_strided(x.shape, x.stride(), dtype=out_dtype, device=x.device)
         else:
-            out = torch.empty(x.shape, dtype=out_dtype, device=x.device)
+            out = x.new_empty(x.shape, dtype=out_dtype)
     elif out.shape != x.shape or (n > 1 and out.stride(-1) != 1):
         raise UnsupportedLayout("softmax: out must match x's shape with a contiguous last dim")
     if x.numel() == 0:
@@ -269,7 +282,7 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
     stat_shape = list(x.shape[:-1]) + ([1] if keepdim else [])
 
     def stat(flag):
-        return torch.empty(stat_shape, dtype=torch.float32, device=x.device) if flag else None
+        return x.new_empty(stat_shape, dtype=torch.float32) if flag else None
 
     mean, rstd, var = stat(want_mean and not rms), stat(want_rstd), stat(want_var)
     lib = load()
@@ -280,7 +293,7 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
                                 (1 if rms else 0) | _NORM_PROLOGUES[prologue], _stream()),
               "b200_norm_fwd")
         return y, mean, rstd, var
-    total = torch.empty(x.shape, dtype=x.dtype, device=x.device) if want_sum else None
+    total = x.new_empty(x.shape, dtype=x.dtype) if want_sum else None
     check(lib.b200_norm_fwd_residual(_ptr(x), _ptr(residual), _ptr(total), _ptr(weight), _ptr(bias), _ptr(y),
                                      _ptr(mean), _ptr(rstd), _ptr(var), rows, n, x_stride, y_stride, _code(x),
                                      w_code, _DTYPE_CODE[out_dtype], float(eps), float(correction),
@@ -318,6 +331,11 @@ def scratch_buffer(device: torch.device, nbytes: int) -> torch.Tensor:
     buf = torch.zeros(max(int(nbytes), SCRATCH_DEFAULT_BYTES), dtype=torch.uint8, device=device)
     bufs.append(buf)  # superseded buffers stay alive: captured graphs may still point at them
     return buf
+
+
+def _behind_barrier_words(scratch: torch.Tensor):
+    """Address and size of what follows the 256 bytes that kernels with a grid barrier keep at zero."""
+    return scratch.data_ptr() + 256, max(0, scratch.numel() * scratch.element_size() - 256)
 
 
 def check_scratch_status(device: torch.device | None = None) -> None:
@@ -358,13 +376,13 @@ def norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor | None, rst
         b, s, h, d = x.shape
         rows, n = b * s, h * d
         x_stride = dy_stride = n
-        dx = torch.empty((b, h, s, d), dtype=x.dtype, device=x.device)
+        dx = x.new_empty((b, h, s, d), dtype=x.dtype)
         seq, head_dim = s, d
         dx_batch, dx_seq, dx_head = h * s * d, d, s * d
     else:
         rows, n, x_stride = _rows_2d(x, "norm_bwd")
         dy_stride = 0 if dy_scalar else _rows_2d(dy, "norm_bwd")[2]
-        dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+        dx = x.new_empty(x.shape, dtype=x.dtype)
         seq, head_dim = 1, n
         dx_batch, dx_seq, dx_head = n, 0, n
     if rstd.dtype != torch.float32 or rstd.numel() != rows or not rstd.is_contiguous():
@@ -377,12 +395,12 @@ def norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor | None, rst
         if weight.dim() != 1 or weight.shape[0] != n or not weight.is_contiguous():
             raise UnsupportedLayout("norm_bwd: weight must be contiguous [n]")
         w_code = _code(weight)
-    dw = torch.empty(n, dtype=torch.float32, device=x.device) if want_dweight else None
-    db = torch.empty(n, dtype=torch.float32, device=x.device) if (want_dbias and not rms) else None
+    dw = x.new_empty(n, dtype=torch.float32) if want_dweight else None
+    db = x.new_empty(n, dtype=torch.float32) if (want_dbias and not rms) else None
     lib = load()
     nbytes = 0
     if dw is not None or db is not None:
-        nbytes = int(lib.b200_norm_bwd_scratch_bytes(n))
+        nbytes = _scratch_bytes("b200_norm_bwd_scratch_bytes", n)
         if scratch is None:
             scratch = scratch_buffer(x.device, nbytes)
         nbytes = scratch.numel() * scratch.element_size()
@@ -431,10 +449,10 @@ def batch_norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Ten
         if stat is not None and (stat.dtype != torch.float32 or stat.shape != (c,) or not stat.is_contiguous()):
             raise UnsupportedLayout("batch_norm_fwd: running statistics must be contiguous fp32 [C]")
     y = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device)
-    mean = torch.empty(c, dtype=torch.float32, device=x.device)
-    invstd = torch.empty(c, dtype=torch.float32, device=x.device)
+    mean = x.new_empty(c, dtype=torch.float32)
+    invstd = x.new_empty(c, dtype=torch.float32)
     lib = load()
-    nbytes = int(lib.b200_batch_norm_scratch_bytes(c))
+    nbytes = _scratch_bytes("b200_batch_norm_scratch_bytes", c)
     if scratch is None:
         scratch = scratch_buffer(x.device, nbytes)
     check(lib.b200_batch_norm_fwd_ex(_ptr(x), _ptr(y), _ptr(weight), _ptr(bias), _ptr(running_mean),
@@ -473,20 +491,19 @@ def batch_norm_bwd(dy: torch.Tensor, x: torch.Tensor, mean: torch.Tensor, invstd
         raise UnsupportedLayout("batch_norm_bwd: H and W must be mergeable into one spatial dimension")
     ss = sw if w > 1 else (sh if h > 1 else 1)
     dx = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) if want_dx else None
-    dw = torch.empty(c, dtype=torch.float32, device=x.device)
-    db = torch.empty(c, dtype=torch.float32, device=x.device)
+    dw = x.new_empty(c, dtype=torch.float32)
+    db = x.new_empty(c, dtype=torch.float32)
     if x.numel() == 0:
         dw.zero_(); db.zero_()
         return dx, dw, db
     lib = load()
-    need = int(lib.b200_batch_norm_bwd_scratch_bytes(c)) + 256
+    need = _scratch_bytes("b200_batch_norm_bwd_scratch_bytes", c) + 256
     if scratch is None:
         scratch = scratch_buffer(x.device, need)
-    usable = scratch[256:]  # the barrier words at the head of the shared buffer stay untouched
     check(lib.b200_batch_norm_bwd_ex(_ptr(dy), _ptr(x), _ptr(act), _ptr(mean), _ptr(invstd), _ptr(weight),
                                      _ptr(dx), _ptr(dw), _ptr(db), n, c, h * w, sn, sc, ss, _code(x),
                                      _code(weight) if weight is not None else F32, float(slope),
-                                     float(inv_count) if inv_count else 0.0, _ptr(usable), usable.numel(), _stream()),
+                                     float(inv_count) if inv_count else 0.0, *_behind_barrier_words(scratch), _stream()),
           "b200_batch_norm_bwd")
     return dx, dw, db
 
@@ -512,7 +529,7 @@ def col_reduce(x: torch.Tensor, op: str, *, out_dtype: torch.dtype | None = None
     if c > 1 and x.stride(2) != 1:
         raise UnsupportedLayout("col_reduce: the kept dimension must be contiguous")
     out_dtype = out_dtype or x.dtype
-    out = torch.empty((b, c), dtype=out_dtype, device=x.device)
+    out = x.new_empty((b, c), dtype=out_dtype)
     if out.numel() == 0:
         return out[0] if squeeze else out
     if r == 0:
@@ -522,12 +539,10 @@ def col_reduce(x: torch.Tensor, op: str, *, out_dtype: torch.dtype | None = None
         return out[0] if squeeze else out
     if scratch is None:
         scratch = scratch_buffer(x.device, 1 << 20)
-    # the barrier words at the head of the shared scratch buffer stay untouched
-    usable = scratch[256:]
     lib = load()
     check(lib.b200_col_reduce(_ptr(x), _ptr(out), b, r, c, x.stride(0) if b > 1 else r * x.stride(1),
                               x.stride(1) if r > 1 else c, c, _code(x), _DTYPE_CODE[out_dtype],
-                              _COL_CODES[op], _ptr(usable), usable.numel(), _stream()),
+                              _COL_CODES[op], *_behind_barrier_words(scratch), _stream()),
           "b200_col_reduce")
     return out[0] if squeeze else out
 
@@ -542,7 +557,7 @@ def permute_copy(x: torch.Tensor, dims, *, scale: float | None = None,
     _require_cuda(x)
     out_dtype = out_dtype or x.dtype
     view = x.permute(*dims)
-    out = torch.empty(view.shape, dtype=out_dtype, device=x.device)
+    out = x.new_empty(view.shape, dtype=out_dtype)
     if out.numel() == 0:
         return out
     shape, (strides,) = _collapse_all(tuple(view.shape), [tuple(view.stride())])
@@ -726,7 +741,7 @@ def dropout_add(x: torch.Tensor, residual: torch.Tensor, seeds: torch.Tensor, se
         raise UnsupportedLayout("dropout_add: tensors must be contiguous")
     if not 0 <= seed_index < seeds.numel():
         raise native.KernelArgumentError("dropout_add: seed index outside the seed tensor")
-    keep = torch.empty(residual.shape, dtype=torch.bool, device=x.device)
+    keep = x.new_empty(residual.shape, dtype=torch.bool)
     total = torch.empty_like(residual)
     lib = load()
     check(lib.b200_dropout_add(_ptr(x), _ptr(residual), _ptr(seeds), int(seed_index), float(p), _ptr(keep),
