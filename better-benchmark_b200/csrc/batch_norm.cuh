@@ -92,15 +92,16 @@ __device__ __forceinline__ void bn_channel_stats(const BatchNormParams& p, int c
 }
 
 // Adds up what the threads of a CTA hold: `one` and `two` are flat arrays of blockDim.x * V values each, of
-// which value f belongs to channel f % channels (blockDim.x * V is a multiple of the channel count). As many
-// threads share a channel as there are; fp64, fixed order. `part`: 2 * blockDim.x doubles. One thread per channel
-// made this a chain of blockDim.x * V / channels additions: bf16 channels-last [N, 16, 7, 7] of 1 MB forward
-// 11.8 us, so 8.0 us.
+// which value f belongs to channel f % channels (blockDim.x * V is a multiple of the channel count). fp64, fixed order.
+// With at most a quarter as many channels as threads, as many threads share a channel as there are: one thread per channel is
+// a chain of blockDim.x * V / channels additions there (bf16 channels-last [N, 16, 7, 7] of 1 MB forward 10.9 us, so
+// 7.6; 36 channels 8.8 and 7.6). With more channels the second step costs more than the chain (92 channels, 12 MB:
+// 14.7 us in one step, 16.2 in two; 256 channels, 2 MB: 8.3 and 9.4). `part`: 2 * blockDim.x doubles.
 template <typename Out, int V>
 __device__ __forceinline__ void bn_fold_channels(const float* one, const float* two, double* part, int channels,
                                                  Out* row_one, Out* row_two) {
   const int tid = threadIdx.x, threads = blockDim.x, values = threads * V;
-  const int share = channels <= threads ? threads / channels : 1;  // threads per channel
+  const int share = 4 * channels <= threads ? threads / channels : 1;  // threads per channel
   if (share == 1) {
     for (int c = tid; c < channels; c += threads) {
       double a = 0.0, b = 0.0;
