@@ -183,9 +183,9 @@ def softmax(x: torch.Tensor, *, mask: torch.Tensor | None = None, scale: float |
     out_dtype = out_dtype or x.dtype
     if out is None:
         if _is_dense(x):
-            out = torch.empty_strided(x.shape, x.stride(), dtype=out_dtype, device=x.device)
+            out = torch.empty_like(x, dtype=out_dtype)  # its strides
         else:
-            out = x.new_empty(x.shape, dtype=out_dtype)
+            out = torch.empty_like(x, dtype=out_dtype, memory_format=torch.contiguous_format)
     elif out.shape != x.shape or (n > 1 and out.stride(-1) != 1):
         raise UnsupportedLayout("softmax: out must match x's shape with a contiguous last dim")
     if x.numel() == 0:
@@ -293,7 +293,7 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
                                 (1 if rms else 0) | _NORM_PROLOGUES[prologue], _stream()),
               "b200_norm_fwd")
         return y, mean, rstd, var
-    total = x.new_empty(x.shape, dtype=x.dtype) if want_sum else None
+    total = torch.empty_like(x, memory_format=torch.contiguous_format) if want_sum else None
     check(lib.b200_norm_fwd_residual(_ptr(x), _ptr(residual), _ptr(total), _ptr(weight), _ptr(bias), _ptr(y),
                                      _ptr(mean), _ptr(rstd), _ptr(var), rows, n, x_stride, y_stride, _code(x),
                                      w_code, _DTYPE_CODE[out_dtype], float(eps), float(correction),
@@ -382,7 +382,7 @@ def norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor | None, rst
     else:
         rows, n, x_stride = _rows_2d(x, "norm_bwd")
         dy_stride = 0 if dy_scalar else _rows_2d(dy, "norm_bwd")[2]
-        dx = x.new_empty(x.shape, dtype=x.dtype)
+        dx = torch.empty_like(x, memory_format=torch.contiguous_format)
         seq, head_dim = 1, n
         dx_batch, dx_seq, dx_head = n, 0, n
     if rstd.dtype != torch.float32 or rstd.numel() != rows or not rstd.is_contiguous():
@@ -448,7 +448,7 @@ def batch_norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Ten
     for stat in (running_mean, running_var):
         if stat is not None and (stat.dtype != torch.float32 or stat.shape != (c,) or not stat.is_contiguous()):
             raise UnsupportedLayout("batch_norm_fwd: running statistics must be contiguous fp32 [C]")
-    y = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device)
+    y = torch.empty_like(x)  # x is dense: its strides
     mean = x.new_empty(c, dtype=torch.float32)
     invstd = x.new_empty(c, dtype=torch.float32)
     lib = load()
@@ -617,7 +617,7 @@ def cast_scale(x: torch.Tensor, out_dtype: torch.dtype, *, scale: float | None =
     _require_cuda(x)
     if not _is_dense(x):
         raise UnsupportedLayout("cast_scale: x must be dense")
-    out = torch.empty_strided(x.shape, x.stride(), dtype=out_dtype, device=x.device)
+    out = torch.empty_like(x, dtype=out_dtype)  # x is dense: its strides
     lib = load()
     check(lib.b200_cast_scale(_ptr(x), _ptr(out), x.numel(), _code(x), _DTYPE_CODE[out_dtype],
                               float(scale) if scale is not None else 1.0,
