@@ -147,7 +147,7 @@ int32_t b200_norm_bwd(const void* x, const void* dy, const void* weight, const f
                       int64_t dx_batch_stride, int64_t dx_seq_stride, int64_t dx_head_stride,
                       void* scratch, int64_t scratch_bytes, int32_t flags, void* stream);
 
-/* Same counter for b200_batch_norm_fwd's fused kernel. */
+/* Same counter for b200_batch_norm_fwd: 0, none of its kernels waits on a copy barrier or on other CTAs. */
 int64_t b200_batch_norm_wait_timeouts(void);
 
 /* Scratch bytes that let b200_batch_norm_fwd run its largest grid for `channels` channels. With less (down
@@ -294,9 +294,7 @@ int32_t b200_batch_norm_bwd_ex(const void* dy, const void* x, const void* act, c
  * device address and should be made before any stream capture. All calls on a device share the
  * array: calls that overlap on the GPU race and must be ordered by the caller. Allocates nothing.
  * Above 512 channels the array is smaller than b200_batch_norm_scratch_bytes: see there.
- * The caller has no scratch pointer to hand to b200_check_status here (and the barrier words are
- * cleared at every call): a bounded device-side wait that ran out shows in
- * b200_batch_norm_wait_timeouts(), which stays at 0 in normal operation.
+ * No kernel of BatchNorm forward waits on another CTA, so there is no status to check.
  * This entry point has no counterpart in the reference. */
 int32_t b200_batch_norm_fwd_static_scratch(const void* x, void* y, const void* weight, const void* bias,
                                            float* running_mean, float* running_var, float* save_mean,
