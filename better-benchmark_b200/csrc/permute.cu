@@ -438,11 +438,12 @@ __global__ void __launch_bounds__(256) transpose_small_kernel(const TransposePar
   }
 }
 
-// Stores N values as Tout with the widest stores that their alignment (that of N * sizeof(Tout), at most 32 bytes) allows.
-template <typename Tout, int N>
+// Stores N values as Tout. WIDE: p lies on a 32-byte boundary, 32 bytes at a time where there are as many; otherwise p need
+// only lie on min(16, N * sizeof(Tout)) bytes (8 values widened to fp32 are two stores of 16).
+template <typename Tout, int N, bool WIDE>
 __device__ __forceinline__ void store_unit(Tout* p, const f32x2 (&o)[N / 2]) {
   constexpr int BYTES = N * (int)sizeof(Tout);
-  if constexpr (BYTES <= 16) {
+  if constexpr (!WIDE || BYTES <= 16) {
     store_pairs<Tout, N>(p, o);
   } else {
     uint32_t w[BYTES / 4];
@@ -547,7 +548,7 @@ __global__ void __launch_bounds__(256, ACT >= 4 ? 5 : 4) cast_scale_kernel(const
                 o[v * (VIN / 2) + i] = apply_activation2<Tout, ACT>(pack2(f[2 * i], f[2 * i + 1]));
             }
           }
-          store_unit<Tout, NV * VIN>(dst + u * (NV * VIN), o);
+          store_unit<Tout, NV * VIN, NV == 2>(dst + u * (NV * VIN), o);
         }
       }
     }

@@ -240,6 +240,31 @@ def test_casts_on_both_sides_of_the_32_byte_path(dtype, out, activation):
                 assert torch.equal(got, (torch.relu(t) if activation else t).to(out)), (n, start)
 
 
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.float32), (torch.float16, torch.float32), (torch.float32, torch.float32),
+                                       (torch.float32, torch.bfloat16), (torch.float16, torch.float16)])
+@pytest.mark.parametrize("mode", [0, 2, 8])
+def test_casts_through_the_entry_point_to_results_of_every_alignment(dtype, out, mode):
+    """A caller's result may start anywhere on its type's grid: 16 bytes off a 32-byte boundary 8 values widened to fp32
+    leave as two stores. The bits are those of the aligned call, and nothing beside the result is written."""
+    k = _kernels()
+    unit = 32 // dtype.itemsize
+    x = _randn((4099 * unit + 64,), dtype, 5, 2.0)
+    y = torch.empty(x.numel() + 64, dtype=out, device="cuda")
+    assert x.data_ptr() % 256 == 0 and y.data_ptr() % 256 == 0
+    activation = {0: None, 2: "relu", 8: "silu"}[mode]
+    for n in (0, 1, 8, 77, 1000, 4096 * unit - 1, 4096 * unit, 4099 * unit + 5):
+        want = k.cast_scale(x[:n].clone(), out, activation=activation)
+        for x_start in (0, unit // 2):
+            x[x_start:x_start + n].copy_(x[:n].clone())
+            for offset in (0, 4, 8, 16, 20, 32, 48):
+                start = offset // y.element_size()
+                y.fill_(7.0)
+                k.check(k.load().b200_cast_scale(x.data_ptr() + x_start * x.element_size(), y.data_ptr() + offset, n, k._code(x),
+                                                 k._DTYPE_CODE[out], 1.0, mode, k._stream()), "b200_cast_scale")
+                assert torch.equal(y[start:start + n], want), (n, x_start, offset)
+                assert (y[:start] == 7).all() and (y[start + n:] == 7).all(), (n, x_start, offset)
+
+
 @pytest.mark.parametrize("dtype,n,c,hw", [(torch.bfloat16, 1001, 92, 196), (torch.bfloat16, 336, 92, 196),
                                           (torch.float32, 80, 485, 256), (torch.bfloat16, 64, 1022, 49)])
 def test_batch_norm_takes_the_same_path_with_the_advertised_scratch(dtype, n, c, hw):
