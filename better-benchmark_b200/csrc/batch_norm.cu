@@ -405,9 +405,12 @@ __device__ __forceinline__ void bn_ring_issue(const uint4* x, uint32_t mine, int
 }
 
 // MAXT: 256 threads, or 512 for patterns of more than 256 vectors.
-template <typename T, int MAXT>
-__global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total,
-                                                                                   int PV, int rows_shift) {
+// SHIFT: by what a channel's sums are shifted (batch_norm.cuh): kShiftRow0 by its element of row 0, asked for in front of the first
+// copies; kShiftRows by the mean of its first sixteen rows, asked for behind them; kShiftRowsFirst by the same, in front of them.
+enum { kShiftRow0 = 0, kShiftRows = 1, kShiftRowsFirst = 2 };
+template <typename T, int MAXT, int SHIFT>
+__global__ void __launch_bounds__(MAXT, 512 / MAXT)
+batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total, int PV) {
   wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -419,33 +422,47 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_sums_cl_ring_kern
   const uint32_t mine = smem_u32(smem) + (uint32_t)tid * 16u;
   const long long step = (long long)gridDim.x * kRingU * T_;
   long long v = (long long)blockIdx.x * kRingU * T_ + tid;
+  T first[SHIFT == kShiftRowsFirst ? BN_SHIFT_ROWS : V];
+  if constexpr (SHIFT == kShiftRowsFirst) {  // the launcher sees to C <= blockDim.x
+    if (tid < C) bn_shift_load<T>(xe, tid, C, p.rows, first);
+  } else if constexpr (SHIFT == kShiftRow0) {
+    int c = ph * V % C;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      first[i] = ld_here(xe + c);
+      if (++c == C) c = 0;
+    }
+  }
 #pragma unroll
   for (int s = 0; s < kRingS - 1; ++s) bn_ring_issue<false>(x, mine, s, v + s * step, total, T_);
-  // The shift of every channel (bn_shift_scalar: mean of its first sixteen rows, eight significant
-  // bits; the finalize kernel forms the same value) is computed once per CTA into shared memory,
-  // at most MAXT * V channels per round, and every thread picks up its V channels.
   f32x2 shift[V / 2], s1[V / 2], s2[V / 2], t1[V / 2], t2[V / 2];
   f32x2 upper[V / 2];
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) shift[i] = s1[i] = s2[i] = t1[i] = t2[i] = upper[i] = splat2(0.f);
-  if (!rows_shift) {  // short chains (small tensors): the channel's element of row 0 will do
+  if constexpr (SHIFT == kShiftRow0) {
 #pragma unroll
-    for (int i = 0; i < V / 2; ++i)
-      shift[i] = pack2(Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i) % C)), Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i + 1) % C)));
-  }
-  for (int c0 = 0; rows_shift && c0 < C; c0 += MAXT * V) {
-    for (int c = c0 + tid; c < C && c < c0 + MAXT * V; c += T_) red[c - c0] = bn_shift_scalar<T>(xe, c, C, p.rows);
-    __syncthreads();
+    for (int i = 0; i < V / 2; ++i) shift[i] = pack2(Elem<T>::to_f32(first[2 * i]), Elem<T>::to_f32(first[2 * i + 1]));
+  } else {
+    // The shift of every channel (the finalize kernel forms the same value) is computed once per CTA into shared
+    // memory, at most MAXT * V channels per round, and every thread picks up its V channels.
+    for (int c0 = 0; c0 < C; c0 += MAXT * V) {
+      if constexpr (SHIFT == kShiftRowsFirst) {
+        if (tid < C) red[tid] = bn_shift_of<T>(first);
+      } else {
+        for (int c = c0 + tid; c < C && c < c0 + MAXT * V; c += T_) red[c - c0] = bn_shift_scalar<T>(xe, c, C, p.rows);
+      }
+      __syncthreads();
 #pragma unroll
-    for (int i = 0; i < V / 2; ++i) {
-      const int ca = (ph * V + 2 * i) % C, cb = (ph * V + 2 * i + 1) % C;
-      float lo, hi;
-      unpack2(shift[i], lo, hi);
-      if (ca >= c0 && ca < c0 + MAXT * V) lo = red[ca - c0];
-      if (cb >= c0 && cb < c0 + MAXT * V) hi = red[cb - c0];
-      shift[i] = pack2(lo, hi);
+      for (int i = 0; i < V / 2; ++i) {
+        const int ca = (ph * V + 2 * i) % C, cb = (ph * V + 2 * i + 1) % C;
+        float lo, hi;
+        unpack2(shift[i], lo, hi);
+        if (ca >= c0 && ca < c0 + MAXT * V) lo = red[ca - c0];
+        if (cb >= c0 && cb < c0 + MAXT * V) hi = red[cb - c0];
+        shift[i] = pack2(lo, hi);
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
   // Additions of squares of 16-bit values are biased, in proportion to the length of the chain they
   // join: two stages' squares are summed by themselves, sixteen of those join one chain, the chains a third.
@@ -618,6 +635,17 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_apply_cl_ring_ker
   copy_async_wait<0>();
 }
 
+// With row 0 alone the error of invstd depends on where that row lies: five standard deviations off the mean it is 1.5e-7
+// instead of 2.9e-8 (rms, bf16), so row 0 is only for what cannot afford more. More than 32 vectors a thread (39 MB): the
+// sixteen rows, asked for behind the copies (bf16 64 channels, 100 MB 46.9 us; in front of them 48.6). From 8 MB on, up to 256
+// channels (at most one a thread): in front, where they cost nothing (64 channels, 12 / 18.5 / 30 MB: row 0 13.3 / 16.4 / 20.7, so
+// 13.2 / 16.2 / 20.1, behind the copies 13.8 / 17.2 / 21.3; 256 channels 14.7 / 17.8 / 22.3 and 14.5 / 17.3 / 21.6). Below 8 MB they would
+// cost 0.2 to 0.7 of 7 to 10 us, with 1024 channels of up to 39 MB 2.5 of 20.
+static int bn_shift_kind(long long channels, long long vectors, long long all_threads) {
+  if (vectors > 32 * all_threads) return kShiftRows;
+  return channels <= 256 && vectors * 16 >= 8000000 ? kShiftRowsFirst : kShiftRow0;
+}
+
 // Returns false when the shape or the scratch does not fit, or the kernels above are faster (the caller takes them).
 template <typename T>
 static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_bytes, cudaStream_t st, int* rc) {
@@ -640,10 +668,12 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   if (splits * threads * 8 > total) splits = (total + threads * 8 - 1) / (threads * 8);
   if (splits > room / (2 * C)) return false;  // the kernels above make do with fewer partial rows
   p.stats = p.partials + splits * 2 * C;
-  const int rows_shift = total > 32LL * threads * splits ? 1 : 0;  // more than 32 vectors per thread
+  const int kind = bn_shift_kind(C, total, (long long)threads * splits);
   auto run = [&](auto maxt_tag) {
     constexpr int MAXT = decltype(maxt_tag)::value;
-    auto sums = batch_norm_sums_cl_ring_kernel<T, MAXT>;
+    auto sums = kind == kShiftRow0   ? batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRow0>
+                : kind == kShiftRows ? batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRows>
+                                     : batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRowsFirst>;
     auto apply = batch_norm_apply_cl_ring_kernel<T, MAXT>;
     const size_t ring = (size_t)kRingBytesPerThread * MAXT;  // 96 KB, or 192 KB: two CTAs, or one, per SM
     const size_t with_shifts = ring + (size_t)MAXT * V * sizeof(float);
@@ -660,10 +690,11 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
       *rc = fail((int)e, "b200_batch_norm_fwd: cannot reserve %zu bytes of shared memory: %s", with_shifts, cudaGetErrorString(e));
       return;
     }
-    launch_dependent(sums, (unsigned)splits, threads, with_shifts, st, p, total, (int)PV, rows_shift);
+    launch_dependent(sums, (unsigned)splits, threads, with_shifts, st, p, total, (int)PV);
     *rc = launch_status("b200_batch_norm_fwd sums [channels-last, flat vectors, copy rings]");
     if (*rc != B200_OK) return;
-    launch_dependent(batch_norm_finalize_ring_kernel<T>, dim3((unsigned)p.channels), dim3(256), 0, st, p, (int)splits, rows_shift);
+    launch_dependent(batch_norm_finalize_ring_kernel<T>, dim3((unsigned)p.channels), dim3(256), 0, st, p, (int)splits,
+                     kind != kShiftRow0 ? 1 : 0);
     *rc = launch_status("b200_batch_norm_fwd finalize");
     if (*rc != B200_OK || !p.y) return;
     launch_dependent(apply, dim3((unsigned)splits), dim3((unsigned)threads), ring, st, p, total, (int)PV);

@@ -45,17 +45,27 @@ __device__ __forceinline__ float bn_round_shift(float v) {
 }
 
 template <typename T>
-__device__ __forceinline__ float bn_shift_scalar(const T* x, int c, int channels, long long rows) {
-  float v[BN_SHIFT_ROWS];
+__device__ __forceinline__ void bn_shift_load(const T* x, int c, int channels, long long rows, T (&v)[BN_SHIFT_ROWS]) {
 #pragma unroll
   for (int r = 0; r < BN_SHIFT_ROWS; ++r) {
     const long long rr = r < rows ? r : rows - 1;
-    v[r] = Elem<T>::to_f32(__ldg(x + rr * channels + c));
+    v[r] = ld_here(x + rr * channels + c);
   }
+}
+
+template <typename T>
+__device__ __forceinline__ float bn_shift_of(const T (&v)[BN_SHIFT_ROWS]) {
   float s = 0.f;
 #pragma unroll
-  for (int r = 0; r < BN_SHIFT_ROWS; ++r) s = __fadd_rn(s, v[r]);
+  for (int r = 0; r < BN_SHIFT_ROWS; ++r) s = __fadd_rn(s, Elem<T>::to_f32(v[r]));
   return bn_round_shift(__fmul_rn(s, 1.0f / BN_SHIFT_ROWS));
+}
+
+template <typename T>
+__device__ __forceinline__ float bn_shift_scalar(const T* x, int c, int channels, long long rows) {
+  T v[BN_SHIFT_ROWS];
+  bn_shift_load<T>(x, c, channels, rows, v);
+  return bn_shift_of<T>(v);
 }
 
 // Turns the fp64 totals of the shifted sums of one channel into mean / invstd and, for the one

@@ -175,6 +175,24 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
   return r;
 }
 
+// One value of 2 or 4 bytes, asked for where the call stands: neither in front of wait_for_previous_kernel nor behind
+// the copies that are to follow it.
+template <typename T>
+__device__ __forceinline__ T ld_here(const T* p) {
+  static_assert(sizeof(T) == 2 || sizeof(T) == 4, "scalars");
+  T r;
+  if constexpr (sizeof(T) == 2) {
+    unsigned short u;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(u) : "l"(p));
+    r = *reinterpret_cast<const T*>(&u);
+  } else {
+    uint32_t u;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(u) : "l"(p));
+    r = *reinterpret_cast<const T*>(&u);
+  }
+  return r;
+}
+
 __device__ __forceinline__ uint4 ld_keep(const void* p) {
   return __ldg(reinterpret_cast<const uint4*>(p));
 }

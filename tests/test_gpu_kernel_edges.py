@@ -415,6 +415,25 @@ def test_batch_norm_channels_last_of_few_channels_and_power_of_two_counts(n, c, 
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("c", [64, 92, 256])
+@pytest.mark.parametrize("mb", [10, 24, 36])
+def test_batch_norm_statistics_with_a_first_row_far_from_the_mean(mb, c, dtype):
+    """The sums are shifted by the mean of sixteen rows, not by the first one: here that is five standard deviations off, which
+    would multiply the error of invstd. Half an fp32 step (2^-24 of the value) for its rounding and as much for the sums."""
+    n = int(mb * 1e6 / dtype.itemsize / c / 49) // 8 * 8
+    x = _randn((n, c, 7, 7), torch.float32, mb + c, 2.0).add_(0.5)
+    side = torch.arange(c, device="cuda") % 2 * 2.0 - 1.0
+    x[0, :, 0, 0] = 0.5 + 2.0 * 5 * side
+    x = x.to(dtype).contiguous(memory_format=torch.channels_last)
+    ones = torch.ones(c, device="cuda")
+    _, mean, invstd = _kernels().batch_norm_fwd(x, ones, ones, None, None, eps=1e-5, momentum=0.1)
+    var64, mean64 = torch.var_mean(x.double(), (0, 2, 3), unbiased=False)
+    worst = (invstd.double() * torch.sqrt(var64 + 1e-5) - 1).abs().max().item()
+    assert worst <= 2.0 ** -23, f"invstd off by {worst:.2e}"
+    assert ((mean.double() - mean64) / var64.sqrt()).abs().max().item() <= 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_log_softmax_in_fp32_has_no_biased_sum(dtype):
     """Mean error of fp32 log-probabilities over 100 000 rows of 1003. An exponential whose errors have a mean shifts
     every row alike: 2.7e-8 with the pair exponential of 16-bit results, 1.3e-8 with expf (rounding of the logits'
