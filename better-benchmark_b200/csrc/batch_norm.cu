@@ -407,6 +407,9 @@ __device__ __forceinline__ void bn_ring_issue(const uint4* x, uint32_t mine, int
 // MAXT: 256 threads, or 512 for patterns of more than 256 vectors.
 // SHIFT: by what a channel's sums are shifted (batch_norm.cuh): kShiftRow0 by its element of row 0, asked for in front of the first
 // copies; kShiftRows by the mean of its first sixteen rows, asked for behind them; kShiftRowsFirst by the same, in front of them.
+// 85 registers: two CTAs of 256 threads then leave room on their SM for two CTAs of the finalize kernel (256 threads, 40 registers)
+// while they drain; above 88 there is room for one, and 149 to 296 channels need two (bf16, 256 channels, 2 / 4 MB: 9.0 / 9.5 us
+// with 102 registers, 8.0 / 8.7 so).
 enum { kShiftRow0 = 0, kShiftRows = 1, kShiftRowsFirst = 2 };
 template <typename T, int MAXT, int SHIFT>
 __global__ void __launch_bounds__(MAXT, 512 / MAXT)

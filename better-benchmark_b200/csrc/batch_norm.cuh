@@ -104,9 +104,9 @@ __device__ __forceinline__ void bn_channel_stats(const BatchNormParams& p, int c
 // Adds up what the threads of a CTA hold: `one` and `two` are flat arrays of blockDim.x * V values each, of
 // which value f belongs to channel f % channels (blockDim.x * V is a multiple of the channel count). fp64, fixed order.
 // With at most a quarter as many channels as threads, as many threads share a channel as there are: one thread per channel is
-// a chain of blockDim.x * V / channels additions there (bf16 channels-last [N, 16, 7, 7] of 1 MB forward 10.9 us, so
-// 7.6; 36 channels 8.8 and 7.6). With more channels the second step costs more than the chain (92 channels, 12 MB:
-// 14.7 us in one step, 16.2 in two; 256 channels, 2 MB: 8.3 and 9.4). `part`: 2 * blockDim.x doubles.
+// a chain of blockDim.x * V / channels additions there (forward, bf16 [N, 16, 7, 7] of 0.5 MB 10.8 us, so 7.4; 36 channels
+// 8.5 and 7.4). With more channels the second step costs more than the chain (92 channels, 12 / 45 MB: bf16 14.2 / 28.0 us in one
+// step, 14.4 / 28.6 in two, f32 12.4 / 23.6 and 13.1 / 24.4). `part`: 2 * blockDim.x doubles.
 template <typename Out, int V>
 __device__ __forceinline__ void bn_fold_channels(const float* one, const float* two, double* part, int channels,
                                                  Out* row_one, Out* row_two) {
