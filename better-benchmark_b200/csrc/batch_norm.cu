@@ -649,7 +649,8 @@ static int bn_shift_kind(long long channels, long long vectors, long long all_th
   return channels <= 256 && vectors * 16 >= 8000000 ? kShiftRowsFirst : kShiftRow0;
 }
 
-// Returns false when the shape or the scratch does not fit, or the kernels above are faster (the caller takes them).
+// Returns false when the shape or the scratch does not fit (not one partial row), or the kernels above are faster (the
+// caller takes them).
 template <typename T>
 static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_bytes, cudaStream_t st, int* rc) {
   constexpr int V = Elem<T>::V;
@@ -662,14 +663,23 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   if (PV > 512 || elems % (PV * V) != 0) return false;  // whole periods only
   if (ring_is_slower(C, elems * (long long)sizeof(T))) return false;
   const long long total = elems / V;
-  const int threads = (int)(PV <= 256 ? 256 / PV * PV : PV);
   const long long stats_floats = 2 * C;
   const long long room = ((long long)scratch_bytes - 256) / (long long)sizeof(float) - stats_floats;
   if (room < 2 * C) return false;
+  const long long most = room / (2 * C);  // partial rows that the scratch holds
+  int threads = (int)(PV <= 256 ? 256 / PV * PV : PV);
   long long splits = (threads <= 256 ? 2LL : 1LL) * dev.sm_count;  // all CTAs resident
   // at least 8 vectors per thread: small tensors get few partial rows and a short finalize
-  if (splits * threads * 8 > total) splits = (total + threads * 8 - 1) / (threads * 8);
-  if (splits > room / (2 * C)) return false;  // the kernels above make do with fewer partial rows
+  auto useful = [&](long long ctas) { return ctas * threads * 8 > total ? (total + threads * 8 - 1) / (threads * 8) : ctas; };
+  splits = useful(splits);
+  if (splits > most) {
+    // No room for two partial rows per SM: one CTA per SM with the threads of both, and fewer of those when there is not even
+    // room for that. bf16 64 channels, 148 rows, 10 / 30 / 100 MB: 12.3 / 19.9 / 48.6 us (CTAs of 256 threads 13.2 / 24.2 / 57.8, the flat
+    // kernels on as few CTAs 19.5 / 39.6 / 109.6); 20 rows, 100 MB: 209 (288, 611).
+    threads = (int)(512 / PV * PV);
+    splits = useful(dev.sm_count);
+    if (splits > most) splits = most;
+  }
   p.stats = p.partials + splits * 2 * C;
   const int kind = bn_shift_kind(C, total, (long long)threads * splits);
   auto run = [&](auto maxt_tag) {

@@ -433,6 +433,28 @@ def test_batch_norm_statistics_with_a_first_row_far_from_the_mean(mb, c, dtype):
     assert ((mean.double() - mean64) / var64.sqrt()).abs().max().item() <= 2.0 ** -24
 
 
+@pytest.mark.parametrize("dtype,c", [(torch.bfloat16, 64), (torch.float32, 92), (torch.float16, 320), (torch.bfloat16, 1022)])
+@pytest.mark.parametrize("partial_rows", [295, 148, 5, 1])
+def test_batch_norm_with_room_for_few_partial_rows(partial_rows, dtype, c):
+    """A caller's scratch of less than two partial rows per SM, down to one: the copy rings on fewer, wider CTAs, the statistics as
+    close to fp64 as with all of them. Nothing behind the buffer is written."""
+    k = _kernels()
+    n = int(12e6 / dtype.itemsize / c / 49) // 8 * 8
+    x = _randn((n, c, 7, 7), dtype, c, 2.0).contiguous(memory_format=torch.channels_last)
+    w, b = _randn((c,), torch.float32, c + 3), _randn((c,), torch.float32, c + 4)
+    size = 256 + (partial_rows + 1) * 2 * c * 4
+    scratch = torch.full((size + 4096,), 77, dtype=torch.uint8, device="cuda")
+    y, mean, invstd = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1, scratch=scratch[:size])
+    assert b"copy rings" in k.load().b200_last_kernel(), k.load().b200_last_kernel()
+    assert (scratch[size:] == 77).all() and (scratch[:256] == 77).all()
+    var64, mean64 = torch.var_mean(x.double(), (0, 2, 3), unbiased=False)
+    # 2^-24 for the rounding of a result; the longest chains here are of 5000 vectors in one CTA, in three levels of sums
+    assert (invstd.double() * torch.sqrt(var64 + 1e-5) - 1).abs().max().item() <= 2.0 ** -22
+    assert ((mean.double() - mean64) / var64.sqrt()).abs().max().item() <= 2.0 ** -23
+    col = lambda t: t.double().view(1, c, 1, 1)  # noqa: E731
+    _near(y, (x.double() - col(mean64)) * col(torch.rsqrt(var64 + 1e-5)) * col(w) + col(b), f"y {partial_rows} rows", floor=2e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_log_softmax_in_fp32_has_no_biased_sum(dtype):
     """Mean error of fp32 log-probabilities over 100 000 rows of 1003. An exponential whose errors have a mean shifts
