@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1) batch_norm_sums_cl_
   if (!rows_shift) {  // short chains (small tensors): the channel's element of row 0 will do
 #pragma unroll
     for (int i = 0; i < V / 2; ++i)
-      shift[i] = pack2(Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i) % C)), Elem<T>::to_f32(__ldg(xe + (ph * V + 2 * i + 1) % C)));
+      shift[i] = pack2(Elem<T>::to_f32(ld_here(xe + (ph * V + 2 * i) % C)), Elem<T>::to_f32(ld_here(xe + (ph * V + 2 * i + 1) % C)));
   }
   for (int c0 = 0; rows_shift && c0 < C; c0 += 2 * MAXT * V) {
     for (int c = c0 + tid; c < C && c < c0 + 2 * MAXT * V; c += T_) red[c - c0] = bn_shift_scalar<T>(xe, c, C, p.rows);
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_ring_kernel(const Bat
   const T* x = reinterpret_cast<const T*>(p.x);
   if (tid < BN_SHIFT_ROWS) {
     const long long r = rows_shift ? (tid < p.rows ? tid : p.rows - 1) : 0;
-    first_rows[tid] = Elem<T>::to_f32(__ldg(x + r * p.channels + c));
+    first_rows[tid] = Elem<T>::to_f32(ld_here(x + r * p.channels + c));
   }
   wait_for_previous_kernel();
   let_next_kernel_start();

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) bn_bwd_sums_cl_kernel(const 
   f32x2 mean2[V / 2], s1[V / 2], s2[V / 2];
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) {
-    mean2[i] = pack2(__ldg(p.mean + (ph * V + 2 * i) % C), __ldg(p.mean + (ph * V + 2 * i + 1) % C));
+    mean2[i] = pack2(ld_here(p.mean + (ph * V + 2 * i) % C), ld_here(p.mean + (ph * V + 2 * i + 1) % C));
     s1[i] = s2[i] = splat2(0.f);
   }
   const long long step = (long long)gridDim.x * kChunk * T_;
@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(256) bn_bwd_finalize_kernel(const BnBwdParams 
   // what thread 0 needs after the sums: requested now, so that it does not cost a round trip then
   float invstd = 0.f, w = 1.f, mean = 0.f;
   if (tid == 0) {
-    invstd = __ldg(p.invstd + c);
-    mean = __ldg(p.mean + c);
+    invstd = ld_here(p.invstd + c);
+    mean = ld_here(p.mean + c);
     if (p.weight) w = load_param1(p.weight, p.w_dtype, c);
   }
   wait_for_previous_kernel();
@@ -456,10 +456,10 @@ bn_bwd_nchw_cluster_kernel(const BnBwdParams p, const int imgs_per_cta, const in
   const T* xc = reinterpret_cast<const T*>(p.x) + (long long)c * hw;
   const T* actc = HAS_ACT ? reinterpret_cast<const T*>(p.act) + (long long)c * hw : nullptr;
   T* dxc = p.dx ? reinterpret_cast<T*>(p.dx) + (long long)c * hw : nullptr;
-  const float mean = __ldg(p.mean + c);
+  const float mean = ld_here(p.mean + c);
   const f32x2 mean2 = splat2(mean);
   const float slope = p.slope;
-  const float invstd = __ldg(p.invstd + c);  // needed after the sums: requested now
+  const float invstd = ld_here(p.invstd + c);  // needed after the sums: requested now
   const float w = p.weight ? load_param1(p.weight, p.w_dtype, c) : 1.f;
 
   // ---- pass 1 ----------------------------------------------------------------------------------
@@ -595,8 +595,8 @@ __global__ void __launch_bounds__(1024) bn_bwd_nchw_small_kernel(const BnBwdPara
       if constexpr (HAS_ACT) a_raw[k] = *reinterpret_cast<const Vec*>(actc + off[k]);
     }
   }
-  const float mean = __ldg(p.mean + c);
-  const float invstd = __ldg(p.invstd + c);
+  const float mean = ld_here(p.mean + c);
+  const float invstd = ld_here(p.invstd + c);
   const float w = p.weight ? load_param1(p.weight, p.w_dtype, c) : 1.f;
   float g[K][W], xm[K][W];
   float s1 = 0.f, s2 = 0.f;

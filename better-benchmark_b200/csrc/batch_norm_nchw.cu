@@ -118,7 +118,7 @@ batch_norm_nchw_cluster_kernel(const BatchNormParams p, const int imgs_per_cta, 
 #define B200_NMARK(i)
 #endif
   B200_NMARK(0)
-  const float shift = Elem<T>::to_f32(__ldg(xc));  // the channel's first element: every CTA of the cluster reads the same one
+  const float shift = Elem<T>::to_f32(ld_here(xc));  // the channel's first element: every CTA of the cluster reads the same one
   const f32x2 shift2 = splat2(shift);
   // everything pass 2 and the statistics need besides x is requested now, so that it arrives
   // while pass 1 runs instead of costing a round trip of its own later

@@ -176,7 +176,8 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
 }
 
 // One value of 2 or 4 bytes, asked for where the call stands: neither in front of wait_for_previous_kernel nor behind
-// the copies that are to follow it.
+// the copies that are to follow it. (Not __ldg: it promises the compiler data that does not change while the kernel runs, which
+// here begins before the kernel that writes it has ended.) Registers and times are those of __ldg.
 template <typename T>
 __device__ __forceinline__ T ld_here(const T* p) {
   static_assert(sizeof(T) == 2 || sizeof(T) == 4, "scalars");
@@ -194,7 +195,9 @@ __device__ __forceinline__ T ld_here(const T* p) {
 }
 
 __device__ __forceinline__ uint4 ld_keep(const void* p) {
-  return __ldg(reinterpret_cast<const uint4*>(p));
+  uint4 r;
+  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
 }
 
 // Plain (coherent) 16-byte load: for data another CTA of the same grid wrote earlier.

@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(128) softmax_dropout_kernel(SoftmaxDropoutPara
         float f[8], bv[8];
         const uint4 raw = ld_stream(x + base + 8 * v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) bv[j] = __ldg(brow + (long long)(8 * v + j) * p.sk);
+        for (int j = 0; j < 8; ++j) bv[j] = ld_here(brow + (long long)(8 * v + j) * p.sk);
         Elem<T>::unpack(raw, f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {

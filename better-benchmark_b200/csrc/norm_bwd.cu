@@ -92,8 +92,8 @@ norm_bwd_kernel(const NormBwdParams p) {
         }
       }
     }
-    const float rstd = __ldg(p.rstd + row);
-    const float mean = LN ? __ldg(p.mean + row) : 0.f;
+    const float rstd = ld_here(p.rstd + row);
+    const float mean = LN ? ld_here(p.mean + row) : 0.f;
 
     float xf[CH][V], gf[CH][V];
     float s1 = 0.f, s2 = 0.f;
@@ -290,8 +290,8 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
     const bool arrived = mbar_wait(&full[st], phase);
     const unsigned char* sx = smem + (size_t)st * 2 * row_bytes;
     const unsigned char* sy = sx + row_bytes;
-    const float rstd = __ldg(p.rstd + row);
-    const float mean = LN ? __ldg(p.mean + row) : 0.f;
+    const float rstd = ld_here(p.rstd + row);
+    const float mean = LN ? ld_here(p.mean + row) : 0.f;
     const f32x2 rstd2 = splat2(rstd), mean2 = splat2(mean);
 
     f32x2 xv[CH][V / 2], gv[CH][V / 2];
@@ -572,8 +572,8 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
     float rstd[R], mean[LN ? R : 1];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      rstd[r] = r < nrows ? __ldg(p.rstd + row0 + r) : 0.f;
-      if constexpr (LN) mean[r] = r < nrows ? __ldg(p.mean + row0 + r) : 0.f;
+      rstd[r] = r < nrows ? ld_here(p.rstd + row0 + r) : 0.f;
+      if constexpr (LN) mean[r] = r < nrows ? ld_here(p.mean + row0 + r) : 0.f;
     }
     const bool arrived = mbar_wait(&full[st], phase);
     const unsigned char* sx = smem + (size_t)st * stage_bytes + (size_t)(grp * R) * row_bytes + (size_t)tid * 16;
@@ -852,13 +852,13 @@ __global__ void __launch_bounds__(G == 0 ? 512 : 256, G == 0 ? 1 : 2) norm_bwd_r
   auto fetch = [&](long long row) {
     const T* x = reinterpret_cast<const T*>(p.x) + row * p.x_row_stride;
     const T* dy = reinterpret_cast<const T*>(p.dy) + row * p.dy_row_stride;
-    rstd_next = __ldg(p.rstd + row);
-    if constexpr (LN) mean_next = __ldg(p.mean + row);
+    rstd_next = ld_here(p.rstd + row);
+    if constexpr (LN) mean_next = ld_here(p.mean + row);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int i = e * gs + lane;
-      nx[e] = i < n ? __ldg(x + i) : Elem<T>::from_f32(0.f);
-      ny[e] = i < n ? __ldg(dy + (p.dy_elem_stride ? i : 0)) : Elem<T>::from_f32(0.f);
+      nx[e] = i < n ? ld_here(x + i) : Elem<T>::from_f32(0.f);
+      ny[e] = i < n ? ld_here(dy + (p.dy_elem_stride ? i : 0)) : Elem<T>::from_f32(0.f);
     }
   };
   if (AHEAD && first < p.rows) fetch(first);

@@ -98,7 +98,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
       for (int i = 0; i < P; ++i) wv[c][i] = pack2(wf[2 * i], wf[2 * i + 1]);
     }
   }
-  const float dyf = DYS ? Elem<T>::to_f32(__ldg(dyg)) : 0.f;
+  const float dyf = DYS ? Elem<T>::to_f32(ld_here(dyg)) : 0.f;
   // the other lanes first touch the barriers after the __syncthreads below
   int issued = 0;
   if (lane == 0) {
@@ -178,13 +178,13 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   int row = gwarp;
 
   // the row statistics are fetched one row ahead, so that their latency is never waited for
-  float rstd_next = my_rows > 0 ? __ldg(p.rstd + row) : 0.f;
-  float mean_next = (LN && my_rows > 0) ? __ldg(p.mean + row) : 0.f;
+  float rstd_next = my_rows > 0 ? ld_here(p.rstd + row) : 0.f;
+  float mean_next = (LN && my_rows > 0) ? ld_here(p.mean + row) : 0.f;
   for (int k = 0; k < my_rows; ++k, row += gstep) {
     const float rstd = rstd_next, mean = mean_next;
     if (k + 1 < my_rows) {
-      rstd_next = __ldg(p.rstd + row + gstep);
-      if constexpr (LN) mean_next = __ldg(p.mean + row + gstep);
+      rstd_next = ld_here(p.rstd + row + gstep);
+      if constexpr (LN) mean_next = ld_here(p.mean + row + gstep);
     }
     const bool arrived = __all_sync(0xffffffffu, mbar_wait(&full[slot], phase));
     if (!arrived) {

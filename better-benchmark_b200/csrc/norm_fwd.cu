@@ -989,11 +989,11 @@ norm_fwd_ragged_kernel(const NormFwdParams p) {
   const int n = p.n;
   float f[E];
 #pragma unroll
-  for (int e = 0; e < E; ++e) f[e] = e * gs + lane < n ? Elem<Tin>::to_f32(__ldg(x + e * gs + lane)) : 0.f;
+  for (int e = 0; e < E; ++e) f[e] = e * gs + lane < n ? Elem<Tin>::to_f32(ld_here(x + e * gs + lane)) : 0.f;
   if (res) {
     float r[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) r[e] = e * gs + lane < n ? Elem<Tin>::to_f32(__ldg(res + e * gs + lane)) : 0.f;
+    for (int e = 0; e < E; ++e) r[e] = e * gs + lane < n ? Elem<Tin>::to_f32(ld_here(res + e * gs + lane)) : 0.f;
     Tin* so = p.sum_out && valid ? reinterpret_cast<Tin*>(p.sum_out) + row * (long long)n : nullptr;
 #pragma unroll
     for (int e = 0; e < E; ++e) {

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) transpose16_ragged_kernel(const Transpose
     for (int i = 0; i < 8; ++i) {  // rows 2 (4 warp + i / 2) + (i & 1)
       const int r = warp * 8 + i;
       w[i] = r < np && 2 * lane < nc
-                 ? __ldg(reinterpret_cast<const uint32_t*>(src + (long long)r * p.in_row_stride) + lane) : 0u;
+                 ? ld_here(reinterpret_cast<const uint32_t*>(src + (long long)r * p.in_row_stride) + lane) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(256) transpose16_ragged_kernel(const Transpose
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = warp * 8 + i, c = lane + 32 * h;
-        e[h][i] = r < np && c < nc ? __ldg(src + (long long)r * p.in_row_stride + c) : (unsigned short)0;
+        e[h][i] = r < np && c < nc ? ld_here(src + (long long)r * p.in_row_stride + c) : (unsigned short)0;
       }
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(256) transpose_pairs_kernel(const TransposePar
     const unsigned char* block = pairs_smem + (size_t)slot * span;
     if (tid * 2 < bytes - whole)  // the last group may end between two 16-byte boundaries
       *reinterpret_cast<unsigned short*>(pairs_smem + (size_t)slot * span + whole + tid * 2) =
-          __ldg(reinterpret_cast<const unsigned short*>(reinterpret_cast<const unsigned char*>(p.x) +
+          ld_here(reinterpret_cast<const unsigned short*>(reinterpret_cast<const unsigned char*>(p.x) +
                                                         g * group * p.in_batch_stride * 2 + whole) + tid);
     if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the block before has left
     __syncthreads();

@@ -376,7 +376,8 @@ __device__ __forceinline__ void load_param(const void* base, int dtype, long lon
       uint4 r = ld_keep(q);
       w[0] = r.x; w[1] = r.y; w[2] = r.z; w[3] = r.w;
     } else {
-      uint2 r = __ldg(reinterpret_cast<const uint2*>(q));
+      uint2 r;
+      asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(q));
       w[0] = r.x; w[1] = r.y;
     }
 #pragma unroll
@@ -395,10 +396,10 @@ __device__ __forceinline__ void load_param(const void* base, int dtype, long lon
 
 // Scalar parameter load with run-time dtype.
 __device__ __forceinline__ float load_param1(const void* base, int dtype, long long idx) {
-  if (dtype == B200_F32) return __ldg(reinterpret_cast<const float*>(base) + idx);
+  if (dtype == B200_F32) return ld_here(reinterpret_cast<const float*>(base) + idx);
   if (dtype == B200_BF16)
-    return __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(base) + idx));
-  return __half2float(__ldg(reinterpret_cast<const __half*>(base) + idx));
+    return __bfloat162float(ld_here(reinterpret_cast<const __nv_bfloat16*>(base) + idx));
+  return __half2float(ld_here(reinterpret_cast<const __half*>(base) + idx));
 }
 
 // N parameters at a distance of `step`, those at n and beyond as 0: the type is asked for once, so that all loads are
@@ -410,7 +411,7 @@ __device__ __forceinline__ void load_params_strided(const void* base, int dtype,
     const P* p = reinterpret_cast<const P*>(base);
     P raw[N];
 #pragma unroll
-    for (int e = 0; e < N; ++e) raw[e] = first + e * step < n ? __ldg(p + first + e * step) : Elem<P>::from_f32(0.f);
+    for (int e = 0; e < N; ++e) raw[e] = first + e * step < n ? ld_here(p + first + e * step) : Elem<P>::from_f32(0.f);
 #pragma unroll
     for (int e = 0; e < N; ++e) out[e] = Elem<P>::to_f32(raw[e]);
   };

@@ -367,11 +367,11 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 ? 2 : 0)
     Tin xv[E], mv[E];
 #pragma unroll
     for (int e = 0; e < E; ++e)
-      if (e * gs + lane < p.n) xv[e] = __ldg(x + e * gs + lane);
+      if (e * gs + lane < p.n) xv[e] = ld_here(x + e * gs + lane);
     if (m) {
 #pragma unroll
       for (int e = 0; e < E; ++e)
-        if (e * gs + lane < p.n) mv[e] = __ldg(m + e * gs + lane);
+        if (e * gs + lane < p.n) mv[e] = ld_here(m + e * gs + lane);
     }
 #pragma unroll
     for (int e = 0; e < E; ++e) {

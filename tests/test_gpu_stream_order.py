@@ -17,6 +17,9 @@ def _calls():
     rstd, mean = torch.full((2000,), 0.7, device="cuda"), torch.full((2000,), 0.1, device="cuda")
     cl = lambda t: t.view(8, 28, 28, 64).permute(0, 3, 1, 2)  # noqa: E731
     ones = torch.ones(64, device="cuda")
+    seeds = torch.tensor([11, 12], device="cuda")
+    res = torch.linspace(-1, 1, 2000 * 512, device="cuda").view(2000, 512)
+    bias = torch.linspace(-2, 2, 64 * 256, device="cuda").view(1, 1, 64, 256).expand(2, 12, 64, 256)
     return {
         "cast": ((2000, 768), torch.float32, lambda x: k.cast_scale(x, torch.bfloat16)),
         "silu": ((2000, 768), torch.bfloat16, lambda x: k.cast_scale(x, torch.bfloat16, activation="silu")),
@@ -35,11 +38,22 @@ def _calls():
         "batch norm nchw": ((8, 64, 28, 28), torch.float32,
                             lambda x: k.batch_norm_fwd(x, ones, ones, None, None, eps=1e-5, momentum=0.1)),
         "transpose": ((64, 49, 128), torch.bfloat16, lambda x: k.permute_copy(x, (0, 2, 1))),
+        # kernels for ragged rows and columns: scalar loads, of vectors along the row as well as of the row itself
+        "softmax ragged, masked": ((700, 1003), torch.float16, lambda x: k.softmax(x, mask=x)),
+        "layer norm ragged": ((2000, 767), torch.bfloat16, lambda x: k.norm_fwd(x, x[0], x[1], eps=1e-5, want_rstd=True)[:3:2]),
+        "norm backward ragged": ((2000, 767), torch.bfloat16,
+                                 lambda x: k.norm_bwd(x, x, x[0], rstd, mean=mean, rms=False, want_dbias=True)),
+        "transpose ragged": ((16, 501, 333), torch.float16, lambda x: k.permute_copy(x, (0, 2, 1))),
+        "dropout norm": ((2000, 512), torch.bfloat16, lambda x: k.dropout_rms_norm(x, res, w[:512], seeds, 0, 1, p=0.1, eps=1e-6)),
+        "softmax dropout": ((24, 64, 256), torch.bfloat16, lambda x: k.softmax_dropout(x, bias, seeds, 1, p=0.1)),
     }
 
 
 NAMES = ["cast", "silu", "row sum", "column sum", "softmax", "softmax ragged", "layer norm", "residual", "norm backward",
-         "norm backward, weight", "batch norm", "batch norm backward", "batch norm nchw", "transpose"]
+         "norm backward, weight", "batch norm", "batch norm backward", "batch norm nchw", "transpose",
+         "softmax ragged, masked", "layer norm ragged", "norm backward ragged", "transpose ragged", "dropout norm", "softmax dropout"]
+KERNELS = {"softmax ragged, masked": b"b200_softmax [elements in registers]", "layer norm ragged": b"b200_norm_fwd [elements in registers]",
+           "norm backward ragged": b"b200_norm_bwd finalize", "transpose ragged": b"b200_transpose_copy [ragged 16-bit tiles]"}
 
 
 def _list(out):
@@ -56,20 +70,31 @@ def test_inputs_changed_just_before_the_call(name):
         torch.cuda.synchronize()
         want.append(_list(call(s)))
     torch.cuda.synchronize()
+    if name in KERNELS:
+        from better_benchmark_b200 import native
+        assert KERNELS[name] in native.load().b200_last_kernel(), native.load().b200_last_kernel()
     x = torch.empty_like(sources[0])
+    side, main = torch.cuda.Stream(), torch.cuda.current_stream()
     got = []
-    for i in range(40):   # a device copy, or a kernel, or both, and the call right behind it
-        if i % 3 == 0:
-            x.copy_(sources[i % 4])
-        elif i % 3 == 1:
-            torch.add(sources[i % 4], 0, out=x)
-        else:
+    for i in range(48):   # a device copy, a kernel, both, or a kernel of another stream, and the call right behind it
+        new = sources[i // 4 % 4]
+        if i % 4 == 0:
+            x.copy_(new)
+        elif i % 4 == 1:
+            torch.add(new, 0, out=x)
+        elif i % 4 == 2:
             x.zero_()
-            torch.mul(sources[i % 4], 1, out=x)
+            torch.mul(new, 1, out=x)
+        else:   # an event wait lies between what wrote x and the call
+            x.zero_()
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                torch.add(new, 0, out=x)
+            main.wait_stream(side)
         got.append(_list(call(x)))
     torch.cuda.synchronize()
     for i, out in enumerate(got):
-        for a, b in zip(out, want[i % 4]):
+        for a, b in zip(out, want[i // 4 % 4]):
             assert torch.equal(a, b), f"{name}, call {i}"
 
 
