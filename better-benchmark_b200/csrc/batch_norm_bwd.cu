@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) bn_bwd_finalize_kernel(const BnBwdParams 
     if (p.weight) w = load_param1(p.weight, p.w_dtype, c);
   }
   wait_for_previous_kernel();
-  let_next_kernel_start();
+  if (p.dx) let_next_kernel_start();  // without dx this is the call's last kernel
   double s1 = 0.0, s2 = 0.0;
   for (int g0 = tid; g0 < p.splits; g0 += 256 * 4) {
     double a[4], b[4];

@@ -45,13 +45,16 @@ def _calls():
                                  lambda x: k.norm_bwd(x, x, x[0], rstd, mean=mean, rms=False, want_dbias=True)),
         "transpose ragged": ((16, 501, 333), torch.float16, lambda x: k.permute_copy(x, (0, 2, 1))),
         "dropout norm": ((2000, 512), torch.bfloat16, lambda x: k.dropout_rms_norm(x, res, w[:512], seeds, 0, 1, p=0.1, eps=1e-6)),
+        "batch norm backward, sums": ((8, 28, 28, 64), torch.bfloat16,
+                                      lambda x: k.batch_norm_bwd(cl(x), cl(x), ones, ones, ones, want_dx=False)),
         "softmax dropout": ((24, 64, 256), torch.bfloat16, lambda x: k.softmax_dropout(x, bias, seeds, 1, p=0.1)),
     }
 
 
 NAMES = ["cast", "silu", "row sum", "column sum", "softmax", "softmax ragged", "layer norm", "residual", "norm backward",
          "norm backward, weight", "batch norm", "batch norm backward", "batch norm nchw", "transpose",
-         "softmax ragged, masked", "layer norm ragged", "norm backward ragged", "transpose ragged", "dropout norm", "softmax dropout"]
+         "softmax ragged, masked", "layer norm ragged", "norm backward ragged", "transpose ragged", "dropout norm", "softmax dropout",
+         "batch norm backward, sums"]
 KERNELS = {"softmax ragged, masked": b"b200_softmax [elements in registers]", "layer norm ragged": b"b200_norm_fwd [elements in registers]",
            "norm backward ragged": b"b200_norm_bwd finalize", "transpose ragged": b"b200_transpose_copy [ragged 16-bit tiles]"}
 
@@ -96,6 +99,38 @@ def test_inputs_changed_just_before_the_call(name):
     for i, out in enumerate(got):
         for a, b in zip(out, want[i // 4 % 4]):
             assert torch.equal(a, b), f"{name}, call {i}"
+
+
+@pytest.mark.parametrize("channels", [64, 768])
+def test_results_of_one_call_read_by_the_next(channels):
+    """The statistics of a backward without dx are written by its last kernel, and read by the call right behind it."""
+    import better_benchmark_b200.kernels as k
+    g = torch.Generator(device="cuda").manual_seed(9)
+    images = [torch.randn((16, channels, 14, 14), generator=g, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+              for _ in range(5)]
+    dy = images.pop()
+    mean, invstd = torch.full((channels,), 0.1, device="cuda"), torch.full((channels,), 0.7, device="cuda")
+    row = torch.randn((300, channels), generator=g, device="cuda")
+    readers = {
+        "cast": lambda dw, db: k.cast_scale(dw, torch.bfloat16),
+        "row": lambda dw, db: k.row_reduce(db.view(1, -1), "sum"),
+        "weight": lambda dw, db: k.norm_fwd(row, dw, db, eps=1e-5)[0],
+        "batch norm": lambda dw, db: k.batch_norm_bwd(dy, images[0], mean, invstd, dw)[0],
+    }
+    for name, reader in readers.items():
+        want = []
+        for x in images:
+            _, dw, db = k.batch_norm_bwd(dy, x, mean, invstd, None, want_dx=False)
+            torch.cuda.synchronize()
+            want.append(reader(dw, db))
+            torch.cuda.synchronize()
+        got = []
+        for i in range(32):
+            _, dw, db = k.batch_norm_bwd(dy, images[i % 4], mean, invstd, None, want_dx=False)
+            got.append(reader(dw, db))
+        torch.cuda.synchronize()
+        for i, out in enumerate(got):
+            assert torch.equal(out, want[i % 4]), f"{name}, call {i}"
 
 
 @pytest.mark.parametrize("name", ["cast", "layer norm", "norm backward", "batch norm", "batch norm backward", "softmax ragged"])
