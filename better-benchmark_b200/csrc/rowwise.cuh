@@ -198,8 +198,9 @@ __device__ __forceinline__ float hsum2(f32x2 v) {
 // units, |r| < 2^-20), 2^yh comes from the hardware approximation (relative error 2^-22) and the
 // result is 2^yh * (1 + r). Relative error below 3.5e-7 for arguments down to -17 (below 6e-7 over
 // the whole range): the accuracy class of expf (2 ulp), three orders of magnitude below half a
-// bf16/fp16 ulp. The argument must be finite (inf - inf inside the fma would give NaN where
-// exp(-inf) is 0): callers clamp to a finite floor first; NaN stays NaN.
+// bf16/fp16 ulp. x * log2(e) must not overflow, which it does below -2.36e38 and for -inf: inf - inf inside
+// the fma then gives NaN where the exponential is 0. Callers clamp to a floor above that first, or look for the NaN and take the
+// elements again with the floor (softmax_rows_kernel). NaN stays NaN.
 // .ftz: results below 2^-126 become 0 instead of denormals; nothing a 16-bit output or the row sum
 // can see.
 __device__ __forceinline__ f32x2 exp_pair_compensated(f32x2 x) {

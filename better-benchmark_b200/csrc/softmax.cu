@@ -455,10 +455,11 @@ __global__ void __launch_bounds__(1024) softmax_streaming_kernel(const SoftmaxPa
 //     of four bytes). The outputs of a thread's vector are handed over by warp shuffles to where the
 //     next aligned chunk of the output starts, so stores are whole chunks; only a warp's first and
 //     last elements leave one by one.
-// What bounds it: issue slots next to HBM (on the case below the traffic takes 75 us and the instructions about as long), with
-// three CTAs per SM that load, reduce twice and store; scale and log are template parameters, and nothing is clamped
-// unless a difference is infinite. Measured: bf16 [4096, 20005] (rows 20 008 apart) -> fp32 log_softmax 183.7 us with the
-// two-sweep kernel below, 109 us with run-time switches and clamps, 103 here; bf16 [2000, 32001] softmax 192.6 -> 54.6 us.
+// What bounds it: three CTAs per SM, as many as their registers allow, each of which loads its row, reduces it twice and stores it. Their
+// phases cover one another in part: on the case below DRAM is 51 % busy, the issue slots 63 %, no pipe more than 42 %. Scale and log
+// are template parameters, and nothing is clamped as long as the sum of a thread is a number (it is not when a difference lies
+// below -2.36e38). Measured: bf16 [4096, 20005] (rows 20 008 apart) -> fp32 log_softmax 183.7 us with the two-sweep
+// kernel below, 109 us with run-time switches and clamps, 104 here; bf16 [2000, 32001] softmax 192.6 -> 54.6 us.
 // Not taken: the next row brought in by a bulk copy meanwhile (121 us: the loads are not what it waits for), stores
 // whose shift is known at compile time (98.6 us where these take 95.8, rows 20 005 apart).
 // ----------------------------------------------------------------------------------------------
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   constexpr int V = Elem<Tin>::V;
   constexpr int P = V / 2;
   constexpr int VO = V * (int)sizeof(Tout) <= 16 ? V : 16 / (int)sizeof(Tout);
-  constexpr float kFloor = -1e30f;  // differences from the maximum are clamped here: the exponential needs finite ones
+  constexpr float kFloor = -1e30f;  // where differences from the maximum are clamped for the pair exponential
   __shared__ float red[32];
   __shared__ float pairs[2][8];  // cluster: (maximum, sum) of every CTA of the row
   const int tid = threadIdx.x, lane = tid & 31, T_ = blockDim.x;
@@ -655,9 +656,9 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   };
   // fp32 results sum expf, log_softmax too: the errors of the pair exponential have a mean of -4e-8, which the sum
   // keeps (mean error of the log-probabilities of 1003 standard normals times two +2.7e-8, against -1.3e-8; without that
-  // mean it would take 4 % less, with errors up to 2 % larger in some cases and smaller in others). expf takes infinite
-  // differences as they are; the pair exponential does not: a thread whose sum is not a number takes its elements
-  // again with a floor under them.
+  // mean it would take 4 % less, with errors up to 2 % larger in some cases and smaller in others). expf takes
+  // differences of any size; the pair exponential none below -2.36e38: a thread whose sum is not a number takes its
+  // elements again with a floor under them.
   float s;
   bool finite = true;
   if constexpr (sizeof(Tout) == 4) {
@@ -725,7 +726,7 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
     }
   };
   if constexpr (sizeof(Tout) == 2 && !LOG) {
-    // the differences of the sum were finite; in a cluster they were taken from another maximum
+    // the differences of the sum were in its range; in a cluster they were taken from another maximum
     if (!CLUSTER && __all_sync(0xffffffffu, finite)) store_all(std::true_type{});
     else store_all(std::false_type{});
   } else {

@@ -602,6 +602,29 @@ def test_softmax_rows_with_infinite_logits(n, dtype, out):
             _near(g[finite], w[finite], f"softmax with -inf, {n} log={log} scale={scale}", floor=2e-6 if log else 1.2e-7)
 
 
+@pytest.mark.parametrize("dtype,out", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32),
+                                       (torch.bfloat16, torch.float32), (torch.float32, torch.float16)])
+@pytest.mark.parametrize("n", [1003, 20483, 30001, 70001])
+def test_softmax_rows_with_logits_as_low_as_the_type_goes(n, dtype, out):
+    """Finite differences whose product with log2(e) is not: probability 0, whatever the exponential makes of them on the way."""
+    x = _randn((5, n), dtype, n, 2.0)
+    x[0, 3:200] = -3e38
+    x[1, 1:] = -3e38
+    x[2, ::3] = -2.4e38
+    x[2, 0] = 1e38          # the difference itself overflows
+    x[3] = -3e38            # all alike: 1 / n
+    x[4, :n // 2] = -1e30
+    d = x.double()
+    for scale in (None, 0.5):
+        t = d if scale is None else d * scale
+        _near(_kernels().softmax(x, out_dtype=out, scale=scale), torch.softmax(t, -1), f"low logits {n} {scale}", floor=1.2e-7)
+        if out != torch.float16:
+            got, want = _kernels().softmax(x, log=True, out_dtype=out, scale=scale), torch.log_softmax(t, -1)
+            inside = want > -3.38e38
+            _near(got[inside], want[inside], f"low logits, log {n} {scale}", floor=2e-6)
+            assert (got[~inside] <= -3.38e38).all()
+
+
 @pytest.mark.parametrize("mask_shape", [(1, 1, 1), (4, 1, 1), (1, 3, 1), (1, 1, 5), (4, 1, 5), (4, 3, 1), (1, 3, 5), (4, 3, 5)])
 @pytest.mark.parametrize("n", [64, 100, 1000])
 def test_softmax_of_every_broadcast_mask_and_outer_order(n, mask_shape):
