@@ -282,7 +282,7 @@ def check_device_waits():
     lib = native.load()
     kernels.check_scratch_status()
     gave_up = {name: int(getattr(lib, name)()) for name in
-               ("b200_norm_fwd_wait_timeouts", "b200_norm_bwd_wait_timeouts", "b200_batch_norm_wait_timeouts")}
+               ("b200_norm_fwd_wait_timeouts", "b200_norm_bwd_wait_timeouts")}
     if any(gave_up.values()):
         raise RuntimeError(f"device-side waits ran out during the timed region: {gave_up}")
 

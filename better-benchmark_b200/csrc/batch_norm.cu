@@ -19,7 +19,6 @@
 #include "batch_norm.cuh"
 #include "tile_stream.cuh"
 
-#include <cstdlib>
 #include <mutex>
 #include <type_traits>
 
@@ -52,9 +51,7 @@ __device__ __forceinline__ uint4 relu_packed(uint4 packed) {
   return packed;
 }
 
-template <typename T, bool VECTOR>
-__device__ __forceinline__ void bn_finalize_channel(const BatchNormParams& p, int c, int num_partials,
-                                                    float shift) {
+__device__ __forceinline__ void bn_finalize_channel(const BatchNormParams& p, int c, int num_partials, float shift) {
   // Called by one warp per channel: lanes split the partials, fp64 accumulation, fixed order.
   const int lane = threadIdx.x & 31;
   float old_mean = 0.f, old_var = 0.f;  // requested now, so that they do not cost a round trip after the sums
@@ -84,7 +81,7 @@ __device__ __forceinline__ void bn_finalize_channel(const BatchNormParams& p, in
   }
   if (lane == 0) {
     float mean, invstd;
-    bn_channel_stats(p, c, s1, s2, shift, true, &mean, &invstd, true, old_mean, old_var);
+    bn_channel_stats(p, c, s1, s2, shift, true, &mean, &invstd, old_mean, old_var);
     p.stats[c] = mean;
     p.stats[p.channels + c] = invstd;
   }
@@ -131,7 +128,7 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_general_kernel(const 
   if (c >= p.channels) return;
   const T* x = reinterpret_cast<const T*>(p.x);
   const float shift = rows_shift ? bn_shift_scalar<T>(x, c, p.channels, p.rows) : Elem<T>::to_f32(x[(long long)c * p.sc]);
-  bn_finalize_channel<T, false>(p, c, num_partials, shift);
+  bn_finalize_channel(p, c, num_partials, shift);
 }
 
 template <typename T>
@@ -352,7 +349,7 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
   if (*rc != B200_OK) return true;
   launch_dependent(batch_norm_finalize_general_kernel<T>, (p.channels + 7) / 8, 256, 0, st, p, (int)splits, rows_shift);
   *rc = launch_status("b200_batch_norm_fwd finalize");
-  if (*rc != B200_OK || !p.y) return true;
+  if (*rc != B200_OK) return true;
   if (threads <= 256) launch_dependent(batch_norm_apply_cl_flat_kernel<T, 256>, (unsigned)splits, threads, 0, st, p, per, (int)PV);
   else launch_dependent(batch_norm_apply_cl_flat_kernel<T, 512>, (unsigned)splits, threads, 0, st, p, per, (int)PV);
   *rc = launch_status("b200_batch_norm_fwd apply [channels-last, flat vectors]");
@@ -577,7 +574,7 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_ring_kernel(const Bat
       shift = bn_round_shift(__fmul_rn(shift, 1.0f / BN_SHIFT_ROWS));
     }
     float mean, invstd;
-    bn_channel_stats(p, c, s1, s2, shift, true, &mean, &invstd, true, old_mean, old_var);
+    bn_channel_stats(p, c, s1, s2, shift, true, &mean, &invstd, old_mean, old_var);
     p.stats[c] = mean;
     p.stats[p.channels + c] = invstd;
   }
@@ -709,7 +706,7 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
     launch_dependent(batch_norm_finalize_ring_kernel<T>, dim3((unsigned)p.channels), dim3(256), 0, st, p, (int)splits,
                      kind != kShiftRow0 ? 1 : 0);
     *rc = launch_status("b200_batch_norm_fwd finalize");
-    if (*rc != B200_OK || !p.y) return;
+    if (*rc != B200_OK) return;
     launch_dependent(apply, dim3((unsigned)splits), dim3((unsigned)threads), ring, st, p, total, (int)PV);
     *rc = launch_status("b200_batch_norm_fwd apply [channels-last, flat vectors, copy rings]");
   };
@@ -747,20 +744,16 @@ static int launch_batch_norm(BatchNormParams p, bool channels_last, size_t scrat
   launch_dependent(batch_norm_finalize_general_kernel<T>, (p.channels + 7) / 8, 256, 0, st, p, (int)splits, 0);
   rc = launch_status("b200_batch_norm_fwd finalize");
   if (rc != B200_OK) return rc;
-  if (p.y) {
-    launch_dependent(batch_norm_apply_general_kernel<T>, dim3(p.channels, (unsigned)splits), 256, 0, st, p);
-    rc = launch_status("b200_batch_norm_fwd apply [strided, element-wise]");
-  }
-  return rc;
+  launch_dependent(batch_norm_apply_general_kernel<T>, dim3(p.channels, (unsigned)splits), 256, 0, st, p);
+  return launch_status("b200_batch_norm_fwd apply [strided, element-wise]");
 }
 
 }  // namespace b200
 
 using namespace b200;
 
-// Bounded waits that ran out since the library was loaded: none of these kernels waits on a copy barrier, so 0.
-// Synchronises the device.
-extern "C" int64_t b200_batch_norm_wait_timeouts(void) { return (int64_t)read_wait_timeouts(); }
+// Bounded waits that ran out since the library was loaded: none of these kernels has one.
+extern "C" int64_t b200_batch_norm_wait_timeouts(void) { return 0; }
 
 static int64_t batch_norm_scratch_for(int64_t rows, int64_t channels) {  // so many partial rows, and the statistics
   return 256 + (rows * 2 * channels + 2 * channels) * (int64_t)sizeof(float);

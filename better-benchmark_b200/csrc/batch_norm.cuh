@@ -70,11 +70,11 @@ __device__ __forceinline__ float bn_shift_scalar(const T* x, int c, int channels
 
 // Turns the fp64 totals of the shifted sums of one channel into mean / invstd and, for the one
 // caller that owns the channel's global outputs, writes the saved and running statistics.
-// have_old: the caller already holds the channel's running statistics (fetched while the sums
-// were being formed, so that their latency is not waited for here).
+// old_mean, old_var: the channel's running statistics, which the caller fetched while the sums were being formed, so that
+// their latency is not waited for here.
 __device__ __forceinline__ void bn_channel_stats(const BatchNormParams& p, int c, double s1, double s2, float shift,
                                                  bool write_global, float* mean_out, float* invstd_out,
-                                                 bool have_old = false, float old_mean = 0.f, float old_var = 0.f) {
+                                                 float old_mean, float old_var) {
   // On the critical path of every launch (one thread per channel computes this while the others
   // wait), so no fp64 division or square root: a product with 1/count and the fp64 rsqrt.
   const double mean_shifted = s1 * p.inv_count;
@@ -91,10 +91,6 @@ __device__ __forceinline__ void bn_channel_stats(const BatchNormParams& p, int c
     if (p.save_mean) p.save_mean[c] = mean;
     if (p.save_invstd) p.save_invstd[c] = invstd;
     if (p.running_mean) {
-      if (!have_old) {
-        old_mean = p.running_mean[c];
-        old_var = p.running_var[c];
-      }
       p.running_mean[c] = mean * p.momentum + old_mean * p.one_minus_momentum;
       p.running_var[c] = (varf * p.unbias) * p.momentum + old_var * p.one_minus_momentum;
     }

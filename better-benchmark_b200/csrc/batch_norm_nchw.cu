@@ -189,7 +189,7 @@ batch_norm_nchw_cluster_kernel(const BatchNormParams p, const int imgs_per_cta, 
         t2 += remote[1];
       }
       float mean, invstd;
-      bn_channel_stats(p, c, t1, t2, shift, cluster.block_rank() == 0, &mean, &invstd, true, old_mean, old_var);
+      bn_channel_stats(p, c, t1, t2, shift, cluster.block_rank() == 0, &mean, &invstd, old_mean, old_var);
       stat[0] = mean;
       stat[1] = invstd;
     }
@@ -197,7 +197,7 @@ batch_norm_nchw_cluster_kernel(const BatchNormParams p, const int imgs_per_cta, 
   } else {
     if (tid == 0) {
       float mean, invstd;
-      bn_channel_stats(p, c, cta_tot[0], cta_tot[1], shift, true, &mean, &invstd, true, old_mean, old_var);
+      bn_channel_stats(p, c, cta_tot[0], cta_tot[1], shift, true, &mean, &invstd, old_mean, old_var);
       stat[0] = mean;
       stat[1] = invstd;
     }

@@ -200,16 +200,6 @@ __device__ __forceinline__ uint4 ld_keep(const void* p) {
   return r;
 }
 
-// Plain (coherent) 16-byte load: for data another CTA of the same grid wrote earlier.
-__device__ __forceinline__ uint4 ld_coherent(const void* p) {
-  uint4 r;
-  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(p)
-               : "memory");
-  return r;
-}
-
 __device__ __forceinline__ void st_stream(void* p, const uint4& v) {
 #ifdef B200_ST_STREAM_DEFAULT
   // build variant for measurements: write-once results with the default cache policy
@@ -233,16 +223,7 @@ __device__ __forceinline__ void st_stream32(void* p, const uint4& a, const uint4
                : "memory");
 }
 
-__device__ __forceinline__ void st_default(void* p, const uint4& v) {
-  *reinterpret_cast<uint4*>(p) = v;
-}
-
 // L2 eviction-priority policies (createpolicy) for data that should stay in, or leave, L2.
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-  uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
-}
 __device__ __forceinline__ uint64_t l2_policy_evict_normal() {
   uint64_t pol;
   asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
@@ -261,12 +242,6 @@ __device__ __forceinline__ uint4 ld_policy(const void* p, uint64_t pol) {
                : "memory");
   return r;
 }
-__device__ __forceinline__ void st_policy(void* p, const uint4& v, uint64_t pol) {
-  asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "r"(v.x),
-               "r"(v.y), "r"(v.z), "r"(v.w), "l"(pol)
-               : "memory");
-}
-
 // ----------------------------------------------------------------------------------------
 // Reductions. Orders are fixed (butterfly within a warp, then warp 0..n-1 in sequence), so
 // every launch of the same shape produces the same bits.

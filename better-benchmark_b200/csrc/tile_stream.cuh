@@ -64,16 +64,6 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, 
       : "memory");
 }
 
-// The same copy with an L2 eviction-priority policy (createpolicy) attached.
-__device__ __forceinline__ void bulk_load_hint(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar,
-                                               uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::
-          "r"(smem_u32(smem_dst)),
-      "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
-      : "memory");
-}
-
 // 16-byte asynchronous copies that a thread issues for itself. They complete in groups; a thread that
 // only ever reads its own slots needs no barrier after copy_async_wait (which leaves the N newest groups
 // in flight).

@@ -725,7 +725,7 @@ def device_wait_failures() -> dict:
     except native.KernelArgumentError as e:
         found["grid_barrier"] = str(e)[:200]
     seen = getattr(device_wait_failures, "_seen", {})
-    for name in ("b200_norm_fwd_wait_timeouts", "b200_norm_bwd_wait_timeouts", "b200_batch_norm_wait_timeouts"):
+    for name in ("b200_norm_fwd_wait_timeouts", "b200_norm_bwd_wait_timeouts"):
         total = int(getattr(lib, name)())
         if total > seen.get(name, 0):
             found[name] = total - seen.get(name, 0)
