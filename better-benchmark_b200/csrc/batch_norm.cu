@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_ring_kernel(const Bat
     if (rows_shift) {
       shift = 0.f;
       for (int r = 0; r < BN_SHIFT_ROWS; ++r) shift = __fadd_rn(shift, first_rows[r]);
-      shift = bn_round_shift(__fmul_rn(shift, 1.0f / BN_SHIFT_ROWS));
+      shift = bn_shift_of_sum(shift, first_rows[0]);
     }
     float mean, invstd;
     bn_channel_stats(p, c, s1, s2, shift, true, &mean, &invstd, old_mean, old_var);

@@ -44,6 +44,12 @@ __device__ __forceinline__ float bn_round_shift(float v) {
   return __uint_as_float((__float_as_uint(v) + 0x8000u) & 0xffff0000u);
 }
 
+// The shift from the sum of the sixteen rows; row 0 where that overflows although the values are finite (a channel of 3e37).
+__device__ __forceinline__ float bn_shift_of_sum(float sum, float row0) {
+  const float mean = bn_round_shift(__fmul_rn(sum, 1.0f / BN_SHIFT_ROWS));
+  return fabsf(mean) < INFINITY ? mean : row0;
+}
+
 template <typename T>
 __device__ __forceinline__ void bn_shift_load(const T* x, int c, int channels, long long rows, T (&v)[BN_SHIFT_ROWS]) {
 #pragma unroll
@@ -58,7 +64,7 @@ __device__ __forceinline__ float bn_shift_of(const T (&v)[BN_SHIFT_ROWS]) {
   float s = 0.f;
 #pragma unroll
   for (int r = 0; r < BN_SHIFT_ROWS; ++r) s = __fadd_rn(s, Elem<T>::to_f32(v[r]));
-  return bn_round_shift(__fmul_rn(s, 1.0f / BN_SHIFT_ROWS));
+  return bn_shift_of_sum(s, Elem<T>::to_f32(v[0]));
 }
 
 template <typename T>

@@ -433,6 +433,23 @@ def test_batch_norm_statistics_with_a_first_row_far_from_the_mean(mb, c, dtype):
     assert ((mean.double() - mean64) / var64.sqrt()).abs().max().item() <= 2.0 ** -24
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("mb", [4, 10, 60])   # the three kinds of shift
+def test_batch_norm_of_channels_whose_rows_add_up_to_more_than_fp32_holds(mb, dtype):
+    """Sixteen rows of 3e37 have a finite mean but not a finite sum: mean 3e37 and variance 0 all the same, beside ordinary channels."""
+    n = int(mb * 1e6 / dtype.itemsize / 64 / 49) // 8 * 8
+    x = _randn((n, 64, 7, 7), dtype, mb, 2.0)
+    x[:, 5] = 3e37
+    x[:, 63] = -3e37
+    x = x.contiguous(memory_format=torch.channels_last)
+    ones = torch.ones(64, device="cuda")
+    y, mean, invstd = _kernels().batch_norm_fwd(x, ones, ones, None, None, eps=1e-5, momentum=0.1)
+    var64, mean64 = torch.var_mean(x.double(), (0, 2, 3), unbiased=False)
+    _near(mean, mean64, "mean", floor=2e-6)
+    _near(invstd, torch.rsqrt(var64 + 1e-5), "invstd", floor=2e-6)
+    assert (y[:, [5, 63]] == 1).all()
+
+
 @pytest.mark.parametrize("dtype,c", [(torch.bfloat16, 64), (torch.float32, 92), (torch.float16, 320), (torch.bfloat16, 1022)])
 @pytest.mark.parametrize("partial_rows", [295, 148, 5, 1])
 def test_batch_norm_with_room_for_few_partial_rows(partial_rows, dtype, c):
