@@ -64,7 +64,7 @@ def measured_peak():
 
 
 def recorded_traffic(workload):
-    """The committed ncu capture of this workload's kernel (one launch from a flushed L2):
+    """The committed ncu capture of this workload's kernel (one launch from a flushed L2, unless its record gives other conditions):
     {"traffic": read + write DRAM bytes, "traffic_read", "traffic_write", "input_bytes",
     "output_bytes"}, or {} without a capture. A capture ends with the kernel, when part of the
     output is still dirty in L2, so only the read side can be compared with the algorithmic bytes

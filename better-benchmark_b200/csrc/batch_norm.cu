@@ -366,18 +366,19 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
 // copies, read only by the thread that issued them: no barrier, no registers), which keeps about 160 KB
 // per SM on the way whatever the arithmetic does. The three kernels are chained by programmatic
 // dependent launch; apply fills its ring before the statistics are there.
-// Measured against the kernels above: bf16 [672, 96, 28, 28] (101 MB) 87.7 -> 51.5 us, [1010, 92, 14, 14] (36 MB)
-// 48.1 -> 24.5, [161, 96, 28, 28] (24 MB) 34.6 -> 19.5, [64, 120, 28, 28] (12 MB) 20.4 -> 14.5, [40, 480, 7, 7]
-// (2 MB) 12.7 -> 8.6, [8, 24, 7, 7] (20 KB) 11.5 -> 9.3; f32 [1402, 92, 14, 14] (101 MB) 74.8 -> 51.3,
-// [168, 92, 14, 14] (12 MB) 18.3 -> 12.5. Against one cooperative launch for power-of-two vector counts from 8 MB up
+// Measured against the kernels above: bf16 [672, 96, 28, 28] (101 MB) 86.7 -> 49.2 us, [1010, 92, 14, 14] (36 MB)
+// 48.1 -> 24.0, [161, 96, 28, 28] (24 MB) 34.2 -> 19.2, [64, 120, 28, 28] (12 MB) 19.8 -> 13.7, [40, 480, 7, 7]
+// (2 MB) 10.3 -> 8.6, [8, 24, 7, 7] (20 KB) 11.3 -> 7.3; f32 [1402, 92, 14, 14] (101 MB) 74.7 -> 51.6,
+// [168, 92, 14, 14] (12 MB) 18.1 -> 12.5. Against one cooperative launch for power-of-two vector counts from 8 MB up
 // (the tensor's end in shared memory between the passes, two grid barriers): bf16 64 channels 12 / 30 / 60 / 100 / 200 MB
-// 20.0 / 26.3 / 36.7 / 55.5 / 107.7 -> 14.1 / 21.5 / 30.8 / 47.2 / 102.0, 256 channels 52.7 / 60.0 / 70.6 / 87.1 / 140.7 ->
-// 15.8 / 23.7 / 33.9 / 51.1 / 104.6. The same with this file's copies in one cooperative launch: 18.6 / 26.2 / 35.6 / 49.4 / 103.0.
-// What bounds it on 100 MB: the first pass reads x next to the write-back of the last y, the second finds half of x in L2.
+// 20.9 / 27.3 / 37.7 / 56.0 / 107.5 -> 13.3 / 20.8 / 30.8 / 46.7 / 102.5, 256 channels 52.5 / 60.0 / 70.6 / 90.2 / 142.6 ->
+// 14.6 / 22.4 / 32.8 / 51.3 / 104.5. The same with this file's copies in one cooperative launch: 18.6 / 26.2 / 35.6 / 49.4 / 103.0.
+// What bounds it on 100 MB: the first pass reads x next to the write-back of the last y, the second finds 60 % of x in L2.
 // apply reads x evict-first, as nothing reads it again: 53.2 -> 52.0 us (back to back) on bf16 [256, 64, 56, 56].
 // With more than 1024 channels and less than 12 MB the CTAs of the finalize are the larger part of it, and the
-// kernels above stay (bf16 [40, 2040, 7, 7] 19.9 us there, 22.0 here; 16 MB: 33.7 and 27.6; 1020 channels, 8 MB:
-// 18.8 and 17.9; f32 1000 channels, 8 MB: 15.5 and 15.8).
+// kernels above stay (bf16 [40, 2040, 7, 7] 19.0 us there, 20.9 here, [20, 4080, 7, 7] 19.9 and 23.9; 16 MB of 2040 channels 32.8 and 26.6;
+// 1020 channels, 8 MB: 17.8 and 16.5; f32 1000 channels, 8 MB: 14.2 and 14.9). Just above 1024 channels the line could lie lower
+// (1200 channels, 9.4 MB: 24.5 there, 20.4 here).
 // ----------------------------------------------------------------------------------------------
 static bool ring_is_slower(long long channels, long long bytes) { return channels > 1024 && bytes < 12000000; }
 

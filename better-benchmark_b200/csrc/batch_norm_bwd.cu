@@ -84,9 +84,11 @@ __device__ __forceinline__ void bn_bwd_prologue(f32x2 (&g)[Elem<T>::V / 2], cons
 // f32 [200, 485, 8, 8], element-wise before, 145 -> 28. The same kernels with 8 CTAs per SM in turn: 93.6 us
 // where these take 85.9 (bf16 [992, 64, 28, 28]).
 constexpr int kChunk = 4;  // vectors of each tensor in flight per thread
-// What the apply kernel finds in L2: the tensors' last 80 MB, provided that nothing pushes them out. The rest is
-// loaded evict-first, and so is everything in the apply kernel without act: bf16
-// [256, 64, 56, 56] 90.4 -> 82.6 us, half of that size 53.3 -> 46.6 (60 MB a tensor).
+// What the apply kernel finds in L2 (126 MB): the tensors' last 80 MB, provided that nothing pushes them out. The rest is
+// loaded evict-first, and so is everything in the apply kernel without act: bf16 [256, 64, 56, 56] 90.4 -> 82.6 us, half of
+// that size 53.3 -> 46.6; with act, where a tensor keeps a third of it and apply has no policy, 20 / 45 / 100 MB a tensor
+// 29.3 / 56.0 / 117.1 -> 26.0 / 52.4 / 115.1 (64 channels; 480 channels 34.0 / 59.7 / 121.8 -> 30.7 / 56.1 / 119.2). 50 / 65 / 80 / 95 / 110 MB kept, 45 MB a
+// tensor: 38.1 / 36.2 / 35.3 / 35.5 / 35.5 us, with act 55.0 / 53.1 / 52.2 / 51.7 / 51.8.
 constexpr long long kStaysBytes = 80000000;
 
 // MAXT: 256 threads, or 512 for patterns of more than 256 vectors (one CTA per SM of as many threads).

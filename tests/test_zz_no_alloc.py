@@ -48,7 +48,7 @@ def _inputs(shape, dtype, channels_last, seed):
 
 
 @pytest.mark.parametrize("shape,dtype,channels_last", [
-    ((16, 64, 28, 28), torch.bfloat16, True),     # fused cooperative path
+    ((16, 64, 28, 28), torch.bfloat16, True),     # channels-last, copy rings
     ((8, 40, 13, 13), torch.float32, False),      # NCHW path (needs no scratch at all)
     ((6, 20, 5, 5), torch.float32, True),         # channel count that is no multiple of the vector: three-launch path
 ])
