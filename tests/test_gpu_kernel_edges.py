@@ -433,6 +433,27 @@ def test_batch_norm_statistics_with_a_first_row_far_from_the_mean(mb, c, dtype):
     assert ((mean.double() - mean64) / var64.sqrt()).abs().max().item() <= 2.0 ** -24
 
 
+@pytest.mark.parametrize("c,mb,dtype", [(8, 300, torch.bfloat16), (64, 300, torch.float32), (1024, 300, torch.bfloat16)])
+def test_batch_norm_statistics_of_long_sums(c, mb, dtype):
+    """Hundreds of additions per thread, in three levels of fp32 sums below fp64 ones: through the wrapper, and through the entry point
+    that brings room for 160 partial rows of 1024 channels. Half an fp32 step for the rounding of a result, as much for the sums."""
+    k = _kernels()
+    n = int(mb * 1e6 / dtype.itemsize / c / 49) // 8 * 8
+    x = _randn((n, c, 7, 7), dtype, c, 2.0).contiguous(memory_format=torch.channels_last)
+    ones = torch.ones(c, device="cuda")
+    results = [k.batch_norm_fwd(x, ones, ones, None, None, eps=1e-5, momentum=0.1)[1:]]
+    y, mean, invstd = torch.empty_like(x), torch.empty(c, device="cuda"), torch.empty(c, device="cuda")
+    k.check(k.load().b200_batch_norm_fwd_static_scratch(
+        x.data_ptr(), y.data_ptr(), ones.data_ptr(), ones.data_ptr(), None, None, mean.data_ptr(), invstd.data_ptr(), n, c, 49,
+        x.stride(0), x.stride(1), x.stride(3), k._code(x), k.F32, 1e-5, 0.1, 0, k._stream()), "b200_batch_norm_fwd_static_scratch")
+    results.append((mean, invstd))
+    var64, mean64 = torch.var_mean(x.double(), (0, 2, 3), unbiased=False)
+    for mean, invstd in results:
+        worst = (invstd.double() * torch.sqrt(var64 + 1e-5) - 1).abs().max().item()
+        assert worst <= 2.0 ** -23, f"invstd off by {worst:.2e}"
+        assert ((mean.double() - mean64) / var64.sqrt()).abs().max().item() <= 2.0 ** -24
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("mb", [4, 10, 60])   # the three kinds of shift
 def test_batch_norm_of_channels_whose_rows_add_up_to_more_than_fp32_holds(mb, dtype):
