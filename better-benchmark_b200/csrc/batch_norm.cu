@@ -131,6 +131,16 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_general_kernel(const 
   bn_finalize_channel(p, c, num_partials, shift);
 }
 
+// One element of y, at `off` in both tensors.
+template <typename T>
+__device__ __forceinline__ void bn_apply_one(const BatchNormParams& p, long long off, int c) {
+  const float w = p.weight ? load_param1(p.weight, p.w_dtype, c) : 1.f;
+  const float b = p.bias ? load_param1(p.bias, p.w_dtype, c) : 0.f;
+  float o = ((Elem<T>::to_f32(reinterpret_cast<const T*>(p.x)[off]) - p.stats[c]) * p.stats[p.channels + c]) * w + b;
+  if (p.relu) o = o < 0.f ? 0.f : o;
+  reinterpret_cast<T*>(p.y)[off] = Elem<T>::from_f32(o);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) batch_norm_apply_general_kernel(const BatchNormParams p) {
   wait_for_previous_kernel();
@@ -357,7 +367,8 @@ static bool try_launch_batch_norm_cl_flat(BatchNormParams p, size_t scratch_byte
 }
 
 // ----------------------------------------------------------------------------------------------
-// The same three steps as they are taken for most tensors:
+// The same three steps as they are taken for most tensors. These kernels need no whole number of periods or vectors (odd channel
+// counts whose rows are no multiple of 8: bf16 [39, 287, 7, 7] 18.6 us element by element, 8.1 so):
 //   sums      all CTAs are resident and take chunks b, b + grid, ...: the launch moves through the tensor
 //             from front to back as a whole, and what it leaves in L2 is the tensor's last part
 //   finalize  a CTA per channel
@@ -409,9 +420,10 @@ __device__ __forceinline__ void bn_ring_issue(const uint4* x, uint32_t mine, int
 // while they drain; above 88 there is room for one, and 149 to 296 channels need two (bf16, 256 channels, 2 / 4 MB: 9.0 / 9.5 us
 // with 102 registers, 8.0 / 8.7 so).
 enum { kShiftRow0 = 0, kShiftRows = 1, kShiftRowsFirst = 2 };
-template <typename T, int MAXT, int SHIFT>
+// REST: there are elements behind the last whole vector.
+template <typename T, int MAXT, int SHIFT, bool REST>
 __global__ void __launch_bounds__(MAXT, 512 / MAXT)
-batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total, int PV) {
+batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total, int PV, int tail) {
   wait_for_previous_kernel();
   constexpr int V = Elem<T>::V;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -503,6 +515,19 @@ batch_norm_sums_cl_ring_kernel(const BatchNormParams p, long long total, int PV)
     }
     if (++slot == kRingS) slot = 0;
   }
+  if (REST && blockIdx.x == 0 && tid == tail) {  // what is behind the last whole vector
+    const int rest = (int)(p.rows * C - total * V);
+    f32x2 f[V / 2];
+    Pairs<T>::unpack(load_first<T>(xe + total * V, rest), f);
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {
+      float lo, hi;
+      unpack2(sub2(f[i], shift[i]), lo, hi);
+      const f32x2 d = pack2(2 * i < rest ? lo : 0.f, 2 * i + 1 < rest ? hi : 0.f);
+      t1[i] = add2(t1[i], d);
+      t2[i] = fma2(d, d, t2[i]);
+    }
+  }
   let_next_kernel_start();
   __syncthreads();  // every thread has read its ring: the memory is reused
   float* r1 = reinterpret_cast<float*>(smem);  // [2][MAXT][V], then [2][MAXT] fp64
@@ -581,9 +606,9 @@ __global__ void __launch_bounds__(256) batch_norm_finalize_ring_kernel(const Bat
   }
 }
 
-template <typename T, int MAXT>
+template <typename T, int MAXT, bool REST>
 __global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_apply_cl_ring_kernel(const BatchNormParams p, long long total,
-                                                                                    int PV) {
+                                                                                    int PV, int rest) {
   constexpr int V = Elem<T>::V;
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, T_ = blockDim.x, C = p.channels;
@@ -633,6 +658,7 @@ __global__ void __launch_bounds__(MAXT, 512 / MAXT) batch_norm_apply_cl_ring_ker
     }
     if (++slot == kRingS) slot = 0;
   }
+  if (REST && blockIdx.x == 0 && tid < rest) bn_apply_one<T>(p, total * V + tid, (int)((total * V + tid) % C));
   copy_async_wait<0>();
 }
 
@@ -658,8 +684,9 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   while (h) { const long long t = g % h; g = h; h = t; }
   const long long PV = C / g;
   const long long elems = p.rows * C;
-  if (PV > 512 || elems % (PV * V) != 0) return false;  // whole periods only
-  if (ring_is_slower(C, elems * (long long)sizeof(T))) return false;
+  if (PV > 512 || elems < V) return false;
+  // the flat kernels above need whole periods
+  if (elems % (PV * V) == 0 && ring_is_slower(C, elems * (long long)sizeof(T))) return false;
   const long long total = elems / V;
   const long long stats_floats = 2 * C;
   const long long room = ((long long)scratch_bytes - 256) / (long long)sizeof(float) - stats_floats;
@@ -680,12 +707,15 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   }
   p.stats = p.partials + splits * 2 * C;
   const int kind = bn_shift_kind(C, total, (long long)threads * splits);
-  auto run = [&](auto maxt_tag) {
+  // The elements behind the last whole vector belong to the thread of CTA 0 that has the phase of the vector they begin.
+  const int rest = (int)(elems % V), tail = rest ? (int)(total % threads) : -1;
+  auto run = [&](auto maxt_tag, auto rest_tag) {
     constexpr int MAXT = decltype(maxt_tag)::value;
-    auto sums = kind == kShiftRow0   ? batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRow0>
-                : kind == kShiftRows ? batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRows>
-                                     : batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRowsFirst>;
-    auto apply = batch_norm_apply_cl_ring_kernel<T, MAXT>;
+    constexpr bool REST = decltype(rest_tag)::value;
+    auto sums = kind == kShiftRow0   ? batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRow0, REST>
+                : kind == kShiftRows ? batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRows, REST>
+                                     : batch_norm_sums_cl_ring_kernel<T, MAXT, kShiftRowsFirst, REST>;
+    auto apply = batch_norm_apply_cl_ring_kernel<T, MAXT, REST>;
     const size_t ring = (size_t)kRingBytesPerThread * MAXT;  // 96 KB, or 192 KB: two CTAs, or one, per SM
     const size_t with_shifts = ring + (size_t)MAXT * V * sizeof(float);
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(sums), with_shifts);
@@ -701,18 +731,20 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
       *rc = fail((int)e, "b200_batch_norm_fwd: cannot reserve %zu bytes of shared memory: %s", with_shifts, cudaGetErrorString(e));
       return;
     }
-    launch_dependent(sums, (unsigned)splits, threads, with_shifts, st, p, total, (int)PV);
+    launch_dependent(sums, (unsigned)splits, threads, with_shifts, st, p, total, (int)PV, tail);
     *rc = launch_status("b200_batch_norm_fwd sums [channels-last, flat vectors, copy rings]");
     if (*rc != B200_OK) return;
     launch_dependent(batch_norm_finalize_ring_kernel<T>, dim3((unsigned)p.channels), dim3(256), 0, st, p, (int)splits,
                      kind != kShiftRow0 ? 1 : 0);
     *rc = launch_status("b200_batch_norm_fwd finalize");
     if (*rc != B200_OK) return;
-    launch_dependent(apply, dim3((unsigned)splits), dim3((unsigned)threads), ring, st, p, total, (int)PV);
+    launch_dependent(apply, dim3((unsigned)splits), dim3((unsigned)threads), ring, st, p, total, (int)PV, rest);
     *rc = launch_status("b200_batch_norm_fwd apply [channels-last, flat vectors, copy rings]");
   };
-  if (threads <= 256) run(std::integral_constant<int, 256>{});
-  else run(std::integral_constant<int, 512>{});
+  using Narrow = std::integral_constant<int, 256>;
+  using Wide = std::integral_constant<int, 512>;
+  if (rest) threads <= 256 ? run(Narrow{}, std::true_type{}) : run(Wide{}, std::true_type{});
+  else threads <= 256 ? run(Narrow{}, std::false_type{}) : run(Wide{}, std::false_type{});
   return true;
 }
 

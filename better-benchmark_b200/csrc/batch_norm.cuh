@@ -146,6 +146,21 @@ __device__ __forceinline__ void bn_fold_channels(const float* one, const float* 
   }
 }
 
+// A tensor whose elements are no whole number of vectors ends with fewer than V of them. The sums pass reads them
+// one by one, in the thread whose next vector they would begin; the rest of that vector is zero.
+template <typename T>
+__device__ __forceinline__ uint4 load_first(const T* src, int count) {
+  constexpr int V = Elem<T>::V;
+  union {
+    T e[V];
+    uint4 raw;
+  } u;
+  u.raw = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int i = 0; i < V - 1; ++i)
+    if (i < count) u.e[i] = ld_here(src + i);
+  return u.raw;
+}
 // Contiguous NCHW tensors (batch_norm_nchw.cu): one launch, the CTAs that share a channel form a
 // thread-block cluster. Returns false when the shape does not fit (the caller takes another path).
 template <typename T>
