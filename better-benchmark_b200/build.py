@@ -1,7 +1,8 @@
 """Build recipe for the CUDA library: nvcc, sm_100a only, one object per family, in-tree output.
 
 ``python -m better_benchmark_b200.build`` (or ``build_library()``) compiles every ``csrc/*.cu``
-file to an object in ``csrc/_build/`` in parallel and links ``csrc/libb200_oracles.so``.
+file to an object in ``csrc/_build/`` in parallel and links ``csrc/libb200_oracles.so``, and compiles
+``csrc/calls.cpp``, the host side of the most frequent calls, to the extension module ``csrc/b200_calls.so``.
 Objects are rebuilt only when their source (or a shared header) is newer.
 """
 from __future__ import annotations
@@ -16,6 +17,7 @@ from pathlib import Path
 CSRC = Path(__file__).resolve().parent / "csrc"
 BUILD_DIR = CSRC / "_build"
 LIB_PATH = CSRC / "libb200_oracles.so"
+CALLS_PATH = CSRC / "b200_calls.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -40,6 +42,26 @@ def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
     return any(dep.stat().st_mtime > t for dep in [src, *headers, Path(__file__)])
 
 
+def build_calls(force: bool = False) -> Path:
+    """The extension module, against the torch that runs this. It holds no device code."""
+    src = CSRC / "calls.cpp"
+    if not force and not _stale(CALLS_PATH, src, [CSRC.parent.parent / "include" / "b200_oracles.h"]):
+        return CALLS_PATH
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include",
+                Path(sysconfig.get_paths()["include"]), Path(_nvcc()).resolve().parent.parent / "include"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in includes), str(src),
+           "-o", str(CALLS_PATH), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {src.name}:\n{res.stdout}\n{res.stderr}")
+    return CALLS_PATH
+
+
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     BUILD_DIR.mkdir(exist_ok=True)
@@ -58,12 +80,14 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
         obj.with_suffix(".ptxas").write_text(res.stderr)   # registers and spills of every kernel
         return src, res
 
-    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as pool:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, 1 + len(jobs))) as pool:
+        calls = pool.submit(build_calls, force)
         for src, res in pool.map(compile_one, jobs):
             if verbose and res.stderr:
                 print(res.stderr, file=sys.stderr)
             if res.returncode != 0:
                 raise RuntimeError(f"nvcc failed on {src.name}:\n{res.stdout}\n{res.stderr}")
+        calls.result()
 
     objs = [BUILD_DIR / (s.stem + ".o") for s in sources]
     if force or jobs or not LIB_PATH.exists():

@@ -29,6 +29,14 @@ def residual_forward(inputs, *, eps, returns=("y2",)):
     returns, in its order: ``sum3`` / ``sum2`` (the rounded sum, 3-D / 2-D), ``mean`` / ``rstd``
     (``[B, S, 1]`` fp32), ``y3`` / ``y2`` (the output, 3-D / its 2-D view - the same buffer)."""
     x, res, weight, bias, shape3, shape2 = inputs[:6]
+    if ("y3" in returns) != ("y2" in returns) and "sum2" not in returns:
+        # one form of each output: allocated in that form instead of viewed
+        got = kernels.residual_layer_norm_as(x, res, weight, bias, shape3, shape2, eps=eps, y_in_second="y2" in returns,
+                                             want_sum="sum3" in returns, want_mean="mean" in returns, want_rstd="rstd" in returns)
+        if got is not None:
+            pick = {"y3": got[0], "y2": got[0], "mean": got[1], "rstd": got[2], "sum3": got[-1]}
+            got = tuple([pick[name] for name in returns])
+            return got[0] if len(got) == 1 else got
     x3 = x.view(_resolve(shape3, x.numel()))
     want_sum = "sum3" in returns or "sum2" in returns
     # both forms of the sum, selected per element: the form that passes the reference's element-wise

@@ -10,7 +10,7 @@ from .. import kernels
 def head_split_forward(inputs):
     x, _flat3, split4, out3 = inputs[:4]
     b, s, h, d = split4
-    return kernels.permute_copy(x.view(b, s, h, d), (0, 2, 1, 3)).view(out3)
+    return kernels.permute_copy_as(x.view(b, s, h, d), (0, 2, 1, 3), out3)
 
 
 def head_merge_forward(inputs):
@@ -26,4 +26,4 @@ def transpose_forward(inputs):
     x, out_shape = inputs[:2]
     nd = x.dim()
     dims = list(range(nd - 2)) + [nd - 1, nd - 2]
-    return kernels.permute_copy(x, dims).view(out_shape)
+    return kernels.permute_copy_as(x, dims, out_shape)

@@ -4,6 +4,10 @@ Each function validates device, dtype and layout, allocates its outputs with tor
 graph capture sees ordinary caching-allocator memory), and launches on the current CUDA stream
 without synchronising. Layouts the kernels cannot address directly raise ``UnsupportedLayout``;
 nothing is ever copied, made contiguous or computed by torch behind the caller's back.
+
+The usual form of the most frequent calls is taken by native code (``csrc/calls.cpp``), which does the same
+in a third of the time and returns None, having done nothing, for every other form; what is written
+here is the whole rule, and raises every error.
 """
 from __future__ import annotations
 
@@ -12,7 +16,7 @@ import functools
 import torch
 
 from . import native
-from .native import F32, BF16, F16, check, i64_array, load
+from .native import F32, BF16, F16, check, i64_array, load, load_calls
 
 _DTYPE_CODE = {torch.float32: F32, torch.bfloat16: BF16, torch.float16: F16}
 
@@ -26,6 +30,16 @@ SOFTMAX_ROUND = 4        # multiply/add in the 16-bit input dtype, results round
 
 class UnsupportedLayout(ValueError):
     """The tensor's strides or dtype have no kernel; the caller must pick another oracle."""
+
+
+_calls = None   # csrc/calls.cpp, loaded by the first call
+_scratch_by_device: dict = {}   # (type, index) -> [buffers, newest and largest last]; see scratch_buffer
+
+
+def _load_calls():
+    global _calls
+    _calls = load_calls(_scratch_by_device)
+    return _calls
 
 
 def _code(t: torch.Tensor) -> int:
@@ -137,6 +151,9 @@ def _numel(shape) -> int:
 def row_reduce(x: torch.Tensor, op: str, *, keepdim: bool = False,
                out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """sum / mean / amax / amin over the last dimension (which must have stride 1)."""
+    got = (_calls or _load_calls()).row_reduce(x, _REDUCE_CODES.get(op, -1), keepdim, out_dtype)
+    if got is not None:
+        return got
     _require_cuda(x)
     if x.dim() < 1:
         raise UnsupportedLayout("row_reduce needs at least one dimension")
@@ -176,6 +193,10 @@ def softmax(x: torch.Tensor, *, mask: torch.Tensor | None = None, scale: float |
     With ``round_intermediates`` the scaled and masked values are rounded to x's dtype the way the
     eager 16-bit graph materialises them.
     """
+    if out is None:
+        got = (_calls or _load_calls()).softmax(x, mask, scale, log, out_dtype, round_intermediates)
+        if got is not None:
+            return got
     _require_cuda(x, mask, out)
     n = x.shape[-1]
     if n > 1 and x.stride(-1) != 1:
@@ -257,6 +278,11 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
     Returns (y, mean, rstd, var) with None for the outputs not requested. Statistics are fp32 with
     x's outer shape (plus a trailing 1 when ``keepdim``).
     """
+    got = (_calls or _load_calls()).norm_fwd(
+        x, weight, bias, eps, rms, out_dtype, want_y, want_mean, want_rstd, want_var, correction, keepdim,
+        _NORM_PROLOGUES.get(prologue, -1), residual, want_sum, _SUM_FORMS.get(round_sum, -1), None, False)
+    if got is not None:
+        return got
     _require_cuda(x, weight, bias, residual)
     rows, n, x_stride = _rows_2d(x, "norm_fwd")
     if residual is not None:
@@ -302,6 +328,14 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
     return (y, mean, rstd, var, total) if want_sum else (y, mean, rstd, var)
 
 
+def residual_layer_norm_as(x, residual, weight, bias, shape, shape2, *, eps: float, y_in_second: bool, want_sum: bool,
+                           want_mean: bool, want_rstd: bool):
+    """``norm_fwd`` of ``x.view(shape) + residual.view(shape)`` with ``round_sum="both"`` and y seen as ``shape`` or ``shape2``, which both
+    have to fit: (y, mean, rstd, var[, sum]), or None where the tensors are not of the usual form."""
+    return (_calls or _load_calls()).norm_fwd(x, weight, bias, eps, False, None, True, want_mean, want_rstd, False, 0.0, True, 0,
+                                              residual, want_sum, _SUM_FORMS["both"], (shape, shape2), y_in_second)
+
+
 # ---------------------------------------------------------------------------------------------
 # Scratch memory. Kernels that combine per-CTA partial results take a caller-provided scratch
 # buffer. One zero-initialised buffer per device is kept here; the first 256 bytes hold the
@@ -312,7 +346,6 @@ def norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Tensor | 
 # Growing while the current stream is being captured is refused (the new buffer would belong to
 # that graph's private pool while later, uncaptured calls keep using it).
 # ---------------------------------------------------------------------------------------------
-_scratch_by_device: dict = {}   # (type, index) -> [buffers, newest and largest last]
 SCRATCH_DEFAULT_BYTES = 64 << 20  # covers every kernel of the library for rows of up to 4096 elements
 
 
@@ -365,6 +398,9 @@ def norm_bwd(x: torch.Tensor, dy: torch.Tensor, weight: torch.Tensor | None, rst
     for LayerNorm) are fp32 with one value per row. Returns (dx, dweight, dbias); the gradients of
     weight and bias are fp32 [n].
     """
+    got = (_calls or _load_calls()).norm_bwd(x, dy, weight, rstd, mean, rms, heads, want_dweight, want_dbias, two_launch, scratch)
+    if got is not None:
+        return got
     _require_cuda(x, dy, weight, rstd, mean, scratch)
     # a 0-dim (or fully expanded one-element) dy is read as a scalar by the kernel: nothing is materialised
     dy_scalar = dy.numel() == 1 or (dy.shape == x.shape and all(st == 0 for st in dy.stride()))
@@ -425,6 +461,10 @@ def batch_norm_fwd(x: torch.Tensor, weight: torch.Tensor | None, bias: torch.Ten
     ``unbiased_factor`` replaces n / (n - 1) in the running-variance update: a captured graph
     holds that factor as a literal of the shape it was captured at.
     """
+    got = (_calls or _load_calls()).batch_norm_fwd(x, weight, bias, running_mean, running_var, eps, momentum, relu, unbiased_factor,
+                                                   scratch)
+    if got is not None:
+        return got
     _require_cuda(x, weight, bias, running_mean, running_var, scratch)
     if x.dim() != 4:
         raise UnsupportedLayout("batch_norm_fwd: expected a 4-D [N, C, H, W] tensor")
@@ -475,6 +515,9 @@ def batch_norm_bwd(dy: torch.Tensor, x: torch.Tensor, mean: torch.Tensor, invstd
     ``inv_count`` replaces 1 / (N*H*W): a captured graph holds it as a literal of the shape it was
     captured at.
     """
+    got = (_calls or _load_calls()).batch_norm_bwd(dy, x, mean, invstd, weight, act, slope, want_dx, inv_count, scratch)
+    if got is not None:
+        return got
     _require_cuda(dy, x, mean, invstd, weight, act, scratch)
     if x.dim() != 4 or dy.shape != x.shape or dy.dtype != x.dtype or dy.stride() != x.stride():
         raise UnsupportedLayout("batch_norm_bwd: dy and x must be 4-D with the same shape, dtype and strides")
@@ -554,6 +597,9 @@ def permute_copy(x: torch.Tensor, dims, *, scale: float | None = None,
     Up to four dimensions after adjacent dimensions that stay adjacent have been merged. A swap of
     the two innermost dimensions goes through the shared-memory transpose kernel.
     """
+    got = (_calls or _load_calls()).permute_copy(x, dims, scale, out_dtype, None)
+    if got is not None:
+        return got
     _require_cuda(x)
     out_dtype = out_dtype or x.dtype
     view = x.permute(*dims)
@@ -582,6 +628,12 @@ def permute_copy(x: torch.Tensor, dims, *, scale: float | None = None,
                                 _DTYPE_CODE[out_dtype], sc, has_scale, _stream()),
           "b200_permute_copy")
     return out
+
+
+def permute_copy_as(x: torch.Tensor, dims, shape) -> torch.Tensor:
+    """``permute_copy(x, dims).view(shape)`` without the view."""
+    got = (_calls or _load_calls()).permute_copy(x, dims, None, None, shape)
+    return got if got is not None else permute_copy(x, dims).view(shape)
 
 
 def _collapse_all(shape, strides_list):
@@ -614,6 +666,9 @@ def cast_scale(x: torch.Tensor, out_dtype: torch.dtype, *, scale: float | None =
     order; the result keeps x's strides."""
     if relu:
         activation = "relu"
+    got = (_calls or _load_calls()).cast_scale(x, out_dtype, scale, _ACTIVATIONS.get(activation, -1))
+    if got is not None:
+        return got
     _require_cuda(x)
     if not _is_dense(x):
         raise UnsupportedLayout("cast_scale: x must be dense")

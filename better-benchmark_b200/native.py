@@ -7,6 +7,8 @@ fallback of any kind: if the library is missing or a symbol cannot be resolved, 
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import threading
 from ctypes import c_char_p, c_double, c_int32, c_int64, c_void_p
 from pathlib import Path
@@ -15,6 +17,9 @@ import os
 
 # B200_ORACLES_LIB names another build of the library (a measurement variant); default: the in-tree one
 LIB_PATH = Path(os.environ.get("B200_ORACLES_LIB") or Path(__file__).resolve().parent / "csrc" / "libb200_oracles.so")
+
+# The host side of the most frequent calls (csrc/calls.cpp), an extension module that works on the library loaded here
+CALLS_PATH = Path(__file__).resolve().parent / "csrc" / "b200_calls.so"
 
 # dtype codes shared with csrc/common.cuh
 F32, BF16, F16 = 0, 1, 2
@@ -134,6 +139,31 @@ def load() -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = lib
         return lib
+
+
+_calls = None
+_BOUND = ("b200_row_reduce", "b200_softmax", "b200_norm_fwd_residual", "b200_norm_bwd", "b200_norm_bwd_scratch_bytes",
+          "b200_batch_norm_fwd_ex", "b200_batch_norm_scratch_bytes", "b200_batch_norm_bwd_ex",
+          "b200_batch_norm_bwd_scratch_bytes", "b200_transpose_copy", "b200_permute_copy", "b200_cast_scale")
+
+
+def load_calls(scratch_by_device: dict):
+    """Load csrc/calls.cpp's module once per process and hand it the library's entry points."""
+    global _calls
+    lib = load()
+    with _lock:
+        if _calls is None:
+            if not CALLS_PATH.exists():
+                raise NativeLibraryError(f"{CALLS_PATH} is not built. Run `python -m better_benchmark_b200.build`.")
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("b200_calls", str(CALLS_PATH))
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200_calls", loader))
+                loader.exec_module(module)
+            except ImportError as e:
+                raise NativeLibraryError(f"cannot load {CALLS_PATH}: {e}") from e
+            module.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _BOUND}, check, scratch_by_device)
+            _calls = module
+        return _calls
 
 
 def last_error() -> str:
