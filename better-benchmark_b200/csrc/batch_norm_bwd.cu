@@ -761,7 +761,7 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
   constexpr int V = Elem<T>::V;
   const DeviceInfo& dev = device_info();
   const long long coef_floats = 4LL * p.channels;
-  if (fast) {
+  while (fast) {
     long long g = p.channels, h = V;  // gcd(C, V)
     while (h) { const long long t = g % h; g = h; h = t; }
     const int vpr = (int)(p.channels / g);  // PV: vectors after which the channel pattern repeats
@@ -775,8 +775,12 @@ static int launch_bn_bwd(BnBwdParams p, bool fast, size_t scratch_bytes, cudaStr
     if (chunks <= 2 * splits) splits = chunks <= splits ? chunks : (chunks + 1) / 2;
     if (splits < 1) splits = 1;
     const long long need = splits * 2 * p.channels * (long long)sizeof(double) + coef_floats * (long long)sizeof(float);
-    if ((long long)scratch_bytes < need)
-      return fail(B200_ERR_WORKSPACE, "b200_batch_norm_bwd: scratch of %zu bytes, need %lld", scratch_bytes, need);
+    if ((long long)scratch_bytes < need) {
+      if (p.rows * p.channels % ((long long)vpr * V) == 0)
+        return fail(B200_ERR_WORKSPACE, "b200_batch_norm_bwd: scratch of %zu bytes, need %lld", scratch_bytes, need);
+      p.rows /= p.spatial;  // no whole number of periods: the strided kernels make do with less
+      break;
+    }
     p.splits = (int)splits;
     p.coef = reinterpret_cast<float*>(p.partials + splits * 2 * p.channels);
     // the elements behind the last whole vector belong to the thread of CTA 0 that has the phase of the vector they begin

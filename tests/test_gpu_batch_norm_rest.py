@@ -66,3 +66,21 @@ def test_backward(dtype, shape):
                 _close(dx, want, dt, "dx")
             else:
                 assert dx is None
+
+
+def test_backward_with_a_small_scratch():
+    """Room for the few partial rows of the strided kernels only: still taken, with the same result."""
+    from better_benchmark_b200 import kernels as k
+    shape, c = (69, 401, 14, 14), 401
+    x, dy = (_image(shape, torch.bfloat16, s) for s in (1, 2))
+    mean, invstd = torch.zeros(c, device="cuda"), torch.ones(c, device="cuda")
+    want = k.batch_norm_bwd(dy, x, mean, invstd, None)
+    splits = 69 * 196 // 16384 or 1
+    small = torch.zeros(256 + splits * 2 * c * 8 + 4 * c * 4, dtype=torch.uint8, device="cuda")
+    got = k.batch_norm_bwd(dy, x, mean, invstd, None, scratch=small)
+    assert b"strided" in k.load().b200_last_kernel()
+    _close(got[0], want[0].double(), torch.bfloat16, "dx")
+    for a, b in zip(got[1:], want[1:]):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-2)
+    with pytest.raises(ValueError, match="scratch"):
+        k.batch_norm_bwd(dy, x, mean, invstd, None, scratch=small[:-16])
