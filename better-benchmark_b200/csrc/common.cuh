@@ -309,61 +309,6 @@ __device__ __forceinline__ float group_reduce(float v, float* scratch) {
   }
 }
 
-// ----------------------------------------------------------------------------------------
-// Grid-wide barrier for cooperative (co-resident) launches, with a bounded wait.
-// `bar` points at four 32-bit words of global scratch that are zero before the launch:
-//   [0] arrival counter, [1] error flag, [2] departure counter, [3] work counter of kernels that
-//   hand out blocks dynamically (reset with the others).
-// Each use of the barrier within one launch passes the next `phase` (1, 2, ..): the arrival
-// counter only grows, and phase p completes when it reaches p * gridDim.x. Every CTA calls
-// grid_barrier_depart() once after its last barrier; the last CTA to depart puts the counters
-// back to zero, so the next launch on the same stream needs no memset. A wait that runs out
-// sets the error flag (which stays set until the host clears the words) and returns false;
-// callers then skip the remaining work, so the context stays usable and the host can report
-// B200_ERR_DEVICE_WAIT.
-// ----------------------------------------------------------------------------------------
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int phase, int* smem_flag) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&bar[0], 1u);
-    const unsigned int target = phase * gridDim.x;
-    int ok = 1;
-    unsigned int spins = 0;
-    while (true) {
-      unsigned int seen;
-      asm volatile("ld.global.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-      if (seen >= target) break;
-      unsigned int err;
-      asm volatile("ld.global.relaxed.gpu.u32 %0, [%1];" : "=r"(err) : "l"(bar + 1) : "memory");
-      if (err != 0u || ++spins > (1u << 22)) {  // ~4M polls: a fraction of a second
-        atomicExch(&bar[1], 1u);
-        ok = 0;
-        break;
-      }
-      if (spins > 4096) __nanosleep(64);  // poll tightly at first: the usual wait is a few microseconds
-    }
-    __threadfence();
-    *smem_flag = ok;
-  }
-  __syncthreads();
-  return *smem_flag != 0;
-}
-
-__device__ __forceinline__ void grid_barrier_depart(unsigned int* bar) {
-  if (threadIdx.x == 0) {
-    const unsigned int old = atomicAdd(&bar[2], 1u);
-    if (old == gridDim.x - 1) {
-      // Everyone has left every barrier of this launch (or gave up): reset for the next one.
-      // The error flag is left alone on purpose.
-      atomicExch(&bar[0], 0u);
-      atomicExch(&bar[2], 0u);
-      atomicExch(&bar[3], 0u);
-      __threadfence();
-    }
-  }
-}
-
 // Programmatic dependent launch: a kernel launched by launch_dependent may be set up while the kernel before it in
 // the stream, ours or not, drains. Every kernel of the library is launched so and begins with
 // wait_for_previous_kernel, after which everything before it has completed and is visible; only kernels in
@@ -408,16 +353,6 @@ inline cudaError_t launch_clusters(dim3 cluster, void (*kernel)(Formal...), dim3
   attr.val.clusterDim.z = cluster.z;
   return launch_with(&attr, kernel, grid, block, smem, st, args...);
 }
-// All CTAs resident at the same time, so that they may wait on one another (grid_barrier).
-template <typename... Formal, typename... Actual>
-inline cudaError_t launch_cooperative(void (*kernel)(Formal...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                      Actual... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeCooperative;
-  attr.val.cooperative = 1;
-  return launch_with(&attr, kernel, grid, block, smem, st, args...);
-}
-
 // Lets a kernel be launched with `bytes` of dynamic shared memory. The limit is an attribute of the function, not of
 // a launch: set to each launch's own size, one host thread would lower it between another's set and launch.
 // So it is set once per kernel and device, to all that the device leaves beside the kernel's static

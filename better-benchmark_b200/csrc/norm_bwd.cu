@@ -16,9 +16,9 @@
 // Structure: a persistent grid; each group of threads (a CTA for long rows, a warp for short
 // ones) walks rows group, group+G, ..., keeps the next row's loads in flight while it reduces the
 // current one, and accumulates its columns of dw/db in registers over all its rows. Each group
-// then writes one fp32 partial row to scratch; after a grid-wide barrier (cooperative launch)
-// the partial rows are summed in fp64, in a fixed order, into dw/db. No atomics: results are
-// bit-reproducible. A two-launch variant (main + finalize) does the same without the barrier.
+// then writes one fp32 partial row to scratch; CTAs of the same launch that start after these
+// sum the partial rows in fp64, in a fixed order, into dw/db (the two roles of norm_bwd.cuh). No atomics on results:
+// they are bit-reproducible. A two-launch variant (main + finalize) does the same.
 #include "norm_bwd.cuh"
 
 #include <cstdlib>
@@ -33,13 +33,19 @@ norm_bwd_kernel(const NormBwdParams p) {
   constexpr int V = Elem<T>::V;
   __shared__ float2 red[2][16];
   __shared__ double fin[16 * 64];
-  __shared__ int bar_ok;
+  __shared__ int bar_ok, ticket;
   const int lane = group_lane<BLOCK>();
   const int G = group_size<BLOCK>();
   const int nv = p.n / V;
-  const long long group = BLOCK ? (long long)blockIdx.x
-                                : (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const long long group_stride = BLOCK ? (long long)gridDim.x : (long long)gridDim.x * (blockDim.x >> 5);
+  bwd_draw_ticket(p, &ticket);
+  __syncthreads();
+  const int cta = bwd_cta(&ticket);
+  if (cta >= p.workers) {
+    bwd_finalize(p, cta, LN ? p.db : nullptr, fin, &bar_ok);
+    return;
+  }
+  const long long group = BLOCK ? (long long)cta : (long long)cta * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const long long group_stride = BLOCK ? (long long)p.workers : (long long)p.workers * (blockDim.x >> 5);
 
   float acc_w[CH][V], acc_b[LN ? CH : 1][V];
 #pragma unroll
@@ -198,11 +204,7 @@ norm_bwd_kernel(const NormBwdParams p) {
       }
     }
   }
-  if (p.fused) {
-    const bool ok = grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
-    grid_barrier_depart(p.bar);
-  }
+  bwd_worker_done(p);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -220,8 +222,6 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
   constexpr int V = Elem<T>::V;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(16) float2 red[2][16];
-  __shared__ double fin[16 * 64];
-  __shared__ int bar_ok;
   const int tid = threadIdx.x;
   const int T_ = blockDim.x;
   const int nv = p.n / V;
@@ -229,7 +229,8 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)stages * 2 * row_bytes);
   const T* xg = reinterpret_cast<const T*>(p.x);
   const T* dyg = reinterpret_cast<const T*>(p.dy);
-  const long long my_rows = p.rows > blockIdx.x ? (p.rows - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const int rows = (int)p.rows;  // the launcher admits fewer than 2^31
+  const int my_rows = rows > (int)blockIdx.x ? (rows - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
   if (tid == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
@@ -237,19 +238,16 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
   }
   __syncthreads();
 
-  auto issue = [&](long long k, int slot) {  // thread 0 only; slot = k mod stages, tracked incrementally
-    const long long row = (long long)blockIdx.x + k * gridDim.x;
+  auto issue = [&](int k, int slot) {  // thread 0 only; slot = k mod stages
+    const long long row = (long long)blockIdx.x + (long long)k * gridDim.x;
     uint64_t* bar = &full[slot];
     unsigned char* dst = smem + (size_t)slot * 2 * row_bytes;
     mbar_arrive_expect_tx(bar, 2 * row_bytes);
     bulk_load(dst, xg + row * p.x_row_stride, row_bytes, bar);
     bulk_load(dst + row_bytes, dyg + row * p.dy_row_stride, row_bytes, bar);
   };
-  long long issued = 0;
-  int issue_slot = 0;
   if (tid == 0) {
-    for (; issued < my_rows && issued < stages; ++issued) issue(issued, (int)issued);
-    issue_slot = (int)(issued % stages);
+    for (int k = 0; k < my_rows && k < stages; ++k) issue(k, k);
   }
 
   // A thread owns the same columns in every row: its slice of the weight stays in registers.
@@ -285,8 +283,8 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
   int parity = 0;
   int st = 0;
   uint32_t phase = 0;
-  for (long long k = 0; k < my_rows; ++k) {
-    const long long row = (long long)blockIdx.x + k * gridDim.x;
+  for (int k = 0; k < my_rows; ++k) {
+    const long long row = (long long)blockIdx.x + (long long)k * gridDim.x;
     const bool arrived = mbar_wait(&full[st], phase);
     const unsigned char* sx = smem + (size_t)st * 2 * row_bytes;
     const unsigned char* sy = sx + row_bytes;
@@ -339,21 +337,19 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
       failed = true;
       if (tid == 0) {
         note_wait_timeout();
-        atomicExch(&p.bar[1], 1u);  // lets the other CTAs leave the grid barrier at once
+        if (p.bar) atomicExch(&p.bar[1], 1u);  // nobody is to wait for this CTA
         int ds = st;
         uint32_t dp = phase;
-        for (long long d = k; d < issued; ++d) {
+        for (int d = k; d < my_rows && d < k + stages; ++d) {
           mbar_wait(&full[ds], dp);
           if (++ds == stages) { ds = 0; dp ^= 1u; }
         }
       }
       break;
     }
-    if (tid == 0 && issued < my_rows) {  // every thread holds its part of this stage in registers
+    if (tid == 0 && k + stages < my_rows) {  // every thread holds its part of this stage in registers
       fence_proxy_async_smem();
-      issue(issued, issue_slot);
-      ++issued;
-      if (++issue_slot == stages) issue_slot = 0;
+      issue(k + stages, st);
     }
     t1 = 0.f;
     t2 = 0.f;
@@ -408,6 +404,7 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
     }
   }
 
+  if (p.dw || p.db) let_next_kernel_start();  // the finalize
   if (!failed && (p.dw || p.db)) {
     float* pw = p.partials + (long long)blockIdx.x * p.n;
     float* pb = p.partials + ((long long)p.groups + blockIdx.x) * p.n;
@@ -432,11 +429,6 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
         }
       }
     }
-  }
-  if (p.fused) {
-    const bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
-    grid_barrier_depart(p.bar);
   }
 }
 
@@ -468,10 +460,6 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
   constexpr int MAX_GROUPS = GROUPED ? 8 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(16) float red[2][MAX_GROUPS][NVAL][16];
-  __shared__ int bar_ok;
-  // the fp64 area of the final column sums reuses the ring once the last tile has been consumed
-  // (the launcher keeps the ring at 8 KB or more)
-  double* fin = reinterpret_cast<double*>(smem);
   const int lane = threadIdx.x & 31;
   // group of this thread = (warp index) / (warps per group), as a multiplication by the 16.16
   // reciprocal the launcher passes: a plain division here gets recomputed in the loop when
@@ -519,10 +507,10 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
       }
     }
   };
-  int issued = 0, issue_slot = 0;
+  // What has been issued follows from the tile at hand, max(k - 1, 0) + stages tiles before tile k: counted in two variables it cost the
+  // kernel up to 20 registers (fp32 64 -> 45, 16-bit RMSNorm 64 and spills -> 60).
   if (threadIdx.x == 0) {
-    for (; issued < my_tiles && issued < stages; ++issued) issue(issued, issued);
-    issue_slot = issued % stages;
+    for (int k = 0; k < my_tiles && k < stages; ++k) issue(k, k);
   }
 
   // A thread owns the same V columns in every row: weight slice and gradient sums in registers.
@@ -576,8 +564,8 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
       if constexpr (LN) mean[r] = r < nrows ? ld_here(p.mean + row0 + r) : 0.f;
     }
     const bool arrived = mbar_wait(&full[st], phase);
-    const unsigned char* sx = smem + (size_t)st * stage_bytes + (size_t)(grp * R) * row_bytes + (size_t)tid * 16;
-    const unsigned char* sy = sx + (size_t)TR * row_bytes;
+    const uint32_t sx = smem_u32(smem) + (uint32_t)st * stage_bytes + (uint32_t)(grp * R) * row_bytes + (uint32_t)tid * 16u;
+    const uint32_t sy = sx + (uint32_t)TR * row_bytes;
     const bool whole = active && nrows == R;  // uniform per warp except in the last warp of a ragged row
 
     // Pass 1: the row sums of this thread's columns.
@@ -587,8 +575,8 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
       f32x2 s1 = splat2(0.f), s2 = splat2(0.f);
       if (whole || (active && r < nrows)) {
         f32x2 x2[V / 2], dy2[V / 2];
-        Pairs<T>::unpack(*reinterpret_cast<const uint4*>(sx + (size_t)r * row_bytes), x2);
-        Pairs<T>::unpack(*reinterpret_cast<const uint4*>(sy + (size_t)r * row_bytes), dy2);
+        Pairs<T>::unpack(lds128(sx + (uint32_t)r * row_bytes), x2);
+        Pairs<T>::unpack(lds128(sy + (uint32_t)r * row_bytes), dy2);
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) {
           const f32x2 g2 = mul2(dy2[i], weight(i));
@@ -610,10 +598,10 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
       failed = true;
       if (threadIdx.x == 0) {
         note_wait_timeout();
-        atomicExch(&p.bar[1], 1u);  // lets the other CTAs leave the grid barrier at once
+        if (p.bar) atomicExch(&p.bar[1], 1u);  // nobody is to wait for this CTA
         int ds = st;
         uint32_t dp = phase;
-        for (int d = k; d < issued; ++d) {
+        for (int d = k; d < my_tiles && d < (k > 0 ? k - 1 : 0) + stages; ++d) {
           mbar_wait(&full[ds], dp);
           if (++ds == stages) { ds = 0; dp ^= 1u; }
         }
@@ -622,11 +610,9 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
     }
     // The second pass reads this stage again; what the barrier proves is that the PREVIOUS tile's
     // stage has been read to the end by every thread: that one is refilled.
-    if (threadIdx.x == 0 && k >= 1 && issued < my_tiles) {
+    if (threadIdx.x == 0 && k >= 1 && k - 1 + stages < my_tiles) {
       fence_proxy_async_smem();
-      issue(issued, issue_slot);
-      ++issued;
-      if (++issue_slot == stages) issue_slot = 0;
+      issue(k - 1 + stages, st == 0 ? stages - 1 : st - 1);
     }
 
     // Second stage of the reduction: lane l sums PER consecutive entries of the [value][warp]
@@ -670,8 +656,8 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
           off = bi * (uint32_t)p.dx_batch_stride + si * (uint32_t)p.dx_seq_stride + dx_col;
         }
         f32x2 x2[V / 2], dy2[V / 2], o2[V / 2];
-        Pairs<T>::unpack(*reinterpret_cast<const uint4*>(sx + (size_t)r * row_bytes), x2);
-        Pairs<T>::unpack(*reinterpret_cast<const uint4*>(sy + (size_t)r * row_bytes), dy2);
+        Pairs<T>::unpack(lds128(sx + (uint32_t)r * row_bytes), x2);
+        Pairs<T>::unpack(lds128(sy + (uint32_t)r * row_bytes), dy2);
         const f32x2 rstd2 = splat2(rstd[r]);
         if constexpr (LN) {
           // The division by n of the aten graph is a multiplication by 1/n here (exact for
@@ -708,6 +694,7 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
   }
 
   // Per-CTA partial rows: the row groups are folded in a fixed order through the ring (free now).
+  if (p.dw || p.db) let_next_kernel_start();  // the finalize
   if (!failed && (p.dw || p.db)) {
     __syncthreads();  // every group is done with its last tile
     float* fold_w = reinterpret_cast<float*>(smem);             // [GROUPS][n]
@@ -736,11 +723,14 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
       }
     }
   }
-  if (p.fused) {
-    const bool ok = !failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
-    grid_barrier_depart(p.bar);
-  }
+}
+
+// The finalize of the streaming and row-tile kernels, whose registers leave no room for the tickets: a unit of columns per CTA.
+__global__ void __launch_bounds__(256) norm_bwd_finalize_units_kernel(const NormBwdParams p) {
+  wait_for_previous_kernel();
+  __shared__ double fin[8 * 64];
+  if (p.bar[1] != 0u) return;  // a worker gave up: the host is told (b200_check_status)
+  finalize_units(p.partials, p.groups, p.n, p.dw, p.db, p.width, blockIdx.x, gridDim.x, fin);
 }
 
 __global__ void __launch_bounds__(512) norm_bwd_finalize_kernel(const NormBwdParams p) {
@@ -954,10 +944,17 @@ static int tile_rows_override() {
   return v;
 }
 
+static int launch_finalize_units(NormBwdParams p, const char* what, cudaStream_t st) {
+  bwd_plan_finalize(p, 8LL * device_info().sm_count);
+  const int units = p.finalizers;
+  p.finalizers = 0;
+  launch_dependent(norm_bwd_finalize_units_kernel, (unsigned)units, 256, 0, st, p);
+  return launch_status(what);
+}
+
 // CTA-per-row streaming launch; returns false when the shape does not fit (caller falls back).
 template <typename T, int CH, bool LN>
-static bool try_launch_norm_bwd_stream(NormBwdParams p, int threads, size_t scratch_bytes, bool cooperative,
-                                       cudaStream_t st, int* rc) {
+static bool try_launch_norm_bwd_stream(NormBwdParams p, int threads, size_t scratch_bytes, cudaStream_t st, int* rc) {
   constexpr int V = Elem<T>::V;
   if (streaming_disabled() || p.rows < 1024) return false;
   const DeviceInfo& dev = device_info();
@@ -984,32 +981,17 @@ static bool try_launch_norm_bwd_stream(NormBwdParams p, int threads, size_t scra
     if (max_groups < 1) return false;
     if (grid > max_groups) grid = max_groups;
   }
-  p.groups = (int)grid;
-  p.fused = cooperative ? 1 : 0;
-  if (cooperative) {
-    e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(threads), smem, st, p, stages);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      *rc = fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
-      return true;
-    }
-    note_launch("b200_norm_bwd [streaming, CTA per row, fused finalize]");
-    *rc = B200_OK;
-    return true;
-  }
+  p.groups = p.workers = (int)grid;
   launch_dependent(kernel, (unsigned)grid, threads, smem, st, p, stages);
-  *rc = launch_status("b200_norm_bwd (streaming)");
-  if (*rc == B200_OK && (p.dw || p.db)) {
-    launch_dependent(norm_bwd_finalize_kernel, (p.n + 63) / 64, 512, 0, st, p);
-    *rc = launch_status("b200_norm_bwd finalize");
-  }
+  *rc = launch_status("b200_norm_bwd [streaming, CTA per row]");
+  if (*rc == B200_OK && (p.dw || p.db)) *rc = launch_finalize_units(p, "b200_norm_bwd finalize [streaming, CTA per row]", st);
   return true;
 }
 
 // Row-tile streaming launch (one vector per thread); returns false when the shape does not fit.
 template <typename T, int R, bool LN>
-static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratch_bytes, bool cooperative,
-                                     cudaStream_t st, int* rc, int want_groups = 0) {
+static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratch_bytes, cudaStream_t st, int* rc,
+                                     int want_groups = 0) {
   constexpr int V = Elem<T>::V;
   if (streaming_disabled() || p.rows < 1024 || threads > 512) return false;
   {  // the kernel addresses dx with 32-bit element offsets
@@ -1059,31 +1041,16 @@ static bool try_launch_norm_bwd_tile(NormBwdParams p, int threads, size_t scratc
     if (max_groups < 1) return false;
     if (grid > max_groups) grid = max_groups;
   }
-  p.groups = (int)grid;
-  p.fused = cooperative ? 1 : 0;
+  p.groups = p.workers = (int)grid;
   int tg_arg = tg, groups_arg = groups_per_cta, wpg_inv_arg = (65536 + tg / 32 - 1) / (tg / 32);
-  if (cooperative) {
-    e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(threads), smem, st, p, stages, tg_arg, groups_arg, wpg_inv_arg);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      *rc = fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
-      return true;
-    }
-    note_launch(groups_per_cta > 1 ? "b200_norm_bwd [row tiles, row groups, fused finalize]" : "b200_norm_bwd [row tiles, fused finalize]");
-    *rc = B200_OK;
-    return true;
-  }
   launch_dependent(kernel, (unsigned)grid, threads, smem, st, p, stages, tg_arg, groups_arg, wpg_inv_arg);
-  *rc = launch_status("b200_norm_bwd (row tiles)");
-  if (*rc == B200_OK && (p.dw || p.db)) {
-    launch_dependent(norm_bwd_finalize_kernel, (p.n + 63) / 64, 512, 0, st, p);
-    *rc = launch_status("b200_norm_bwd finalize");
-  }
+  *rc = launch_status("b200_norm_bwd [row tiles]");
+  if (*rc == B200_OK && (p.dw || p.db)) *rc = launch_finalize_units(p, "b200_norm_bwd finalize [row tiles]", st);
   return true;
 }
 
 template <typename T, int CH, bool BLOCK, bool LN>
-static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_bytes, bool cooperative,
+static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_bytes, bool fused,
                                 cudaStream_t st) {
   auto kernel = norm_bwd_kernel<T, CH, BLOCK, LN>;
   const int sms = device_info().sm_count;
@@ -1102,15 +1069,11 @@ static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_byt
     if (grid * groups_per_cta > max_groups) grid = max_groups / groups_per_cta;
   }
   p.groups = (int)(grid * groups_per_cta);
-  p.fused = cooperative ? 1 : 0;
-  if (cooperative) {
-    const cudaError_t e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(threads), 0, st, p);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
-    }
-    note_launch(BLOCK ? "b200_norm_bwd [registers, CTA per row, fused finalize]" : "b200_norm_bwd [registers, warp per row, fused finalize]");
-    return B200_OK;
+  p.workers = (int)grid;
+  if (fused) {
+    bwd_plan_finalize(p, (long long)per_sm * sms);
+    launch_dependent(kernel, (unsigned)(grid + p.finalizers), threads, 0, st, p);
+    return launch_status(BLOCK ? "b200_norm_bwd [registers, CTA per row, fused finalize]" : "b200_norm_bwd [registers, warp per row, fused finalize]");
   }
   launch_dependent(kernel, (unsigned)grid, threads, 0, st, p);
   int rc = launch_status("b200_norm_bwd");
@@ -1170,7 +1133,7 @@ static bool try_launch_norm_bwd_ragged(NormBwdParams p, size_t scratch_bytes, cu
       if (max_groups < 1) return false;
       if (grid > max_groups) grid = max_groups;
     }
-    p.groups = (int)grid;
+    p.groups = p.workers = (int)grid;
     launch_dependent(kernel, (unsigned)grid, threads, smem, st, p);
     *rc = launch_status("b200_norm_bwd [ragged rows, elements in registers]");
     if (*rc == B200_OK && sums) {
@@ -1186,7 +1149,7 @@ static bool try_launch_norm_bwd_ragged(NormBwdParams p, size_t scratch_bytes, cu
 }
 
 template <typename T, bool LN>
-static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes, bool cooperative,
+static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes, bool fused,
                            cudaStream_t st) {
   constexpr int V = Elem<T>::V;
   if (p.rows > 0x7fffffffLL) return fail(B200_ERR_UNSUPPORTED, "norm_bwd: too many rows");
@@ -1194,7 +1157,7 @@ static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes
   if (vector_ok && p.n % V == 0 && p.head_dim % V == 0 && nv <= 2048) {
     {  // rows of 33..256 vectors: warp per row, per-warp copy rings (norm_bwd_warp.cu)
       int rc = B200_OK;
-      if (try_launch_norm_bwd_warp<T, LN>(p, scratch_bytes, cooperative, st, &rc)) return rc;
+      if (try_launch_norm_bwd_warp<T, LN>(p, scratch_bytes, fused, st, &rc)) return rc;
     }
   }
   // a broadcast scalar dy is read by the warp-per-row kernel above and by the element-wise kernels
@@ -1207,12 +1170,12 @@ static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes
         // four rows per group and barrier when two stages of that fit (with fewer groups if need
         // be: more work per barrier beats more groups), else two rows
         for (int g = 512 / narrow; g >= 3; --g)
-          if (try_launch_norm_bwd_tile<T, 4, LN>(p, narrow, scratch_bytes, cooperative, st, &rc, g)) return rc;
-        if (try_launch_norm_bwd_tile<T, 2, LN>(p, narrow, scratch_bytes, cooperative, st, &rc)) return rc;
+          if (try_launch_norm_bwd_tile<T, 4, LN>(p, narrow, scratch_bytes, st, &rc, g)) return rc;
+        if (try_launch_norm_bwd_tile<T, 2, LN>(p, narrow, scratch_bytes, st, &rc)) return rc;
       }
-      if (nv <= 32) return launch_norm_bwd_fast<T, 1, false, LN>(p, 256, scratch_bytes, cooperative, st);
-      if (nv <= 64) return launch_norm_bwd_fast<T, 2, false, LN>(p, 256, scratch_bytes, cooperative, st);
-      return launch_norm_bwd_fast<T, 4, false, LN>(p, 256, scratch_bytes, cooperative, st);
+      if (nv <= 32) return launch_norm_bwd_fast<T, 1, false, LN>(p, 256, scratch_bytes, fused, st);
+      if (nv <= 64) return launch_norm_bwd_fast<T, 2, false, LN>(p, 256, scratch_bytes, fused, st);
+      return launch_norm_bwd_fast<T, 4, false, LN>(p, 256, scratch_bytes, fused, st);
     }
     int rc = B200_OK;
     if (nv <= 512) {
@@ -1220,23 +1183,23 @@ static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes
       const int wide = (int)((nv + 31) / 32 * 32);
       if (tile_rows_override() != 1) {
         if (tile_rows_override() != 2 &&
-            try_launch_norm_bwd_tile<T, 4, LN>(p, wide, scratch_bytes, cooperative, st, &rc)) return rc;
-        if (try_launch_norm_bwd_tile<T, 2, LN>(p, wide, scratch_bytes, cooperative, st, &rc)) return rc;
+            try_launch_norm_bwd_tile<T, 4, LN>(p, wide, scratch_bytes, st, &rc)) return rc;
+        if (try_launch_norm_bwd_tile<T, 2, LN>(p, wide, scratch_bytes, st, &rc)) return rc;
       }
-      if (try_launch_norm_bwd_stream<T, 1, LN>(p, wide, scratch_bytes, cooperative, st, &rc)) return rc;
+      if (try_launch_norm_bwd_stream<T, 1, LN>(p, wide, scratch_bytes, st, &rc)) return rc;
       int threads = (int)((nv + 1) / 2);
       threads = (threads + 31) / 32 * 32;
-      return launch_norm_bwd_fast<T, 2, true, LN>(p, threads, scratch_bytes, cooperative, st);
+      return launch_norm_bwd_fast<T, 2, true, LN>(p, threads, scratch_bytes, fused, st);
     }
     if (nv <= 1024) {
       int threads = (int)((nv + 1) / 2);
       threads = (threads + 31) / 32 * 32;
-      if (try_launch_norm_bwd_stream<T, 2, LN>(p, threads, scratch_bytes, cooperative, st, &rc)) return rc;
+      if (try_launch_norm_bwd_stream<T, 2, LN>(p, threads, scratch_bytes, st, &rc)) return rc;
     }
     int threads = (int)((nv + 3) / 4);
     threads = (threads + 31) / 32 * 32;
-    if (try_launch_norm_bwd_stream<T, 4, LN>(p, threads, scratch_bytes, cooperative, st, &rc)) return rc;
-    return launch_norm_bwd_fast<T, 4, true, LN>(p, threads, scratch_bytes, cooperative, st);
+    if (try_launch_norm_bwd_stream<T, 4, LN>(p, threads, scratch_bytes, st, &rc)) return rc;
+    return launch_norm_bwd_fast<T, 4, true, LN>(p, threads, scratch_bytes, fused, st);
   }
   {
     int rc = B200_OK;
@@ -1313,8 +1276,8 @@ extern "C" int b200_norm_bwd(const void* x, const void* dy, const void* weight, 
   p.n_f = (float)n;
   p.bar = reinterpret_cast<unsigned int*>(scratch);
   p.partials = scratch ? reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + 256) : nullptr;
-  p.groups = 0; p.fused = 0;
-  const bool cooperative = (flags & 1) == 0 && (dweight || dbias);
+  p.groups = p.workers = 0; p.finalizers = 0; p.width = 0;
+  const bool fused = (flags & 1) == 0 && (dweight || dbias);
 
   const int eb = dtype_size(x_dtype), wb = dtype_size(w_dtype);
   const int v = 16 / eb;
@@ -1326,8 +1289,8 @@ extern "C" int b200_norm_bwd(const void* x, const void* dy, const void* weight, 
 
 #define B200_NBWD_CASE(TT, DT)                                                              \
   if (x_dtype == DT)                                                                        \
-    return rms ? launch_norm_bwd<TT, false>(p, vec, (size_t)scratch_bytes, cooperative, st) \
-               : launch_norm_bwd<TT, true>(p, vec, (size_t)scratch_bytes, cooperative, st);
+    return rms ? launch_norm_bwd<TT, false>(p, vec, (size_t)scratch_bytes, fused, st) \
+               : launch_norm_bwd<TT, true>(p, vec, (size_t)scratch_bytes, fused, st);
   B200_NBWD_CASE(float, B200_F32)
   B200_NBWD_CASE(__nv_bfloat16, B200_BF16)
   B200_NBWD_CASE(__half, B200_F16)

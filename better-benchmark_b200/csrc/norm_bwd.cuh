@@ -28,10 +28,76 @@ struct NormBwdParams {
   long long dx_batch_stride, dx_seq_stride, dx_head_stride;
   float n_f;
   float* partials;    // [groups][n] for dw, followed by [groups][n] for db
-  unsigned int* bar;  // grid barrier words (cooperative variant)
+  unsigned int* bar;  // words that are zero between launches: [0] workers done, [1] error, [2] CTAs gone, [3] tickets
   int groups;
-  int fused;  // 1: barrier + finalize inside this launch
+  int workers;  // CTAs that walk the rows
+  // The finalize in the same launch (0: none, or a launch of its own): this many CTAs beside the workers, a unit of
+  // `width` columns at a time.
+  int finalizers;
+  int width;
 };
+
+// ----------------------------------------------------------------------------------------------
+// One launch, two roles. The first `workers` CTAs that START are workers: they walk the rows, and the partial row that each
+// leaves has the number of its ticket. The CTAs that start after them add the partial rows up once all workers have arrived.
+// A worker waits for nobody, and a CTA that waits has started after every worker has: whatever else occupies the GPU,
+// the wait ends, so that the launch need not be cooperative. (Cooperative launches with a grid barrier took
+// 2 to 3 us more back to back, 10.4 us for a few hundred rows whose kernel runs 7.7, and the CTAs that had finished
+// early did nothing.) Tickets decide who owns which rows, so the result does not depend on which CTA draws which.
+// ----------------------------------------------------------------------------------------------
+// A CTA's number, among the workers or, from p.workers on, the finalizers: thread 0 draws it, the others know it after the CTA's next
+// barrier. The shuffle tells the compiler that it is the same in a warp, so that what depends on it can live in uniform registers, as
+// what depends on blockIdx does. (All the same the kernels of 64 registers spilled: RMSNorm backward bf16 [4, 4096, 32, 128] 70 ->
+// 78 us. Those have a finalize of their own, chained to them.)
+__device__ __forceinline__ void bwd_draw_ticket(const NormBwdParams& p, int* ticket) {
+  if (threadIdx.x == 0) *ticket = p.finalizers > 0 ? (int)atomicAdd(&p.bar[3], 1u) : (int)blockIdx.x;
+}
+__device__ __forceinline__ int bwd_cta(const int* ticket) { return __shfl_sync(0xffffffffu, *ticket, 0); }
+
+// The last CTA puts the words back to zero (the error flag stays until the host has seen it).
+__device__ __forceinline__ void bwd_depart(const NormBwdParams& p) {
+  if (threadIdx.x == 0 && atomicAdd(&p.bar[2], 1u) == gridDim.x - 1) {
+    atomicExch(&p.bar[0], 0u);
+    atomicExch(&p.bar[2], 0u);
+    atomicExch(&p.bar[3], 0u);
+    __threadfence();
+  }
+}
+
+// A worker's partial row is written: every thread of the CTA calls this.
+__device__ __forceinline__ void bwd_worker_done(const NormBwdParams& p) {
+  if (p.finalizers == 0) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&p.bar[0], 1u);
+  }
+  bwd_depart(p);
+}
+
+// Waits until all workers have arrived; false when one has given up or the bound ran out (some seconds: with a scratch for few
+// partial rows there are few workers, which may take long).
+__device__ __forceinline__ bool bwd_wait_for_workers(const NormBwdParams& p, int* flag) {
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    for (unsigned int spins = 0;; ++spins) {
+      unsigned int seen, err;
+      asm volatile("ld.global.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(p.bar) : "memory");
+      asm volatile("ld.global.relaxed.gpu.u32 %0, [%1];" : "=r"(err) : "l"(p.bar + 1) : "memory");
+      if (err == 0u && seen >= (unsigned int)p.workers) break;
+      if (err != 0u || spins > (1u << 24)) {
+        atomicExch(&p.bar[1], 1u);
+        ok = 0;
+        break;
+      }
+      __nanosleep(spins > 4096 ? 256 : 32);  // the workers' copies have the memory system
+    }
+    __threadfence();
+    *flag = ok;
+  }
+  __syncthreads();
+  return *flag != 0;
+}
 
 template <int V>
 __device__ __forceinline__ void zero(float (&a)[V]) {
@@ -79,11 +145,9 @@ __device__ __forceinline__ void finalize_columns(const float* partials, int grou
   }
 }
 
-// The same inside a cooperative launch, after its grid barrier, for rows of n % 4 == 0 columns: the
-// columns of dw and db are dealt out in units of 8 (a 32-byte sector of a partial row), so that the whole grid takes
-// part (192 CTAs for 768 columns of both) and no second level, with a second grid barrier, is needed
-// (LayerNorm backward bf16 [32768, 768], together with the copies that start before the weights are
-// staged: 45.1 us with the two levels, 39.0 us so). Where that makes more units than CTAs, units of 16, 32 or 64
+// The same by the finalizers of the launch, for rows of n % 4 == 0 columns: the
+// columns of dw and db are dealt out in units of 8 (a 32-byte sector of a partial row), a finalizer each
+// (192 CTAs for 768 columns of both). Where that makes more units than CTAs that fit, units of 16, 32 or 64
 // columns: a unit is two barriers and a load latency, whatever its width (LayerNorm f32 [256, 8192]: 27.9 us with
 // 2048 units of 8, 17.2 us with two times 128 of 64).
 // width / 4 threads share a partial row's unit, the CTA's threads split the partial rows. fp64, fixed order.
@@ -91,12 +155,13 @@ __device__ __forceinline__ void finalize_columns(const float* partials, int grou
 // registers than the kernels around it (the streaming kernel of fp32 RMSNorm 82 -> 120, so that one CTA of 288 threads
 // fitted an SM instead of two: f32 [16352, 2052] 86 -> 112 us).
 __device__ __forceinline__ void finalize_units(const float* partials, int groups, int n, float* dw, float* db,
-                                               const int width, double* smem /* [warps][width] */) {
+                                               const int width, const int first, const int step,
+                                               double* smem /* [warps][width] */) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int share = width / 4, units = (n + width - 1) / width, rows_at_once = blockDim.x / share;
   const int sub = tid & (share - 1);
   const int total = units * ((dw ? 1 : 0) + (db ? 1 : 0));
-  for (int s = blockIdx.x; s < total; s += gridDim.x) {
+  for (int s = first; s < total; s += step) {
     const bool is_db = !dw || s >= units;
     const int col = (dw && s >= units ? s - units : s) * width;
     const int c = col + 4 * sub;
@@ -140,20 +205,20 @@ __device__ __forceinline__ void finalize_units(const float* partials, int groups
   }
 }
 
-// A call, so that the width that a few calls need stays out of the registers and the code of the kernels.
-static __device__ __noinline__ void finalize_wide_units(const float* partials, int groups, int n, float* dw, float* db,
-                                                        double* smem) {
-  const int planes = (dw ? 1 : 0) + (db ? 1 : 0);
-  int width = 16;
-  while (width < 64 && (n + width - 1) / width * planes > (int)gridDim.x) width *= 2;
-  finalize_units(partials, groups, n, dw, db, width, smem);
+// What a CTA with a ticket beyond the workers' does: waits, adds up, leaves.
+__device__ __forceinline__ void bwd_finalize(const NormBwdParams& p, int cta, float* db, double* smem, int* flag) {
+  if (bwd_wait_for_workers(p, flag))
+    finalize_units(p.partials, p.groups, p.n, p.dw, db, p.width, cta - p.workers, p.finalizers, smem);
+  bwd_depart(p);
 }
 
-__device__ __forceinline__ void finalize_grid(const NormBwdParams& p, float* db, double* smem /* [warps][64] */) {
-  if ((p.n + 7) / 8 * ((p.dw ? 1 : 0) + (db ? 1 : 0)) <= (int)gridDim.x)
-    finalize_units(p.partials, p.groups, p.n, p.dw, db, 8, smem);
-  else
-    finalize_wide_units(p.partials, p.groups, p.n, p.dw, db, smem);
+// Host: how many finalizers a launch of rows of n columns gets, and the width of their units. `room`: CTAs of the kernel that fit.
+inline void bwd_plan_finalize(NormBwdParams& p, long long room) {
+  const int planes = (p.dw ? 1 : 0) + (p.db ? 1 : 0);
+  p.width = 8;
+  while (p.width < 64 && (long long)(p.n + p.width - 1) / p.width * planes > room) p.width *= 2;
+  const long long units = (long long)(p.n + p.width - 1) / p.width * planes;
+  p.finalizers = (int)(units < room ? units : room);
 }
 
 // Warp reduction of N (2, 4 or 8) values per lane at once: in every step a lane keeps one half of
@@ -188,7 +253,7 @@ __device__ __forceinline__ float warp_reduce_multi(float (&v)[N], int lane) {
 // Returns false when the shape does not fit (the caller takes another kernel); otherwise *rc is
 // the launch status.
 template <typename T, bool LN>
-bool try_launch_norm_bwd_warp(NormBwdParams p, size_t scratch_bytes, bool cooperative, cudaStream_t st, int* rc);
+bool try_launch_norm_bwd_warp(NormBwdParams p, size_t scratch_bytes, bool fused, cudaStream_t st, int* rc);
 
 unsigned int norm_bwd_warp_wait_timeouts();  // bounded waits of that kernel that ran out
 

@@ -7,7 +7,7 @@
 // norm_bwd.cu (same evaluation order as the decomposed aten graphs, see there).
 //
 // Structure
-//   * Persistent cooperative grid of 256-thread CTAs. Warp g of the grid takes rows g, g + G, ...
+//   * Persistent 256-thread CTAs. Warp g of the workers takes rows g, g + G, ...
 //   * A stage of a warp's ring holds one row of x and one row of dy, brought in by two bulk
 //     asynchronous copies that lane 0 issues; the warp waits on the stage's mbarrier. There is no
 //     CTA barrier in the row loop, and the bytes in flight (stages - 1 rows per warp) do not
@@ -19,10 +19,10 @@
 //   * Two sweeps over the stage: row sums first (one batched warp reduction), then dx and the
 //     gradient sums. The stage is refilled as soon as the second sweep has read it.
 //   * At the end the warps of a CTA fold their sums in a fixed order through shared memory into
-//     ONE fp32 partial row per CTA; after the grid barrier the partial rows are added in fp64 by
-//     the whole grid. No atomics: results are bit-reproducible.
+//     ONE fp32 partial row per CTA; CTAs that start after the workers add the partial rows in fp64
+//     (the two roles of norm_bwd.cuh). No atomics on results: they are bit-reproducible.
 // Every wait is bounded; a wait that runs out makes the warp stop, wait (bounded) for its own
-// copies and raise the error word of the grid barrier, so that all CTAs leave.
+// copies and raise the error word, so that nobody waits for it.
 #include "norm_bwd.cuh"
 
 namespace b200 {
@@ -41,7 +41,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;  // fp32 pairs per vector
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ int bar_ok;
+  __shared__ int bar_ok, ticket;
   __shared__ int cta_failed;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = p.n / V;
@@ -52,10 +52,8 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + ring_bytes) + warp * 8;
   float* wsm = reinterpret_cast<float*>(smem + ring_bytes + kWarps * 8 * sizeof(uint64_t));
   const int rows = (int)p.rows;  // the launcher admits fewer than 2^31 rows
-  const int gwarp = (int)blockIdx.x * kWarps + warp;
-  const int gstep = (int)gridDim.x * kWarps;
-  const int my_rows = rows > gwarp ? (rows - gwarp + gstep - 1) / gstep : 0;
 
+  bwd_draw_ticket(p, &ticket);
   if (threadIdx.x == 0) cta_failed = 0;
   if (lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
@@ -64,6 +62,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
 
   const T* xg = reinterpret_cast<const T*>(p.x);
   const T* dyg = reinterpret_cast<const T*>(p.dy);
+  int gwarp = 0, gstep = 1;
   auto issue = [&](int k, int slot) {  // lane 0 only
     const long long row = (long long)gwarp + (long long)k * gstep;
     unsigned char* dst = ring + (size_t)slot * stage_bytes;
@@ -99,12 +98,18 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     }
   }
   const float dyf = DYS ? Elem<T>::to_f32(ld_here(dyg)) : 0.f;
-  // the other lanes first touch the barriers after the __syncthreads below
-  int issued = 0;
-  if (lane == 0) {
-    for (; issued < my_rows && issued < stages; ++issued) issue(issued, issued);
+  __syncthreads();  // the ticket is there
+  const int cta = bwd_cta(&ticket);
+  if (cta >= p.workers) {
+    bwd_finalize(p, cta, LN ? p.db : nullptr, reinterpret_cast<double*>(smem), &bar_ok);
+    return;
   }
-  issued = __shfl_sync(0xffffffffu, issued, 0);
+  gwarp = cta * kWarps + warp;
+  gstep = p.workers * kWarps;
+  const int my_rows = rows > gwarp ? (rows - gwarp + gstep - 1) / gstep : 0;
+  if (lane == 0) {
+    for (int k = 0; k < my_rows && k < stages; ++k) issue(k, k);
+  }
   const f32x2 dy_all = splat2(dyf);
 
   // LayerNorm keeps its weight slice in shared memory (it already keeps two gradient sums per column in
@@ -190,11 +195,11 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     if (!arrived) {
       if (lane == 0) {
         note_wait_timeout();
-        atomicExch(&p.bar[1], 1u);  // lets the other CTAs leave the grid barrier at once
+        if (p.bar) atomicExch(&p.bar[1], 1u);  // nobody is to wait for this CTA
         atomicExch(&cta_failed, 1);
         int ds = slot;
         uint32_t dp = phase;
-        for (int d = k; d < issued; ++d) {  // none of this warp's copies may be in flight at exit
+        for (int d = k; d < my_rows && d < k + stages; ++d) {  // none of this warp's copies may be in flight at exit
           mbar_wait(&full[ds], dp);
           if (++ds == stages) { ds = 0; dp ^= 1u; }
         }
@@ -335,12 +340,9 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
 
     // every lane has read the stage: refill it with the row `stages` further on
     __syncwarp();
-    if (k + stages < my_rows) {
-      if (lane == 0) {
-        fence_proxy_async_smem();
-        issue(k + stages, slot);
-      }
-      ++issued;
+    if (lane == 0 && k + stages < my_rows) {
+      fence_proxy_async_smem();
+      issue(k + stages, slot);
     }
     if (++slot == stages) {
       slot = 0;
@@ -390,17 +392,11 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
         float4 out;
         unpack2(lo, out.x, out.y);
         unpack2(hi, out.z, out.w);
-        *reinterpret_cast<float4*>(p.partials + ((long long)plane * p.groups + blockIdx.x) * p.n + col) = out;
+        *reinterpret_cast<float4*>(p.partials + ((long long)plane * p.groups + cta) * p.n + col) = out;
       }
     }
-    __syncthreads();  // the fold area doubles as the fp64 area of the finalize
   }
-  if (p.fused) {
-    double* fin = reinterpret_cast<double*>(smem);  // [warps][64] fp64, inside the ring
-    const bool ok = !any_failed && grid_barrier(p.bar, 1u, &bar_ok);
-    if (ok) finalize_grid(p, LN ? p.db : nullptr, fin);
-    grid_barrier_depart(p.bar);
-  }
+  bwd_worker_done(p);
 }
 
 template <typename T, int CH, bool LN, bool DYS>
@@ -411,7 +407,7 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
   const size_t stage_bytes = (DYS ? 1 : 2) * (size_t)nv * 16;
   // barriers (+ fp32 weight slots; a second table of the same size for LayerNorm with a scalar dy)
   const size_t fixed = kWarps * 8 * sizeof(uint64_t) + (LN ? (size_t)(DYS ? 2 : 1) * CH * 32 * V * sizeof(float) : 0);
-  // the ring doubles as the fold area [2][kWarps][CH * 32 * V] fp32 and as the fp64 area of the finalize
+  // the ring doubles as the fold area [2][kWarps][CH * 32 * V] fp32 and as the finalizers' fp64 area
   size_t floor_bytes = 2 * (size_t)kWarps * CH * 32 * V * sizeof(float);
   if (floor_bytes < 16 * 64 * sizeof(double)) floor_bytes = 16 * 64 * sizeof(double);
   int stages = 0, ctas_per_sm = (LN && DYS) ? 3 : 2;  // the scalar-dy LayerNorm form needs fewer registers
@@ -444,17 +440,11 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
     if (max_groups < 1) return false;
     if (grid > max_groups) grid = max_groups;
   }
-  p.groups = (int)grid;
-  p.fused = 1;
-  e = launch_cooperative(kernel, dim3((unsigned)grid), dim3(kWarps * 32), smem, st, p, stages, (int)ring_bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    *rc = fail((int)e, "b200_norm_bwd: cooperative launch failed: %s", cudaGetErrorString(e));
-    return true;
-  }
-  note_launch(DYS ? "b200_norm_bwd [warp per row, warp rings, scalar dy, fused finalize]"
-                  : "b200_norm_bwd [warp per row, warp rings, fused finalize]");
-  *rc = B200_OK;
+  p.groups = p.workers = (int)grid;
+  bwd_plan_finalize(p, (long long)per_sm * dev.sm_count);
+  launch_dependent(kernel, (unsigned)(grid + p.finalizers), kWarps * 32, smem, st, p, stages, (int)ring_bytes);
+  *rc = launch_status(DYS ? "b200_norm_bwd [warp per row, warp rings, scalar dy, fused finalize]"
+                          : "b200_norm_bwd [warp per row, warp rings, fused finalize]");
   return true;
 }
 
@@ -467,13 +457,13 @@ bool launch_warp_kernel(NormBwdParams p, size_t scratch_bytes, cudaStream_t st, 
 }  // namespace
 
 template <typename T, bool LN>
-bool try_launch_norm_bwd_warp(NormBwdParams p, size_t scratch_bytes, bool cooperative, cudaStream_t st, int* rc) {
+bool try_launch_norm_bwd_warp(NormBwdParams p, size_t scratch_bytes, bool fused, cudaStream_t st, int* rc) {
   constexpr int V = Elem<T>::V;
   static const bool off = [] {
     const char* e = getenv("B200_NORM_BWD_NO_WARP_RINGS");
     return e && e[0] == '1';
   }();
-  if (off || !cooperative || !(p.dw || p.db)) return false;  // the kernel is the fused, single-launch form
+  if (off || !fused || !(p.dw || p.db)) return false;  // the kernel is the fused, single-launch form
   const long long nv = p.n / V;
   if (nv <= 32 || nv > (V == 4 ? 256 : 128) || p.rows >= 0x7fffffffLL) return false;
   {  // dx is addressed with 32-bit element offsets
