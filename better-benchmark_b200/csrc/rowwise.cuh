@@ -480,6 +480,65 @@ inline bool pick_row_geometry(long long nv, RowGeometry* g) {
   return true;
 }
 
+// ----------------------------------------------------------------------------------------------
+// Rows that start and end anywhere, as the 16-byte vectors of memory that they touch: vector j holds the row's elements
+// j V - off .. j V - off + V - 1. Only the first and the last one may hold others beside them; those two are
+// read and written element by element, so that nothing outside the row is touched. Tensors with the same `off` in every
+// row share the vectors.
+// ----------------------------------------------------------------------------------------------
+struct RowSpan {
+  int off;   // elements between the 16-byte boundary and the row's first one
+  int nv;    // vectors
+  int last;  // elements of the last vector that lie in front of the row's end
+
+  template <typename T>
+  __device__ __forceinline__ static RowSpan of(const T* row, int n) {
+    constexpr int V = Elem<T>::V;
+    RowSpan s;
+    s.off = (int)((reinterpret_cast<uintptr_t>(row) & 15u) / sizeof(T));
+    s.nv = (n + s.off + V - 1) / V;
+    s.last = n + s.off - (s.nv - 1) * V;
+    return s;
+  }
+  // The elements of vector j that belong to the row: [lo(j), hi(j)).
+  __device__ __forceinline__ int lo(int j) const { return j == 0 ? off : 0; }
+  template <int V>
+  __device__ __forceinline__ int hi(int j) const {
+    return j == nv - 1 ? last : V;
+  }
+  template <int V>
+  __device__ __forceinline__ bool whole(int j) const {
+    return (j != 0 || off == 0) && (j != nv - 1 || last == V);
+  }
+};
+
+// Elements [lo, hi) of the vector at p, zeros beside them.
+template <typename T>
+__device__ __forceinline__ uint4 load_part(const T* p, int lo, int hi) {
+  constexpr int V = Elem<T>::V;
+  union {
+    T e[V];
+    uint4 raw;
+  } u;
+  u.raw = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if (i >= lo && i < hi) u.e[i] = ld_here(p + i);
+  return u.raw;
+}
+template <typename T>
+__device__ __forceinline__ void store_part(T* p, const uint4& raw, int lo, int hi) {
+  constexpr int V = Elem<T>::V;
+  union {
+    T e[V];
+    uint4 raw;
+  } u;
+  u.raw = raw;
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if (i >= lo && i < hi) p[i] = u.e[i];
+}
+
 template <int G>
 __device__ __forceinline__ int glane() {
   return G == 0 ? (int)threadIdx.x : (int)(threadIdx.x & (G - 1));

@@ -342,7 +342,7 @@ __device__ __forceinline__ float softmax_logit(const SoftmaxParams& p, const Tin
   return t;
 }
 
-// Rows with a mask (or short ones) that the vector path cannot take: a warp per row (n <= 512) or a
+// Rows with a mask (or short ones) that neither the vector path nor softmax_span_kernel takes: a warp per row (n <= 512) or a
 // CTA per row, E elements per thread at a distance of the group, held in registers: one read of the
 // row and of its mask instead of the three sweeps below, every access of a warp one coalesced stretch
 // whatever the alignment. Bound by the number of 2-byte accesses and the exponentials. Measured with a key mask: fp16
@@ -404,6 +404,302 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 ? 2 : 0)
     const int i = e * gs + lane;
     if (i < p.n) y[i] = Elem<Tout>::from_f32(p.log_mode ? t[e] - ls : (sizeof(Tout) == 4 ? t[e] / s : t[e] * inv));
   }
+}
+
+// 16-bit rows at one distance, off the 16-byte grid, whose result has their alignment (contiguous rows of an odd length, in the input's
+// dtype): the row as the vectors it touches (RowSpan), in registers from the load to the store. A group of G lanes takes
+// `reps` rows that are a multiple of eight apart and so have the same alignment: what belongs to a column, the mask, stays in its registers
+// as long as the rows share it, and holds -inf where a vector reaches beyond the row, so that no other part of the loop asks what is
+// inside. The next row is on its way meanwhile. Numerics as in softmax_rows_kernel: the maximum keeps NaN, differences are
+// clamped for the pair exponential. Bound by instructions (the same with every edge asked for in every row: 709 a warp and row of 333
+// elements, 84 % of the issue slots), so the mask stays packed, four CTAs of 256 threads an SM up to two vectors a lane. Key mask,
+// fp16, against softmax_ragged_kernel: [60000, 333] 53.9 -> 32.8 us, [20000, 716] 39.4 -> 21.5, [60000, 1001] 146 -> 67,
+// [60000, 114] 19.6 -> 13.3.
+template <typename T, int K, int G>
+__global__ void __launch_bounds__(256, K <= 2 ? 4 : K == 3 ? 3 : 2) softmax_span_kernel(const SoftmaxParams p, const int reps) {
+  wait_for_previous_kernel();
+  static_assert(sizeof(T) == 2, "pairs of 16-bit elements");
+  constexpr int V = Elem<T>::V;
+  constexpr int P = V / 2;
+  constexpr float kFloor = -1e30f;
+  const int lane = glane<G>();
+  constexpr int gs = G, step = 256 / G;  // rows that the CTA takes at a time: a multiple of eight
+  const int rows = (int)p.rows;
+  int row = (int)blockIdx.x * reps * step + (int)threadIdx.x / G;
+  const T* x0 = reinterpret_cast<const T*>(p.x);
+  const long long pitch = p.xmap.s0;
+  const RowSpan span = RowSpan::of(x0 + row * pitch, p.n);
+  // whole vectors are read where all of them lies between the first row's start and the last row's end
+  const uintptr_t x_first = reinterpret_cast<uintptr_t>(x0), x_end = reinterpret_cast<uintptr_t>(x0 + (rows - 1) * pitch + p.n);
+  auto fetch = [&](int r, uint4 (&raw)[K]) {
+    const T* x = x0 + r * pitch - span.off + (long long)lane * V;
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      const int j = c * gs + lane;
+      const T* at = x + (long long)c * gs * V;
+      raw[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < rows && j < span.nv) {
+        const uintptr_t u = reinterpret_cast<uintptr_t>(at);
+        if (u >= x_first && u + 16 <= x_end) raw[c] = ld_stream(at);
+        else raw[c] = load_part(at, span.lo(j), span.hi<V>(j));
+      }
+    }
+  };
+  // which halves of the words of the first and the last vector belong to the row
+  uint32_t in_first[P], in_last[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    in_first[i] = (2 * i >= span.off ? 0xffffu : 0u) | (2 * i + 1 >= span.off ? 0xffff0000u : 0u);
+    in_last[i] = (2 * i < span.last ? 0xffffu : 0u) | (2 * i + 1 < span.last ? 0xffff0000u : 0u);
+  }
+  uint4 m[K];
+  auto set_mask = [&](const T* mask) {
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      const int j = c * gs + lane;
+      const int lo = span.lo(j), hi = j < span.nv ? span.hi<V>(j) : 0;
+      union {
+        T e[V];
+        uint4 raw;
+      } u;
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        u.e[i] = Elem<T>::from_f32(-INFINITY);
+        if (i >= lo && i < hi) u.e[i] = mask ? ld_here(mask - span.off + (long long)j * V + i) : Elem<T>::from_f32(0.f);
+      }
+      m[c] = u.raw;
+    }
+  };
+  uint4 next[K];
+  fetch(row, next);
+  long long mask_at = -1;
+  if (!p.mask) set_mask(nullptr);
+  const f32x2 scale2 = splat2(p.has_scale ? p.scale : 1.f);
+
+  for (int rep = 0; rep < reps; ++rep, row += step) {
+    const bool valid = row < rows;
+    if (!__any_sync(0xffffffffu, valid)) break;
+    uint4 raw[K];
+#pragma unroll
+    for (int c = 0; c < K; ++c) raw[c] = next[c];
+    if (rep + 1 < reps) fetch(row + step, next);
+    if (p.mask && valid) {
+      const long long at = row_offset(p.mmap, row);
+      if (at != mask_at) {
+        mask_at = at;
+        set_mask(reinterpret_cast<const T*>(p.mask) + at);
+      }
+    }
+    f32x2 t[K][P];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      uint32_t w[P] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+      if (c == 0 && lane == 0) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) w[i] &= in_first[i];
+      }
+      if (c * gs + lane == span.nv - 1) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) w[i] &= in_last[i];
+      }
+      f32x2 mc[P];
+      Pairs<T>::unpack(m[c], mc);
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        t[c][i] = add2(mul2(Pairs<T>::word(w[i]), scale2), mc[i]);
+        float a, b;
+        unpack2(t[c][i], a, b);
+        mx = MaxOp::apply(mx, MaxOp::apply(a, b));
+      }
+    }
+    mx = greduce<MaxOp, G>(mx, nullptr);
+
+    auto finish = [&](auto log_tag) {
+      constexpr bool LOG = decltype(log_tag)::value;
+      const f32x2 mx2 = splat2(mx);
+      f32x2 s2 = splat2(0.f);
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          t[c][i] = sub2(t[c][i], mx2);
+          float a, b;
+          unpack2(t[c][i], a, b);
+          const f32x2 e = exp_pair_compensated(pack2(fmaxf(a, kFloor), fmaxf(b, kFloor)));
+          s2 = add2(s2, e);
+          if constexpr (!LOG) t[c][i] = e;
+        }
+      }
+      float s = greduce<SumOp, G>(hsum2(s2), nullptr);
+      if (!(fabsf(mx) < INFINITY)) s = NAN;  // aten's x - max is NaN for a row of -inf and where x is inf; a NaN poisons its row
+      if (!valid) return;
+      const f32x2 k2 = splat2(LOG ? logf(s) : __frcp_rn(s));
+      T* y = reinterpret_cast<T*>(p.y) + row * p.ymap.s0 - span.off + (long long)lane * V;
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        const int j = c * gs + lane;
+        if (j < span.nv) {
+          f32x2 o[P];
+#pragma unroll
+          for (int i = 0; i < P; ++i) o[i] = LOG ? sub2(t[c][i], k2) : mul2(t[c][i], k2);
+          const uint4 out = Pairs<T>::pack(o);
+          if (span.whole<V>(j)) st_stream(y + (long long)c * gs * V, out);
+          else store_part(y + (long long)c * gs * V, out, span.lo(j), span.hi<V>(j));
+        }
+      }
+    };
+    if (p.log_mode) finish(std::true_type{});
+    else finish(std::false_type{});
+  }
+}
+
+// The same for longer rows: a CTA per row, as many of them as the SM holds; the mask is read element by element through L1, where
+// eight such loads a vector take as long as HBM takes for the vector and its result. (With eight rows per CTA in turn, as above:
+// [20000, 1241] 50.3 us.) fp16 with a key mask: [20000, 1241] 64 -> 39 us, [20000, 2047] 98 -> 62, [5000, 5001] 69 -> 36.
+template <typename T, int K>
+__global__ void __launch_bounds__(512) softmax_span_row_kernel(const SoftmaxParams p) {
+  wait_for_previous_kernel();
+  static_assert(sizeof(T) == 2, "pairs of 16-bit elements");
+  constexpr int V = Elem<T>::V;
+  constexpr int P = V / 2;
+  constexpr float kFloor = -1e30f;
+  __shared__ float red[32];
+  const int lane = (int)threadIdx.x, gs = (int)blockDim.x;
+  const long long row = blockIdx.x;
+  const T* x = reinterpret_cast<const T*>(p.x) + row_offset(p.xmap, row);
+  const RowSpan span = RowSpan::of(x, p.n);
+  x -= span.off;
+  uint4 raw[K];
+#pragma unroll
+  for (int c = 0; c < K; ++c) {
+    const int j = c * gs + lane;
+    raw[c] = make_uint4(0u, 0u, 0u, 0u);
+    if (j < span.nv) {
+      if (span.whole<V>(j)) raw[c] = ld_stream(x + (long long)j * V);
+      else raw[c] = load_part(x + (long long)j * V, span.lo(j), span.hi<V>(j));
+    }
+  }
+  const T* m = p.mask ? reinterpret_cast<const T*>(p.mask) + row_offset(p.mmap, row) - span.off : nullptr;
+  T* y = reinterpret_cast<T*>(p.y) + row_offset(p.ymap, row) - span.off;
+
+  f32x2 t[K][P];
+  float mx = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < K; ++c) {
+    const int j = c * gs + lane;
+    float f[V];
+    Elem<T>::unpack(raw[c], f);
+    if (p.has_scale) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) f[i] = f[i] * p.scale;
+    }
+    if (j < span.nv) {
+      const int lo = span.lo(j), hi = span.hi<V>(j);
+      if (m) {
+        const T* mj = m + (long long)j * V;
+        T mv[V];
+        if (span.whole<V>(j)) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) mv[i] = ld_here(mj + i);
+        } else {
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            mv[i] = Elem<T>::from_f32(0.f);
+            if (i >= lo && i < hi) mv[i] = ld_here(mj + i);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) f[i] = f[i] + Elem<T>::to_f32(mv[i]);
+      }
+      if (!span.whole<V>(j)) {
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+          if (i < lo || i >= hi) f[i] = -INFINITY;
+      }
+#pragma unroll
+      for (int i = 0; i < V; ++i) mx = MaxOp::apply(mx, f[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i) f[i] = -INFINITY;
+    }
+#pragma unroll
+    for (int i = 0; i < P; ++i) t[c][i] = pack2(f[2 * i], f[2 * i + 1]);
+  }
+  mx = block_reduce<MaxOp>(mx, red);
+
+  auto finish = [&](auto log_tag) {
+    constexpr bool LOG = decltype(log_tag)::value;
+    const f32x2 mx2 = splat2(mx);
+    f32x2 s2 = splat2(0.f);
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        t[c][i] = sub2(t[c][i], mx2);
+        float a, b;
+        unpack2(t[c][i], a, b);
+        const f32x2 e = exp_pair_compensated(pack2(fmaxf(a, kFloor), fmaxf(b, kFloor)));
+        s2 = add2(s2, e);
+        if constexpr (!LOG) t[c][i] = e;
+      }
+    }
+    float s = block_reduce<SumOp>(hsum2(s2), red);
+    if (!(fabsf(mx) < INFINITY)) s = NAN;  // as above
+    const f32x2 k2 = splat2(LOG ? logf(s) : __frcp_rn(s));
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      const int j = c * gs + lane;
+      if (j < span.nv) {
+        f32x2 o[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i) o[i] = LOG ? sub2(t[c][i], k2) : mul2(t[c][i], k2);
+        const uint4 out = Pairs<T>::pack(o);
+        if (span.whole<V>(j)) st_stream(y + (long long)j * V, out);
+        else store_part(y + (long long)j * V, out, span.lo(j), span.hi<V>(j));
+      }
+    }
+  };
+  if (p.log_mode) finish(std::true_type{});
+  else finish(std::false_type{});
+}
+
+// Whether the two kernels above take the rows: x and y have the same alignment in every row, and there are enough of them (what
+// belongs to a column costs the groups 1 us once; fp16 rows from which on they are ahead of softmax_ragged_kernel: about 7000 of 41 to 249
+// elements, 2000 of 333, 600 of 501 to 1001, 300 beyond: [2000, 333] 3.88 -> 3.75 us, [2000, 716] 6.1 -> 4.5, [64, 716] 2.5 -> 3.6).
+// Up to 1017 elements (four vectors a lane) groups, above that CTAs.
+template <typename T>
+static bool try_launch_softmax_span(const SoftmaxParams& p, cudaStream_t st) {
+  constexpr int V = Elem<T>::V;
+  const long long sms = device_info().sm_count;
+  const int nv = (p.n + 2 * (V - 1)) / V;  // vectors that a row touches at most
+  auto flat = [](const RowMap& m) { return m.d1.d == 1 && m.d2.d == 1 && m.s0 >= 0; };
+  if (!flat(p.xmap) || !flat(p.ymap) || (reinterpret_cast<uintptr_t>(p.x) & 15u) != (reinterpret_cast<uintptr_t>(p.y) & 15u) ||
+      (p.xmap.s0 - p.ymap.s0) % V != 0 || p.rows > 0x7fff0000LL)
+    return false;
+  if (p.rows < (p.n <= 256 ? 48 : p.n <= 384 ? 14 : nv <= 128 ? 5 : 2) * sms) return false;
+  if (nv > 128) {
+    if (nv <= 512) launch_dependent(softmax_span_row_kernel<T, 2>, (unsigned)p.rows, (nv + 63) / 64 * 32, 0, st, p);
+    else if (nv <= 2048) launch_dependent(softmax_span_row_kernel<T, 4>, (unsigned)p.rows, (nv + 127) / 128 * 32, 0, st, p);
+    else return false;
+    return true;
+  }
+  auto launch = [&](auto kernel, int lanes) {
+    const int at_once = 256 / lanes;
+    const long long resident = sms * cached_occupancy(reinterpret_cast<const void*>(kernel), 256);
+    long long reps = p.rows / (at_once * resident);
+    reps = reps < 1 ? 1 : (reps > 16 ? 16 : reps);
+    launch_dependent(kernel, (unsigned)((p.rows + at_once * reps - 1) / (at_once * reps)), 256, 0, st, p, (int)reps);
+    return true;
+  };
+  if (nv <= 8) return launch(softmax_span_kernel<T, 1, 8>, 8);
+  if (nv <= 16) return launch(softmax_span_kernel<T, 2, 8>, 8);
+  if (nv <= 24) return launch(softmax_span_kernel<T, 3, 8>, 8);
+  if (nv <= 32) return launch(softmax_span_kernel<T, 2, 16>, 16);
+  if (nv <= 48) return launch(softmax_span_kernel<T, 3, 16>, 16);
+  if (nv <= 64) return launch(softmax_span_kernel<T, 2, 32>, 32);
+  if (nv <= 96) return launch(softmax_span_kernel<T, 3, 32>, 32);
+  return launch(softmax_span_kernel<T, 4, 32>, 32);
 }
 
 template <typename Tin, typename Tout, bool PACKED>
@@ -1045,6 +1341,9 @@ static int launch_softmax(const SoftmaxParams& p, bool vector_ok, cudaStream_t s
     launch_dependent(softmax_long_kernel<Tin, Tout>, (unsigned)p.rows, threads, 0, st, p);
   } else if (p.n <= 8192) {
     set_path_tag("elements in registers");
+    if constexpr (std::is_same<Tin, Tout>::value && sizeof(Tin) == 2 && !PACKED) {
+      if (try_launch_softmax_span<Tin>(p, st)) return launch_status("b200_softmax");
+    }
     if (p.n > 64 && p.n <= 2048 && p.rows <= (p.n <= 512 ? 4LL : 2LL) * device_info().sm_count) {
       launch_dependent(softmax_ragged_kernel<Tin, Tout, PACKED, 2, 0>, (unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st, p);
     } else if (p.n <= 512) {

@@ -1,0 +1,63 @@
+"""Masked softmax of many 16-bit rows off the 16-byte grid: groups of lanes that keep the mask, and a CTA per row."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(rows, n, dtype, mask, scale, start, log, batches=4):
+    """x, out and what lies around them in one storage each, so that an access outside is seen (NaN in, a changed guard out)."""
+    from better_benchmark_b200 import kernels as k
+    g = torch.Generator(device="cuda").manual_seed(n + rows)
+    size = rows * n
+    xs = torch.full((size + 64,), float("nan"), device="cuda", dtype=dtype)
+    xs[start:start + size] = (torch.randn(size, generator=g, device="cuda") * 3).to(dtype)
+    ys = torch.full((size + 64,), 7.0, device="cuda", dtype=dtype)
+    x, y = (t[start:start + size].view(batches, rows // batches, n) for t in (xs, ys))
+    k.softmax(x, mask=mask, scale=scale, log=log, out=y)
+    assert bool((ys[:start] == 7).all()) and bool((ys[start + size:] == 7).all()), "nothing beside the rows is written"
+    t = x.double() * (1.0 if scale is None else scale)
+    if mask is not None:
+        t = t + mask.double()
+    return y, torch.log_softmax(t, -1) if log else torch.softmax(t, -1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=str)
+@pytest.mark.parametrize("n", [1, 7, 9, 50, 57, 58, 114, 121, 122, 185, 249, 250, 257, 377, 378, 505, 506, 761, 762, 1017, 1018, 1241, 2047, 4089, 4090, 8191])
+def test_spans(dtype, n):
+    """Both sides of every change of geometry; every alignment of the first row; masks per batch, per row and none."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = ((48 if n <= 256 else 14 if n <= 384 else 5 if n <= 1017 else 2) * sms + 15) // 4 * 4
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    g = torch.Generator(device="cuda").manual_seed(n)
+    key = torch.where(torch.rand(4, 1, n, generator=g, device="cuda") < 0.7, 0.0, -10000.0).to(dtype)
+    per_row = torch.randn(4, rows // 4, n, generator=g, device="cuda").to(dtype)
+    cases = [(key, 0.125, 0, False), (None, None, 3, False), (per_row, None, 0, True), (key, 0.5, 5, True)]
+    for start in (1, 2, 4, 6, 7):
+        cases.append((key, None, start, False))
+    for mask, scale, start, log in cases:
+        y, want = _run(rows, n, dtype, mask, scale, start, log)
+        # one rounding of the result, and fp32 steps in front of it (of a log-probability also in its terms, which may be 1e4)
+        bound = ulp * want.abs() + (4e-6 * want.abs().clamp(max=1e4) + 2e-5 if log else 2e-6 * want + 6.2e-8)
+        assert bool(((y.double() - want).abs() <= bound).all()), (n, start, log, ((y.double() - want).abs() - bound).max().item())
+
+
+@pytest.mark.parametrize("n", [41, 333, 1001, 1241])
+def test_special_values(n):
+    """Masks of -inf and of the type's lowest value, rows without a key, infinities and NaN in one row, which stay there."""
+    from better_benchmark_b200 import kernels as k
+    rows = 8000
+    x = torch.randn(2, rows // 2, n, device="cuda").half()
+    x[0, 5, 3], x[0, 6, 0], x[1, 7, n - 1], x[1, 9] = float("nan"), float("inf"), float("-inf"), float("-inf")
+    for low in (float("-inf"), torch.finfo(torch.float16).min):
+        mask = torch.zeros(2, 1, n, device="cuda", dtype=torch.float16)
+        mask[0, :, n // 2:] = low
+        mask[1, :, 1:] = low
+        for log in (False, True):
+            got = k.softmax(x, mask=mask, scale=0.5, log=log)
+            t = x.double() * 0.5 + mask.double()
+            want = torch.log_softmax(t, -1) if log else torch.softmax(t, -1)
+            assert torch.equal(torch.isnan(got), torch.isnan(want))
+            assert torch.allclose(got.double(), want.to(got.dtype).double(), rtol=2e-3, atol=1e-6 if not log else 2e-2, equal_nan=True)
+    full = torch.full((2, 1, n), float("-inf"), device="cuda", dtype=torch.float16)
+    assert bool(torch.isnan(k.softmax(x, mask=full)).all())
