@@ -11,73 +11,13 @@
 // The variance is the centred second pass over the row held in registers (squares accumulated with
 // fused multiply-adds: aten's var_mean has no multiply/add sequence to mirror). Statistics are fp32.
 // Any of y, mean, rstd, var may be null (var_mean alone = no y, no rstd).
-#include "rowwise.cuh"
+#include "norm_fwd.cuh"
 #include "tile_stream.cuh"
 
 #include <cstdlib>
 #include <type_traits>
 
 namespace b200 {
-
-struct NormFwdParams {
-  const void* x;
-  const void* w;  // may be null
-  const void* b;  // may be null
-  void* y;        // may be null
-  float* mean_out;
-  float* rstd_out;
-  float* var_out;
-  long long rows;
-  int n;
-  long long x_row_stride, y_row_stride;  // elements
-  int w_dtype;
-  float eps;
-  float inv_n;      // 1 / n
-  float inv_denom;  // 1 / (n - correction)
-  int rms;
-  int prologue;     // 0: none; 1: exact (erf) GELU of x, rounded to x's dtype, is what gets normalised
-  // Residual prologue (the post-LayerNorm blocks, repros/canonical/var_mean_0ada225c0a04/repro.py:26-27):
-  // what gets normalised is T(x + res); res has x's dtype and row stride. sum_out (may be null)
-  // receives that rounded sum, rows of n elements, contiguous.
-  const void* res;
-  void* sum_out;
-  // 1: the sum is rounded to x's dtype before it is normalised, as the eager graph materialises it;
-  // 0: it stays in fp32, as in Inductor's fused kernel - the form the reference's fp64-anchored gate
-  // accepts (the fp64 evaluation of the graph has no such rounding);
-  // 2 (what the stubs use; LayerNorm of 16-bit tensors): both rows are normalised, each with its own
-  // statistics, and every element takes the fp32 form where that form's rounded output exceeds 3 in
-  // magnitude and the rounded form elsewhere - the rule of the reference's oracle for these regions
-  // (repros/canonical/var_mean_45f7dfd4a983/oracle.py:96-107). Small outputs then equal the eager
-  // module's (its element-wise check allows 1e-2 + 1e-2 |y|, less than two 16-bit steps between 1.3
-  // and 2 and between 2.6 and 4), large ones, which decide the maximum error against the fp64 graph,
-  // carry no intermediate rounding. The statistics that are returned are those of the fp32 sum.
-  int res_round;
-};
-
-// Pointwise prologue of the LayerNorm regions that normalise an activation
-// (repros/canonical/var_mean_af505388b035/repro.py:27-33): (x * 0.5) * (erf(x * 0.7071067811865476) + 1)
-// in fp32, in that order, then rounded to the tensor dtype - the graph materialises the
-// activation as a 16-bit tensor before the statistics are taken.
-// (16-bit tensors: gelu_pair, whose fp32 result is as close to the fp64 one as that expression's.)
-template <typename Tin>
-__device__ __forceinline__ f32x2 gelu_erf_rounded2(f32x2 v) {
-  if constexpr (sizeof(Tin) == 2) {
-    return Pairs<Tin>::word(Pairs<Tin>::narrow(gelu_pair(v)));
-  } else {
-    float a, b;
-    unpack2(v, a, b);
-    return pack2((a * 0.5f) * (erff(a * 0.7071067811865476f) + 1.0f), (b * 0.5f) * (erff(b * 0.7071067811865476f) + 1.0f));
-  }
-}
-template <typename Tin>
-__device__ __forceinline__ float gelu_erf_rounded(float x) {
-  float a, b;
-  unpack2(gelu_erf_rounded2<Tin>(splat2(x)), a, b);
-  return a;
-}
-
-// rsqrtf is the 2-ulp hardware approximation aten's CUDA rsqrt uses as well.
-__device__ __forceinline__ float precise_rsqrt(float v) { return rsqrtf(v); }
 
 template <typename Tin, typename Tout, int CH, int G, bool GELU, bool RES>
 // Residual instantiations with sub-warp rows: three CTAs of 256 threads per SM (80 registers, a few
@@ -637,16 +577,6 @@ static bool try_launch_norm_fwd_stream(const NormFwdParams& p, cudaStream_t st, 
 // ----------------------------------------------------------------------------------------------
 constexpr int kResWarps = 8;  // warps per CTA
 
-// |a| > 3 per 16-bit half: all ones or zeros (zeros for NaN)
-template <typename T>
-__device__ __forceinline__ uint32_t beyond_three(uint32_t a) {
-  if constexpr (std::is_same<T, __half>::value) {
-    return __hgt2_mask(__habs2(*reinterpret_cast<const __half2*>(&a)), __float2half2_rn(3.0f));
-  } else {
-    return __hgt2_mask(__habs2(*reinterpret_cast<const __nv_bfloat162*>(&a)), __float2bfloat162_rn(3.0f));
-  }
-}
-
 template <typename T, int CH, bool EXACT, bool BOTH>
 __global__ void __launch_bounds__(kResWarps * 32, 3)
 residual_norm_warp_kernel(const NormFwdParams p, const int stages) {
@@ -963,6 +893,7 @@ __global__ void __launch_bounds__(1024) norm_fwd_streaming_kernel(const NormFwdP
 // elements per thread at a distance of the group, so that every access of a warp is one coalesced
 // stretch of 2- or 4-byte elements whatever the row's alignment. The row is read once; the element-wise
 // sweeps below read it two to six times and are left with rows of more than 16 384 elements (16 a thread).
+// Many rows of a 16-bit type, and long ones of fp32, go by the vector instead (norm_fwd_span.cu, with both sides' times).
 // Bound by the number of those accesses: about 1.6 TB/s for 16-bit elements, 3.3 TB/s for fp32.
 // Measured against the sweeps: LayerNorm bf16 [4800, 769] 114 -> 17.5 us, [4800, 8191] 246 -> 158, RMSNorm f32 [4800, 1001]
 // 82 -> 14.6 us, residual LayerNorm (both forms) bf16 [18682, 449] 322 -> 52 us.
@@ -1128,6 +1059,9 @@ static int launch_norm_fwd(const NormFwdParams& p, bool vector_ok, cudaStream_t 
 #undef B200_NF_LAUNCH
   } else if (p.n <= 16384) {
     set_path_tag(p.res ? "residual add, elements in registers" : "elements in registers");
+    if constexpr (kResBuilt) {
+      if (try_launch_norm_fwd_span<Tin>(p, st)) return launch_status("b200_norm_fwd");
+    }
     if (p.n > 128 && p.n <= 2048 && p.rows <= (p.n <= 512 ? 8LL : 2LL) * device_info().sm_count) {
       launch_dependent(norm_fwd_ragged_kernel<Tin, Tout, 2, 0>, (unsigned)p.rows, ((p.n + 1) / 2 + 31) / 32 * 32, 0, st, p);
     } else if (p.n <= 512) {  // a warp per row

@@ -539,6 +539,50 @@ __device__ __forceinline__ void store_part(T* p, const uint4& raw, int lo, int h
     if (i >= lo && i < hi) p[i] = u.e[i];
 }
 
+// Which halves (fp32: words) of the first and the last vector belong to the row.
+template <typename T>
+__device__ __forceinline__ void span_edges(const RowSpan& span, uint32_t (&in_first)[4], uint32_t (&in_last)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (sizeof(T) == 2) {
+      in_first[i] = (2 * i >= span.off ? 0xffffu : 0u) | (2 * i + 1 >= span.off ? 0xffff0000u : 0u);
+      in_last[i] = (2 * i < span.last ? 0xffffu : 0u) | (2 * i + 1 < span.last ? 0xffff0000u : 0u);
+    } else {
+      in_first[i] = i >= span.off ? 0xffffffffu : 0u;
+      in_last[i] = i < span.last ? 0xffffffffu : 0u;
+    }
+  }
+}
+
+// The vectors of row r, whole where all of them lies between the first row's start and the last row's end.
+template <typename T, int K>
+__device__ __forceinline__ void span_fetch(const void* base, long long pitch, long long rows, int n, long long r, bool there,
+                                           const RowSpan& span, int lane, int gs, uint4 (&raw)[K]) {
+  constexpr int V = Elem<T>::V;
+  const T* x0 = reinterpret_cast<const T*>(base);
+  const uintptr_t first = reinterpret_cast<uintptr_t>(x0), end = reinterpret_cast<uintptr_t>(x0 + (rows - 1) * pitch + n);
+  const T* x = x0 + r * pitch - span.off + (long long)lane * V;
+  const int nv = there ? span.nv : 0;
+#pragma unroll
+  for (int c = 0; c < K; ++c) raw[c] = make_uint4(0u, 0u, 0u, 0u);
+  if (r > 0 && r + 1 < rows && pitch >= n) {  // rows on both sides
+#pragma unroll
+    for (int c = 0; c < K; ++c)
+      if (c * gs + lane < nv) raw[c] = ld_stream(x + (long long)c * gs * V);
+  } else {
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      const int j = c * gs + lane;
+      const T* at = x + (long long)c * gs * V;
+      if (j < nv) {
+        const uintptr_t u = reinterpret_cast<uintptr_t>(at);
+        if (u >= first && u + 16 <= end) raw[c] = ld_stream(at);
+        else raw[c] = load_part(at, span.lo(j), span.hi<V>(j));
+      }
+    }
+  }
+}
+
 template <int G>
 __device__ __forceinline__ int glane() {
   return G == 0 ? (int)threadIdx.x : (int)(threadIdx.x & (G - 1));
