@@ -814,6 +814,7 @@ __global__ void __launch_bounds__(128) norm_bwd_cols_general_kernel(const NormBw
 // row, E elements per thread at a distance of the group: every access of a warp is one coalesced
 // stretch whatever the alignment, a thread's columns are the same in every row, so its weights and its
 // sums of dweight / dbias stay in registers. One partial row per CTA, added up by the finalize launch.
+// (More rows of more than 512 columns by the vector: norm_bwd_span.cu, with both sides' times.)
 // Bound by the number of 2- and 4-byte accesses, about half of HBM speed. Measured against the three
 // passes (with the finalize below): LayerNorm bf16 [20000, 449] 121 -> 34.4 us, [300, 513] 9.8 -> 6.8, [1397, 3001] 40.5 ->
 // 24.9, RMSNorm f32 [20000, 769] 191 -> 55 us.
@@ -1136,16 +1137,20 @@ static bool try_launch_norm_bwd_ragged(NormBwdParams p, size_t scratch_bytes, cu
     p.groups = p.workers = (int)grid;
     launch_dependent(kernel, (unsigned)grid, threads, smem, st, p);
     *rc = launch_status("b200_norm_bwd [ragged rows, elements in registers]");
-    if (*rc == B200_OK && sums) {
+    return true;
+  };
+  auto finalize = [&](bool launched) {
+    if (launched && *rc == B200_OK && sums) {
       launch_dependent(norm_bwd_finalize_ragged_kernel, dim3((p.n + 15) / 16, (p.dw ? 1 : 0) + (p.db ? 1 : 0)), 512, 0, st, p);
       *rc = launch_status("b200_norm_bwd finalize");
     }
-    return true;
+    return launched;
   };
-  if (p.n <= 128) return launch(norm_bwd_ragged_kernel<T, LN, 4, 32>, 256);
-  if (p.n <= 256) return launch(norm_bwd_ragged_kernel<T, LN, 8, 32>, 256);
-  if (p.n <= 512) return launch(norm_bwd_ragged_kernel<T, LN, 16, 32>, 256);
-  return launch(norm_bwd_ragged_kernel<T, LN, 8, 0>, ((p.n + 7) / 8 + 31) / 32 * 32);
+  if (try_launch_norm_bwd_span<T, LN>(p, scratch_bytes, st, rc)) return finalize(true);
+  if (p.n <= 128) return finalize(launch(norm_bwd_ragged_kernel<T, LN, 4, 32>, 256));
+  if (p.n <= 256) return finalize(launch(norm_bwd_ragged_kernel<T, LN, 8, 32>, 256));
+  if (p.n <= 512) return finalize(launch(norm_bwd_ragged_kernel<T, LN, 16, 32>, 256));
+  return finalize(launch(norm_bwd_ragged_kernel<T, LN, 8, 0>, ((p.n + 7) / 8 + 31) / 32 * 32));
 }
 
 template <typename T, bool LN>

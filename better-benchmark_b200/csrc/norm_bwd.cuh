@@ -257,4 +257,9 @@ bool try_launch_norm_bwd_warp(NormBwdParams p, size_t scratch_bytes, bool fused,
 
 unsigned int norm_bwd_warp_wait_timeouts();  // bounded waits of that kernel that ran out
 
+// Rows off the 16-byte grid whose dy and dx have their alignment (norm_bwd_span.cu): the rows and p.groups partial rows. False: the caller
+// takes another kernel.
+template <typename T, bool LN>
+bool try_launch_norm_bwd_span(NormBwdParams& p, size_t scratch_bytes, cudaStream_t st, int* rc);
+
 }  // namespace b200
