@@ -1178,7 +1178,7 @@ static int launch_norm_bwd(NormBwdParams p, bool vector_ok, size_t scratch_bytes
           if (try_launch_norm_bwd_tile<T, 4, LN>(p, narrow, scratch_bytes, st, &rc, g)) return rc;
         if (try_launch_norm_bwd_tile<T, 2, LN>(p, narrow, scratch_bytes, st, &rc)) return rc;
       }
-      if (nv <= 32) return launch_norm_bwd_fast<T, 1, false, LN>(p, 256, scratch_bytes, fused, st);
+      if (nv <= 32) return launch_norm_bwd_narrow<T, LN>(p, scratch_bytes, fused, st);
       if (nv <= 64) return launch_norm_bwd_fast<T, 2, false, LN>(p, 256, scratch_bytes, fused, st);
       return launch_norm_bwd_fast<T, 4, false, LN>(p, 256, scratch_bytes, fused, st);
     }
@@ -1239,8 +1239,8 @@ extern "C" int64_t b200_norm_bwd_wait_timeouts(void) {
 
 // Bytes of scratch that let every path run its largest grid for rows of n elements: the barrier
 // words and two planes (dweight, dbias) of one fp32 partial row per group. A group is a CTA (at most eight resident
-// per SM), except in the warp-per-row register kernel that takes rows of up to 256 elements, where it is a warp (64 per
-// SM). The launchers shrink their grids to whatever scratch they are given, so a smaller buffer
+// per SM), except in the warp-per-row register kernel, which takes rows of up to 256 elements where the copy rings do not
+// fit, where it is a warp (64 per SM). (Rows of at most 32 vectors: fp64, at most six per SM.) The launchers shrink their grids to whatever scratch they are given, so a smaller buffer
 // costs speed, never correctness.
 extern "C" int64_t b200_norm_bwd_scratch_bytes(int64_t n) {
   const int64_t groups = (n <= 256 ? 64 : 8) * (int64_t)device_info().sm_count;

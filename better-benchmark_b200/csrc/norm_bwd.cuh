@@ -257,6 +257,10 @@ bool try_launch_norm_bwd_warp(NormBwdParams p, size_t scratch_bytes, bool fused,
 
 unsigned int norm_bwd_warp_wait_timeouts();  // bounded waits of that kernel that ran out
 
+// Rows of at most 32 vectors (norm_bwd_narrow.cu).
+template <typename T, bool LN>
+int launch_norm_bwd_narrow(NormBwdParams p, size_t scratch_bytes, bool fused, cudaStream_t st);
+
 // Rows off the 16-byte grid whose dy and dx have their alignment (norm_bwd_span.cu): the rows and p.groups partial rows. False: the caller
 // takes another kernel.
 template <typename T, bool LN>
