@@ -934,6 +934,10 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
     unpack2(d, a, b);
     return pack2(expf(a), expf(b));
   };
+  // fp32 rows with 16-bit results keep their exponentials where the row was, and multiply them by the sum's inverse at the end (f32 -> bf16
+  // [2000, 10698] 32.5 -> 29.3 us, [4000, 2909] 15.9 -> 14.7; with fp32 results, where the division takes as long as expf, they stand
+  // in the way: 46.6 -> 50.5 us; and a cluster would have to agree on the maximum first: [1425, 29114] 72 -> 80).
+  constexpr bool KEEP = sizeof(Tin) == 4 && sizeof(Tout) == 2 && !LOG && !CLUSTER;
   auto add_up = [&](auto exponential) {
     const f32x2 own = splat2(M);
     f32x2 sum = splat2(0.f);
@@ -942,10 +946,19 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
       if (c * T_ + tid < cnt) {
         f32x2 t[P];
         logits(c, t);
-        f32x2 part = exponential(sub2(t[0], own));
+        if constexpr (KEEP) {
+          const f32x2 e0 = exponential(sub2(t[0], own)), e1 = exponential(sub2(t[1], own));
+          sum = add2(sum, add2(e0, e1));
+          float a, b, c2, d;
+          unpack2(e0, a, b);
+          unpack2(e1, c2, d);
+          raw[c] = make_uint4(__float_as_uint(a), __float_as_uint(b), __float_as_uint(c2), __float_as_uint(d));
+        } else {
+          f32x2 part = exponential(sub2(t[0], own));
 #pragma unroll
-        for (int i = 1; i < P; ++i) part = add2(part, exponential(sub2(t[i], own)));
-        sum = add2(sum, part);
+          for (int i = 1; i < P; ++i) part = add2(part, exponential(sub2(t[i], own)));
+          sum = add2(sum, part);
+        }
       }
     }
     return hsum2(sum);
@@ -959,6 +972,8 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
   bool finite = true;
   if constexpr (sizeof(Tout) == 4) {
     s = add_up(exp_exact);
+  } else if constexpr (KEEP) {  // no second try: the row is gone
+    s = add_up([&](f32x2 d) { return exp_pair_compensated(clamped(d)); });
   } else {
     s = add_up([](f32x2 d) { return exp_pair_compensated(d); });
     finite = s == s;
@@ -1000,10 +1015,14 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
       f32x2 t[P], o[P];
       const bool valid = j < cnt;
       if (!valid) raw[c] = make_uint4(0u, 0u, 0u, 0u);
-      logits(c, t);
+      if constexpr (KEEP) Pairs<Tin>::unpack(raw[c], t);
+      else logits(c, t);
       if constexpr (LOG) {
 #pragma unroll
         for (int i = 0; i < P; ++i) o[i] = sub2(sub2(t[i], M2), log_sum2);
+      } else if constexpr (KEEP) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) o[i] = mul2(t[i], inv2);
       } else if constexpr (sizeof(Tout) == 4) {
 #pragma unroll
         for (int i = 0; i < P; ++i) {
@@ -1049,19 +1068,26 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
 //     SM four times (bf16 [1024, 131075]: 4 CTAs 193 us, 8 CTAs 182, two sweeps 317).
 //   * No more than half as many rows as SMs: 8 CTAs once a row has 1024 vectors (bf16 [8, 131072] 7.4 us, two
 //     sweeps 17.6; [64, 65536] 9.4 and 12.3; [16, 20005] 4.8, one CTA 5.7; f32 [16, 4099] 4.4 and 5.6).
-//   * Otherwise aligned rows of more than 8192 vectors are read twice: the second sweep finds the row in L2, and a
-//     CTA per row loads and stores at its own pace where a cluster waits for its slowest CTA twice a row
-//     (bf16 [1024, 131072]: two sweeps 134 us, clusters 144; [682, 196608] 132 and 188; [512, 262136] 143 and
-//     168; f32 [1024, 65536] 148 and 161). fp32 log-probabilities of 16-bit rows are the exception, their
-//     sweeps being bound by expf (bf16 -> f32 log [1024, 131072]: 250 and 187 us, [682, 196608]: 246 and 241).
-//   * fp32 rows of more than 16 384 vectors are read twice on any alignment (f32 [682, 98307] 208 us, 231 as clusters).
+//   * Up to one row per SM, aligned rows of more than 8192 vectors are read twice: the second sweep finds the row in L2, and a CTA per row
+//     loads and stores at its own pace where a cluster waits for its slowest CTA twice a row (f32 [100, 98304] 31 us, clusters 35). So
+//     are fp32 rows of more than 16384 vectors on any alignment.
+//   * With more rows than SMs (the CTAs of a second wave, or the second row of some SMs, cost the sweeps a whole row's time), only aligned
+//     ones of more than 16384 vectors (12288 of 16 bits with fp32 results) are: bf16 [682, 196608] two sweeps 132 us, clusters 171;
+//     f32 [682, 98304] 148 and 182. Shorter ones: f32 [1500, 40000] 156 and 136, [195, 65536] 43 and 33; bf16 [300, 98304] 44 and 36; bf16 ->
+//     f32 [2000, 67584] 266 and 254, but [1024, 131072] 216 and 219. fp32 rows with 16-bit results of any length: [195, 113832]
+//     68 and 48, [682, 98304] 144 and 137. fp32 rows off the grid: [195, 113835] 98 and 64, -> bf16 96 and 48; [682, 98307] 207 and
+//     183, -> bf16 198 and 138.
+//   * fp32 log-probabilities of 16-bit rows are the exception, their sweeps being bound by expf (bf16 -> f32 log [1024, 131072]:
+//     250 and 177 us, [682, 196608]: 246 and 237).
 template <typename Tin, typename Tout>
 static int softmax_ctas_per_row(long long nvec, long long rows, bool aligned, bool log_mode) {
   if (nvec > 8 * 4096) return 0;
   if (2 * rows <= device_info().sm_count && nvec >= 1024) return 8;
   if (nvec > 8192) {
-    if (aligned && !(log_mode && sizeof(Tin) == 2 && sizeof(Tout) == 4)) return 0;
-    if (sizeof(Tin) == 4 && nvec > 16384) return 0;
+    constexpr bool IN16 = sizeof(Tin) == 2, OUT16 = sizeof(Tout) == 2;
+    const bool many = rows > device_info().sm_count;
+    if (aligned && !(log_mode && IN16 && !OUT16) && !(many && ((!IN16 && OUT16) || nvec <= (IN16 && !OUT16 ? 12288 : 16384)))) return 0;
+    if (!IN16 && nvec > 16384 && !many) return 0;
     return 8;
   }
   return nvec > (log_mode && sizeof(Tin) == 2 && sizeof(Tout) == 4 ? 2560 : 4096) ? 2 : 1;
@@ -1100,8 +1126,8 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
 }
 
 // ----------------------------------------------------------------------------------------------
-// Rows that softmax_ctas_per_row leaves (beyond 32768 vectors, that is 262 144 16-bit columns; long aligned ones and long
-// fp32 ones when there are many): one CTA per row, two sweeps.
+// Rows that softmax_ctas_per_row leaves (beyond 32768 vectors, that is 262 144 16-bit columns; long aligned ones, and fp32
+// ones when there are few): one CTA per row, two sweeps.
 //   sweep 1: every thread keeps a running maximum m and the sum of exp(t - m) of its elements,
 //            rescaling the sum when the maximum grows; the CTA then combines the (m, s) pairs:
 //            M = max m_i, S = sum s_i * exp(m_i - M)

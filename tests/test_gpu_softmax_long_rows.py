@@ -1,0 +1,41 @@
+"""Softmax of long rows with more rows than SMs: clusters or two sweeps; fp32 rows with 16-bit results that keep their exponentials."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("log", [False, True])
+@pytest.mark.parametrize("n,dtype,out_dtype,path", [
+    (32772, torch.float32, torch.float32, b"cluster"), (65536, torch.float32, torch.float32, b"cluster"),
+    (65540, torch.float32, torch.float32, b"two sweeps"), (65537, torch.float32, torch.float32, b"cluster"),
+    (131072, torch.float32, torch.float16, b"cluster"), (131075, torch.float32, torch.bfloat16, b"cluster"),
+    (131076, torch.float32, torch.bfloat16, b"two sweeps"), (65544, torch.bfloat16, torch.bfloat16, b"cluster"),
+    (131072, torch.float16, torch.float16, b"cluster"), (131080, torch.bfloat16, torch.bfloat16, b"two sweeps"),
+    (2909, torch.float32, torch.bfloat16, b"registers of a CTA"), (16384 + 3, torch.float32, torch.float16, b"registers of a CTA"),
+], ids=str)
+def test_many_long_rows(n, dtype, out_dtype, path, log):
+    from better_benchmark_b200 import kernels as k
+    rows = torch.cuda.get_device_properties(0).multi_processor_count + 1
+    x = (torch.randn(rows, n, device="cuda") * 3).to(dtype)
+    x[3, : n // 2] = float("-inf")
+    x[4, 5], x[5, n - 1], x[6] = float("nan"), float("inf"), float("-inf")
+    if dtype != torch.float16 and path != b"two sweeps":
+        x[7], x[7, 9] = -3e38, 3e38    # differences beyond what fp32 holds
+    got = k.softmax(x, log=log, out_dtype=out_dtype)
+    assert path in k.load().b200_last_kernel(), k.load().b200_last_kernel()
+    want = torch.log_softmax(x.double(), -1) if log else torch.softmax(x.double(), -1)
+    poisoned = torch.isnan(got).all(-1)
+    assert bool(poisoned[4:7].all()) and int(poisoned.sum()) == 3
+    ok = ~poisoned
+    ulp = {torch.float32: 2.0 ** -23, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[out_dtype]
+    got, want = got[ok].double(), want[ok]
+    if log:
+        # the difference, the logarithm of the sum and their difference, each rounded once, and 2e-6 for the sum's own error
+        finite = torch.isfinite(got) & (want.abs() < 1e30)
+        bound = ulp * want.abs() + 2.0 ** -23 * want.abs() + 4e-6
+        assert bool(((got - want).abs() <= bound)[finite].all())
+        assert bool((got[~finite] < -6e4).all())
+    else:
+        # the exponent's difference may be off by half an ulp of 30 and the exponential by two of its own
+        assert bool(((got - want).abs() <= ulp * want + 4e-6 * want + 6.2e-8 * (out_dtype == torch.float16) + 1e-38).all())
