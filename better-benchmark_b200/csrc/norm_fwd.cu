@@ -299,13 +299,13 @@ norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contig
   // Weight and bias are asked for first: behind the first copies of all CTAs (30 MB) they took 4 us to arrive, and no
   // row is worked on before they are there.
   fetch_params(threadIdx.x);
-  int issued = 0;
-  int issue_slot = 0;  // stage the next copy goes to
+  // What has been issued follows from the tile at hand: max(k - 1, 0) + stages tiles before tile k. (Thread 0's counters of it cost every
+  // thread eight registers: 32768 rows, LayerNorm bf16 640 columns 20.1 -> 19.3 us, behind GELU 768 32.6 -> 31.7 and f32 1024 57.5 -> 54.0;
+  // at most 1 % slower anywhere, RMSNorm f32 640.)
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
     mbar_init_fence();
-    for (; issued < my_tiles_i && issued < stages; ++issued) issue(issued, issued);
-    issue_slot = issued % stages;
+    for (int k = 0; k < my_tiles_i && k < stages; ++k) issue(k, k);
   }
 
   for (int j = threadIdx.x; j < nv; j += blockDim.x) {
@@ -347,7 +347,7 @@ norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contig
         note_wait_timeout();
         int ds = st;
         uint32_t dp = phase;
-        for (int d = k; d < issued; ++d) {
+        for (int d = k; d < my_tiles_i && d < (k > 0 ? k - 1 : 0) + stages; ++d) {
           mbar_wait(&full[ds], dp);
           if (++ds == stages) { ds = 0; dp ^= 1u; }
         }
@@ -355,11 +355,9 @@ norm_fwd_stream_kernel(const NormFwdParams p, const int stages, const int contig
       return;
     }
     // Everyone has passed the barrier, so everyone is done with tile k-1: refill its stage.
-    if (threadIdx.x == 0 && k >= 1 && issued < my_tiles_i) {
+    if (threadIdx.x == 0 && k >= 1 && k - 1 + stages < my_tiles_i) {
       fence_proxy_async_smem();
-      issue(issued, issue_slot);
-      ++issued;
-      if (++issue_slot == stages) issue_slot = 0;
+      issue(k - 1 + stages, st == 0 ? stages - 1 : st - 1);
     }
     const bool valid = row < rows_i;
 
