@@ -72,6 +72,20 @@ cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes) {
   return e;
 }
 
+static std::mutex& launch_order(cudaStream_t st) {
+  static std::mutex mutexes[64];
+  uintptr_t key = reinterpret_cast<uintptr_t>(st);
+  if (st == nullptr || st == cudaStreamLegacy) {  // one stream per device under two names
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+    key = (uintptr_t)dev << 4;
+  }
+  return mutexes[((key >> 4) * 0x9e3779b97f4a7c15ull) >> 58];
+}
+
+LaunchesTogether::LaunchesTogether(cudaStream_t st) : held_(&launch_order(st)) { static_cast<std::mutex*>(held_)->lock(); }
+LaunchesTogether::~LaunchesTogether() { static_cast<std::mutex*>(held_)->unlock(); }
+
 int cached_occupancy(const void* fn, int threads, size_t smem) {
   struct Entry { const void* fn; int threads, device; size_t smem; int blocks; };
   static Entry cache[256];

@@ -847,6 +847,7 @@ extern "C" int b200_batch_norm_fwd_ex(const void* x, void* y, const void* weight
   const bool cl_vector = cl && aligned16(x) && aligned16(y);
   p.rows = batch;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const LaunchesTogether together(st);
   switch (x_dtype) {
     case B200_F32: return launch_batch_norm<float>(p, cl_vector, (size_t)scratch_bytes, st);
     case B200_BF16: return launch_batch_norm<__nv_bfloat16>(p, cl_vector, (size_t)scratch_bytes, st);

@@ -878,6 +878,7 @@ extern "C" int b200_batch_norm_bwd_ex(const void* dy, const void* x, const void*
   const bool fast = cl && pv >= 1 && pv <= 512 && batch * spatial * channels >= v && aligned16(dy) &&
                     aligned16(x) && (!act || aligned16(act)) && (!dx || aligned16(dx));
   p.rows = fast ? batch * spatial : batch;
+  const LaunchesTogether together(st);
   switch (x_dtype) {
     case B200_F32: return launch_bn_bwd<float>(p, fast, (size_t)scratch_bytes, st);
     case B200_BF16: return launch_bn_bwd<__nv_bfloat16>(p, fast, (size_t)scratch_bytes, st);

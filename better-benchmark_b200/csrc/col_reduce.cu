@@ -310,6 +310,7 @@ extern "C" int b200_col_reduce(const void* x, void* out, int64_t batch, int64_t 
                    cols % (16 / eb) == 0;
   const size_t sb = scratch ? (size_t)scratch_bytes : 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const LaunchesTogether together(st);
   switch (x_dtype) {
     case B200_F32: return launch_col_reduce<float>(p, vec, sb, st);
     case B200_BF16: return launch_col_reduce<__nv_bfloat16>(p, vec, sb, st);

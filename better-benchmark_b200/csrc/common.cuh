@@ -362,6 +362,21 @@ cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
 // Sets a function attribute that is the same for every launch, once per kernel and device.
 cudaError_t set_function_attribute_once(const void* kernel, cudaFuncAttribute attr, int value);
 
+// Held by every entry point that takes scratch memory while it launches. The kernels of one call hand partial results to each other
+// in the scratch, and callers on one stream share a scratch: with launches of two host threads mixed (rows of A, rows of B, finalize
+// of A) A would get B's sums. Keyed by the stream (the legacy default stream by its device): threads on
+// different streams, which need a scratch each, do not wait for one another, unless their streams share one of the 64 locks.
+class LaunchesTogether {
+ public:
+  explicit LaunchesTogether(cudaStream_t st);
+  ~LaunchesTogether();
+  LaunchesTogether(const LaunchesTogether&) = delete;
+  LaunchesTogether& operator=(const LaunchesTogether&) = delete;
+
+ private:
+  void* held_;
+};
+
 // Resident CTAs per SM (at least 1): a host-side calculation, cached per (kernel, block size, smem, device). In abi.cu.
 int cached_occupancy(const void* fn, int threads, size_t smem = 0);
 

@@ -1292,6 +1292,7 @@ extern "C" int b200_norm_bwd(const void* x, const void* dy, const void* weight, 
              (dx_seq_stride * eb) % 16 == 0 && (dx_head_stride * eb) % 16 == 0;
   if (weight) vec = vec && reinterpret_cast<uintptr_t>(weight) % w_chunk == 0;
 
+  const LaunchesTogether together(st);
 #define B200_NBWD_CASE(TT, DT)                                                              \
   if (x_dtype == DT)                                                                        \
     return rms ? launch_norm_bwd<TT, false>(p, vec, (size_t)scratch_bytes, fused, st) \

@@ -340,7 +340,8 @@ def residual_layer_norm_as(x, residual, weight, bias, shape, shape2, *, eps: flo
 # Scratch memory. Kernels that combine per-CTA partial results take a caller-provided scratch
 # buffer. One zero-initialised buffer per device is kept here; the first 256 bytes hold the
 # grid-barrier words, which every kernel leaves at zero when it finishes. Kernels on one stream run
-# in order, so sharing the buffer is safe there; callers that launch on several streams at once must
+# in order, and the library lets no launch of another thread in between those of one call, so sharing the buffer is safe
+# there; callers that launch on several streams at once must
 # pass their own ``scratch``. A request for more bytes than the buffer holds allocates a larger one,
 # but the smaller ones are never released: a CUDA graph captured earlier still holds their address.
 # Growing while the current stream is being captured is refused (the new buffer would belong to

@@ -20,7 +20,8 @@
  *   - Kernels that combine per-CTA partial results take a caller-provided `scratch` buffer
  *     (16-byte aligned). Its first 256 bytes hold grid-barrier words that must be zero before
  *     the first use; every kernel leaves them zero. Concurrent launches on different streams
- *     need different scratch buffers.
+ *     need different scratch buffers. Calls on one stream may share one, from several host threads
+ *     too: the launches of a call follow one another in the stream.
  *   - Accumulation is fp32 (fp64 where partial results of many CTAs are combined), no fast-math,
  *     no fused multiply-add contraction; reductions have a fixed order (bit-reproducible).
  */
