@@ -410,18 +410,17 @@ __global__ void __launch_bounds__(G == 0 ? 1024 : 256, G == 0 && E == 8 ? 2 : 0)
 // dtype): the row as the vectors it touches (RowSpan), in registers from the load to the store. A group of G lanes takes
 // `reps` rows that are a multiple of eight apart and so have the same alignment: what belongs to a column, the mask, stays in its registers
 // as long as the rows share it, and holds -inf where a vector reaches beyond the row, so that no other part of the loop asks what is
-// inside. The next row is on its way meanwhile. Numerics as in softmax_rows_kernel: the maximum keeps NaN, differences are
-// clamped for the pair exponential. Bound by instructions (the same with every edge asked for in every row: 709 a warp and row of 333
-// elements, 84 % of the issue slots), so the mask stays packed, four CTAs of 256 threads an SM up to two vectors a lane. Key mask,
-// fp16, against softmax_ragged_kernel: [60000, 333] 53.9 -> 32.8 us, [20000, 716] 39.4 -> 21.5, [60000, 1001] 146 -> 67,
-// [60000, 114] 19.6 -> 13.3.
+// inside. The next row is on its way meanwhile. Numerics as in softmax_ragged_kernel, expf included (the pair exponential, 5 to 15 % faster, is
+// less exact and loses subnormal bf16 probabilities); the maximum keeps NaN. Bound by instructions (with every edge asked for
+// in every row 709 a warp and row of 333 elements, 84 % of the issue slots), so the mask stays packed, four CTAs of 256 threads an SM up to two
+// vectors a lane (three vectors: 8 bytes of spills at three CTAs, four: 24 at two). Key mask, fp16, against softmax_ragged_kernel: [60000, 333]
+// 52.8 -> 35.2 us, [20000, 716] 38.5 -> 23.2, [60000, 1001] 141 -> 73, [60000, 114] 18.6 -> 14.3.
 template <typename T, int K, int G>
 __global__ void __launch_bounds__(256, K <= 2 ? 4 : K == 3 ? 3 : 2) softmax_span_kernel(const SoftmaxParams p, const int reps) {
   wait_for_previous_kernel();
   static_assert(sizeof(T) == 2, "pairs of 16-bit elements");
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;
-  constexpr float kFloor = -1e30f;
   const int lane = glane<G>();
   constexpr int gs = G, step = 256 / G;  // rows that the CTA takes at a time: a multiple of eight
   const int rows = (int)p.rows;
@@ -526,7 +525,7 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K == 3 ? 3 : 2) softmax_span
           t[c][i] = sub2(t[c][i], mx2);
           float a, b;
           unpack2(t[c][i], a, b);
-          const f32x2 e = exp_pair_compensated(pack2(fmaxf(a, kFloor), fmaxf(b, kFloor)));
+          const f32x2 e = pack2(expf(a), expf(b));
           s2 = add2(s2, e);
           if constexpr (!LOG) t[c][i] = e;
         }
@@ -555,15 +554,14 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K == 3 ? 3 : 2) softmax_span
 }
 
 // The same for longer rows: a CTA per row, as many of them as the SM holds; the mask is read element by element through L1, where
-// eight such loads a vector take as long as HBM takes for the vector and its result. (With eight rows per CTA in turn, as above:
-// [20000, 1241] 50.3 us.) fp16 with a key mask: [20000, 1241] 64 -> 39 us, [20000, 2047] 98 -> 62, [5000, 5001] 69 -> 36.
+// eight such loads a vector take as long as HBM takes for the vector and its result. (Eight rows per CTA in turn, as above, took 1.3 times
+// as long.) fp16 with a key mask: [20000, 1241] 61.9 -> 40.3 us, [20000, 2047] 95.2 -> 63.9, [20000, 3001] 147 -> 80.
 template <typename T, int K>
 __global__ void __launch_bounds__(512) softmax_span_row_kernel(const SoftmaxParams p) {
   wait_for_previous_kernel();
   static_assert(sizeof(T) == 2, "pairs of 16-bit elements");
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;
-  constexpr float kFloor = -1e30f;
   __shared__ float red[32];
   const int lane = (int)threadIdx.x, gs = (int)blockDim.x;
   const long long row = blockIdx.x;
@@ -639,7 +637,7 @@ __global__ void __launch_bounds__(512) softmax_span_row_kernel(const SoftmaxPara
         t[c][i] = sub2(t[c][i], mx2);
         float a, b;
         unpack2(t[c][i], a, b);
-        const f32x2 e = exp_pair_compensated(pack2(fmaxf(a, kFloor), fmaxf(b, kFloor)));
+        const f32x2 e = pack2(expf(a), expf(b));
         s2 = add2(s2, e);
         if constexpr (!LOG) t[c][i] = e;
       }

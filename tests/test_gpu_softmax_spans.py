@@ -61,3 +61,19 @@ def test_special_values(n):
             assert torch.allclose(got.double(), want.to(got.dtype).double(), rtol=2e-3, atol=1e-6 if not log else 2e-2, equal_nan=True)
     full = torch.full((2, 1, n), float("-inf"), device="cuda", dtype=torch.float16)
     assert bool(torch.isnan(k.softmax(x, mask=full)).all())
+
+
+@pytest.mark.parametrize("n", [41, 100, 333, 716, 1241])
+def test_probabilities_below_the_normal_range(n):
+    """bf16 holds numbers down to 2^-133 and so does fp32 below its normal range: probabilities there are not lost."""
+    from better_benchmark_b200 import kernels as k
+    rows = 200 * torch.cuda.get_device_properties(0).multi_processor_count
+    x = torch.full((rows, n), -80.0, device="cuda", dtype=torch.bfloat16)
+    x[:, 7] = 0.0
+    mask = torch.linspace(0.0, -12.0, n, device="cuda").to(torch.bfloat16)
+    mask[7] = 0.0
+    got, want = k.softmax(x, mask=mask).double(), torch.softmax(x[:1].double() + mask.double(), -1)
+    assert 0 < want.min() < 2.0 ** -130 and int((want < 2.0 ** -126).sum()) > n // 4
+    # bf16's rounding: half a step of eight significant bits, at most 2^-8 of the value, below the normal range half of 2^-133; in front of it
+    # those of fp32's exponential and of its product with the sum's inverse, 2^-21 of the value and steps of 2^-149 there
+    assert bool(((got - want).abs() <= (2.0 ** -8 + 2.0 ** -21) * want + 2.0 ** -134 + 2.0 ** -147).all())
