@@ -368,6 +368,7 @@ bool try_launch_norm_fwd_span(const NormFwdParams& p, cudaStream_t st) {
   } else {
     if (p.n <= 2048 || p.rows < 4 * sms || p.res || p.prologue) return false;
   }
+  set_path_tag(p.res ? "residual add, off-grid rows as vectors" : "off-grid rows as vectors");
   auto go = [&](auto kind_tag) {
     constexpr int KIND = decltype(kind_tag)::value;
     const bool whole = HALF && p.w_dtype == (std::is_same<T, __half>::value ? B200_F16 : B200_BF16) && off(p.w) == 0 && off(p.b) == 0;

@@ -676,10 +676,11 @@ static bool try_launch_softmax_span(const SoftmaxParams& p, cudaStream_t st) {
       (p.xmap.s0 - p.ymap.s0) % V != 0 || p.rows > 0x7fff0000LL)
     return false;
   if (p.rows < (p.n <= 256 ? 48 : p.n <= 384 ? 14 : nv <= 128 ? 5 : 2) * sms) return false;
+  if (nv > 2048) return false;
+  set_path_tag(nv > 128 ? "off-grid rows as vectors, CTA per row" : "off-grid rows as vectors, several rows in turn");
   if (nv > 128) {
     if (nv <= 512) launch_dependent(softmax_span_row_kernel<T, 2>, (unsigned)p.rows, (nv + 63) / 64 * 32, 0, st, p);
-    else if (nv <= 2048) launch_dependent(softmax_span_row_kernel<T, 4>, (unsigned)p.rows, (nv + 127) / 128 * 32, 0, st, p);
-    else return false;
+    else launch_dependent(softmax_span_row_kernel<T, 4>, (unsigned)p.rows, (nv + 127) / 128 * 32, 0, st, p);
     return true;
   }
   auto launch = [&](auto kernel, int lanes) {

@@ -34,7 +34,8 @@ def test_spans(dtype, n):
         stats = torch.empty(3, rows, device="cuda")
         rc = lib.b200_norm_fwd(x.data_ptr(), w.data_ptr() if has_w else None, b.data_ptr() if has_b else None, y.data_ptr(),
                                *(t.data_ptr() for t in stats), rows, n, n, n, code[dtype], code[wdt], code[dtype], eps, 0.0, int(rms), stream)
-        assert rc == 0
+        on_grid = start * x.element_size() % 16 == 0 and n * x.element_size() % 16 == 0
+        assert rc == 0 and (b"off-grid rows as vectors" in lib.b200_last_kernel()) == (n > 57 and not on_grid)
         assert bool((flat[:start] == 7).all()) and bool((flat[start + rows * n:] == 7).all()), "nothing beside the rows is written"
         d = x.double()
         mean = d.mean(-1, keepdim=True) * (0 if rms else 1)
@@ -67,6 +68,7 @@ def test_residual_and_gelu(dtype, n):
     rounded = k.norm_fwd(x, w, b, round_sum=True, **kw)[0]
     both, mean2, rstd2, _, total2 = k.norm_fwd(x, w, b, round_sum="both", **kw)
     gelu = k.norm_fwd(x, w, b, eps=1e-6, prologue="gelu_erf")[0]
+    assert b"[off-grid rows as vectors]" in k.load().b200_last_kernel()
     s = x.float() + r.float()
     bad = torch.zeros(rows, dtype=torch.bool, device="cuda")
     bad[5:8] = True

@@ -15,6 +15,8 @@ def _run(rows, n, dtype, mask, scale, start, log, batches=4):
     ys = torch.full((size + 64,), 7.0, device="cuda", dtype=dtype)
     x, y = (t[start:start + size].view(batches, rows // batches, n) for t in (xs, ys))
     k.softmax(x, mask=mask, scale=scale, log=log, out=y)
+    on_grid = start % 8 == 0 and n % 8 == 0
+    assert (b"off-grid rows as vectors" in k.load().b200_last_kernel()) == ((mask is not None or n < 256) and not on_grid)
     assert bool((ys[:start] == 7).all()) and bool((ys[start + size:] == 7).all()), "nothing beside the rows is written"
     t = x.double() * (1.0 if scale is None else scale)
     if mask is not None:

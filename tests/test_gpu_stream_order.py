@@ -40,9 +40,14 @@ def _calls():
         "transpose": ((64, 49, 128), torch.bfloat16, lambda x: k.permute_copy(x, (0, 2, 1))),
         # kernels for ragged rows and columns: scalar loads, of vectors along the row as well as of the row itself
         "softmax ragged, masked": ((700, 1003), torch.float16, lambda x: k.softmax(x, mask=x)),
-        "layer norm ragged": ((2000, 767), torch.bfloat16, lambda x: k.norm_fwd(x, x[0], x[1], eps=1e-5, want_rstd=True)[:3:2]),
+        "layer norm ragged": ((1000, 767), torch.bfloat16, lambda x: k.norm_fwd(x, x[0], x[1], eps=1e-5, want_rstd=True)[:3:2]),
         "norm backward ragged": ((2000, 767), torch.bfloat16,
                                  lambda x: k.norm_bwd(x, x, x[0], rstd, mean=mean, rms=False, want_dbias=True)),
+        # the same rows by the vector, where there are more of them
+        "softmax as vectors, masked": ((2000, 1003), torch.float16, lambda x: k.softmax(x, mask=x[0])),
+        "layer norm as vectors": ((2000, 767), torch.bfloat16, lambda x: k.norm_fwd(x, x[0], x[1], eps=1e-5, want_rstd=True)[:3:2]),
+        "norm backward as vectors": ((2000, 1601), torch.bfloat16,
+                                     lambda x: k.norm_bwd(x, x, x[0], rstd, mean=mean, rms=False, want_dbias=True)),
         "transpose ragged": ((16, 501, 333), torch.float16, lambda x: k.permute_copy(x, (0, 2, 1))),
         "dropout norm": ((2000, 512), torch.bfloat16, lambda x: k.dropout_rms_norm(x, res, w[:512], seeds, 0, 1, p=0.1, eps=1e-6)),
         "batch norm backward, sums": ((8, 28, 28, 64), torch.bfloat16,
@@ -53,10 +58,12 @@ def _calls():
 
 NAMES = ["cast", "silu", "row sum", "column sum", "softmax", "softmax ragged", "layer norm", "residual", "norm backward",
          "norm backward, weight", "batch norm", "batch norm backward", "batch norm nchw", "transpose",
-         "softmax ragged, masked", "layer norm ragged", "norm backward ragged", "transpose ragged", "dropout norm", "softmax dropout",
+         "softmax ragged, masked", "layer norm ragged", "norm backward ragged", "softmax as vectors, masked", "layer norm as vectors",
+         "norm backward as vectors", "transpose ragged", "dropout norm", "softmax dropout",
          "batch norm backward, sums"]
 KERNELS = {"softmax ragged, masked": b"b200_softmax [elements in registers]", "layer norm ragged": b"b200_norm_fwd [elements in registers]",
-           "norm backward ragged": b"b200_norm_bwd finalize", "transpose ragged": b"b200_transpose_copy [ragged 16-bit tiles]"}
+           "softmax as vectors, masked": b"b200_softmax [off-grid rows as vectors", "layer norm as vectors": b"b200_norm_fwd [off-grid rows as vectors]",
+           "norm backward ragged": b"b200_norm_bwd finalize", "norm backward as vectors": b"b200_norm_bwd finalize", "transpose ragged": b"b200_transpose_copy [ragged 16-bit tiles]"}
 
 
 def _list(out):
