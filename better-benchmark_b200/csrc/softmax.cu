@@ -662,9 +662,40 @@ __global__ void __launch_bounds__(512) softmax_span_row_kernel(const SoftmaxPara
   else finish(std::false_type{});
 }
 
-// Whether the two kernels above take the rows: x and y have the same alignment in every row, and there are enough of them (what
-// belongs to a column costs the groups 1 us once; fp16 rows from which on they are ahead of softmax_ragged_kernel: about 7000 of 41 to 249
-// elements, 2000 of 333, 600 of 501 to 1001, 300 beyond: [2000, 333] 3.88 -> 3.75 us, [2000, 716] 6.1 -> 4.5, [64, 716] 2.5 -> 3.6).
+// Rows per SM from which on the two kernels above are ahead of softmax_ragged_kernel at every number of rows measured (0: never), for rows
+// of n elements that touch nv vectors at most. A group reads its part of the mask once, 1 us; its slots are filled or not, as the other kernel's
+// are. That kernel / this one, us, fp16, rows per SM in front:
+//   n 57    48 2.9 / 2.8, 96 4.4 / 3.6        n 58    80 4.0 / 4.1, 104 4.7 / 4.7         n 121   72 4.6 / 4.3, 104 5.7 / 5.3
+//   n 150   48 4.3 / 4.6, 64 5.3 / 4.6        n 186   200 13.3 / 13.8, 250 16.2 / 15.8    n 249   200 14.7 / 14.0, 300 21.3 / 17.6
+//   n 257   24 3.9 / 4.5, 25 5.5 / 4.5        n 391   40 7.1 / 7.2, 48 7.6 / 8.1, 56 9.4 / 8.4    n 420   20 4.5 / 4.3, 48 7.7 / 7.6
+//   n 601   10 4.4 / 4.6, 11 5.0 / 4.6        n 900   8 4.4 / 4.4, 11 5.6 / 5.1, 18 8.4 / 7.8
+//   n 1241  2 4.1 / 3.7, 135 61.9 / 40.3      n 250   200 14.7 / 18.3, 800 52.6 / 62.2    n 506   64 10.9 / 12.4, 300 45.2 / 47.1
+// The last two are of the rows that fill the other kernel's slots and have just left one of this one's. All with one mask for all rows. With a
+// mask for so many rows as the CTA takes at two times the groups are still ahead ([20000, 1017] 50.6 / 41.3), with one for half as many no longer
+// (50.6 / 53.3), with one for every row they are far behind (49.0 / 73.0, [60000, 249] 29.6 / 36.7).
+static int softmax_span_rows_per_sm(int n, int nv) {
+  if (nv > 128) return 2;
+  if (nv * 8 > (n <= 128 ? 128 : (n + 255) / 256 * 256)) return 0;
+  return n <= 57 ? 48 : n <= 72 ? 200 : n <= 121 ? 88 : n <= 185 ? 64 : n <= 249 ? 300 : n <= 377 ? 25 : n <= 409 ? 50 : n <= 505 ? 5 : 11;
+}
+
+// How many rows that follow one another share their mask.
+static long long softmax_rows_per_mask(const SoftmaxParams& p) {
+  if (!p.mask) return p.rows;
+  const RowMap& m = p.mmap;
+  long long r = 1;
+  if (m.d2.d > 1) {
+    if (m.s2 != 0) return r;
+    r *= m.d2.d;
+  }
+  if (m.d1.d > 1) {
+    if (m.s1 != 0) return r;
+    r *= m.d1.d;
+  }
+  return m.s0 != 0 ? r : p.rows;
+}
+
+// Whether the two kernels above take the rows: x and y have the same alignment in every row, and there are enough of them.
 // Up to 1017 elements (four vectors a lane) groups, above that CTAs.
 template <typename T>
 static bool try_launch_softmax_span(const SoftmaxParams& p, cudaStream_t st) {
@@ -675,7 +706,9 @@ static bool try_launch_softmax_span(const SoftmaxParams& p, cudaStream_t st) {
   if (!flat(p.xmap) || !flat(p.ymap) || (reinterpret_cast<uintptr_t>(p.x) & 15u) != (reinterpret_cast<uintptr_t>(p.y) & 15u) ||
       (p.xmap.s0 - p.ymap.s0) % V != 0 || p.rows > 0x7fff0000LL)
     return false;
-  if (p.rows < (p.n <= 256 ? 48 : p.n <= 384 ? 14 : nv <= 128 ? 5 : 2) * sms) return false;
+  if (nv <= 128 && softmax_rows_per_mask(p) < (nv <= 24 ? 64 : nv <= 48 ? 32 : 16)) return false;  // 2 * 256 / lanes of a group
+  const int rows_per_sm = softmax_span_rows_per_sm(p.n, nv);
+  if (rows_per_sm == 0 || p.rows < rows_per_sm * sms) return false;
   if (nv > 2048) return false;
   set_path_tag(nv > 128 ? "off-grid rows as vectors, CTA per row" : "off-grid rows as vectors, several rows in turn");
   if (nv > 128) {

@@ -15,8 +15,10 @@ def _run(rows, n, dtype, mask, scale, start, log, batches=4):
     ys = torch.full((size + 64,), 7.0, device="cuda", dtype=dtype)
     x, y = (t[start:start + size].view(batches, rows // batches, n) for t in (xs, ys))
     k.softmax(x, mask=mask, scale=scale, log=log, out=y)
-    on_grid = start % 8 == 0 and n % 8 == 0
-    assert (b"off-grid rows as vectors" in k.load().b200_last_kernel()) == ((mask is not None or n < 256) and not on_grid)
+    shared = mask is None and n < 256 or mask is not None and mask.shape[1] == 1
+    fills = n <= 1017 and (n + 14) // 8 * 8 > (128 if n <= 128 else (n + 255) // 256 * 256)   # the other kernel's slots, and one more of this one's
+    by_vectors = (n > 1017 and mask is not None or shared) and not fills and not (start % 8 == 0 and n % 8 == 0)
+    assert (b"off-grid rows as vectors" in k.load().b200_last_kernel()) == by_vectors
     assert bool((ys[:start] == 7).all()) and bool((ys[start + size:] == 7).all()), "nothing beside the rows is written"
     t = x.double() * (1.0 if scale is None else scale)
     if mask is not None:
@@ -29,7 +31,8 @@ def _run(rows, n, dtype, mask, scale, start, log, batches=4):
 def test_spans(dtype, n):
     """Both sides of every change of geometry; every alignment of the first row; masks per batch, per row and none."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    rows = ((48 if n <= 256 else 14 if n <= 384 else 5 if n <= 1017 else 2) * sms + 15) // 4 * 4
+    per_sm = next(r for most, r in ((57, 48), (72, 200), (121, 88), (185, 64), (249, 300), (377, 25), (409, 50), (505, 5), (1017, 11), (8191, 2)) if n <= most)
+    rows = (per_sm * sms + 15) // 4 * 4
     ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     g = torch.Generator(device="cuda").manual_seed(n)
     key = torch.where(torch.rand(4, 1, n, generator=g, device="cuda") < 0.7, 0.0, -10000.0).to(dtype)
@@ -79,3 +82,32 @@ def test_probabilities_below_the_normal_range(n):
     # bf16's rounding: half a step of eight significant bits, at most 2^-8 of the value, below the normal range half of 2^-133; in front of it
     # those of fp32's exponential and of its product with the sum's inverse, 2^-21 of the value and steps of 2^-149 there
     assert bool(((got - want).abs() <= (2.0 ** -8 + 2.0 ** -21) * want + 2.0 ** -134 + 2.0 ** -147).all())
+
+
+@pytest.mark.parametrize("n,group", [(41, 8), (100, 8), (333, 16), (716, 32)])
+def test_masks_that_few_rows_share(n, group):
+    """A group of lanes keeps its part of the mask, so masks for fewer rows than two turns of a CTA go by the element; so do rows that just fill
+    that kernel's slots. The results are the same."""
+    from better_benchmark_b200 import kernels as k
+    rows = 208 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(n)
+    least = 2 * 256 // group
+    x = torch.randn(rows, n, generator=g, device="cuda").half()
+    masks = torch.randn(rows, n, generator=g, device="cuda").half()
+    for share in (1, least // 2, least, 4 * least):
+        for outer in (1, 2):
+            batched = x[:rows // (outer * share) * outer * share].view(outer, -1, share, n)
+            mask = masks[:batched.shape[0] * batched.shape[1]].view(outer, -1, 1, n)
+            got = k.softmax(batched, mask=mask, scale=0.5)
+            assert (b"off-grid rows as vectors" in k.load().b200_last_kernel()) == (share >= least), share
+            want = torch.softmax(batched.double() * 0.5 + mask.double(), -1)
+            assert bool(((got.double() - want).abs() <= (2.0 ** -11 + 2e-6) * want + 6.2e-8).all())
+    every = masks[:1].expand(rows, n)
+    k.softmax(x, mask=every)
+    assert b"off-grid rows as vectors" in k.load().b200_last_kernel(), "one mask for all rows"
+    for full in (125, 251, 509, 765):
+        x = torch.randn(rows, full, generator=g, device="cuda").half()
+        got = k.softmax(x, mask=x[0])
+        assert b"[elements in registers]" in k.load().b200_last_kernel()
+        want = torch.softmax(x.double() + x[0].double(), -1)
+        assert bool(((got.double() - want).abs() <= (2.0 ** -11 + 2e-6) * want + 6.2e-8).all())
