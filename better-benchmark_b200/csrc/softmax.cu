@@ -1169,13 +1169,15 @@ static bool try_launch_softmax_rows(const SoftmaxParams& p, bool aligned, cudaSt
 // element by element) and 16-byte stores when the output row does. No mask; the optional scale is
 // applied in fp32.
 // ----------------------------------------------------------------------------------------------
+// d: differences from a maximum. -inf, and for the pair exponential all that is below its range, has the exponential 0; NaN may be lost.
 template <typename Tout>
 __device__ __forceinline__ f32x2 long_row_exp(f32x2 d) {
+  float a, b;
+  unpack2(d, a, b);
   if constexpr (sizeof(Tout) == 2) {
-    return exp_pair_compensated(d);
+    constexpr float kFloor = -1e30f;
+    return exp_pair_compensated(pack2(fmaxf(a, kFloor), fmaxf(b, kFloor)));
   } else {
-    float a, b;
-    unpack2(d, a, b);
     return pack2(expf(a), expf(b));
   }
 }
@@ -1186,7 +1188,6 @@ __global__ void __launch_bounds__(1024) softmax_long_kernel(const SoftmaxParams 
   constexpr int V = Elem<Tin>::V;
   constexpr int P = V / 2;
   constexpr int U = 4;  // vectors in flight per thread
-  constexpr float kFloor = -1e30f;  // finite stand-in for -inf inside the compensated exponential
   __shared__ float red[64];
   const long long row = blockIdx.x;
   const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
@@ -1200,6 +1201,7 @@ __global__ void __launch_bounds__(1024) softmax_long_kernel(const SoftmaxParams 
 
   // ---- sweep 1 ----------------------------------------------------------------------------------
   float m = -INFINITY, s = 0.f;
+  auto over_m = [&] { return m == -INFINITY ? 0.f : m; };  // nothing but -inf so far: their differences from any number are -inf
   auto absorb = [&](const f32x2 (&t)[P]) {  // one vector of logits into (m, s)
     float vm = -INFINITY;
 #pragma unroll
@@ -1209,19 +1211,13 @@ __global__ void __launch_bounds__(1024) softmax_long_kernel(const SoftmaxParams 
       vm = fmaxf(vm, fmaxf(a, b));
     }
     if (vm > m) {
-      s = s * expf(fmaxf(m, kFloor) - vm);  // m = -inf the first time: the sum is still zero
+      s = s * expf(m - vm);  // m = -inf the first time: the sum is still zero
       m = vm;
     }
-    const f32x2 m2 = splat2(fmaxf(m, kFloor));
+    const f32x2 m2 = splat2(over_m());
     f32x2 acc = splat2(0.f);
 #pragma unroll
-    for (int i = 0; i < P; ++i) {
-      float a, b;
-      unpack2(t[i], a, b);
-      a = fmaxf(a, kFloor);  // NaN would be lost here, so NaN rows are caught through the maximum below
-      b = fmaxf(b, kFloor);
-      acc = add2(acc, long_row_exp<Tout>(sub2(pack2(a, b), m2)));
-    }
+    for (int i = 0; i < P; ++i) acc = add2(acc, long_row_exp<Tout>(sub2(t[i], m2)));
     s += hsum2(acc);
   };
   bool saw_nan = false;
@@ -1257,31 +1253,30 @@ __global__ void __launch_bounds__(1024) softmax_long_kernel(const SoftmaxParams 
     if (scaled) t = t * p.scale;
     saw_nan |= t != t;
     if (t > m) {
-      s = s * expf(fmaxf(m, kFloor) - t);
+      s = s * expf(m - t);
       m = t;
     }
-    s += expf(fmaxf(t, kFloor) - fmaxf(m, kFloor));
+    s += expf(t - over_m());
   }
   // CTA-wide (M, S)
   const float M = block_reduce<FastMax>(m, red);
-  const float contrib = (m == -INFINITY) ? 0.f : s * expf(m - fmaxf(M, kFloor));
+  const float contrib = (m == -INFINITY) ? 0.f : s * expf(m - M);
   float S = block_reduce<SumOp>(contrib, red);
   const float nan_any = block_reduce<FastMax>(saw_nan ? 1.f : 0.f, red);
-  if (M == -INFINITY || nan_any > 0.f) S = NAN;  // aten: x - max is NaN for a row of -inf; NaN logits poison the row
+  if (!(fabsf(M) < INFINITY) || nan_any > 0.f) S = NAN;  // aten: x - max is NaN for a row of -inf and for inf; NaN logits poison the row
 
   // ---- sweep 2 ----------------------------------------------------------------------------------
   const float logS = logf(S);
   const float inv = __frcp_rn(S);
-  const float Mf = fmaxf(M, kFloor);
   const bool log_mode = p.log_mode != 0;
   auto finish = [&](float t) -> float {  // one logit -> one output value
     if (log_mode) return (t - M) - logS;
-    const float e = expf(fmaxf(t, kFloor) - Mf);
+    const float e = expf(t - M);
     return sizeof(Tout) == 4 ? e / S : e * inv;
   };
   constexpr int VO = 16 / (int)sizeof(Tout);           // output elements per 16-byte store
   const bool y_vec = x_vec && (reinterpret_cast<uintptr_t>(y) & 15u) == 0 && V % VO == 0;
-  const f32x2 M2 = splat2(Mf), inv2 = splat2(inv), logS2 = splat2(logS), Mraw2 = splat2(M);
+  const f32x2 M2 = splat2(M), inv2 = splat2(inv), logS2 = splat2(logS);
   if (!y_vec) {
     // The output row does not start on a 16-byte boundary where the input row does (a ragged row
     // length, another element size): vectors are formed on the OUTPUT side - up to the first
@@ -1331,11 +1326,9 @@ __global__ void __launch_bounds__(1024) softmax_long_kernel(const SoftmaxParams 
         for (int i = 0; i < P; ++i) {
           if (scaled) t[i] = mul2(t[i], scale2);
           if (log_mode) {
-            o[i] = sub2(sub2(t[i], Mraw2), logS2);
+            o[i] = sub2(sub2(t[i], M2), logS2);
           } else {
-            float a, b;
-            unpack2(t[i], a, b);
-            const f32x2 e = long_row_exp<Tout>(sub2(pack2(fmaxf(a, kFloor), fmaxf(b, kFloor)), M2));
+            const f32x2 e = long_row_exp<Tout>(sub2(t[i], M2));
             if constexpr (sizeof(Tout) == 4) {
               float ea, eb;
               unpack2(e, ea, eb);

@@ -20,8 +20,10 @@ def test_many_long_rows(n, dtype, out_dtype, path, log):
     x = (torch.randn(rows, n, device="cuda") * 3).to(dtype)
     x[3, : n // 2] = float("-inf")
     x[4, 5], x[5, n - 1], x[6] = float("nan"), float("inf"), float("-inf")
-    if dtype != torch.float16 and path != b"two sweeps":
+    if dtype != torch.float16:
         x[7], x[7, 9] = -3e38, 3e38    # differences beyond what fp32 holds
+        x[8], x[8, 9], x[8, 11] = -3e38, -2e38, float("-inf")   # and rows far below what -inf might be replaced by
+        x[9], x[9, n - 1] = float("-inf"), -3e38
     got = k.softmax(x, log=log, out_dtype=out_dtype)
     assert path in k.load().b200_last_kernel(), k.load().b200_last_kernel()
     want = torch.log_softmax(x.double(), -1) if log else torch.softmax(x.double(), -1)
