@@ -729,7 +729,15 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
 __global__ void __launch_bounds__(256) norm_bwd_finalize_units_kernel(const NormBwdParams p) {
   wait_for_previous_kernel();
   __shared__ double fin[8 * 64];
-  if (p.bar[1] != 0u) return;  // a worker gave up: the host is told (b200_check_status)
+  if (p.words_hold && p.bar[1] != 0u) {  // a worker gave up: the host is told (b200_check_status), and the sums are no numbers
+    if (blockIdx.x == 0) {
+      for (int c = threadIdx.x; c < p.n; c += blockDim.x) {
+        if (p.dw) p.dw[c] = NAN;
+        if (p.db) p.db[c] = NAN;
+      }
+    }
+    return;
+  }
   finalize_units(p.partials, p.groups, p.n, p.dw, p.db, p.width, blockIdx.x, gridDim.x, fin);
 }
 
@@ -1283,6 +1291,7 @@ extern "C" int b200_norm_bwd(const void* x, const void* dy, const void* weight, 
   p.partials = scratch ? reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + 256) : nullptr;
   p.groups = p.workers = 0; p.finalizers = 0; p.width = 0;
   const bool fused = (flags & 1) == 0 && (dweight || dbias);
+  p.words_hold = fused ? 1 : 0;
 
   const int eb = dtype_size(x_dtype), wb = dtype_size(w_dtype);
   const int v = 16 / eb;

@@ -31,6 +31,7 @@ struct NormBwdParams {
   unsigned int* bar;  // words that are zero between launches: [0] workers done, [1] error, [2] CTAs gone, [3] tickets
   int groups;
   int workers;  // CTAs that walk the rows
+  int words_hold;  // the scratch has the zeroed words (all but the two-launch form, which reads none of them)
   // The finalize in the same launch (0: none, or a launch of its own): this many CTAs beside the workers, a unit of
   // `width` columns at a time.
   int finalizers;

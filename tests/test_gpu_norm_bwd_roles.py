@@ -59,3 +59,32 @@ def test_two_streams_at_once():
     for outs in got:
         for which, out in outs:
             assert all(torch.equal(a, b) for a, b in zip(out, want[which]))
+
+
+@pytest.mark.parametrize("rows,n,dtype", [(1100, 4096, torch.bfloat16), (1100, 2056, torch.float32), (1030, 16384, torch.bfloat16), (300, 768, torch.bfloat16),
+                                          (300, 64, torch.bfloat16), (300, 2048, torch.float32)])
+def test_two_launches_need_no_zeroed_words(rows, n, dtype):
+    """The two-launch form neither reads nor writes the words in front of the scratch."""
+    from better_benchmark_b200 import kernels as k
+    x, dy, w, mean, rstd = _inputs(rows, n, dtype, rows)
+    want = k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True, two_launch=True)
+    scratch = torch.full((256 + 600 * 2 * n * 4,), 0xa5, dtype=torch.uint8, device="cuda")
+    got = k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True, two_launch=True, scratch=scratch)
+    for a, b in zip(got, want):
+        assert not bool(torch.isnan(a).any()) and torch.allclose(a.float(), b.float(), rtol=1e-5, atol=1e-3)
+    assert bool((scratch[:256] == 0xa5).all())
+
+
+@pytest.mark.parametrize("rows,n,dtype", [(1100, 4096, torch.bfloat16), (1100, 2056, torch.float32), (1030, 16384, torch.bfloat16)])
+def test_a_noted_error_shows_in_the_sums(rows, n, dtype):
+    """With an error still noted in the words no sums are formed: they are NaN, not what the memory held, and the status says why."""
+    from better_benchmark_b200 import kernels as k
+    from better_benchmark_b200 import native
+    x, dy, w, mean, rstd = _inputs(rows, n, dtype, rows)
+    scratch = torch.zeros(256 + 600 * 2 * n * 4, dtype=torch.uint8, device="cuda")
+    scratch[:16].view(torch.int32)[1] = 1
+    want = k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True)
+    got = k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True, scratch=scratch)
+    assert torch.equal(got[0], want[0]) and bool(torch.isnan(got[1]).all()) and bool(torch.isnan(got[2]).all())
+    assert native.load().b200_check_status(scratch.data_ptr(), torch.cuda.current_stream().cuda_stream) != 0
+    assert int(scratch[:256].count_nonzero()) == 1
