@@ -75,7 +75,7 @@ def test_two_launches_need_no_zeroed_words(rows, n, dtype):
     assert bool((scratch[:256] == 0xa5).all())
 
 
-@pytest.mark.parametrize("rows,n,dtype", [(1100, 4096, torch.bfloat16), (1100, 2056, torch.float32), (1030, 16384, torch.bfloat16)])
+@pytest.mark.parametrize("rows,n,dtype", [(1100, 4096, torch.bfloat16), (1100, 2056, torch.float32)])
 def test_a_noted_error_shows_in_the_sums(rows, n, dtype):
     """With an error still noted in the words no sums are formed: they are NaN, not what the memory held, and the status says why."""
     from better_benchmark_b200 import kernels as k
