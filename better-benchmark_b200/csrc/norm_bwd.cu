@@ -16,9 +16,9 @@
 // Structure: a persistent grid; each group of threads (a CTA for long rows, a warp for short
 // ones) walks rows group, group+G, ..., keeps the next row's loads in flight while it reduces the
 // current one, and accumulates its columns of dw/db in registers over all its rows. Each group
-// then writes one fp32 partial row to scratch; CTAs of the same launch that start after these
-// sum the partial rows in fp64, in a fixed order, into dw/db (the two roles of norm_bwd.cuh). No atomics on results:
-// they are bit-reproducible. A two-launch variant (main + finalize) does the same.
+// then writes one fp32 partial row to scratch; when all are written, the CTAs of the same launch sum them in fp64, in a
+// fixed order, into dw/db (bwd_combine), or a launch chained to it does (row tiles, streaming, rows off the 16-byte grid, and the
+// two-launch variant of the others). No atomics on results: they are bit-reproducible.
 #include "norm_bwd.cuh"
 
 #include <cstdlib>
@@ -33,18 +33,13 @@ norm_bwd_kernel(const NormBwdParams p) {
   constexpr int V = Elem<T>::V;
   __shared__ float2 red[2][16];
   __shared__ double fin[16 * 64];
-  __shared__ int bar_ok, ticket;
+  __shared__ int combine_flag[2];
   const int lane = group_lane<BLOCK>();
   const int G = group_size<BLOCK>();
   const int nv = p.n / V;
-  bwd_draw_ticket(p, &ticket);
-  __syncthreads();
-  const int cta = bwd_cta(&ticket);
-  if (cta >= p.workers) {
-    bwd_finalize(p, cta, LN ? p.db : nullptr, fin, &bar_ok);
-    return;
-  }
-  const long long group = BLOCK ? (long long)cta : (long long)cta * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  bwd_started(p);
+  const bool worker = (int)blockIdx.x < p.workers;  // CTAs behind the workers have no rows; they help to add up the columns
+  const long long group = BLOCK ? (long long)blockIdx.x : (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long group_stride = BLOCK ? (long long)p.workers : (long long)p.workers * (blockDim.x >> 5);
 
   float acc_w[CH][V], acc_b[LN ? CH : 1][V];
@@ -62,7 +57,7 @@ norm_bwd_kernel(const NormBwdParams p) {
   }
 
   uint4 nx[CH], ny[CH];  // next row, in flight
-  long long row = group;
+  long long row = worker ? group : p.rows;
   if (row < p.rows) {
     const T* xr = reinterpret_cast<const T*>(p.x) + row * p.x_row_stride;
     const T* yr = reinterpret_cast<const T*>(p.dy) + row * p.dy_row_stride;
@@ -182,7 +177,7 @@ norm_bwd_kernel(const NormBwdParams p) {
   }
 
   // one partial row per group
-  if (p.dw || p.db) {
+  if (worker && (p.dw || p.db)) {
     float* pw = p.partials + group * p.n;
     float* pb = p.partials + ((long long)p.groups + group) * p.n;
 #pragma unroll
@@ -204,7 +199,7 @@ norm_bwd_kernel(const NormBwdParams p) {
       }
     }
   }
-  bwd_worker_done(p);
+  bwd_combine(p, LN ? p.db : nullptr, fin, combine_flag);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -337,7 +332,7 @@ norm_bwd_stream_kernel(const NormBwdParams p, const int stages) {
       failed = true;
       if (tid == 0) {
         note_wait_timeout();
-        if (p.bar) atomicExch(&p.bar[1], 1u);  // nobody is to wait for this CTA
+        if (p.bar) atomicExch(&p.bar[kBwdError], 1u);  // nobody is to wait for this CTA
         int ds = st;
         uint32_t dp = phase;
         for (int d = k; d < my_rows && d < k + stages; ++d) {
@@ -598,7 +593,7 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
       failed = true;
       if (threadIdx.x == 0) {
         note_wait_timeout();
-        if (p.bar) atomicExch(&p.bar[1], 1u);  // nobody is to wait for this CTA
+        if (p.bar) atomicExch(&p.bar[kBwdError], 1u);  // nobody is to wait for this CTA
         int ds = st;
         uint32_t dp = phase;
         for (int d = k; d < my_tiles && d < (k > 0 ? k - 1 : 0) + stages; ++d) {
@@ -725,17 +720,12 @@ norm_bwd_tile_kernel(const NormBwdParams p, const int stages, const int TG, cons
   }
 }
 
-// The finalize of the streaming and row-tile kernels, whose registers leave no room for the tickets: a unit of columns per CTA.
+// The finalize of the streaming and row-tile kernels, whose registers leave no room for it: a unit of columns per CTA.
 __global__ void __launch_bounds__(256) norm_bwd_finalize_units_kernel(const NormBwdParams p) {
   wait_for_previous_kernel();
   __shared__ double fin[8 * 64];
-  if (p.words_hold && p.bar[1] != 0u) {  // a worker gave up: the host is told (b200_check_status), and the sums are no numbers
-    if (blockIdx.x == 0) {
-      for (int c = threadIdx.x; c < p.n; c += blockDim.x) {
-        if (p.dw) p.dw[c] = NAN;
-        if (p.db) p.db[c] = NAN;
-      }
-    }
+  if (p.words_hold && p.bar[kBwdError] != 0u) {  // a worker gave up: the host is told (b200_check_status), and the sums are no numbers
+    bwd_no_sums(p.dw, p.db, p.n, p.width, blockIdx.x, gridDim.x);
     return;
   }
   finalize_units(p.partials, p.groups, p.n, p.dw, p.db, p.width, blockIdx.x, gridDim.x, fin);
@@ -1080,8 +1070,8 @@ static int launch_norm_bwd_fast(NormBwdParams p, int threads, size_t scratch_byt
   p.groups = (int)(grid * groups_per_cta);
   p.workers = (int)grid;
   if (fused) {
-    bwd_plan_finalize(p, (long long)per_sm * sms);
-    launch_dependent(kernel, (unsigned)(grid + p.finalizers), threads, 0, st, p);
+    const unsigned ctas = bwd_plan_combined(p, (long long)per_sm * sms);
+    launch_dependent(kernel, ctas, threads, 0, st, p);
     return launch_status(BLOCK ? "b200_norm_bwd [registers, CTA per row, fused finalize]" : "b200_norm_bwd [registers, warp per row, fused finalize]");
   }
   launch_dependent(kernel, (unsigned)grid, threads, 0, st, p);

@@ -28,76 +28,31 @@ struct NormBwdParams {
   long long dx_batch_stride, dx_seq_stride, dx_head_stride;
   float n_f;
   float* partials;    // [groups][n] for dw, followed by [groups][n] for db
-  unsigned int* bar;  // words that are zero between launches: [0] workers done, [1] error, [2] CTAs gone, [3] tickets
+  unsigned int* bar;  // words that are zero between launches (BwdWords)
   int groups;
-  int workers;  // CTAs that walk the rows
+  int workers;  // CTAs that walk the rows: the first of the grid
   int words_hold;  // the scratch has the zeroed words (all but the two-launch form, which reads none of them)
-  // The finalize in the same launch (0: none, or a launch of its own): this many CTAs beside the workers, a unit of
-  // `width` columns at a time.
+  // The partial rows are added up in the same launch, by all its CTAs (norm_bwd_narrow.cu: by so many beside the workers), a unit of
+  // `width` columns at a time. 0: not at all, or by a launch of its own.
   int finalizers;
   int width;
 };
 
-// ----------------------------------------------------------------------------------------------
-// One launch, two roles. The first `workers` CTAs that START are workers: they walk the rows, and the partial row that each
-// leaves has the number of its ticket. The CTAs that start after them add the partial rows up once all workers have arrived.
-// A worker waits for nobody, and a CTA that waits has started after every worker has: whatever else occupies the GPU,
-// the wait ends, so that the launch need not be cooperative. (Cooperative launches with a grid barrier took
-// 2 to 3 us more back to back, 10.4 us for a few hundred rows whose kernel runs 7.7, and the CTAs that had finished
-// early did nothing.) Tickets decide who owns which rows, so the result does not depend on which CTA draws which.
-// ----------------------------------------------------------------------------------------------
-// A CTA's number, among the workers or, from p.workers on, the finalizers: thread 0 draws it, the others know it after the CTA's next
-// barrier. The shuffle tells the compiler that it is the same in a warp, so that what depends on it can live in uniform registers, as
-// what depends on blockIdx does. (All the same the kernels of 64 registers spilled: RMSNorm backward bf16 [4, 4096, 32, 128] 70 ->
-// 78 us. Those have a finalize of their own, chained to them.)
-__device__ __forceinline__ void bwd_draw_ticket(const NormBwdParams& p, int* ticket) {
-  if (threadIdx.x == 0) *ticket = p.finalizers > 0 ? (int)atomicAdd(&p.bar[3], 1u) : (int)blockIdx.x;
-}
-__device__ __forceinline__ int bwd_cta(const int* ticket) { return __shfl_sync(0xffffffffu, *ticket, 0); }
+// Words in front of the scratch, zero between launches. The two that CTAs ask for while others work lie in another sector than the rest.
+enum BwdWords { kBwdArrived = 0, kBwdError = 1, kBwdLeft = 32, kBwdStarted = 48 };
 
-// The last CTA puts the words back to zero (the error flag stays until the host has seen it).
-__device__ __forceinline__ void bwd_depart(const NormBwdParams& p) {
-  if (threadIdx.x == 0 && atomicAdd(&p.bar[2], 1u) == gridDim.x - 1) {
-    atomicExch(&p.bar[0], 0u);
-    atomicExch(&p.bar[2], 0u);
-    atomicExch(&p.bar[3], 0u);
-    __threadfence();
-  }
+__device__ __forceinline__ unsigned int bwd_peek(const unsigned int* word) {
+  unsigned int v;
+  asm volatile("ld.global.relaxed.gpu.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+  return v;
 }
-
-// A worker's partial row is written: every thread of the CTA calls this.
-__device__ __forceinline__ void bwd_worker_done(const NormBwdParams& p) {
-  if (p.finalizers == 0) return;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&p.bar[0], 1u);
-  }
-  bwd_depart(p);
-}
-
-// Waits until all workers have arrived; false when one has given up or the bound ran out (some seconds: with a scratch for few
-// partial rows there are few workers, which may take long).
-__device__ __forceinline__ bool bwd_wait_for_workers(const NormBwdParams& p, int* flag) {
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    for (unsigned int spins = 0;; ++spins) {
-      unsigned int seen, err;
-      asm volatile("ld.global.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(p.bar) : "memory");
-      asm volatile("ld.global.relaxed.gpu.u32 %0, [%1];" : "=r"(err) : "l"(p.bar + 1) : "memory");
-      if (err == 0u && seen >= (unsigned int)p.workers) break;
-      if (err != 0u || spins > (1u << 24)) {
-        atomicExch(&p.bar[1], 1u);
-        ok = 0;
-        break;
-      }
-      __nanosleep(spins > 4096 ? 256 : 32);  // the workers' copies have the memory system
-    }
-    __threadfence();
-    *flag = ok;
-  }
-  __syncthreads();
-  return *flag != 0;
+// Workers that have arrived, and with the same trip to memory whether an error is noted.
+__device__ __forceinline__ unsigned int bwd_arrived(const NormBwdParams& p, bool& error) {
+  static_assert(kBwdArrived == 0 && kBwdError == 1, "one aligned pair of words");
+  unsigned long long v;
+  asm volatile("ld.global.acquire.gpu.u64 %0, [%1];" : "=l"(v) : "l"(p.bar) : "memory");
+  error = (v >> 32) != 0;
+  return (unsigned int)v;
 }
 
 template <int V>
@@ -146,9 +101,8 @@ __device__ __forceinline__ void finalize_columns(const float* partials, int grou
   }
 }
 
-// The same by the finalizers of the launch, for rows of n % 4 == 0 columns: the
-// columns of dw and db are dealt out in units of 8 (a 32-byte sector of a partial row), a finalizer each
-// (192 CTAs for 768 columns of both). Where that makes more units than CTAs that fit, units of 16, 32 or 64
+// The same for rows of n % 4 == 0 columns: the columns of dw and db are dealt out in units of 8 (a 32-byte sector of a partial
+// row), a CTA each (192 CTAs for 768 columns of both). Where that makes more units than CTAs that fit, units of 16, 32 or 64
 // columns: a unit is two barriers and a load latency, whatever its width (LayerNorm f32 [256, 8192]: 27.9 us with
 // 2048 units of 8, 17.2 us with two times 128 of 64).
 // width / 4 threads share a partial row's unit, the CTA's threads split the partial rows. fp64, fixed order.
@@ -206,20 +160,109 @@ __device__ __forceinline__ void finalize_units(const float* partials, int groups
   }
 }
 
-// What a CTA with a ticket beyond the workers' does: waits, adds up, leaves.
-__device__ __forceinline__ void bwd_finalize(const NormBwdParams& p, int cta, float* db, double* smem, int* flag) {
-  if (bwd_wait_for_workers(p, flag))
-    finalize_units(p.partials, p.groups, p.n, p.dw, db, p.width, cta - p.workers, p.finalizers, smem);
-  bwd_depart(p);
+// ----------------------------------------------------------------------------------------------
+// Rows and column sums in one launch that need not be cooperative. Every CTA, when its partial row is written, waits until all workers
+// have arrived, and then adds its share of the columns up. The grid is no larger than what fits the GPU, so all of it is normally
+// there; but nothing guarantees it (another stream's kernel may hold SMs), so a CTA that has seen all workers start waits for them,
+// and one that has not leaves after a while, to make room; the CTA that leaves last then adds up all columns, whoever left early.
+// Each wait ends: those it is for have started, and wait themselves for nothing but what has started.
+// (A cooperative launch takes 2.5 us more when calls follow one another. With roles drawn as tickets, the first CTAs that start as
+// workers and those behind them as finalizers, the draw came in front of the first copies and the finalizers' start behind
+// the workers' end: in a graph LayerNorm bf16 [1000, 1024] 11.3 us, cooperative 9.2, so 9.2; [40000, 768] 39.8, 39.3 and 39.5; [40000, 1024] 49.3, 47.1 and 48.6.)
+// ----------------------------------------------------------------------------------------------
+// Asked of every CTA before its first row.
+__device__ __forceinline__ void bwd_started(const NormBwdParams& p) {
+  if (p.finalizers != 0 && threadIdx.x == 0 && (int)blockIdx.x < p.workers)
+    asm volatile("red.global.relaxed.gpu.add.u32 [%0], 1;" ::"l"(p.bar + kBwdStarted) : "memory");
 }
 
-// Host: how many finalizers a launch of rows of n columns gets, and the width of their units. `room`: CTAs of the kernel that fit.
-inline void bwd_plan_finalize(NormBwdParams& p, long long room) {
+// A call, so that the widths that a few calls need stay out of the registers and the code of the kernels (with the width of 8 called
+// too: LayerNorm bf16 [8000, 768] 15.0 -> 15.4 us).
+static __device__ __noinline__ void finalize_any_units(const float* partials, int groups, int n, float* dw, float* db, int width, int first,
+                                                       int step, double* smem) {
+  finalize_units(partials, groups, n, dw, db, width, first, step, smem);
+}
+
+// Sums that cannot be formed are no numbers: the units first, first + step, ... of finalize_units.
+__device__ __forceinline__ void bwd_no_sums(float* dw, float* db, int n, int width, int first, int step) {
+  const int units = (n + width - 1) / width, total = units * ((dw ? 1 : 0) + (db ? 1 : 0));
+  for (int s = first; s < total; s += step) {
+    const bool is_db = !dw || s >= units;
+    const int col = (dw && s >= units ? s - units : s) * width;
+    for (int k = threadIdx.x; k < width && col + k < n; k += blockDim.x) (is_db ? db : dw)[col + k] = NAN;
+  }
+}
+
+// Every thread of every CTA calls this when the CTA's partial row, if it has one, is written. flag: two words of shared memory.
+__device__ __forceinline__ void bwd_combine(const NormBwdParams& p, float* db, double* smem /* [warps][64] */, int* flag) {
+  if (p.finalizers == 0) return;
+  enum { kAddUp, kLeave, kFailed };
+  constexpr unsigned int kPatience = 64;  // polls, some 40 us
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned int workers = (unsigned int)p.workers;
+    if (blockIdx.x < workers) {
+      __threadfence();
+      atomicAdd(&p.bar[kBwdArrived], 1u);
+    }
+    int state = kAddUp;
+    bool all_started = false, error = false;
+    for (unsigned int polls = 0; bwd_arrived(p, error) < workers; ++polls) {
+      if (polls >= kPatience && !all_started) {
+        all_started = bwd_peek(p.bar + kBwdStarted) >= workers;
+        if (!all_started) {
+          state = kLeave;
+          break;
+        }
+      }
+      if (polls > (1u << 24)) {  // some seconds: with a scratch for few partial rows there are few workers, which may take long
+        atomicExch(&p.bar[kBwdError], 1u);
+        error = true;
+        break;
+      }
+      if (polls > 4096) __nanosleep(64);
+    }
+    if (state == kAddUp && error) state = kFailed;
+    __threadfence();
+    flag[0] = state;
+  }
+  __syncthreads();
+  const int state = flag[0];
+  if (state == kAddUp && p.width == 8) finalize_units(p.partials, p.groups, p.n, p.dw, db, 8, (int)blockIdx.x, (int)gridDim.x, smem);
+  else if (state == kAddUp) finalize_any_units(p.partials, p.groups, p.n, p.dw, db, p.width, (int)blockIdx.x, (int)gridDim.x, smem);
+  else if (state == kFailed) bwd_no_sums(p.dw, db, p.n, p.width, (int)blockIdx.x, (int)gridDim.x);
+  if (threadIdx.x == 0) {
+    const unsigned int before = atomicAdd(&p.bar[kBwdLeft], state == kLeave ? 0x10001u : 1u);
+    int missing = 0;
+    if ((before & 0xffffu) == gridDim.x - 1) {  // the last one: no other CTA looks at the words any more
+      missing = (before >> 16) != 0u || state == kLeave;
+      if (missing && bwd_peek(p.bar + kBwdError) != 0u) missing = 2;
+      atomicExch(&p.bar[kBwdArrived], 0u);
+      atomicExch(&p.bar[kBwdStarted], 0u);
+      atomicExch(&p.bar[kBwdLeft], 0u);
+      __threadfence();
+    }
+    flag[1] = missing;
+  }
+  __syncthreads();
+  if (flag[1] == 1) finalize_any_units(p.partials, p.groups, p.n, p.dw, db, p.width, 0, 1, smem);
+  else if (flag[1] == 2) bwd_no_sums(p.dw, db, p.n, p.width, 0, 1);
+}
+
+// Host: the width of the units that rows of n columns are added up in, and how many there are, for `ctas` CTAs.
+inline void bwd_plan_finalize(NormBwdParams& p, long long ctas) {
   const int planes = (p.dw ? 1 : 0) + (p.db ? 1 : 0);
   p.width = 8;
-  while (p.width < 64 && (long long)(p.n + p.width - 1) / p.width * planes > room) p.width *= 2;
-  const long long units = (long long)(p.n + p.width - 1) / p.width * planes;
-  p.finalizers = (int)(units < room ? units : room);
+  while (p.width < 64 && (long long)(p.n + p.width - 1) / p.width * planes > ctas) p.width *= 2;
+  p.finalizers = (p.n + p.width - 1) / p.width * planes;
+}
+// Host: the same for a launch whose CTAs add up themselves, and its grid: the workers where they get by with a unit each, more CTAs, up
+// to what fits, where there are too few of them (LayerNorm f32 [64, 2048]: 6.9 us with 64 units for 64 workers, 7.4 with 256 for 256 CTAs).
+inline unsigned bwd_plan_combined(NormBwdParams& p, long long room) {
+  bwd_plan_finalize(p, p.workers);
+  if (p.finalizers <= p.workers) return (unsigned)p.workers;
+  bwd_plan_finalize(p, room);
+  return (unsigned)(p.finalizers < room ? (p.finalizers > p.workers ? p.finalizers : p.workers) : room);
 }
 
 // Warp reduction of N (2, 4 or 8) values per lane at once: in every step a lane keeps one half of

@@ -5,6 +5,63 @@ namespace b200 {
 
 constexpr int kNarrowThreads = 256;
 
+// ----------------------------------------------------------------------------------------------
+// One launch, two roles. The first `workers` CTAs that START are workers: they walk the rows, and the partial row that each
+// leaves has the number of its ticket. The `finalizers` that start after them add the partial rows up once all workers have arrived.
+// A worker waits for nobody, and a CTA that waits has started after every worker has: whatever else occupies the GPU, and however
+// many waves of CTAs the workers are, the wait ends. Tickets decide who owns which rows, so the result does not
+// depend on which CTA draws which.
+// ----------------------------------------------------------------------------------------------
+enum NarrowWords { kNarrowGone = 2, kNarrowTickets = 3 };  // beside kBwdArrived and kBwdError
+
+// A CTA's number, among the workers or, from p.workers on, the finalizers: thread 0 draws it, the others know it after the CTA's next
+// barrier. The shuffle tells the compiler that it is the same in a warp.
+__device__ __forceinline__ void narrow_draw_ticket(const NormBwdParams& p, int* ticket) {
+  if (threadIdx.x == 0) *ticket = p.finalizers > 0 ? (int)atomicAdd(&p.bar[kNarrowTickets], 1u) : (int)blockIdx.x;
+}
+__device__ __forceinline__ int narrow_cta(const int* ticket) { return __shfl_sync(0xffffffffu, *ticket, 0); }
+
+// The last CTA puts the words back to zero (the error flag stays until the host has seen it).
+__device__ __forceinline__ void narrow_depart(const NormBwdParams& p) {
+  if (threadIdx.x == 0 && atomicAdd(&p.bar[kNarrowGone], 1u) == gridDim.x - 1) {
+    atomicExch(&p.bar[kBwdArrived], 0u);
+    atomicExch(&p.bar[kNarrowGone], 0u);
+    atomicExch(&p.bar[kNarrowTickets], 0u);
+    __threadfence();
+  }
+}
+
+// A worker's partial row is written: every thread of the CTA calls this.
+__device__ __forceinline__ void narrow_worker_done(const NormBwdParams& p) {
+  if (p.finalizers == 0) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&p.bar[kBwdArrived], 1u);
+  }
+  narrow_depart(p);
+}
+
+// Waits until all workers have arrived; false when an error is noted or the bound ran out (some seconds: with a scratch for few
+// partial rows there are few workers, which may take long).
+__device__ __forceinline__ bool narrow_wait_for_workers(const NormBwdParams& p, int* flag) {
+  if (threadIdx.x == 0) {
+    bool error = false;
+    for (unsigned int polls = 0; bwd_arrived(p, error) < (unsigned int)p.workers; ++polls) {
+      if (polls > (1u << 24)) {
+        atomicExch(&p.bar[kBwdError], 1u);
+        error = true;
+        break;
+      }
+      __nanosleep(polls > 4096 ? 256 : 32);  // the workers' loads have the memory system
+    }
+    __threadfence();
+    *flag = error ? 0 : 1;
+  }
+  __syncthreads();
+  return *flag != 0;
+}
+
 // The finalize of this file's partial rows, which are fp64: the columns of dw and db in units of 8, a CTA each. n % 4 == 0.
 __device__ __forceinline__ void finalize_units_f64(const double* partials, int groups, int n, float* dw, float* db, int first, int step,
                                                    double* smem /* [warps][8] */) {
@@ -54,7 +111,7 @@ __device__ __forceinline__ void finalize_units_f64(const double* partials, int g
 
 // A group of G lanes takes a row, a vector a lane, two rows on their way at once; a lane's columns are the same in every row, so its weights
 // and sums stay in registers, and every few rows go to its own words of shared memory. At the end the CTA's groups are added up in
-// fp64 into one partial row, and the partial rows by the launch's finalizers (the two roles of norm_bwd.cuh).
+// fp64 into one partial row, and the partial rows by the launch's finalizers (the two roles above).
 // A warp per row, as before, left up to 28 of its lanes idle and one partial row per warp: the finalizers' reads of up to 9472 of them took
 // longer than the rows. LayerNorm bf16, us: [4000, 64] 13.8 -> 6.9, [24000, 64] 19.1 -> 9.3, [100000, 64] 46 -> 16.5, [100000, 128]
 // 46 -> 25, [4000, 256] 14.7 -> 11.1, [100000, 256] 49 -> 42; RMSNorm [24000, 128] 21 -> 10.5; f32 [24000, 64] 20.0 -> 9.7. A few hundred rows
@@ -66,7 +123,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 3) norm_bwd_narrow_kernel(cons
   __shared__ float fold[LN ? 2 : 1][kGroups][G * V];
   __shared__ double fin[8 * 8];
   __shared__ int bar_ok, ticket;
-  bwd_draw_ticket(p, &ticket);
+  narrow_draw_ticket(p, &ticket);
   const int lane = (int)threadIdx.x & (G - 1), group = (int)threadIdx.x / G, n = p.n;
   const bool live = lane * V < n;
   const int col = live ? lane * V : 0;
@@ -87,12 +144,14 @@ __global__ void __launch_bounds__(kNarrowThreads, 3) norm_bwd_narrow_kernel(cons
   }
   const long long dx_col = (long long)(col / p.head_dim) * p.dx_head_stride + (col % p.head_dim);
   __syncthreads();
-  const int cta = bwd_cta(&ticket);
+  const int cta = narrow_cta(&ticket);
   double* partials = reinterpret_cast<double*>(p.partials);
   if (cta >= p.workers) {
-    if (bwd_wait_for_workers(p, &bar_ok))
+    if (narrow_wait_for_workers(p, &bar_ok))
       finalize_units_f64(partials, p.groups, p.n, p.dw, LN ? p.db : nullptr, cta - p.workers, p.finalizers, fin);
-    bwd_depart(p);
+    else
+      bwd_no_sums(p.dw, LN ? p.db : nullptr, p.n, 8, cta - p.workers, p.finalizers);
+    narrow_depart(p);
     return;
   }
   const T* x = reinterpret_cast<const T*>(p.x) + col;
@@ -189,7 +248,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 3) norm_bwd_narrow_kernel(cons
       partials[((long long)plane * p.groups + cta) * n + (c - plane * n)] = (a[0] + a[1]) + (a[2] + a[3]);
     }
   }
-  bwd_worker_done(p);
+  narrow_worker_done(p);
 }
 
 __global__ void __launch_bounds__(kNarrowThreads) norm_bwd_narrow_finalize_kernel(const NormBwdParams p) {

@@ -19,8 +19,8 @@
 //   * Two sweeps over the stage: row sums first (one batched warp reduction), then dx and the
 //     gradient sums. The stage is refilled as soon as the second sweep has read it.
 //   * At the end the warps of a CTA fold their sums in a fixed order through shared memory into
-//     ONE fp32 partial row per CTA; CTAs that start after the workers add the partial rows in fp64
-//     (the two roles of norm_bwd.cuh). No atomics on results: they are bit-reproducible.
+//     ONE fp32 partial row per CTA; when all are written, the CTAs add them in fp64 (bwd_combine). No atomics on
+//     results: they are bit-reproducible.
 // Every wait is bounded; a wait that runs out makes the warp stop, wait (bounded) for its own
 // copies and raise the error word, so that nobody waits for it.
 #include "norm_bwd.cuh"
@@ -41,7 +41,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   constexpr int V = Elem<T>::V;
   constexpr int P = V / 2;  // fp32 pairs per vector
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ int bar_ok, ticket;
+  __shared__ int combine_flag[2];
   __shared__ int cta_failed;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = p.n / V;
@@ -52,8 +52,12 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + ring_bytes) + warp * 8;
   float* wsm = reinterpret_cast<float*>(smem + ring_bytes + kWarps * 8 * sizeof(uint64_t));
   const int rows = (int)p.rows;  // the launcher admits fewer than 2^31 rows
+  // CTAs behind the workers have no rows; they help to add up the columns
+  const int gwarp = (int)blockIdx.x * kWarps + warp;
+  const int gstep = p.workers * kWarps;
+  const int my_rows = (int)blockIdx.x < p.workers && rows > gwarp ? (rows - gwarp + gstep - 1) / gstep : 0;
 
-  bwd_draw_ticket(p, &ticket);
+  bwd_started(p);
   if (threadIdx.x == 0) cta_failed = 0;
   if (lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
@@ -62,7 +66,6 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
 
   const T* xg = reinterpret_cast<const T*>(p.x);
   const T* dyg = reinterpret_cast<const T*>(p.dy);
-  int gwarp = 0, gstep = 1;
   auto issue = [&](int k, int slot) {  // lane 0 only
     const long long row = (long long)gwarp + (long long)k * gstep;
     unsigned char* dst = ring + (size_t)slot * stage_bytes;
@@ -98,15 +101,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     }
   }
   const float dyf = DYS ? Elem<T>::to_f32(ld_here(dyg)) : 0.f;
-  __syncthreads();  // the ticket is there
-  const int cta = bwd_cta(&ticket);
-  if (cta >= p.workers) {
-    bwd_finalize(p, cta, LN ? p.db : nullptr, reinterpret_cast<double*>(smem), &bar_ok);
-    return;
-  }
-  gwarp = cta * kWarps + warp;
-  gstep = p.workers * kWarps;
-  const int my_rows = rows > gwarp ? (rows - gwarp + gstep - 1) / gstep : 0;
+  // the other lanes first touch the barriers after the __syncthreads below
   if (lane == 0) {
     for (int k = 0; k < my_rows && k < stages; ++k) issue(k, k);
   }
@@ -195,7 +190,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
     if (!arrived) {
       if (lane == 0) {
         note_wait_timeout();
-        if (p.bar) atomicExch(&p.bar[1], 1u);  // nobody is to wait for this CTA
+        if (p.bar) atomicExch(&p.bar[kBwdError], 1u);  // nobody is to wait for this CTA
         atomicExch(&cta_failed, 1);
         int ds = slot;
         uint32_t dp = phase;
@@ -353,7 +348,7 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
   // One partial row per CTA: the warps are folded in a fixed order through the ring (free now).
   __syncthreads();  // every warp is done with its rows (or gave up, with no copy in flight)
   const bool any_failed = cta_failed != 0;
-  if (!any_failed && (p.dw || p.db)) {
+  if (!any_failed && (int)blockIdx.x < p.workers && (p.dw || p.db)) {
     // [kWarps][CH][P][32] fp32 pairs for dw, then the same for db: a lane's pair at the lane's place, no bank conflicts
     constexpr int kPlane = CH * P * 32;
     f32x2* fold = reinterpret_cast<f32x2*>(smem);
@@ -392,11 +387,11 @@ norm_bwd_warp_kernel(const NormBwdParams p, const int stages, const int ring_byt
         float4 out;
         unpack2(lo, out.x, out.y);
         unpack2(hi, out.z, out.w);
-        *reinterpret_cast<float4*>(p.partials + ((long long)plane * p.groups + cta) * p.n + col) = out;
+        *reinterpret_cast<float4*>(p.partials + ((long long)plane * p.groups + blockIdx.x) * p.n + col) = out;
       }
     }
   }
-  bwd_worker_done(p);
+  bwd_combine(p, LN ? p.db : nullptr, reinterpret_cast<double*>(smem), combine_flag);
 }
 
 template <typename T, int CH, bool LN, bool DYS>
@@ -441,8 +436,8 @@ bool launch_warp_kernel_impl(NormBwdParams p, size_t scratch_bytes, cudaStream_t
     if (grid > max_groups) grid = max_groups;
   }
   p.groups = p.workers = (int)grid;
-  bwd_plan_finalize(p, (long long)per_sm * dev.sm_count);
-  launch_dependent(kernel, (unsigned)(grid + p.finalizers), kWarps * 32, smem, st, p, stages, (int)ring_bytes);
+  const unsigned ctas = bwd_plan_combined(p, (long long)per_sm * dev.sm_count);
+  launch_dependent(kernel, ctas, kWarps * 32, smem, st, p, stages, (int)ring_bytes);
   *rc = launch_status(DYS ? "b200_norm_bwd [warp per row, warp rings, scalar dy, fused finalize]"
                           : "b200_norm_bwd [warp per row, warp rings, fused finalize]");
   return true;

@@ -1,4 +1,4 @@
-"""Norm backward whose column sums are added up by CTAs of the same launch that start after the workers, or by a kernel chained to it."""
+"""Norm backward whose column sums are added up by the CTAs of the same launch, by some that start after the workers, or by a kernel chained to it."""
 import pytest
 import torch
 
@@ -75,7 +75,8 @@ def test_two_launches_need_no_zeroed_words(rows, n, dtype):
     assert bool((scratch[:256] == 0xa5).all())
 
 
-@pytest.mark.parametrize("rows,n,dtype", [(1100, 4096, torch.bfloat16), (1100, 2056, torch.float32)])
+@pytest.mark.parametrize("rows,n,dtype", [(1100, 4096, torch.bfloat16), (1100, 2056, torch.float32), (1030, 16384, torch.bfloat16), (300, 768, torch.bfloat16),
+                                          (5000, 264, torch.bfloat16), (300, 64, torch.bfloat16), (300, 2048, torch.float32)])
 def test_a_noted_error_shows_in_the_sums(rows, n, dtype):
     """With an error still noted in the words no sums are formed: they are NaN, not what the memory held, and the status says why."""
     from better_benchmark_b200 import kernels as k
@@ -88,3 +89,27 @@ def test_a_noted_error_shows_in_the_sums(rows, n, dtype):
     assert torch.equal(got[0], want[0]) and bool(torch.isnan(got[1]).all()) and bool(torch.isnan(got[2]).all())
     assert native.load().b200_check_status(scratch.data_ptr(), torch.cuda.current_stream().cuda_stream) != 0
     assert int(scratch[:256].count_nonzero()) == 1
+
+
+@pytest.mark.parametrize("rows,n,dtype", [(3000, 768, torch.bfloat16), (700, 2048, torch.bfloat16), (64, 512, torch.float32), (4000, 128, torch.bfloat16)])
+def test_while_another_stream_holds_the_gpu(rows, n, dtype):
+    """CTAs that find the GPU full of another stream's start late, and those that are there do not wait for them: the last one adds up."""
+    from better_benchmark_b200 import kernels as k
+    x, dy, w, mean, rstd = _inputs(rows, n, dtype, rows)
+    scratch = torch.zeros(16 << 20, dtype=torch.uint8, device="cuda")
+    want = k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True, scratch=scratch)
+    a = torch.randn(4096, 4096, device="cuda")
+    a @ a
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(6):
+        with torch.cuda.stream(side):
+            for _ in range(3):
+                a @ a   # a few ms of every SM
+        for _ in range(12):
+            got.append(k.norm_bwd(x, dy, w, rstd, mean=mean, rms=False, want_dbias=True, scratch=scratch))
+    torch.cuda.synchronize()
+    for outs in got:
+        assert all(torch.equal(p, q) for p, q in zip(outs, want))
+    assert int(scratch[:256].count_nonzero()) == 0
