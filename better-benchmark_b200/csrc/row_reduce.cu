@@ -207,15 +207,110 @@ struct ExtremeChains {
 template <typename Tin, typename Op, SumKind KIND>
 using RowChains = typename std::conditional<Op::is_sum, SumChains<Tin, KIND>, ExtremeChains<Tin, Op>>::type;
 
-// U = 16-byte loads in flight per thread. Warp mode uses U = 4 and at most 32 registers so that
-// 64 warps fit on an SM; block mode uses U = 8.
-// I: index type, long long for rows of 2^30 elements and more.
-template <typename Tin, typename Op, bool BLOCK, typename I>
+// Rows that start on 16-byte boundaries. U = 16-byte loads in flight per thread. Warp mode uses U = 4 and at most 32 registers so that
+// 64 warps fit on an SM; block mode uses U = 8. Bound by HBM: fp32 [8192, 4096] 21.6 us, 6.2 TB/s; with the head and the edges of the
+// kernel below and its joins of the chains 21.8, and where the rows are in L2 up to twice as long (amax bf16 [2400, 8000] 5.9 and 12.1).
+// VEC false: rows that start anywhere, element by element.
+template <typename Tin, typename Op, bool BLOCK, bool VEC>
 __global__ void __launch_bounds__(BLOCK ? 1024 : 256, BLOCK ? 1 : 8)
-row_reduce_kernel(const RowReduceParams p) {
+row_reduce_grid_kernel(const RowReduceParams p) {
   wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
   constexpr int U = BLOCK ? 8 : 4;
+  __shared__ __align__(8) float red[64];
+  const int lane = group_lane<BLOCK>();
+  const int G = group_size<BLOCK>();
+  const long long row = group_row<BLOCK>();
+  if (row >= p.rows) return;
+  const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
+  const long long nv = VEC ? p.n / V : 0;
+
+  float acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = Op::identity();
+  auto walk = [&](auto&& add) {
+    for (long long j0 = lane; j0 < nv; j0 += (long long)G * U) {
+      uint4 raw[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long j = j0 + (long long)u * G;
+        if (j < nv) raw[u] = ld_stream(x + j * V);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long j = j0 + (long long)u * G;
+        if (j < nv) add(raw[u]);
+      }
+    }
+  };
+  if constexpr (!VEC) {
+  } else if constexpr (!Op::is_sum && sizeof(Tin) == 2) {  // exact in the storage type: packed pairs, only the last of a thread is widened
+    using P2 = typename std::conditional<std::is_same<Tin, __half>::value, __half2, __nv_bfloat162>::type;
+    P2 m[4];
+    {
+      const Tin id = Elem<Tin>::from_f32(Op::identity());
+      P2 idp;
+      idp.x = id;
+      idp.y = id;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m[i] = idp;
+    }
+    walk([&](const uint4& v) {
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m[i] = Op::apply2(m[i], *reinterpret_cast<const P2*>(&w[i]));
+    });
+    const P2 a = Op::apply2(Op::apply2(m[0], m[1]), Op::apply2(m[2], m[3]));
+    acc[0] = Op::apply(Elem<Tin>::to_f32(a.x), Elem<Tin>::to_f32(a.y));
+  } else {
+    walk([&](const uint4& v) {
+      float f[V];
+      Elem<Tin>::unpack(v, f);
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] = Op::apply(acc[i], f[i]);
+    });
+  }
+  for (long long i = nv * V + lane; i < p.n; i += G) acc[0] = Op::apply(acc[0], Elem<Tin>::to_f32(x[i]));
+
+  float r;
+  if constexpr (Op::is_sum) {
+    // Chains are short (tens of elements); what is above them is combined in fp64, so that the result is the correctly rounded
+    // sum of the chains.
+    double d = 0.0;
+#pragma unroll
+    for (int i = 0; i < V; ++i) d += (double)acc[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    if constexpr (BLOCK) {
+      double* dred = reinterpret_cast<double*>(red);
+      const int warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+      if ((threadIdx.x & 31) == 0) dred[warp] = d;
+      __syncthreads();
+      d = 0.0;
+      for (int w = 0; w < nwarps; ++w) d += dred[w];
+    }
+    r = (float)d;
+  } else {
+#pragma unroll
+    for (int w = V / 2; w > 0; w >>= 1) {
+#pragma unroll
+      for (int i = 0; i < w; ++i) acc[i] = Op::apply(acc[i], acc[i + w]);
+    }
+    r = group_reduce<Op, BLOCK>(acc[0], red);
+  }
+  if (lane == 0) store_scalar(p.out, p.out_dtype, row * p.out_stride, r * p.post_scale);
+}
+
+// Rows that start and end anywhere. Warp mode: CTAS of 256 threads an SM. Six with U = 4, or four with U = 8, where all rows are then there at
+// once: with the 32 registers of eight CTAs the loads and the edges spill (bf16 sum [5000, 5001] 9.2 us with eight, 7.7 with six). By the
+// element [5000, 5001] takes 15.7, [8192, 1101] fp32 4.7 and 5.1 so, [5000, 2049] fp32 5.6 and 6.5: the two of some 200 shapes that lose.
+// I: index type, long long for rows of 2^30 elements and more.
+template <typename Tin, typename Op, bool BLOCK, typename I, int CTAS = 1>
+__global__ void __launch_bounds__(BLOCK ? 1024 : 256, CTAS)
+row_reduce_kernel(const RowReduceParams p) {
+  wait_for_previous_kernel();
+  constexpr int V = Elem<Tin>::V;
+  constexpr int U = BLOCK || CTAS == 4 ? 8 : 4;
   __shared__ __align__(8) float red[64];
   const int lane = group_lane<BLOCK>();
   const int G = group_size<BLOCK>();
@@ -329,27 +424,11 @@ __global__ void __launch_bounds__(256, K == 4 ? 6 : 4) row_reduce_short_kernel(c
 }
 
 template <typename Tin, typename Op>
-static int launch_row_reduce(const RowReduceParams& p, cudaStream_t st) {
+static int launch_row_reduce(const RowReduceParams& p, bool on_grid, cudaStream_t st) {
   constexpr int V = Elem<Tin>::V;
   const int sms = device_info().sm_count;
   if (p.rows > 0x7fffffffLL) return fail(B200_ERR_UNSUPPORTED, "row_reduce: too many rows");
   const long long nv = p.n / V;
-  // Rows of up to 128 vectors, whatever their number, and of up to 256 from four an SM on: all of a row's loads in one to 32
-  // lanes at once. A CTA (of 64 threads) for each of many short rows costs its launch, 0.6 ns a row over the whole GPU: fp32
-  // [60000, 64] 37.1 us as CTAs, 10.9 with a warp per row, 3.0 so, [64, 64] 1.9, 1.5 and 1.4; [60000, 640] 49.1, 24.0 (chains of fp32
-  // additions) and 23.8, [2000, 946] 3.5, 2.2 and 2.2; bf16 [60000, 512] 46.9, 16.1 and 10.7, [10000, 2048] 11.0, 9.1 and 7.5,
-  // [64, 1500] off the grid 3.3, 2.4 and 2.1.
-  auto short_rows = [&](auto kernel, int lanes) {
-    const int rows_per_cta = 256 / lanes;
-    set_path_tag("several rows a warp");
-    launch_dependent(kernel, (unsigned)((p.rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st, p);
-    return launch_status("b200_row_reduce");
-  };
-  if (nv <= 16) return short_rows(row_reduce_short_kernel<Tin, Op, 4, 4, kKept>, 4);
-  if (nv <= 32) return short_rows(row_reduce_short_kernel<Tin, Op, 8, 4, kKept>, 8);
-  if (nv <= 64) return short_rows(row_reduce_short_kernel<Tin, Op, 16, 4, kKept>, 16);
-  if (nv <= 128) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 4, kKept>, 32);
-  if (nv <= 256 && p.rows >= 4LL * sms) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 8, kPairs>, 32);
   // CTA-per-row geometry: about eight vectors per thread.
   int threads = (int)((nv + 7) / 8);
   threads = (threads + 31) / 32 * 32;
@@ -361,23 +440,62 @@ static int launch_row_reduce(const RowReduceParams& p, cudaStream_t st) {
     const double waves = units / (sms * resident_per_sm);
     return waves <= 1.0 ? 1.0 : waves / (double)(long long)(waves + 0.999999);
   };
-  const double eff_warp = efficiency((double)((p.rows + 7) / 8), 8.0);
   const double eff_block = efficiency((double)p.rows, (double)(2048 / threads > 32 ? 32 : 2048 / threads));
-  const bool warp_mode = nv > 256 && p.rows >= (long long)sms * 16 && p.n <= 16384 && eff_warp + 0.02 >= eff_block;
-  set_path_tag(warp_mode ? "warp per row" : "CTA per row");
-  if (warp_mode) launch_dependent(row_reduce_kernel<Tin, Op, false, int>, (unsigned)((p.rows + 7) / 8), 256, 0, st, p);
+  auto by_warp = [&](double ctas) {
+    return p.rows >= (long long)sms * 16 && p.n <= 16384 && efficiency((double)((p.rows + 7) / 8), ctas) + 0.02 >= eff_block;
+  };
+  // Rows of up to 128 vectors, whatever their number, and of up to 256 from four an SM on: all of a row's loads in one to 32
+  // lanes at once. A CTA (of 64 threads) for each of many short rows costs its launch, 0.6 ns a row over the whole GPU: fp32
+  // [60000, 64] 37.1 us as CTAs, 10.9 with a warp per row, 3.0 so, [64, 64] 1.9, 1.5 and 1.4; [60000, 640] 49.1, 24.0 (chains of fp32
+  // additions) and 23.8, [2000, 946] 3.5, 2.2 and 2.2; bf16 [60000, 512] 46.9, 16.1 and 10.7, [10000, 2048] 11.0, 9.1 and 7.5,
+  // [64, 1500] off the grid 3.3, 2.4 and 2.1.
+  auto short_rows = [&](auto kernel, int lanes) {
+    const int rows_per_cta = 256 / lanes;
+    set_path_tag("several rows a warp");
+    launch_dependent(kernel, (unsigned)((p.rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st, p);
+    return launch_status("b200_row_reduce");
+  };
+  // fp32 sums of 64 to 256 vectors where a warp per row is one well filled wave (2368 to some 9000 rows on 148 SMs) are bound by the
+  // additions that keep what is rounded away: plain chains there, as for longer rows, and element by element off the grid
+  // ([8192, 512] 3.9 us with what is rounded away, so 2.8; [8192, 301] 3.7, as vectors with plain chains 3.4, so 3.0).
+  const bool plain = Op::is_sum && sizeof(Tin) == 4 && nv >= 64 && nv <= 256 && by_warp(8.0);
+  if (nv <= 16) return short_rows(row_reduce_short_kernel<Tin, Op, 4, 4, kKept>, 4);
+  if (nv <= 32) return short_rows(row_reduce_short_kernel<Tin, Op, 8, 4, kKept>, 8);
+  if (nv <= 64 && !plain) return short_rows(row_reduce_short_kernel<Tin, Op, 16, 4, kKept>, 16);
+  if (nv <= 128 && !plain) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 4, kKept>, 32);
+  if (nv <= 256 && !plain && p.rows >= 4LL * sms) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 8, kPairs>, 32);
+  const unsigned warp_ctas = (unsigned)((p.rows + 7) / 8);
+  if (on_grid) {
+    const bool warp_mode = plain || (nv > 256 && by_warp(8.0));
+    set_path_tag(warp_mode ? "vector, warp per row" : "vector, CTA per row");
+    if (warp_mode) launch_dependent(row_reduce_grid_kernel<Tin, Op, false, true>, warp_ctas, 256, 0, st, p);
+    else launch_dependent(row_reduce_grid_kernel<Tin, Op, true, true>, (unsigned)p.rows, threads, 0, st, p);
+    return launch_status("b200_row_reduce");
+  }
+  if constexpr (Op::is_sum && sizeof(Tin) == 4) {
+    if (plain) {
+      set_path_tag("element-wise, warp per row");
+      launch_dependent(row_reduce_grid_kernel<Tin, Op, false, false>, warp_ctas, 256, 0, st, p);
+      return launch_status("b200_row_reduce");
+    }
+  }
+  const bool warp_mode = nv > 256 && by_warp(8.0);
+  set_path_tag(warp_mode ? "off-grid rows as vectors, warp per row" : "off-grid rows as vectors, CTA per row");
+  if (warp_mode && warp_ctas <= 4u * sms) launch_dependent(row_reduce_kernel<Tin, Op, false, int, 4>, warp_ctas, 256, 0, st, p);
+  else if (warp_mode && warp_ctas <= 6u * sms) launch_dependent(row_reduce_kernel<Tin, Op, false, int, 6>, warp_ctas, 256, 0, st, p);
+  else if (warp_mode) launch_dependent(row_reduce_kernel<Tin, Op, false, int, 8>, warp_ctas, 256, 0, st, p);
   else if (p.n < (1 << 30)) launch_dependent(row_reduce_kernel<Tin, Op, true, int>, (unsigned)p.rows, threads, 0, st, p);
   else launch_dependent(row_reduce_kernel<Tin, Op, true, long long>, (unsigned)p.rows, threads, 0, st, p);
   return launch_status("b200_row_reduce");
 }
 
 template <typename Tin>
-static int dispatch_row_reduce_op(const RowReduceParams& p, int op, cudaStream_t st) {
+static int dispatch_row_reduce_op(const RowReduceParams& p, int op, bool on_grid, cudaStream_t st) {
   switch (op) {
     case B200_REDUCE_SUM:
-    case B200_REDUCE_MEAN: return launch_row_reduce<Tin, SumOp>(p, st);
-    case B200_REDUCE_AMAX: return launch_row_reduce<Tin, MaxOp>(p, st);
-    case B200_REDUCE_AMIN: return launch_row_reduce<Tin, MinOp>(p, st);
+    case B200_REDUCE_MEAN: return launch_row_reduce<Tin, SumOp>(p, on_grid, st);
+    case B200_REDUCE_AMAX: return launch_row_reduce<Tin, MaxOp>(p, on_grid, st);
+    case B200_REDUCE_AMIN: return launch_row_reduce<Tin, MinOp>(p, on_grid, st);
   }
   return fail(B200_ERR_INVALID, "b200_row_reduce: unknown op %d", op);
 }
@@ -404,11 +522,13 @@ extern "C" int b200_row_reduce(const void* x, void* out, int64_t rows, int64_t n
   p.out_stride = out_stride; p.out_dtype = out_dtype;
   // mean of an empty row is 0 * (1/0) = NaN, as aten.mean returns
   p.post_scale = op == B200_REDUCE_MEAN ? 1.0f / (float)n : 1.0f;
+  const int ib = dtype_size(x_dtype);
+  const bool on_grid = aligned16(x) && (p.xmap.s0 * ib) % 16 == 0 && (p.xmap.s1 * ib) % 16 == 0 && (p.xmap.s2 * ib) % 16 == 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   switch (x_dtype) {
-    case B200_F32: return dispatch_row_reduce_op<float>(p, op, st);
-    case B200_BF16: return dispatch_row_reduce_op<__nv_bfloat16>(p, op, st);
-    case B200_F16: return dispatch_row_reduce_op<__half>(p, op, st);
+    case B200_F32: return dispatch_row_reduce_op<float>(p, op, on_grid, st);
+    case B200_BF16: return dispatch_row_reduce_op<__nv_bfloat16>(p, op, on_grid, st);
+    case B200_F16: return dispatch_row_reduce_op<__half>(p, op, on_grid, st);
   }
   return fail(B200_ERR_INVALID, "b200_row_reduce: unknown dtype %d", x_dtype);
 }
