@@ -512,6 +512,14 @@ struct RowSpan {
   }
 };
 
+// Turns of a CTA that takes `at_once` rows at a time, at most sixteen, so that the CTAs make whole waves of `resident` (rounded down, 24 rows
+// per SM in CTAs that take 16 at a time an SM were two waves of one turn, 72 two waves of four).
+inline int span_turns(long long rows, int at_once, long long resident) {
+  const long long turns = (rows + at_once * resident - 1) / (at_once * resident);
+  const long long waves = (turns + 15) / 16;
+  return (int)((turns + waves - 1) / waves);
+}
+
 // Elements [lo, hi) of the vector at p, zeros beside them.
 template <typename T>
 __device__ __forceinline__ uint4 load_part(const T* p, int lo, int hi) {

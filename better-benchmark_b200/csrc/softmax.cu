@@ -719,9 +719,8 @@ static bool try_launch_softmax_span(const SoftmaxParams& p, cudaStream_t st) {
   auto launch = [&](auto kernel, int lanes) {
     const int at_once = 256 / lanes;
     const long long resident = sms * cached_occupancy(reinterpret_cast<const void*>(kernel), 256);
-    long long reps = p.rows / (at_once * resident);
-    reps = reps < 1 ? 1 : (reps > 16 ? 16 : reps);
-    launch_dependent(kernel, (unsigned)((p.rows + at_once * reps - 1) / (at_once * reps)), 256, 0, st, p, (int)reps);
+    const int reps = span_turns(p.rows, at_once, resident);
+    launch_dependent(kernel, (unsigned)((p.rows + (long long)at_once * reps - 1) / ((long long)at_once * reps)), 256, 0, st, p, reps);
     return true;
   };
   if (nv <= 8) return launch(softmax_span_kernel<T, 1, 8>, 8);
