@@ -1,4 +1,6 @@
 """Channels-last BatchNorm whose elements are no whole number of channel periods, or of 16-byte vectors."""
+import math
+
 import pytest
 import torch
 
@@ -6,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 DTYPES = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}
 # (n, c, h, w): odd channel counts and row counts, so that 1 to 7 elements are left over; few vectors; more than one wave of chunks
-SHAPES = [(1, 3, 1, 3), (1, 9, 1, 2), (2, 35, 5, 5), (3, 287, 7, 7), (1, 401, 14, 13), (5, 509, 3, 3), (9, 92, 5, 5), (600, 77, 15, 15)]
+SHAPES = [(1, 3, 1, 3), (1, 9, 1, 2), (2, 35, 5, 5), (3, 287, 7, 7), (1, 401, 14, 13), (5, 509, 3, 3), (9, 92, 5, 5), (600, 77, 15, 15),
+          (3, 3, 15, 15), (1, 9, 25, 27), (27, 35, 5, 5), (13, 287, 7, 7), (5, 401, 11, 13), (67, 509, 3, 3), (25, 92, 5, 5)]
 
 
 def _image(shape, dtype, seed, scale=1.0):
@@ -29,8 +32,9 @@ def test_forward(dtype, shape):
     w, b = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
     for relu in (False, True):
         y, mean, invstd = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1, relu=relu)
-        if c > 3:
-            assert b"copy rings" in k.load().b200_last_kernel()
+        rows, v = shape[0] * shape[2] * shape[3], 16 // dt.itemsize
+        if rows * c % (c // math.gcd(c, v) * v) != 0:   # few rows: the strided kernels
+            assert (b"copy rings" in k.load().b200_last_kernel()) == (rows >= 75 * v)
         d = x.double()
         m, v = d.mean((0, 2, 3)), d.var((0, 2, 3), unbiased=False)
         s = torch.rsqrt(v + 1e-5)
