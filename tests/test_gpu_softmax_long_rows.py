@@ -41,3 +41,21 @@ def test_many_long_rows(n, dtype, out_dtype, path, log):
     else:
         # the exponent's difference may be off by half an ulp of 30 and the exponential by two of its own
         assert bool(((got - want).abs() <= ulp * want + 4e-6 * want + 6.2e-8 * (out_dtype == torch.float16) + 1e-38).all())
+
+
+@pytest.mark.parametrize("n,dtype,path", [(98304, torch.bfloat16, b"two sweeps"), (50000, torch.float32, b"two sweeps"), (65536, torch.float32, b"cluster"),
+                                          (81920, torch.float16, b"cluster"), (81928, torch.float16, b"two sweeps"), (98307, torch.bfloat16, b"cluster")])
+def test_full_last_rows(n, dtype, path):
+    """Two rows an SM: the sweeps lose nothing to an SM without a row."""
+    from better_benchmark_b200 import kernels as k
+    rows = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    x = (torch.randn(rows, n, device="cuda") * 3).to(dtype)
+    for log in (False, True):
+        got = k.softmax(x, log=log)
+        assert path in k.load().b200_last_kernel(), k.load().b200_last_kernel()
+        for i in (0, rows - 1):
+            want = torch.log_softmax(x[i].double(), -1) if log else torch.softmax(x[i].double(), -1)
+            ulp = {torch.float32: 2.0 ** -23, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+            # one rounding of the result; in front of it the difference, the exponential and the sum, as above
+            bound = (ulp + 2.0 ** -23) * want.abs() + 4e-6 * (1 if log else want) + 6.2e-8 * (dtype == torch.float16)
+            assert bool(((got[i].double() - want).abs() <= bound + 1e-38).all())
