@@ -381,7 +381,8 @@ B200_CALL(norm_fwd, 18)
     if (rows > 1) stride = x->stride(0);
   }
   if (residual && (residual->scalar_type() != x->scalar_type() || !residual->is_contiguous() || residual->numel() != numel ||
-                   type != x->scalar_type() || (v[16] == Py_None && residual->sizes() != x->sizes())))
+                   type != x->scalar_type() ||
+                   (v[16] == Py_None && (residual->sizes() != x->sizes() || residual->strides() != x->strides()))))
     Py_RETURN_NONE;
   if (want_sum && !residual) Py_RETURN_NONE;
   if ((weight && !vector_of(weight, n)) || (bias && !vector_of(bias, n))) Py_RETURN_NONE;

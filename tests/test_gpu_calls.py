@@ -274,3 +274,14 @@ def test_streams_threads_and_graphs():
     g.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got[:3], want[:3]))
+
+
+def test_residuals_with_strides_of_their_own(monkeypatch):
+    """A residual counts as contiguous whatever the stride of a dimension of size one: the Python code refuses it, and so does the native code."""
+    from better_benchmark_b200 import kernels as k
+    x, w = _t(4, 1, 40, dtype=BF16), _t(40)
+    residual = torch.empty_strided((4, 1, 40), (40, 8, 1), device="cuda", dtype=BF16).copy_(x)
+    assert residual.is_contiguous() and residual.stride() != x.stride()
+    _compare(monkeypatch, lambda: k.norm_fwd(x, w, w, eps=1e-5, residual=residual), native=False)
+    with pytest.raises(k.UnsupportedLayout, match="strides"):
+        k.norm_fwd(x, w, w, eps=1e-5, residual=residual)
