@@ -2,7 +2,8 @@
 
 ``python -m better_benchmark_b200.build`` (or ``build_library()``) compiles every ``csrc/*.cu``
 file to an object in ``csrc/_build/`` in parallel and links ``csrc/libb200_oracles.so``, and compiles
-``csrc/calls.cpp``, the host side of the most frequent calls, to the extension module ``csrc/b200_calls.so``.
+``csrc/calls.cpp``, the host side of the most frequent calls, to an extension module beside it that is named after the torch
+and the Python it is compiled against (``native.calls_path()``).
 Objects are rebuilt only when their source (or a shared header) is newer.
 """
 from __future__ import annotations
@@ -17,7 +18,6 @@ from pathlib import Path
 CSRC = Path(__file__).resolve().parent / "csrc"
 BUILD_DIR = CSRC / "_build"
 LIB_PATH = CSRC / "libb200_oracles.so"
-CALLS_PATH = CSRC / "b200_calls.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -44,9 +44,10 @@ def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
 
 def build_calls(force: bool = False) -> Path:
     """The extension module, against the torch that runs this. It holds no device code."""
-    src = CSRC / "calls.cpp"
-    if not force and not _stale(CALLS_PATH, src, [CSRC.parent.parent / "include" / "b200_oracles.h"]):
-        return CALLS_PATH
+    from .native import calls_path
+    src, out = CSRC / "calls.cpp", calls_path()
+    if not force and not _stale(out, src, [CSRC.parent.parent / "include" / "b200_oracles.h"]):
+        return out
     import sysconfig
 
     import torch
@@ -55,11 +56,11 @@ def build_calls(force: bool = False) -> Path:
                 Path(sysconfig.get_paths()["include"]), Path(_nvcc()).resolve().parent.parent / "include"]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in includes), str(src),
-           "-o", str(CALLS_PATH), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+           "-o", str(out), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed on {src.name}:\n{res.stdout}\n{res.stderr}")
-    return CALLS_PATH
+    return out
 
 
 def build_library(force: bool = False, verbose: bool = False) -> Path:

@@ -9,7 +9,9 @@ from __future__ import annotations
 import ctypes
 import importlib.machinery
 import importlib.util
+import sys
 import threading
+import warnings
 from ctypes import c_char_p, c_double, c_int32, c_int64, c_void_p
 from pathlib import Path
 
@@ -18,8 +20,13 @@ import os
 # B200_ORACLES_LIB names another build of the library (a measurement variant); default: the in-tree one
 LIB_PATH = Path(os.environ.get("B200_ORACLES_LIB") or Path(__file__).resolve().parent / "csrc" / "libb200_oracles.so")
 
-# The host side of the most frequent calls (csrc/calls.cpp), an extension module that works on the library loaded here
-CALLS_PATH = Path(__file__).resolve().parent / "csrc" / "b200_calls.so"
+
+def calls_path() -> Path:
+    """The host side of the most frequent calls (csrc/calls.cpp), an extension module that works on the library loaded here. It is compiled
+    against the C++ headers of one torch and one Python, and looks into their objects: a build for others has another name."""
+    import torch
+    build = f"{sys.implementation.cache_tag}.torch-{torch.__version__}.abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+    return Path(__file__).resolve().parent / "csrc" / f"b200_calls.{build}.so"
 
 # dtype codes shared with csrc/common.cuh
 F32, BF16, F16 = 0, 1, 2
@@ -147,22 +154,36 @@ _BOUND = ("b200_row_reduce", "b200_softmax", "b200_norm_fwd_residual", "b200_nor
           "b200_batch_norm_bwd_scratch_bytes", "b200_transpose_copy", "b200_permute_copy", "b200_cast_scale")
 
 
-def load_calls(scratch_by_device: dict):
-    """Load csrc/calls.cpp's module once per process and hand it the library's entry points."""
+class _LeftToPython:
+    """Stands in for the module where it is not built: every call is left to the Python code of the wrappers."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def load_calls(scratch_by_device: dict, required: bool = False):
+    """Load csrc/calls.cpp's module once per process and hand it the library's entry points. Where it is not built for this torch and this
+    Python the wrappers' Python code takes every call, which it can, at two to four times the host time; with ``required`` that is an error."""
     global _calls
     lib = load()
     with _lock:
         if _calls is None:
-            if not CALLS_PATH.exists():
-                raise NativeLibraryError(f"{CALLS_PATH} is not built. Run `python -m better_benchmark_b200.build`.")
-            try:
-                loader = importlib.machinery.ExtensionFileLoader("b200_calls", str(CALLS_PATH))
-                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200_calls", loader))
-                loader.exec_module(module)
-            except ImportError as e:
-                raise NativeLibraryError(f"cannot load {CALLS_PATH}: {e}") from e
-            module.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _BOUND}, check, scratch_by_device)
-            _calls = module
+            path = calls_path()
+            if path.exists():
+                try:
+                    loader = importlib.machinery.ExtensionFileLoader("b200_calls", str(path))
+                    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200_calls", loader))
+                    loader.exec_module(module)
+                except ImportError as e:
+                    raise NativeLibraryError(f"cannot load {path}: {e}") from e
+                module.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _BOUND}, check, scratch_by_device)
+                _calls = module
+            elif not required:
+                warnings.warn(f"{path} is not built, so every call takes the longer way through Python. "
+                              "Run `python -m better_benchmark_b200.build`.", RuntimeWarning, stacklevel=2)
+                _calls = _LeftToPython()
+        if required and (_calls is None or isinstance(_calls, _LeftToPython)):
+            raise NativeLibraryError(f"{calls_path()} is not built. Run `python -m better_benchmark_b200.build`.")
         return _calls
 
 

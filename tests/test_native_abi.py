@@ -51,3 +51,25 @@ def test_wrappers_refuse_cpu_tensors_and_missing_library(monkeypatch, tmp_path):
     monkeypatch.setattr(native, "LIB_PATH", tmp_path / "absent.so")
     with pytest.raises(native.NativeLibraryError):
         native.load()
+
+
+def test_calls_without_the_extension_module(monkeypatch, tmp_path):
+    """Not built, or built for another torch or Python: the Python code takes every call, and says so once; a build that needs it is told."""
+    import warnings
+
+    import torch
+    from better_benchmark_b200 import kernels, native
+    built = native.calls_path()
+    assert torch.__version__ in built.name
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert native.calls_path() != built and not native.calls_path().exists()
+    monkeypatch.setattr(native, "_calls", None)
+    monkeypatch.setattr(kernels, "_calls", None)
+    with pytest.raises(native.NativeLibraryError, match="not built"):
+        native.load_calls({}, required=True)
+    with pytest.warns(RuntimeWarning, match="not built"), pytest.raises(native.KernelArgumentError):
+        kernels.row_reduce(torch.zeros(4, 4), "sum")   # the wrapper's own rule: no CPU tensors
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        with pytest.raises(native.KernelArgumentError):
+            kernels.softmax(torch.zeros(4, 4))
