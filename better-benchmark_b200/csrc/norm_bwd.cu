@@ -1238,7 +1238,7 @@ extern "C" int64_t b200_norm_bwd_wait_timeouts(void) {
 // Bytes of scratch that let every path run its largest grid for rows of n elements: the barrier
 // words and two planes (dweight, dbias) of one fp32 partial row per group. A group is a CTA (at most eight resident
 // per SM), except in the warp-per-row register kernel, which takes rows of up to 256 elements where the copy rings do not
-// fit, where it is a warp (64 per SM). (Rows of at most 32 vectors: fp64, at most six per SM.) The launchers shrink their grids to whatever scratch they are given, so a smaller buffer
+// fit, where it is a warp (64 per SM). (Rows of at most 32 vectors: fp64, two waves of three per SM at most.) The launchers shrink their grids to whatever scratch they are given, so a smaller buffer
 // costs speed, never correctness.
 extern "C" int64_t b200_norm_bwd_scratch_bytes(int64_t n) {
   const int64_t groups = (n <= 256 ? 64 : 8) * (int64_t)device_info().sm_count;

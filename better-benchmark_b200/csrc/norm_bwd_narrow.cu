@@ -263,12 +263,15 @@ int launch_norm_bwd_narrow(NormBwdParams p, size_t scratch_bytes, bool fused, cu
   constexpr int V = Elem<T>::V;
   const int nv = p.n / V;
   auto launch = [&](auto kernel, int lanes) {
-    const long long room = (long long)cached_occupancy(reinterpret_cast<const void*>(kernel), kNarrowThreads) * device_info().sm_count;
+    // three CTAs an SM, as the kernel's launch bounds say and the advertised scratch counts on, also where a compiler leaves room for more
+    const int resident = cached_occupancy(reinterpret_cast<const void*>(kernel), kNarrowThreads);
+    const long long room = (long long)(resident < 3 ? resident : 3) * device_info().sm_count;
     const int at_once = kNarrowThreads / lanes;
     long long grid = (p.rows + at_once - 1) / at_once;
-    // Rows of 17 vectors and more have a quarter of the groups that those of 8 have: with a second wave of CTAs, up to 42624 rows on
-    // 148 SMs, a group's chain is no longer than a warp's of the kernel that was here (LayerNorm bf16 [8000, 256] 10.8 -> 14.3 us, [20000, 256]
-    // 16.0 -> 18.6, but errors of dweight and dbias up to 15 % larger without). From there on the blocks of rows make up for it.
+    // Rows of 17 vectors and more have a quarter of the groups that those of 8 have. As long as one wave of CTAs would leave a group at most 12
+    // rows (42624 rows on 148 SMs) there are two waves, of chains half as long: without them errors of dweight and dbias are up to 15 % larger
+    // than with a warp per row (LayerNorm bf16 [8000, 256] 10.8 us in one wave, 14.3 so; [20000, 256] 16.0 and 18.6). Longer chains are
+    // cut into blocks of four rows and more, whose sums are added once each, so that the second wave gains nothing there.
     const long long most = lanes == 32 && p.rows <= 12 * room * at_once ? 2 * room : room;
     if (grid > most) grid = most;
     if (p.dw || p.db) {
