@@ -124,7 +124,7 @@ void note_launch(const char* what) {
 
 }  // namespace b200
 
-// Number of kernels this library has launched in this process (cooperative launches included).
+// Number of kernels this library has launched in this process so far.
 extern "C" int64_t b200_launch_count(void) { return b200::g_launches.load(std::memory_order_relaxed); }
 
 // Name of the kernel this thread launched last, with the variant the launcher chose in brackets
@@ -140,7 +140,7 @@ extern "C" int b200_sm_count(void) { return b200::device_info().sm_count; }
 
 extern "C" int b200_l2_bytes(void) { return b200::device_info().l2_bytes; }
 
-// Reads the status words of a scratch buffer used by a cooperative kernel (see grid_barrier).
+// Reads the status words of a scratch buffer used by the norm backward (BwdWords in norm_bwd.cuh).
 // Synchronises the stream: a diagnostic call, never part of a timed or captured region.
 extern "C" int b200_check_status(const void* scratch, void* stream) {
   if (!scratch) return b200::fail(B200_ERR_INVALID, "b200_check_status: null scratch");
@@ -151,6 +151,6 @@ extern "C" int b200_check_status(const void* scratch, void* stream) {
   if (e != cudaSuccess) return b200::fail((int)e, "b200_check_status: %s", cudaGetErrorString(e));
   if (words[1] != 0)
     return b200::fail(B200_ERR_DEVICE_WAIT,
-                      "a grid-wide wait ran out inside a cooperative kernel (arrivals=%u)", words[0]);
+                      "a bounded wait ran out in a norm backward: its column sums were not formed (arrivals=%u)", words[0]);
   return B200_OK;
 }

@@ -841,7 +841,7 @@ extern "C" int b200_batch_norm_fwd_ex(const void* x, void* y, const void* weight
   p.inv_count = 1.0 / count;
   p.unbias = unbiased_factor > 0.0 ? (float)unbiased_factor : (float)(count / (count - 1.0));
   p.relu = relu ? 1 : 0;
-  p.partials = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + 256);  // behind the barrier words of other kernels
+  p.partials = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + 256);  // behind the words that the norm backward keeps at zero
   p.stats = nullptr;
 
   // channels-last: c is the unit-stride dimension, rows are (n, s) pairs with a uniform stride of C

@@ -521,7 +521,7 @@ B200_CALL(batch_norm_bwd, 10)
   const at::Tensor scratch =
       v[9] == Py_None ? shared_scratch(a.device, lib.batch_norm_bwd_scratch_bytes(c) + 256) : own_scratch(a, v[9]);
   if (!scratch.defined()) Py_RETURN_NONE;
-  // behind the 256 bytes that kernels with a grid barrier keep at zero
+  // behind the 256 bytes that the norm backward keeps at zero
   const int64_t bytes = scratch.numel() * scratch.element_size() - 256;
   at::Tensor dx, dw, db;
   int status;

@@ -482,9 +482,10 @@ inline bool pick_row_geometry(long long nv, RowGeometry* g) {
 
 // ----------------------------------------------------------------------------------------------
 // Rows that start and end anywhere, as the 16-byte vectors of memory that they touch: vector j holds the row's elements
-// j V - off .. j V - off + V - 1. Only the first and the last one may hold others beside them; those two are
-// read and written element by element, so that nothing outside the row is touched. Tensors with the same `off` in every
-// row share the vectors.
+// j V - off .. j V - off + V - 1. Only the first and the last one may hold others beside them. Those two are written element by element, so
+// that nothing outside the row changes; they are read whole wherever all of them lies between the first row's start and the last row's
+// end (a neighbour's elements, or the gap of a padded tensor, which are masked out), and element by element elsewhere, so that nothing
+// outside the tensor is read. Tensors with the same `off` in every row share the vectors.
 // ----------------------------------------------------------------------------------------------
 struct RowSpan {
   int off;   // elements between the 16-byte boundary and the row's first one

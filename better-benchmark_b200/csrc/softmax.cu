@@ -670,7 +670,8 @@ __global__ void __launch_bounds__(512) softmax_span_row_kernel(const SoftmaxPara
 //   n 257   24 3.9 / 4.5, 25 5.5 / 4.5        n 391   40 7.1 / 7.2, 48 7.6 / 8.1, 56 9.4 / 8.4    n 420   20 4.5 / 4.3, 48 7.7 / 7.6
 //   n 601   10 4.4 / 4.6, 11 5.0 / 4.6        n 900   8 4.4 / 4.4, 11 5.6 / 5.1, 18 8.4 / 7.8
 //   n 1241  2 4.1 / 3.7, 135 61.9 / 40.3      n 250   200 14.7 / 18.3, 800 52.6 / 62.2    n 506   64 10.9 / 12.4, 300 45.2 / 47.1
-// The last two are of the rows that fill the other kernel's slots and have just left one of this one's. All with one mask for all rows. With a
+// The last two are of the rows that fill the other kernel's slots and have just left one of this one's. All with one mask for all rows, and with
+// turns rounded down, which made waves of CTAs that were not full (n 391, 48 rows per SM; n 900, 18); now nothing from the lines on is slower. With a
 // mask for so many rows as the CTA takes at two times the groups are still ahead ([20000, 1017] 50.6 / 41.3), with one for half as many no longer
 // (50.6 / 53.3), with one for every row they are far behind (49.0 / 73.0, [60000, 249] 29.6 / 36.7).
 static int softmax_span_rows_per_sm(int n, int nv) {

@@ -339,10 +339,9 @@ def residual_layer_norm_as(x, residual, weight, bias, shape, shape2, *, eps: flo
 # ---------------------------------------------------------------------------------------------
 # Scratch memory. Kernels that combine per-CTA partial results take a caller-provided scratch
 # buffer. One zero-initialised buffer per device is kept here; the first 256 bytes hold the
-# grid-barrier words, which every kernel leaves at zero when it finishes. Kernels on one stream run
-# in order, and the library lets no launch of another thread in between those of one call, so sharing the buffer is safe
-# there; callers that launch on several streams at once must
-# pass their own ``scratch``. A request for more bytes than the buffer holds allocates a larger one,
+# words by which the CTAs of a norm backward count one another, which it leaves at zero when it finishes. Kernels on one
+# stream run in order, and the library lets no launch of another thread in between those of one call, so sharing the buffer
+# is safe there; callers that launch on several streams at once must pass their own ``scratch``. A request for more bytes than the buffer holds allocates a larger one,
 # but the smaller ones are never released: a CUDA graph captured earlier still holds their address.
 # Growing while the current stream is being captured is refused (the new buffer would belong to
 # that graph's private pool while later, uncaptured calls keep using it).
@@ -368,12 +367,12 @@ def scratch_buffer(device: torch.device, nbytes: int) -> torch.Tensor:
 
 
 def _behind_barrier_words(scratch: torch.Tensor):
-    """Address and size of what follows the 256 bytes that kernels with a grid barrier keep at zero."""
+    """Address and size of what follows the 256 bytes that the norm backward keeps at zero."""
     return scratch.data_ptr() + 256, max(0, scratch.numel() * scratch.element_size() - 256)
 
 
 def check_scratch_status(device: torch.device | None = None) -> None:
-    """Raise if a cooperative kernel on this device gave up a grid-wide wait (synchronises)."""
+    """Raise if CTAs of a norm backward on this device gave up waiting for copies or for one another (synchronises)."""
     device = device or torch.device("cuda", torch.cuda.current_device())
     lib = load()
     for buf in _scratch_by_device.get(_device_key(device), []):
@@ -383,7 +382,7 @@ def check_scratch_status(device: torch.device | None = None) -> None:
             check(status, "b200_check_status")
 
 
-NORM_BWD_TWO_LAUNCH = 1  # flag: main kernel + finalize kernel instead of one cooperative launch
+NORM_BWD_TWO_LAUNCH = 1  # flag: main kernel + finalize kernel also where one launch does both
 NORM_BWD_DY_SCALAR = 2   # flag: dy is one element that stands for the whole tensor (an expanded 0-dim gradient)
 
 

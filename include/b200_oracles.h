@@ -18,8 +18,8 @@
  *     (B200_ERR_*); > 0 the cudaError_t of a rejected launch. b200_last_error() returns the text
  *     of the calling thread's last failure.
  *   - Kernels that combine per-CTA partial results take a caller-provided `scratch` buffer
- *     (16-byte aligned). Its first 256 bytes hold grid-barrier words that must be zero before
- *     the first use; every kernel leaves them zero. Concurrent launches on different streams
+ *     (16-byte aligned). Its first 256 bytes hold the words by which the CTAs of b200_norm_bwd count one another; they
+ *     must be zero before the first use, and every launch leaves them zero. Concurrent launches on different streams
  *     need different scratch buffers. Calls on one stream may share one, from several host threads
  *     too: the launches of a call follow one another in the stream.
  *   - Accumulation is fp32 (fp64 where partial results of many CTAs are combined), no fast-math,
@@ -67,9 +67,9 @@ int64_t b200_launch_count(void);
  * tell the tuned paths from the element-wise ones. */
 const char* b200_last_kernel(void);
 
-/* Reads the status words of a scratch buffer; returns B200_ERR_DEVICE_WAIT if a grid-wide wait
- * inside a cooperative kernel ran out. Synchronises `stream`: diagnostic use only. No
- * counterpart in the reference (its kernels never wait on one another). */
+/* Reads the status words of a scratch buffer; returns B200_ERR_DEVICE_WAIT if CTAs of b200_norm_bwd gave up
+ * waiting for copies or for one another (dweight and dbias are NaN then, and stay so until the words
+ * are set to zero again). Synchronises `stream`: diagnostic use only. No counterpart in the reference (its kernels never wait on one another). */
 int32_t b200_check_status(const void* scratch, void* stream);
 
 /* Row reduction over the last (unit-stride) dimension: op 0 sum, 1 mean, 2 amax, 3 amin.
@@ -135,8 +135,9 @@ int64_t b200_norm_bwd_scratch_bytes(int64_t n);
  * nullable) as column reductions over all rows. dx element (r, c) is stored at
  *   (r / seq) * dx_batch_stride + (r % seq) * dx_seq_stride + (c / head_dim) * dx_head_stride + c % head_dim
  * which covers both the plain [rows, n] layout (seq = 1, head_dim = n, dx_batch_stride = n) and the
- * fused head-major (B,S,H,D) -> (B,H,S,D) store. flags: 1 = two launches (main + finalize)
- * instead of one cooperative launch; 2 = dy points at ONE element that stands for the whole
+ * fused head-major (B,S,H,D) -> (B,H,S,D) store. flags: 1 = two launches (main + finalize) where one would do
+ * (rows on the 16-byte grid of up to 256 vectors, and those that register kernels take; the others always
+ * have a finalize chained to them), which need no zeroed words in the scratch; 2 = dy points at ONE element that stands for the whole
  * tensor (the reference's captured graphs expand a 0-dim gradient,
  * sum_sum_2cd99e5eb23e/repro.py:26): dy_row_stride is ignored and nothing but that element is read.
  * Replaces sum_sum_2cd99e5eb23e/oracle.py:48-117, sum_sum_sum_3cac3bbf4e8f/oracle.py:100-193 and
