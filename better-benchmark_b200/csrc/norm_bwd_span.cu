@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) norm_bwd_span_kernel(const Norm
 template <typename T, bool LN>
 bool try_launch_norm_bwd_span(NormBwdParams& p, size_t scratch_bytes, cudaStream_t st, int* rc) {
   constexpr int V = Elem<T>::V;
+  
   const DeviceInfo& dev = device_info();
   auto off = [](const void* q) { return reinterpret_cast<uintptr_t>(q) & 15u; };
   if (p.dy_elem_stride != 1 || p.head_dim != p.n || p.n < 2 * V || p.x_row_stride < p.n || p.dy_row_stride < p.n) return false;
@@ -194,10 +195,7 @@ bool try_launch_norm_bwd_span(NormBwdParams& p, size_t scratch_bytes, cudaStream
   constexpr bool HALF = sizeof(T) == 2;
   if (p.n <= (HALF ? 512 : 1024)) return false;
   // Fewer rows would gain up to a fifth, but with chains that are longer than before: RMSNorm's dweight, 1300 x 517, 5.7e-8 instead of 4.8e-8.
-  // RMSNorm in fp32, which has less to compute by the element, gains from more rows on: 24 per SM up to 2048 columns ([2960, 1523] 18.5 / 18.0,
-  // [2368, 1523] 15.7 / 16.6), 14 up to 2560 ([1200, 2305] 13.3 / 14.6).
-  const int rows_per_sm = HALF ? (p.n <= 1010 ? 32 : p.n <= 1522 ? 16 : 8) : LN ? (p.n <= 2048 ? 18 : 8) : (p.n <= 2048 ? 24 : p.n <= 2560 ? 14 : 8);
-  if (p.rows < rows_per_sm * (long long)dev.sm_count) return false;
+  if (p.rows < (HALF ? (p.n <= 1010 ? 32 : p.n <= 1522 ? 16 : 8) : p.n <= 2048 ? 16 : 8) * (long long)dev.sm_count) return false;
   const int nv = (p.n + 2 * (V - 1)) / V;  // vectors that a row touches at most
   const bool sums = p.dw || p.db;
   auto launch = [&](auto kernel, int threads) {
