@@ -685,10 +685,10 @@ static bool try_launch_batch_norm_cl_ring(BatchNormParams p, size_t scratch_byte
   const long long PV = C / g;
   const long long elems = p.rows * C;
   if (PV > 512 || elems < V) return false;
-  // The flat kernels above need whole periods. Where there are none, the strided kernels are faster for few rows, whose channels take a CTA
-  // each and one load a thread (bf16, 401 channels: 147 rows 7.8 us strided, 10.2 so, 441 rows 9.9 and 9.9, 637 rows 11.3 and 10.2; f32
-  // 245 rows 7.7 and 8.2, 343 rows 8.6 and 8.3).
-  if (elems % (PV * V) == 0 ? ring_is_slower(C, elems * (long long)sizeof(T)) : p.rows < 75 * V) return false;
+  // The flat kernels above need whole periods. (Where there are none, the strided kernels are faster for few rows, whose channels take a CTA
+  // each and one load a thread: bf16, 401 channels, 147 rows 7.8 us strided, 10.2 so, 441 rows 9.9 and 9.9, 637 rows 11.3 and 10.2. But
+  // their errors are up to six times as large, the mean's 8.3e-8 at 147 rows and 3.0e-8 so, 2.0e-7 and 4.8e-8 at 405 rows of 101 channels.)
+  if (elems % (PV * V) == 0 && ring_is_slower(C, elems * (long long)sizeof(T))) return false;
   const long long total = elems / V;
   const long long stats_floats = 2 * C;
   const long long room = ((long long)scratch_bytes - 256) / (long long)sizeof(float) - stats_floats;

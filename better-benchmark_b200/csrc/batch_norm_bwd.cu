@@ -875,9 +875,9 @@ extern "C" int b200_batch_norm_bwd_ex(const void* dy, const void* x, const void*
   long long g = channels, h = v;
   while (h) { const long long t = g % h; g = h; h = t; }
   const long long pv = channels / g;
-  // and few rows without whole periods stay with them (bf16 401 channels: 147 rows 7.0 us strided, 8.4 so, 343 rows 9.4 and 8.3; 17 channels:
-  // 441 rows 6.1 and 6.8, 637 rows 6.8 and 6.7; f32 401 channels: 98 rows 6.3 and 6.8, 245 rows 7.5 and 7.0).
-  const bool worth_it = count * channels % (pv * v) == 0 || count >= (channels < 64 ? 640 : 300 * v / 8);
+  // and few rows without whole periods stay with them (bf16 401 channels: 147 rows 7.0 us strided, 8.4 so, 343 rows 9.4 and 8.3;
+  // f32 98 rows 6.3 and 6.8, 245 rows 7.5 and 7.0), whose sums are as exact there (dweight of 401 channels, 147 rows 5.0e-8 and 5.9e-8)
+  const bool worth_it = count * channels % (pv * v) == 0 || count >= 300 * v / 8;
   const bool fast = cl && pv >= 1 && pv <= 512 && count * channels >= v && worth_it && aligned16(dy) &&
                     aligned16(x) && (!act || aligned16(act)) && (!dx || aligned16(dx));
   p.rows = fast ? batch * spatial : batch;

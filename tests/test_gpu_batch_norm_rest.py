@@ -33,9 +33,8 @@ def test_forward(dtype, shape):
     w, b = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
     for relu in (False, True):
         y, mean, invstd = k.batch_norm_fwd(x, w, b, None, None, eps=1e-5, momentum=0.1, relu=relu)
-        rows, v = shape[0] * shape[2] * shape[3], 16 // dt.itemsize
-        if rows * c % (c // math.gcd(c, v) * v) != 0:   # few rows: the strided kernels
-            assert (b"copy rings" in k.load().b200_last_kernel()) == (rows >= 75 * v)
+        if c > 3:
+            assert b"copy rings" in k.load().b200_last_kernel()
         d = x.double()
         m, v = d.mean((0, 2, 3)), d.var((0, 2, 3), unbiased=False)
         s = torch.rsqrt(v + 1e-5)
@@ -62,8 +61,11 @@ def test_backward(dtype, shape):
         xhat = (d - column(m)) * column(s)
         db, dw = g.sum((0, 2, 3)), (g * xhat).sum((0, 2, 3))
         want = (g - column(db) / count - xhat * column(dw) / count) * column(s) * column(w)
+        rows, v = shape[0] * shape[2] * shape[3], 16 // dt.itemsize
         for want_dx in (True, False):
             dx, dweight, dbias = k.batch_norm_bwd(dy, x, m, s, w, act=a, slope=0.25, want_dx=want_dx)
+            if want_dx and rows * c >= v and rows * c % (c // math.gcd(c, v) * v) != 0:   # few rows: the strided kernels
+                assert (b"strided" in k.load().b200_last_kernel()) == (rows < 300 * v // 8)
             # fp32 chains of at most 16 additions a thread below fp64: a few 2^-24 of the magnitudes that are added
             for got, ref, parts in ((dbias, db, g.abs()), (dweight, dw, (g * xhat).abs())):
                 assert bool(((got.double() - ref).abs() <= 40 * 2.0 ** -24 * (parts.sum((0, 2, 3)) + column(s).flatten() * g.abs().sum((0, 2, 3)))).all())
