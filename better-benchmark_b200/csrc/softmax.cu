@@ -1109,9 +1109,9 @@ __global__ void __launch_bounds__(512, 2) softmax_rows_kernel(const SoftmaxParam
 //     f32 [2000, 67584] 266 and 254, but [1024, 131072] 216 and 219. fp32 rows with 16-bit results of any length: [195, 113832]
 //     68 and 48, [682, 98304] 144 and 137. fp32 rows off the grid: [195, 113835] 98 and 64, -> bf16 96 and 48; [682, 98307] 207 and
 //     183, -> bf16 198 and 138.
-//     But where the sweeps' last row of an SM is there for nine SMs in ten, they are ahead of clusters for rows of more than 10240 vectors (fp32 up
-//     to 15000) with results of their size: bf16 [296, 106000] 36.3 and 41.5, [1024, 106000] 116 and 127, [450, 106000] 66 and 59, [888, 80000] 81 and
-//     78; f32 [592, 50000] 73 and 77, [592, 65536] 87 and 85.
+//     But where the sweeps' last row of an SM is there for nine SMs in ten, they are ahead of clusters for 16-bit rows of more than 10240 vectors
+//     with 16-bit results: [296, 106000] 36.3 and 41.5, [1024, 106000] 116 and 127, [450, 106000] 66 and 59, [888, 80000] 81 and
+//     78. (So they are in fp32, [592, 50000] 73 and 77, but with errors of 1.0e-7 instead of 8e-8.)
 //   * fp32 log-probabilities of 16-bit rows are the exception, their sweeps being bound by expf (bf16 -> f32 log [1024, 131072]:
 //     250 and 177 us, [682, 196608]: 246 and 237).
 template <typename Tin, typename Tout>
@@ -1122,7 +1122,7 @@ static int softmax_ctas_per_row(long long nvec, long long rows, bool aligned, bo
     constexpr bool IN16 = sizeof(Tin) == 2, OUT16 = sizeof(Tout) == 2;
     const long long sms = device_info().sm_count;
     const bool many = rows > sms, full = rows * 10 >= (rows + sms - 1) / sms * sms * 9;
-    if (aligned && many && full && IN16 == OUT16 && nvec > 10240 && (IN16 || nvec <= 15000)) return 0;
+    if (aligned && many && full && IN16 && OUT16 && nvec > 10240) return 0;
     if (aligned && !(log_mode && IN16 && !OUT16) && !(many && ((!IN16 && OUT16) || nvec <= (IN16 && !OUT16 ? 12288 : 16384)))) return 0;
     if (!IN16 && nvec > 16384 && !many) return 0;
     return 8;

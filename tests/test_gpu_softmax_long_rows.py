@@ -43,7 +43,7 @@ def test_many_long_rows(n, dtype, out_dtype, path, log):
         assert bool(((got - want).abs() <= ulp * want + 4e-6 * want + 6.2e-8 * (out_dtype == torch.float16) + 1e-38).all())
 
 
-@pytest.mark.parametrize("n,dtype,path", [(98304, torch.bfloat16, b"two sweeps"), (50000, torch.float32, b"two sweeps"), (65536, torch.float32, b"cluster"),
+@pytest.mark.parametrize("n,dtype,path", [(98304, torch.bfloat16, b"two sweeps"), (50000, torch.float32, b"cluster"), (65536, torch.float32, b"cluster"),
                                           (81920, torch.float16, b"cluster"), (81928, torch.float16, b"two sweeps"), (98307, torch.bfloat16, b"cluster")])
 def test_full_last_rows(n, dtype, path):
     """Two rows an SM: the sweeps lose nothing to an SM without a row."""
