@@ -207,23 +207,19 @@ struct ExtremeChains {
 template <typename Tin, typename Op, SumKind KIND>
 using RowChains = typename std::conditional<Op::is_sum, SumChains<Tin, KIND>, ExtremeChains<Tin, Op>>::type;
 
-// Rows that start on 16-byte boundaries. U = 16-byte loads in flight per thread. Warp mode uses U = 4 and at most 32 registers so that
-// 64 warps fit on an SM; block mode uses U = 8. Bound by HBM: fp32 [8192, 4096] 21.6 us, 6.2 TB/s; with the head and the edges of the
-// kernel below and its joins of the chains 21.8, and where the rows are in L2 up to twice as long (amax bf16 [2400, 8000] 5.9 and 12.1).
-// VEC false: rows that start anywhere, element by element.
-template <typename Tin, typename Op, bool BLOCK, bool VEC>
-__global__ void __launch_bounds__(BLOCK ? 1024 : 256, BLOCK ? 1 : 8)
-row_reduce_grid_kernel(const RowReduceParams p) {
+// A warp per row that starts on a 16-byte boundary, four 16-byte loads in flight per lane and at most 32 registers, so that 64 warps fit
+// on an SM. Bound by HBM: fp32 [8192, 4096] 21.5 us, 6.2 TB/s; with the head and the edges of the kernel below and its joins of the chains
+// 21.8, and where the rows are in L2 up to twice as long (amax bf16 [2400, 8000] 5.9 and 12.1).
+template <typename Tin, typename Op>
+__global__ void __launch_bounds__(256, 8) row_reduce_grid_kernel(const RowReduceParams p) {
   wait_for_previous_kernel();
   constexpr int V = Elem<Tin>::V;
-  constexpr int U = BLOCK ? 8 : 4;
-  __shared__ __align__(8) float red[64];
-  const int lane = group_lane<BLOCK>();
-  const int G = group_size<BLOCK>();
-  const long long row = group_row<BLOCK>();
+  constexpr int U = 4, G = 32;
+  const int lane = group_lane<false>();
+  const long long row = group_row<false>();
   if (row >= p.rows) return;
   const Tin* x = reinterpret_cast<const Tin*>(p.x) + row_offset(p.xmap, row);
-  const long long nv = VEC ? p.n / V : 0;
+  const long long nv = p.n / V;
 
   float acc[V];
 #pragma unroll
@@ -243,8 +239,7 @@ row_reduce_grid_kernel(const RowReduceParams p) {
       }
     }
   };
-  if constexpr (!VEC) {
-  } else if constexpr (!Op::is_sum && sizeof(Tin) == 2) {  // exact in the storage type: packed pairs, only the last of a thread is widened
+  if constexpr (!Op::is_sum && sizeof(Tin) == 2) {  // exact in the storage type: packed pairs, only the last of a thread is widened
     using P2 = typename std::conditional<std::is_same<Tin, __half>::value, __half2, __nv_bfloat162>::type;
     P2 m[4];
     {
@@ -281,14 +276,6 @@ row_reduce_grid_kernel(const RowReduceParams p) {
     for (int i = 0; i < V; ++i) d += (double)acc[i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    if constexpr (BLOCK) {
-      double* dred = reinterpret_cast<double*>(red);
-      const int warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
-      if ((threadIdx.x & 31) == 0) dred[warp] = d;
-      __syncthreads();
-      d = 0.0;
-      for (int w = 0; w < nwarps; ++w) d += dred[w];
-    }
     r = (float)d;
   } else {
 #pragma unroll
@@ -296,7 +283,7 @@ row_reduce_grid_kernel(const RowReduceParams p) {
 #pragma unroll
       for (int i = 0; i < w; ++i) acc[i] = Op::apply(acc[i], acc[i + w]);
     }
-    r = group_reduce<Op, BLOCK>(acc[0], red);
+    r = warp_reduce<Op>(acc[0]);
   }
   if (lane == 0) store_scalar(p.out, p.out_dtype, row * p.out_stride, r * p.post_scale);
 }
@@ -440,10 +427,8 @@ static int launch_row_reduce(const RowReduceParams& p, bool on_grid, cudaStream_
     const double waves = units / (sms * resident_per_sm);
     return waves <= 1.0 ? 1.0 : waves / (double)(long long)(waves + 0.999999);
   };
+  const double eff_warp = efficiency((double)((p.rows + 7) / 8), 8.0);
   const double eff_block = efficiency((double)p.rows, (double)(2048 / threads > 32 ? 32 : 2048 / threads));
-  auto by_warp = [&](double ctas) {
-    return p.rows >= (long long)sms * 16 && p.n <= 16384 && efficiency((double)((p.rows + 7) / 8), ctas) + 0.02 >= eff_block;
-  };
   // Rows of up to 128 vectors, whatever their number, and of up to 256 from four an SM on: all of a row's loads in one to 32
   // lanes at once. A CTA (of 64 threads) for each of many short rows costs its launch, 0.6 ns a row over the whole GPU: fp32
   // [60000, 64] 37.1 us as CTAs, 10.9 with a warp per row, 3.0 so, [64, 64] 1.9, 1.5 and 1.4; [60000, 640] 49.1, 24.0 (chains of fp32
@@ -455,32 +440,28 @@ static int launch_row_reduce(const RowReduceParams& p, bool on_grid, cudaStream_
     launch_dependent(kernel, (unsigned)((p.rows + rows_per_cta - 1) / rows_per_cta), 256, 0, st, p);
     return launch_status("b200_row_reduce");
   };
-  // fp32 sums of 64 to 256 vectors where a warp per row is one well filled wave (2368 to some 9000 rows on 148 SMs) are bound by the
-  // additions that keep what is rounded away: plain chains there, as for longer rows, and element by element off the grid
-  // ([8192, 512] 3.9 us with what is rounded away, so 2.8; [8192, 301] 3.7, as vectors with plain chains 3.4, so 3.0).
-  const bool plain = Op::is_sum && sizeof(Tin) == 4 && nv >= 64 && nv <= 256 && by_warp(8.0);
+  // (fp32 sums of 64 to 256 vectors where a warp per row is one well filled wave, 2368 to some 9000 rows on 148 SMs, are bound by the additions that
+  // keep what is rounded away: [8192, 512] 3.9 us, with plain chains of a warp per row 2.8. Those are off by 4.8e-8 instead of 2.5e-8.)
   if (nv <= 16) return short_rows(row_reduce_short_kernel<Tin, Op, 4, 4, kKept>, 4);
   if (nv <= 32) return short_rows(row_reduce_short_kernel<Tin, Op, 8, 4, kKept>, 8);
-  if (nv <= 64 && !plain) return short_rows(row_reduce_short_kernel<Tin, Op, 16, 4, kKept>, 16);
-  if (nv <= 128 && !plain) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 4, kKept>, 32);
-  if (nv <= 256 && !plain && p.rows >= 4LL * sms) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 8, kPairs>, 32);
+  if (nv <= 64) return short_rows(row_reduce_short_kernel<Tin, Op, 16, 4, kKept>, 16);
+  if (nv <= 128) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 4, kKept>, 32);
+  if (nv <= 256 && p.rows >= 4LL * sms) return short_rows(row_reduce_short_kernel<Tin, Op, 32, 8, kPairs>, 32);
   const unsigned warp_ctas = (unsigned)((p.rows + 7) / 8);
-  if (on_grid) {
-    const bool warp_mode = plain || (nv > 256 && by_warp(8.0));
-    set_path_tag(warp_mode ? "vector, warp per row" : "vector, CTA per row");
-    if (warp_mode) launch_dependent(row_reduce_grid_kernel<Tin, Op, false, true>, warp_ctas, 256, 0, st, p);
-    else launch_dependent(row_reduce_grid_kernel<Tin, Op, true, true>, (unsigned)p.rows, threads, 0, st, p);
+  const bool warp_mode = nv > 256 && p.rows >= (long long)sms * 16 && p.n <= 16384 && eff_warp + 0.02 >= eff_block;
+  // Where a warp takes a row of the grid: row_reduce_grid_kernel, but the other kernel for rows of 512 vectors and more that are all there at
+  // once, with registers for more loads (f32 [2400, 8192] 13.2 and 12.3 us, bf16 [2400, 8192] 7.6 and 4.8, [5000, 4096] 6.1 and 5.1; shorter ones f32
+  // [2400, 1500] 2.7 and 3.0, and above four CTAs an SM f32 and extremes [5000, 4000] 12.7 and 13.8), and for sums of 16 bits in whole
+  // batches, whose loop spills in the former ([8192, 4096] 12.3 and 11.6). A CTA per row is faster so on the grid too (f32 [1200, 16384] amax
+  // 14.1 and 12.6, a single row 2.2 and 2.0).
+  const bool sum16 = Op::is_sum && sizeof(Tin) == 2;
+  const bool at_once = nv >= 512 && warp_ctas <= (sum16 ? 6u : 4u) * sms;
+  if (on_grid && warp_mode && !at_once && !(sum16 && nv % 128 == 0)) {
+    set_path_tag("vector, warp per row");
+    launch_dependent(row_reduce_grid_kernel<Tin, Op>, warp_ctas, 256, 0, st, p);
     return launch_status("b200_row_reduce");
   }
-  if constexpr (Op::is_sum && sizeof(Tin) == 4) {
-    if (plain) {
-      set_path_tag("element-wise, warp per row");
-      launch_dependent(row_reduce_grid_kernel<Tin, Op, false, false>, warp_ctas, 256, 0, st, p);
-      return launch_status("b200_row_reduce");
-    }
-  }
-  const bool warp_mode = nv > 256 && by_warp(8.0);
-  set_path_tag(warp_mode ? "off-grid rows as vectors, warp per row" : "off-grid rows as vectors, CTA per row");
+  set_path_tag(warp_mode ? "any alignment, warp per row" : "any alignment, CTA per row");
   if (warp_mode && warp_ctas <= 4u * sms) launch_dependent(row_reduce_kernel<Tin, Op, false, int, 4>, warp_ctas, 256, 0, st, p);
   else if (warp_mode && warp_ctas <= 6u * sms) launch_dependent(row_reduce_kernel<Tin, Op, false, int, 6>, warp_ctas, 256, 0, st, p);
   else if (warp_mode) launch_dependent(row_reduce_kernel<Tin, Op, false, int, 8>, warp_ctas, 256, 0, st, p);

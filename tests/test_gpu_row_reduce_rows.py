@@ -53,20 +53,19 @@ def test_totals_beyond_fp32_on_the_way(n):
 
 @pytest.mark.parametrize("op", ["sum", "amax"])
 @pytest.mark.parametrize("dtype,n,per_sm,path", [
-    ("f32", 512, 17, b"vector, warp per row"), ("f32", 1023, 17, b"element-wise, warp per row"), ("f32", 260, 63, b"vector, warp per row"),
-    ("f32", 512, 8, b"several rows a warp"), ("f32", 512, 90, b"several rows a warp"), ("bf16", 4096, 17, b"vector, warp per row"),
-    ("bf16", 4096, 8, b"vector, CTA per row"), ("bf16", 4001, 17, b"off-grid rows as vectors, warp per row"),
-    ("f16", 4001, 40, b"off-grid rows as vectors, warp per row"), ("f32", 2049, 60, b"off-grid rows as vectors, warp per row"),
-    ("bf16", 5001, 8, b"off-grid rows as vectors, CTA per row")])
+    ("f32", 512, 17, b"several rows a warp"), ("f32", 1023, 17, b"several rows a warp"), ("f32", 1028, 17, b"vector, warp per row"),
+    ("f32", 1024, 3, b"any alignment, CTA per row"), ("f32", 1023, 3, b"any alignment, CTA per row"), ("bf16", 4104, 63, b"vector, warp per row"), ("bf16", 4096, 17, b"any alignment, warp per row"),
+    ("bf16", 4096, 8, b"any alignment, CTA per row"), ("bf16", 4001, 17, b"any alignment, warp per row"),
+    ("f16", 4001, 40, b"any alignment, warp per row"), ("f32", 2049, 60, b"any alignment, warp per row"),
+    ("bf16", 5001, 8, b"any alignment, CTA per row")])
 def test_routes_of_longer_rows(dtype, n, per_sm, path, op):
-    """Each kernel for rows of 64 vectors and more, at a number of rows that it takes; extremes never keep what sums round away."""
+    """Each kernel for rows of 64 vectors and more, at a number of rows that it takes."""
     from better_benchmark_b200 import kernels as k
     dt = DTYPES[dtype]
     rows = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + 3
     x = torch.randn(rows, n, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda").to(dt)
     got = k.row_reduce(x, op, out_dtype=torch.float32)
-    if op == "sum" or n > 1024:
-        assert path in k.load().b200_last_kernel(), k.load().b200_last_kernel()
+    assert path in k.load().b200_last_kernel(), k.load().b200_last_kernel()
     d = x.double()
     if op == "amax":
         assert torch.equal(got, d.amax(-1).float())
