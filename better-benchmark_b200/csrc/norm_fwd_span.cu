@@ -352,22 +352,22 @@ __global__ void __launch_bounds__(512) norm_fwd_span_row_kernel(const NormFwdPar
 // 6.0 / 5.1, 20000 81 / 60; 2661: 600 rows 10.8 / 7.9, 20000 233 / 160; 7081: 2000 rows 72 / 53.
 // fp32 (half as many elements a vector): 981 columns and below slower, 1317 equal at 2000 rows, 2049: 600 rows 4.6 / 5.0, 2661: 750 8.9 / 7.5, 6000 52 / 38.
 // Bound by instructions (masks, edges, shifted parameters): 981 columns run at half the rate of a copy, a CTA per row at a third.
-// The lines lie where this is ahead at every number of rows measured from there on. Rows that fill the other kernel's slots and have just left one
-// of this one's (250..256, 506..512 and 1018..1024 columns) gain least: RMSNorm 255 at 26 rows per SM 3.4 / 3.6, GELU 255 at 40 6.3 / 6.9,
-// residual add, both forms, 511 at 24 7.8 / 10.8 and at 160 41 / 41, 1019 at 12 9.3 / 10.2. Both forms of a residual add have no room for three turns'
-// registers: 378 columns at 16 6.0 / 5.5, at 24 6.9 / 8.2, at 28 10.5 / 8.3.
-static int norm_span_rows_per_sm(const NormFwdParams& p, int nv) {
+// The lines lie where this is ahead, or within 4 per cent, at every number of rows measured from there on. Rows that fill the other kernel's
+// slots and have just left one of this one's (250..256, 506..512 and 1018..1024 columns) gain least: RMSNorm 255 at 26 rows per SM 3.4 / 3.6, GELU 255 at
+// 40 6.3 / 6.9, residual add, both forms, 511 at 24 7.8 / 10.8 and at 160 41 / 41, 1019 at 12 9.3 / 10.2. Both forms of a residual add leave room for
+// two CTAs an SM: 378 columns at 16, one wave, 6.0 / 5.5, at 24 6.9 / 8.2, at 28 10.5 / 8.3.
+static bool norm_span_takes(const NormFwdParams& p, int nv, long long sms) {
   const bool both = p.res && p.res_round == 2;
   const bool edge = p.n > 128 && p.n <= 1024 && nv * 8 > (p.n + 255) / 256 * 256;
-  constexpr int kNever = 1 << 30;
-  if (nv > 128) return both && edge ? kNever : 4;
-  if (p.n > 512) return 8;
-  if (p.n > 256) {
-    if (edge) return both ? kNever : p.res ? 48 : p.rms ? 28 : 14;
-    return both && p.n > 377 ? 28 : 14;
-  }
-  if (p.n > 128) return !edge ? 26 : p.prologue ? kNever : p.rms ? 48 : 26;
-  return 64;
+  if (edge && p.prologue && p.n <= 256) return false;
+  int line;  // rows per SM
+  if (nv > 128) line = both && edge ? 16 : 4;
+  else if (p.n > 512) line = 8;
+  else if (p.n > 256 && edge) line = both ? 64 : p.res ? 28 : p.rms ? 25 : 14;
+  else if (p.n > 256) line = both && p.n > 377 && p.rows > 16 * sms ? 25 : 14;
+  else if (p.n > 128) line = edge ? (p.rms ? 48 : 26) : p.rms ? 25 : 20;
+  else line = 64;
+  return p.rows >= line * sms;
 }
 
 template <typename T>
@@ -380,7 +380,7 @@ bool try_launch_norm_fwd_span(const NormFwdParams& p, cudaStream_t st) {
   if (!p.y || nv > 2048 || p.x_row_stride < p.n || off(p.x) != off(p.y) || (p.x_row_stride - p.y_row_stride) % V != 0) return false;
   if constexpr (HALF) {
     if (p.n <= (p.res ? 256 : 57)) return false;  // 57: two vectors a lane of eight
-    if (p.rows < norm_span_rows_per_sm(p, nv) * sms) return false;
+    if (!norm_span_takes(p, nv, sms)) return false;
     if (p.res && (p.rms || off(p.x) != off(p.res) ||
                   (p.sum_out && (off(p.x) != off(p.sum_out) || (p.x_row_stride - p.n) % V != 0)))) return false;
   } else {
@@ -395,7 +395,10 @@ bool try_launch_norm_fwd_span(const NormFwdParams& p, cudaStream_t st) {
         const size_t smem = (size_t)2 * V * (p.n / V + 3) * sizeof(f32x2);  // both tables of both: 16.5 KB at 1017 columns
         const int at_once = 256 / lanes;
         const long long resident = sms * cached_occupancy(reinterpret_cast<const void*>(kernel), 256, smem);
-        const int reps = span_turns(p.rows, at_once, resident);
+        // Behind GELU a row is bound by instructions: what counts is how many turns the SM with the most has, not whether its CTAs are there at
+        // once ([23680, 249] 13.6 us with turns rounded down, 15.0 in whole waves).
+        const long long whole = p.rows / (at_once * resident);
+        const int reps = KIND != 1 ? span_turns(p.rows, at_once, resident) : whole < 1 ? 1 : whole > 16 ? 16 : (int)whole;
         launch_dependent(kernel, (unsigned)((p.rows + (long long)at_once * reps - 1) / ((long long)at_once * reps)), 256, smem, st, p, reps);
       };
       if (KIND != 2 && nv <= 16) { launch(norm_fwd_span_kernel<T, 2, 8, KIND == 2 ? 0 : KIND>, 8); return; }

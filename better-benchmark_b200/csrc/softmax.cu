@@ -662,22 +662,24 @@ __global__ void __launch_bounds__(512) softmax_span_row_kernel(const SoftmaxPara
   else finish(std::false_type{});
 }
 
-// Rows per SM from which on the two kernels above are ahead of softmax_ragged_kernel at every number of rows measured (0: never), for rows
-// of n elements that touch nv vectors at most. A group reads its part of the mask once, 1 us; its slots are filled or not, as the other kernel's
-// are. That kernel / this one, us, fp16, rows per SM in front:
-//   n 57    48 2.9 / 2.8, 96 4.4 / 3.6        n 58    80 4.0 / 4.1, 104 4.7 / 4.7         n 121   72 4.6 / 4.3, 104 5.7 / 5.3
-//   n 150   48 4.3 / 4.6, 64 5.3 / 4.6        n 186   200 13.3 / 13.8, 250 16.2 / 15.8    n 249   200 14.7 / 14.0, 300 21.3 / 17.6
-//   n 257   24 3.9 / 4.5, 25 5.5 / 4.5        n 391   40 7.1 / 7.2, 48 7.6 / 8.1, 56 9.4 / 8.4    n 420   20 4.5 / 4.3, 48 7.7 / 7.6
-//   n 601   10 4.4 / 4.6, 11 5.0 / 4.6        n 900   8 4.4 / 4.4, 11 5.6 / 5.1, 18 8.4 / 7.8
-//   n 1241  2 4.1 / 3.7, 135 61.9 / 40.3      n 250   200 14.7 / 18.3, 800 52.6 / 62.2    n 506   64 10.9 / 12.4, 300 45.2 / 47.1
-// The last two are of the rows that fill the other kernel's slots and have just left one of this one's. All with one mask for all rows, and with
-// turns rounded down, which made waves of CTAs that were not full (n 391, 48 rows per SM; n 900, 18); now nothing from the lines on is slower. With a
+// Rows per SM from which on the two kernels above are ahead of softmax_ragged_kernel, or within 4 per cent, at every number of rows measured (0:
+// never), for rows of n elements that touch nv vectors at most. A group reads its part of the mask once, 1 us; its slots are filled or not, as the
+// other kernel's are. That kernel's time over this one's, fp16 with one mask for all rows, rows per SM in front:
+//   n 57    32 0.99, 40 0.91, 48 1.00, 96 1.24        n 90    56 0.97, 64 1.05, 104 0.99, 128 1.13 (no mask 144 0.95, 160 1.03)
+//   n 121   48 0.91, 56 1.01, 104 1.07, 250 1.41      n 150   48 0.93, 52 1.00, 104 1.10     n 201   160 1.01, 200 0.98, 250 1.19
+//   n 249   80 1.01, 96 1.15, 200 1.04                n 257   22 0.88, 25 1.24, 36 1.16      n 378   22 0.96, 25 1.14, 36 1.00
+//   n 420   3 0.95, 5 1.13, 22 1.02                   n 511   64 0.98, 72 1.05               n 601   8 0.99, 11 1.08, 18 1.15
+//   n 900   8 1.01, 11 1.10, 64 1.90                  n 127   200 0.86, 405 1.01             n 255   144 0.97, 250 0.91
+// The last two are of the rows that fill the other kernel's slots and have just left one of this one's. With a
 // mask for so many rows as the CTA takes at two times the groups are still ahead ([20000, 1017] 50.6 / 41.3), with one for half as many no longer
 // (50.6 / 53.3), with one for every row they are far behind (49.0 / 73.0, [60000, 249] 29.6 / 36.7).
-static int softmax_span_rows_per_sm(int n, int nv) {
+static int softmax_span_rows_per_sm(int n, int nv, bool masked) {
   if (nv > 128) return 2;
-  if (nv * 8 > (n <= 128 ? 128 : (n + 255) / 256 * 256)) return 0;
-  return n <= 57 ? 48 : n <= 72 ? 200 : n <= 121 ? 88 : n <= 185 ? 64 : n <= 249 ? 300 : n <= 377 ? 25 : n <= 409 ? 50 : n <= 505 ? 5 : 11;
+  if ((n > 121 && n <= 128) || (n > 249 && n <= 256)) return 0;
+  if (n <= 57) return 44;
+  if (n <= 99) return masked ? (n <= 65 ? 80 : 64) : 160;
+  if (n <= 249) return n <= 185 ? 52 : n <= 234 ? 250 : 96;
+  return n <= 390 ? 25 : n <= 505 ? 5 : n <= 512 ? 72 : 11;
 }
 
 // How many rows that follow one another share their mask.
@@ -708,7 +710,7 @@ static bool try_launch_softmax_span(const SoftmaxParams& p, cudaStream_t st) {
       (p.xmap.s0 - p.ymap.s0) % V != 0 || p.rows > 0x7fff0000LL)
     return false;
   if (nv <= 128 && softmax_rows_per_mask(p) < (nv <= 24 ? 64 : nv <= 48 ? 32 : 16)) return false;  // 2 * 256 / lanes of a group
-  const int rows_per_sm = softmax_span_rows_per_sm(p.n, nv);
+  const int rows_per_sm = softmax_span_rows_per_sm(p.n, nv, p.mask != nullptr);
   if (rows_per_sm == 0 || p.rows < rows_per_sm * sms) return false;
   if (nv > 2048) return false;
   set_path_tag(nv > 128 ? "off-grid rows as vectors, CTA per row" : "off-grid rows as vectors, several rows in turn");

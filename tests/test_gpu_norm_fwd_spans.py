@@ -20,7 +20,7 @@ def test_spans(dtype, n):
     """Both sides of every change of geometry; what lies beside the rows is NaN and stays out; parameters of either type, off the grid, none."""
     from better_benchmark_b200 import native
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    rows = (64 if n <= 128 else 26 if n < 250 else 48 if n <= 256 else 14 if n <= 505 else 28 if n <= 512 else 8 if n <= 1017 else 5) * sms + 3
+    rows = (64 if n <= 128 else 25 if n < 250 else 48 if n <= 256 else 14 if n <= 505 else 25 if n <= 512 else 8 if n <= 1017 else 5) * sms + 3
     lib, stream = native.load(), torch.cuda.current_stream().cuda_stream
     eps, code = 1e-5, {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
     ulp = {torch.float32: 2.0 ** -23, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
@@ -59,7 +59,7 @@ def test_residual_and_gelu(dtype, n):
     """The three forms of the sum, the sum itself, the GELU prologue, and rows with infinities and NaN, which stay theirs."""
     from better_benchmark_b200 import kernels as k
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    rows = (14 if n <= 377 else 28 if n <= 505 else 48 if n <= 512 else 8 if n <= 1017 else 4) * sms + 1
+    rows = (14 if n <= 505 and n != 378 else 25 if n <= 505 else 64 if n <= 512 else 8 if n <= 1017 else 4) * sms + 1
     x, r = _storage(rows, n, dtype, 0, n), _storage(rows, n, dtype, 0, n + 1)
     x[5, n - 1], x[6, 0], x[7, n // 2] = float("nan"), float("inf"), float("-inf")
     w, b = torch.randn(n, device="cuda").to(dtype), torch.randn(n, device="cuda").to(dtype)
@@ -67,7 +67,7 @@ def test_residual_and_gelu(dtype, n):
     full, mean, rstd, _, total = k.norm_fwd(x, w, b, **kw)
     rounded = k.norm_fwd(x, w, b, round_sum=True, **kw)[0]
     both, mean2, rstd2, _, total2 = k.norm_fwd(x, w, b, round_sum="both", **kw)
-    assert (b"residual add, off-grid rows as vectors" in k.load().b200_last_kernel()) == (n != 506), "506: by the element for both forms"
+    assert b"residual add, off-grid rows as vectors" in k.load().b200_last_kernel()
     gelu = k.norm_fwd(x, w, b, eps=1e-6, prologue="gelu_erf")[0]
     assert b"[off-grid rows as vectors]" in k.load().b200_last_kernel()
     s = x.float() + r.float()
@@ -78,14 +78,8 @@ def test_residual_and_gelu(dtype, n):
     assert not bool(torch.isnan(gelu[~bad]).any())
     ok = ~bad
     assert torch.equal(total[ok], s.to(dtype)[ok]) and torch.equal(total2[ok], total[ok])
-    if n != 506:
-        assert torch.equal(mean[ok], mean2[ok]) and torch.equal(rstd[ok], rstd2[ok])
-        assert torch.equal(both[ok], torch.where(full.float().abs() > 3, full, rounded)[ok])
-    else:   # another kernel, whose sums have another order: the statistics agree to some ulp, an output to one of its own in either form
-        assert torch.allclose(mean[ok], mean2[ok], rtol=0, atol=1e-5) and torch.allclose(rstd[ok], rstd2[ok], rtol=1e-5)
-        step = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
-        f, q, o = full[ok].float(), rounded[ok].float(), both[ok].float()
-        assert bool((torch.minimum((o - f).abs(), (o - q).abs()) <= step * o.abs() + 1e-4).all())
+    assert torch.equal(mean[ok], mean2[ok]) and torch.equal(rstd[ok], rstd2[ok])
+    assert torch.equal(both[ok], torch.where(full.float().abs() > 3, full, rounded)[ok])
     ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     act = torch.nn.functional.gelu(x.double()).to(dtype)
     for got, at in ((full, x.double() + r.double()), (rounded, s.to(dtype).double()), (gelu, act.double())):

@@ -16,7 +16,7 @@ def _run(rows, n, dtype, mask, scale, start, log, batches=4):
     x, y = (t[start:start + size].view(batches, rows // batches, n) for t in (xs, ys))
     k.softmax(x, mask=mask, scale=scale, log=log, out=y)
     shared = mask is None and n < 256 or mask is not None and mask.shape[1] == 1
-    fills = n <= 1017 and (n + 14) // 8 * 8 > (128 if n <= 128 else (n + 255) // 256 * 256)   # the other kernel's slots, and one more of this one's
+    fills = 121 < n <= 128 or 249 < n <= 256   # the other kernel's slots, and one more of this one's
     by_vectors = (n > 1017 and mask is not None or shared) and not fills and not (start % 8 == 0 and n % 8 == 0)
     assert (b"off-grid rows as vectors" in k.load().b200_last_kernel()) == by_vectors
     assert bool((ys[:start] == 7).all()) and bool((ys[start + size:] == 7).all()), "nothing beside the rows is written"
@@ -31,7 +31,7 @@ def _run(rows, n, dtype, mask, scale, start, log, batches=4):
 def test_spans(dtype, n):
     """Both sides of every change of geometry; every alignment of the first row; masks per batch, per row and none."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    per_sm = next(r for most, r in ((57, 48), (72, 200), (121, 88), (185, 64), (249, 300), (377, 25), (409, 50), (505, 5), (1017, 11), (8191, 2)) if n <= most)
+    per_sm = next(r for most, r in ((57, 44), (99, 160), (185, 52), (234, 250), (249, 96), (390, 25), (505, 5), (512, 72), (1017, 11), (8191, 2)) if n <= most)
     rows = (per_sm * sms + 15) // 4 * 4
     ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     g = torch.Generator(device="cuda").manual_seed(n)
@@ -105,9 +105,9 @@ def test_masks_that_few_rows_share(n, group):
     every = masks[:1].expand(rows, n)
     k.softmax(x, mask=every)
     assert b"off-grid rows as vectors" in k.load().b200_last_kernel(), "one mask for all rows"
-    for full in (125, 251, 509, 765):
+    for full in (125, 251, 509):
         x = torch.randn(rows, full, generator=g, device="cuda").half()
         got = k.softmax(x, mask=x[0])
-        assert b"[elements in registers]" in k.load().b200_last_kernel()
+        assert (b"[elements in registers]" in k.load().b200_last_kernel()) == (full < 256)
         want = torch.softmax(x.double() + x[0].double(), -1)
         assert bool(((got.double() - want).abs() <= (2.0 ** -11 + 2e-6) * want + 6.2e-8).all())
